@@ -398,7 +398,7 @@ __global__ void rowsum_coef_refine_kernel(const double2* __restrict__ tr, const 
     const double2 v = tr[t];
     re += cr * v.x - ci * v.y;
     im += cr * v.y + ci * v.x;
-    sc += sqrt(cr * cr + ci * ci) * trabs[t];
+    sc += (double)sqrtf(coef[2 * r] * coef[2 * r] + coef[2 * r + 1] * coef[2 * r + 1]) * trabs[t];
   }
   out[(size_t)p * nout + o] = make_double2(re, im);
   // flagged: an error estimate above the tolerance, a NaN (a product whose

@@ -1514,6 +1514,41 @@ __global__ void __launch_bounds__(TG_THREADS) trace_groups_kernel(
   }
 }
 
+// Warp sums of eight FP64 values by reduce-scatter: each lane returns the sum of
+// value lane >> 2 (the four lanes of a group hold the same bits).
+__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
+  double a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const double keep = (lane & 16) ? v[4 + i] : v[i], give = (lane & 16) ? v[i] : v[4 + i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const double keep = (lane & 8) ? a[2 + i] : a[i], give = (lane & 8) ? a[i] : a[2 + i];
+    b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+  }
+  const double keep = (lane & 4) ? b[1] : b[0], give = (lane & 4) ? b[0] : b[1];
+  double s = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
+// The same for four FP32 values: each lane returns the sum of value lane >> 3.
+__device__ __forceinline__ float warp_sum4(const float (&v)[4], int lane) {
+  float a[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const float keep = (lane & 16) ? v[2 + i] : v[i], give = (lane & 16) ? v[i] : v[2 + i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+  }
+  const float keep = (lane & 8) ? a[1] : a[0], give = (lane & 8) ? a[0] : a[1];
+  float s = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
 // Quad groups: at most 2 A blocks and 2 B blocks and the (up to 4) traces
 // between them.  One CTA per (pair, group) walks the nev*nev elements with U
 // independent streams a thread; each element of the group's (at most 4) blocks
@@ -1579,36 +1614,38 @@ __global__ void __launch_bounds__(TPB) trace_quads_kernel(const TraceGroup* __re
       }
     }
   }
-  __shared__ double red[4][3][NW];
+  // A warp's FP64 add holds the FP64 pipe for 16 clocks, so the eight sums go
+  // through a reduce-scatter (4 + 2 + 1 + 1 + 1 adds a warp instead of 8 x 5) and
+  // the four error scales, which need a few bits, stay in FP32.
+  __shared__ double red[NW][8];
+  __shared__ float reda[NW][4];
+  const int lane = threadIdx.x & 31;
+  double v[8];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    if (!((mask >> k) & 1u)) continue;
-    double re = (double)sr[k] + (double)er[k], im = (double)si[k] + (double)ei[k], ab = (double)sa[k];
-    for (int o = 16; o; o >>= 1) {
-      re += __shfl_down_sync(0xffffffffu, re, o);
-      im += __shfl_down_sync(0xffffffffu, im, o);
-      ab += __shfl_down_sync(0xffffffffu, ab, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      red[k][0][threadIdx.x >> 5] = re;
-      red[k][1][threadIdx.x >> 5] = im;
-      red[k][2][threadIdx.x >> 5] = ab;
-    }
+    v[2 * k] = (double)sr[k] + (double)er[k];
+    v[2 * k + 1] = (double)si[k] + (double)ei[k];
   }
+  const double tot = warp_sum8(v, lane);
+  const float tota = warp_sum4(sa, lane);
+  if ((lane & 3) == 0) red[threadIdx.x >> 5][lane >> 2] = tot;
+  if ((lane & 7) == 0) reda[threadIdx.x >> 5][lane >> 3] = tota;
   __syncthreads();
   if (threadIdx.x < nt) {
     const int t = threadIdx.x, k = G.ta[t] * 2 + G.tb[t];
-    double re = 0.0, im = 0.0, ab = 0.0;
-    for (int w = 0; w < NW; w++) {
-      re += red[k][0][w];
-      im += red[k][1][w];
-      ab += red[k][2][w];
+    double re = red[0][2 * k], im = red[0][2 * k + 1];
+    float ab = reda[0][k];
+#pragma unroll
+    for (int w = 1; w < NW; w++) {
+      re += red[w][2 * k];
+      im += red[w][2 * k + 1];
+      ab += reda[w][k];
     }
     const int r = G.tr[t];
     const TraceRow T = rt[r];
     const double2 c = make_double2((double)T.coef[0], (double)T.coef[1]);
     rows[(size_t)q * nrows + r] = cmul(c, make_double2(re, im));
-    rabs[(size_t)q * nrows + r] = sqrt(c.x * c.x + c.y * c.y) * ab;
+    rabs[(size_t)q * nrows + r] = (double)(sqrtf(T.coef[0] * T.coef[0] + T.coef[1] * T.coef[1]) * ab);
   }
 }
 
@@ -2131,6 +2168,14 @@ int launch_trace_groups(const TraceGroup* d_groups, int ngroups, int maxcols, co
   return CTR_OK;
 }
 
+// Up to this Nev a group gets one warp: its Nev^2 elements are too few to pay
+// for a cross-warp reduction, and with 32 CTAs an SM the loads in flight still
+// cover the latency.  Measured (rho, 256 pairs, trace_quads in us; one warp /
+// 128 threads / 64 threads before the reduce-scatter): Nev = 16: 272 / 1175 /
+// 731, 32: 548 / 1417 / 1047, 64: 1887 / 2288 / 2173.  The gain over 128 threads
+// is down to the shorter reduction by Nev = 64, so larger blocks keep them.
+constexpr int TRACE_WARP_NEV = 64;
+
 int launch_trace_quads(const TraceGroup* d_groups, int ngroups, const TraceRow* d_rows, int nrows,
                        const float4* const* d_abase, const float4* const* d_bbase, int lda, int ldb, int npair,
                        int nev, double2* rows, double* rabs, int variant, cudaStream_t s) {
@@ -2138,7 +2183,10 @@ int launch_trace_quads(const TraceGroup* d_groups, int ngroups, const TraceRow* 
   const long long nblk = (long long)npair * ngroups;
   if (nblk > 0x7fffffffLL) return fail(CTR_ERR_ARG, "trace quads: grid too large");
   TimedLaunch tl(s, "trace_quads");
-  if (variant == 0)
+  if (nev <= TRACE_WARP_NEV)
+    trace_quads_kernel<32, 4><<<(unsigned)nblk, 32, 0, s>>>(d_groups, ngroups, d_rows, nrows, d_abase, d_bbase, lda,
+                                                            ldb, nev, rows, rabs);
+  else if (variant == 0)
     trace_quads_kernel<128, 2><<<(unsigned)nblk, 128, 0, s>>>(d_groups, ngroups, d_rows, nrows, d_abase, d_bbase,
                                                                 lda, ldb, nev, rows, rabs);
   else

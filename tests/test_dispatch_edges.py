@@ -1,0 +1,29 @@
+"""The kernels' dispatch rules at the sizes where they switch: each side of a
+size rule, remainders of its tiles and the ends of its range, against the
+oracle or a plain FP64 restatement."""
+import numpy as np
+import pytest
+import torch
+
+from contractions_code_scattering_gb300 import api, synth
+from oracle import pyoracle as O
+from tests import parity as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a, cuda):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+
+@pytest.mark.parametrize("n", [2, 31, 33, 64, 65])
+def test_quad_traces_one_warp_or_one_block_a_group(cuda, n):
+    """trace_quads gives a group one warp up to Nev = 64 and a block above."""
+    nt = 2
+    prop = synth.make_prop(nt, n, seed=500 + n)
+    rng = np.random.default_rng(501 + n)
+    mom2 = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(2)], axis=1)
+    got = api.run_contract_sigma(_dev(prop, cuda), _dev(mom2, cuda), engine="split").cpu().numpy()
+    rc = [O.sigma_row(prop, np.ascontiguousarray(mom2), tf) for tf in range(nt)]
+    P.entrywise(got, np.stack([c for _, c in rc]), 1e-9, np.stack([P.sigma_rows_abs(r) for r, _ in rc]),
+                "sigma Nev=%d" % n)
