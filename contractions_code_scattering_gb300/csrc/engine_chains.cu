@@ -1620,23 +1620,7 @@ int rhopi_sigmapi_sets(int N, int Nt, int tf_begin, int tf_end, const double* pr
 // -------------------------------------------------------------- loop unity
 // lib/calculate_loop_unity_core.h: L(t) = sum_s Tr[taud(t)_{ss} Phi(t)] (trace of a product: Nev^2 work).
 int loop_unity_fp64(int N, int Nt, const double* prop_diag, const double* mom, double* loop, cudaStream_t s) {
-  Ctx c{N, Nt, (size_t)N * N, s, CTR_ENGINE_FP64};
-  const double2 *diag = (const double2*)prop_diag, *P = (const double2*)mom;
-  void* trm;
-  CTR_TRY(workspace(WS_ROWS).get((size_t)Nt * 4 * sizeof(double2), &trm));
-  std::vector<TraceTask> tt;
-  for (int t = 0; t < Nt; t++)
-    for (int sp = 0; sp < 4; sp++)
-      tt.push_back(tr(diag + ((size_t)t * 16 + sp * 5) * c.N2, P + (size_t)t * c.N2, (double2*)trm + t * 4 + sp, 1.f,
-                      0.f, 1));
-  std::vector<int> csr(Nt + 1 + Nt * 4);
-  for (int t = 0; t <= Nt; t++) csr[t] = 4 * t;
-  for (int k = 0; k < Nt * 4; k++) csr[Nt + 1 + k] = k;
-  void* d_csr;
-  CTR_TRY(upload(WS_MISC, csr.data(), csr.size() * sizeof(int), &d_csr, s));
-  CTR_TRY(run_traces(c, tt));
-  return launch_rowsum((double2*)trm, Nt * 4, (const int*)d_csr, (const int*)d_csr + Nt + 1, Nt, 1, (double2*)loop,
-                       Nt, s);
+  return launch_loop_unity((const double2*)prop_diag, (const double2*)mom, N, Nt, (double2*)loop, s);
 }
 
 }  // namespace ctr

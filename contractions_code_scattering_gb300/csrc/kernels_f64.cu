@@ -10,6 +10,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include "kernels.h"
 
 namespace ctr {
@@ -338,6 +340,62 @@ __global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restr
   }
 }
 
+// ---------------------------------------------------------- unit-spin loop
+// loop[t] = sum_s Tr[tau(t,t)_ss Phi(t)] = Tr[(sum_s tau(t,t)_ss) Phi(t)].  The
+// FP64 pipe is the bound: summing the four spin blocks first takes 6 adds + 4
+// FMAs an element where four traces take 16 FMAs (10.7 against 17 us of the pipe
+// at Nev = 100, Lt = 64).  One cluster of up to 8 CTAs a time slice, each over a
+// range of the Nev^2 elements; CTA 0 adds the CTAs' partial sums in rank order
+// through distributed shared memory, so there is one launch, no table to upload
+// and a fixed summation order.
+constexpr int LOOP_TPB = 128;
+
+__global__ void __launch_bounds__(LOOP_TPB) loop_unity_kernel(const double2* __restrict__ diag,
+                                                              const double2* __restrict__ mom, int N, int ncta,
+                                                              double2* __restrict__ loop) {
+  __shared__ double red[LOOP_TPB / 32][2];
+  __shared__ double part[2];
+  const int t = blockIdx.x / ncta, rank = blockIdx.x - t * ncta;
+  const size_t n2 = (size_t)N * N;
+  const double2* T = diag + (size_t)t * 16 * n2;
+  const double2* P = mom + (size_t)t * n2;
+  const size_t e1 = n2 * (rank + 1) / ncta;
+  double re = 0.0, im = 0.0;
+#pragma unroll 2
+  for (size_t e = n2 * rank / ncta + threadIdx.x; e < e1; e += LOOP_TPB) {
+    const size_t i = e / N, j = e - i * N;
+    const double2 a = T[e], b = T[e + 5 * n2], c = T[e + 10 * n2], d = T[e + 15 * n2], y = P[j * N + i];
+    const double xr = (a.x + b.x) + (c.x + d.x), xi = (a.y + b.y) + (c.y + d.y);
+    re = fma(xr, y.x, re);
+    re = fma(-xi, y.y, re);
+    im = fma(xr, y.y, im);
+    im = fma(xi, y.x, im);
+  }
+  // lanes 0-15 take the sum of re, lanes 16-31 that of im
+  const int lane = threadIdx.x & 31;
+  double s = ((lane & 16) ? im : re) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? re : im, 16);
+  for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((lane & 15) == 0) red[threadIdx.x >> 5][lane >> 4] = s;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double v = red[0][threadIdx.x];
+    for (int w = 1; w < LOOP_TPB / 32; w++) v += red[w][threadIdx.x];
+    part[threadIdx.x] = v;
+  }
+  if (ncta == 1) {
+    if (threadIdx.x < 2) ((double*)(loop + t))[threadIdx.x] = part[threadIdx.x];
+    return;
+  }
+  auto cl = cooperative_groups::this_cluster();
+  cl.sync();
+  if (rank == 0 && threadIdx.x < 2) {
+    double v = part[threadIdx.x];
+    for (int r = 1; r < ncta; r++) v += cl.map_shared_rank(part, r)[threadIdx.x];
+    ((double*)(loop + t))[threadIdx.x] = v;
+  }
+  cl.sync();  // the other CTAs' partial sums stay in place until they are read
+}
+
 // ------------------------------------------------------------- row sums
 // out[p][o] = sum_{k in [off[o], off[o+1])} rows[p][idx[k]]  (ascending idx)
 __global__ void rowsum_kernel(const double2* __restrict__ rows, int nrows, const int* __restrict__ off,
@@ -513,6 +571,35 @@ int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s)
   TimedLaunch tl(s, "trace_f64");
   trace_f64_kernel<<<ntask, 256, 0, s>>>(d_tasks, ntask, N);
   CTR_CUDA(cudaGetLastError());
+  return CTR_OK;
+}
+
+int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s) {
+  int dev = 0, nsm = 0;
+  CTR_CUDA(cudaGetDevice(&dev));
+  CTR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // CTAs a time slice (at most 8, the portable cluster size, and no less than a
+  // CTA's worth of elements each): the split whose most loaded SM has the least
+  // work, ceil(Nt c / SMs) / c, the smaller one of equals.  At Lt = 64 that is 7
+  // (448 CTAs, at most 3 an SM); 8 would put 4 on some.
+  int best = 1;
+  const long long most = std::min<long long>(8, ((long long)N * N + LOOP_TPB - 1) / LOOP_TPB);
+  for (int c = 2; c <= most; c++) {
+    const long long a = ((long long)Nt * c + nsm - 1) / nsm * best, b = ((long long)Nt * best + nsm - 1) / nsm * c;
+    if (a < b) best = c;
+  }
+  TimedLaunch tl(s, "loop_unity");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)Nt * best);
+  cfg.blockDim = dim3(LOOP_TPB);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = best;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CTR_CUDA(cudaLaunchKernelEx(&cfg, loop_unity_kernel, diag, mom, N, best, loop));
   return CTR_OK;
 }
 

@@ -27,3 +27,18 @@ def test_quad_traces_one_warp_or_one_block_a_group(cuda, n):
     rc = [O.sigma_row(prop, np.ascontiguousarray(mom2), tf) for tf in range(nt)]
     P.entrywise(got, np.stack([c for _, c in rc]), 1e-9, np.stack([P.sigma_rows_abs(r) for r, _ in rc]),
                 "sigma Nev=%d" % n)
+
+
+@pytest.mark.parametrize("nt,n", [(1, 1), (5, 11), (3, 12), (22, 37), (64, 100), (200, 9)])
+def test_loop_unity_cluster_sizes(cuda, nt, n):
+    """One CTA a time slice up to a cluster of 8, ragged element ranges; per
+    entry to the FP64 rounding floor of its 4 rows of Nev^2 terms."""
+    rng = np.random.default_rng(600 + n)
+    diag = rng.normal(size=(nt, 4, 4, n, n)) + 1j * rng.normal(size=(nt, 4, 4, n, n))
+    mom = rng.normal(size=(nt, n, n)) + 1j * rng.normal(size=(nt, n, n))
+    got = api.run_contract_loop_unity(_dev(diag, cuda), _dev(mom, cuda)).cpu().numpy()
+    wide = np.clongdouble
+    ref = np.einsum("tssij,tji->t", diag.astype(wide), mom.astype(wide)).astype(complex)
+    # each sum adds at most Nev^2 / 128 + 11 rounded terms in sequence
+    terms = np.einsum("tssij,tji->t", np.abs(diag), np.abs(mom))
+    assert np.all(np.abs(got - ref) <= 2.0 ** -53 * (n * n / 128 + 16) * terms)
