@@ -32,8 +32,11 @@ struct ElTask {
   const double2* y[3];
   double w[3];
   int nterm;
-  int p;  // momentum index into the phase table
+  int p;     // momentum index into the phase table
+  int self;  // 1: out[c][r] = sign conj(out[r][c]), so only the tiles on and above the diagonal are computed
+  double sign;
   double2* out;
+  double2* mirror;  // not null: mirror[c][r] = sign conj(out[r][c]), the elemental of -p
 };
 
 // phase[p][s] = exp(-i 2 pi n / V) with n = (x p_x n_y n_z + y p_y n_x n_z + z p_z n_x n_y) mod V,
@@ -113,21 +116,34 @@ __global__ void el_covderiv_kernel(const double2* __restrict__ v, const double2*
   }
 }
 
-// One CTA per (TE x TE output tile, task): out[r][c] = sum_q w_q sum_k conj(X_q[r][k]) ph[k / 3] Y_q[c][k].
+// One CTA per (TE x TE output tile, task, K piece): the piece's share of
+// out[r][c] = sum_q w_q sum_k conj(X_q[r][k]) ph[k / 3] Y_q[c][k].  The task's
+// nterm K products run through nterm * nsplit pieces, so that every CTA of the
+// launch has about the same work whatever the task's number of terms: with one
+// CTA a tile, tasks of 1 to 3 terms left the last wave nearly empty (4 time
+// slices of 16^3: 0.95 TFLOP/s; with pieces 1.17).  The partial tiles are added in
+// piece order by el_sum_kernel.
 // Thread (tx, ty) owns rows tx + TX a (a < RX) and columns ty + TY b (b < RY); K
 // is staged KC at a time in shared memory, the phase and weight applied to Y as
 // it is staged.  FP64 FMAs only in the product (the FP64 pipe is the bound).
+struct ElPiece {
+  int task, tile, piece;
+  int part;  // partial tile's slot
+};
+
 template <int TE, int RX, int RY>
-__global__ void __launch_bounds__((TE / RX) * (TE / RY)) el_gemm_kernel(const ElTask* __restrict__ tasks, int nev,
-                                                                          long long K,
+__global__ void __launch_bounds__((TE / RX) * (TE / RY)) el_gemm_kernel(const ElTask* __restrict__ tasks,
+                                                                          const ElPiece* __restrict__ pieces, int nev,
+                                                                          long long K, int nsplit,
                                                                           const double2* __restrict__ phase,
-                                                                          long long V) {
+                                                                          long long V, double2* __restrict__ part) {
   constexpr int TX = TE / RX, TY = TE / RY, NTH = TX * TY, KC = 8;
   __shared__ double2 xs[KC][TE + 1];
   __shared__ double2 ys[KC][TE + 1];
-  const ElTask& T = tasks[blockIdx.y];
+  const ElPiece pc = pieces[blockIdx.x];
+  const ElTask& T = tasks[pc.task];
   const int nti = (nev + TE - 1) / TE;
-  const int r0 = (blockIdx.x / nti) * TE, c0 = (blockIdx.x % nti) * TE;
+  const int r0 = (pc.tile / nti) * TE, c0 = (pc.tile % nti) * TE;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const double2* ph = phase + (size_t)T.p * V;
   double2 acc[RX][RY];
@@ -135,65 +151,131 @@ __global__ void __launch_bounds__((TE / RX) * (TE / RY)) el_gemm_kernel(const El
   for (int a = 0; a < RX; a++)
 #pragma unroll
     for (int b = 0; b < RY; b++) acc[a][b] = make_double2(0.0, 0.0);
-  for (int q = 0; q < T.nterm; q++) {
-    const double2* X = T.x[q];
-    const double2* Y = T.y[q];
-    const double w = T.w[q];
-    for (long long k0 = 0; k0 < K; k0 += KC) {
-      for (int e = threadIdx.x; e < TE * KC; e += NTH) {
-        const int i = e / KC, kk = e - i * KC;  // consecutive threads along k
-        const long long k = k0 + kk;
-        const int r = r0 + i, c = c0 + i;
-        xs[kk][i] = (r < nev && k < K) ? X[(size_t)r * K + k] : make_double2(0.0, 0.0);
-        double2 y = make_double2(0.0, 0.0);
-        if (c < nev && k < K) {
-          const double2 yv = Y[(size_t)c * K + k], f = ph[k / 3];
-          y = make_double2(w * (f.x * yv.x - f.y * yv.y), w * (f.x * yv.y + f.y * yv.x));
-        }
-        ys[kk][i] = y;
+  const int q = pc.piece / nsplit, sp = pc.piece - q * nsplit;
+  const long long kb = K * sp / nsplit, ke = K * (sp + 1) / nsplit;
+  const double2* X = T.x[q];
+  const double2* Y = T.y[q];
+  const double w = T.w[q];
+  for (long long k0 = kb; k0 < ke; k0 += KC) {
+    for (int e = threadIdx.x; e < TE * KC; e += NTH) {
+      const int i = e / KC, kk = e - i * KC;  // consecutive threads along k
+      const long long k = k0 + kk;
+      const int r = r0 + i, c = c0 + i;
+      xs[kk][i] = (r < nev && k < ke) ? X[(size_t)r * K + k] : make_double2(0.0, 0.0);
+      double2 y = make_double2(0.0, 0.0);
+      if (c < nev && k < ke) {
+        const double2 yv = Y[(size_t)c * K + k], f = ph[k / 3];
+        y = make_double2(w * (f.x * yv.x - f.y * yv.y), w * (f.x * yv.y + f.y * yv.x));
       }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < KC; kk++) {
-        double2 xv[RX], yv[RY];
-#pragma unroll
-        for (int a = 0; a < RX; a++) xv[a] = xs[kk][tx + TX * a];
-#pragma unroll
-        for (int b = 0; b < RY; b++) yv[b] = ys[kk][ty + TY * b];
-#pragma unroll
-        for (int a = 0; a < RX; a++)
-#pragma unroll
-          for (int b = 0; b < RY; b++) {
-            // acc += conj(x) y
-            acc[a][b].x = fma(xv[a].x, yv[b].x, acc[a][b].x);
-            acc[a][b].x = fma(xv[a].y, yv[b].y, acc[a][b].x);
-            acc[a][b].y = fma(xv[a].x, yv[b].y, acc[a][b].y);
-            acc[a][b].y = fma(-xv[a].y, yv[b].x, acc[a][b].y);
-          }
-      }
-      __syncthreads();
+      ys[kk][i] = y;
     }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < KC; kk++) {
+      double2 xv[RX], yv[RY];
+#pragma unroll
+      for (int a = 0; a < RX; a++) xv[a] = xs[kk][tx + TX * a];
+#pragma unroll
+      for (int b = 0; b < RY; b++) yv[b] = ys[kk][ty + TY * b];
+#pragma unroll
+      for (int a = 0; a < RX; a++)
+#pragma unroll
+        for (int b = 0; b < RY; b++) {
+          // acc += conj(x) y
+          acc[a][b].x = fma(xv[a].x, yv[b].x, acc[a][b].x);
+          acc[a][b].x = fma(xv[a].y, yv[b].y, acc[a][b].x);
+          acc[a][b].y = fma(xv[a].x, yv[b].y, acc[a][b].y);
+          acc[a][b].y = fma(-xv[a].y, yv[b].x, acc[a][b].y);
+        }
+    }
+    __syncthreads();
   }
+  double2* o = part + (size_t)pc.part * TE * TE;
 #pragma unroll
   for (int a = 0; a < RX; a++)
 #pragma unroll
-    for (int b = 0; b < RY; b++) {
-      const int r = r0 + tx + TX * a, c = c0 + ty + TY * b;
-      if (r < nev && c < nev) T.out[(size_t)r * nev + c] = acc[a][b];
-    }
+    for (int b = 0; b < RY; b++) o[(tx + TX * a) * TE + ty + TY * b] = acc[a][b];
 }
 
+// One CTA per (output tile, task): adds the tile's partial sums in piece order
+// and writes the elemental, its lower triangle where the task is self-conjugate,
+// and the elemental of the opposite momentum.
+template <int TE>
+__global__ void __launch_bounds__(256) el_sum_kernel(const ElTask* __restrict__ tasks, const int4* __restrict__ tiles,
+                                                     int nev, const double2* __restrict__ part) {
+  const int4 tl = tiles[blockIdx.x];  // task, tile, first partial slot, number of pieces
+  const ElTask& T = tasks[tl.x];
+  const int nti = (nev + TE - 1) / TE;
+  const int r0 = (tl.y / nti) * TE, c0 = (tl.y % nti) * TE;
+  for (int e = threadIdx.x; e < TE * TE; e += 256) {
+    const int r = r0 + e / TE, c = c0 + e % TE;
+    if (r >= nev || c >= nev) continue;
+    double2 v = part[(size_t)tl.z * TE * TE + e];
+    for (int q = 1; q < tl.w; q++) {
+      const double2 u = part[(size_t)(tl.z + q) * TE * TE + e];
+      v.x += u.x;
+      v.y += u.y;
+    }
+    const double2 m = make_double2(T.sign * v.x, -T.sign * v.y);
+    T.out[(size_t)r * nev + c] = v;
+    if (T.self && r0 != c0) T.out[(size_t)c * nev + r] = m;
+    if (T.mirror) T.mirror[(size_t)c * nev + r] = m;
+  }
+}
+
+// Launches of at most EL_PART_BYTES of partial tiles each.
+constexpr size_t EL_PART_BYTES = (size_t)512 << 20;
+
 template <int TE, int RX, int RY>
-int launch_el_gemm(const ElTask* d_tasks, int ntask, int nev, long long K, const double2* phase, long long V,
+int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const double2* phase, long long V,
                    cudaStream_t s) {
   const int nti = (nev + TE - 1) / TE;
-  for (int t0 = 0; t0 < ntask; t0 += 65535) {  // grid.y limit
-    const int nb = std::min(65535, ntask - t0);
-    TimedLaunch tl(s, "el_gemm");
-    el_gemm_kernel<TE, RX, RY><<<dim3(nti * nti, nb), (TE / RX) * (TE / RY), 0, s>>>(d_tasks + t0, nev, K, phase, V);
-    CTR_CUDA(cudaGetLastError());
+  int dev = 0, nsm = 0;
+  CTR_CUDA(cudaGetDevice(&dev));
+  CTR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  long long units = 0;  // products of one tile
+  for (const ElTask& T : tasks) units += (long long)T.nterm * (T.self ? nti * (nti + 1) / 2 : nti * nti);
+  // pieces a product: enough that the launch has about 16 CTAs an SM (its last
+  // wave then costs a few percent), none shorter than 512 of K
+  const int nsplit = (int)std::max<long long>(1, std::min((16LL * nsm + units - 1) / units, K / 512));
+  void* d_tasks;
+  CTR_TRY(upload(WS_TASKS, tasks.data(), tasks.size() * sizeof(ElTask), &d_tasks, s));
+  const size_t max_parts = EL_PART_BYTES / ((size_t)TE * TE * sizeof(double2));
+  std::vector<ElPiece> pieces;
+  std::vector<int4> tiles;
+  auto flush = [&]() -> int {
+    if (pieces.empty()) return CTR_OK;
+    void *d[2], *part;
+    CTR_TRY(upload_group(WS_TASKS2, {{pieces.data(), pieces.size() * sizeof(ElPiece)},
+                                     {tiles.data(), tiles.size() * sizeof(int4)}}, d, s));
+    CTR_TRY(workspace(WS_ROWS).get(pieces.size() * TE * TE * sizeof(double2), &part));
+    {
+      TimedLaunch tl(s, "el_gemm");
+      el_gemm_kernel<TE, RX, RY><<<(unsigned)pieces.size(), (TE / RX) * (TE / RY), 0, s>>>(
+          (const ElTask*)d_tasks, (const ElPiece*)d[0], nev, K, nsplit, phase, V, (double2*)part);
+      CTR_CUDA(cudaGetLastError());
+    }
+    {
+      TimedLaunch tl(s, "el_sum");
+      el_sum_kernel<TE><<<(unsigned)tiles.size(), 256, 0, s>>>((const ElTask*)d_tasks, (const int4*)d[1], nev,
+                                                               (const double2*)part);
+      CTR_CUDA(cudaGetLastError());
+    }
+    pieces.clear();
+    tiles.clear();
+    return CTR_OK;
+  };
+  for (size_t k = 0; k < tasks.size(); k++) {
+    const ElTask& T = tasks[k];
+    for (int tile = 0; tile < nti * nti; tile++) {
+      if (T.self && tile / nti > tile % nti) continue;
+      const int np = T.nterm * nsplit;
+      if (pieces.size() + np > max_parts) CTR_TRY(flush());
+      tiles.push_back(make_int4((int)k, tile, (int)pieces.size(), np));
+      for (int q = 0; q < np; q++) pieces.push_back(ElPiece{(int)k, tile, q, (int)pieces.size()});
+    }
   }
-  return CTR_OK;
+  return flush();
 }
 
 }  // namespace
@@ -237,18 +319,41 @@ int ctr_elementals(int nev, int nt, int nx, int ny, int nz, const double* evec, 
         v, (const double2*)links, nev, nt, nx, ny, nz, dv);
     CTR_CUDA(cudaGetLastError());
   }
+  // Reversed momenta: with the phase of -p the complex conjugate of p's,
+  // Phi_{0,1}(-p) = Phi_{0,1}(p)^dag and Phi_{2+j}(-p) = -Phi_{2+j}(p)^dag, so one of
+  // the two is computed and the other written with it; a p with the phases of
+  // its own -p needs the tiles on and above the diagonal only.  The seven
+  // momenta |p|^2 <= 1 then take 37.5 products of the five operators instead of 70.
+  const int L[3] = {nx, ny, nz};
+  auto reversed = [&](int a, int b) {
+    for (int d = 0; d < 3; d++)
+      if (((long long)mom[3 * a + d] + mom[3 * b + d]) % L[d] != 0) return false;
+    return true;
+  };
+  std::vector<int> mirror(nmom, -1);
+  std::vector<char> done(nmom, 0);
+  for (int p = 0; p < nmom; p++) {
+    if (done[p] || reversed(p, p)) continue;
+    for (int b = p + 1; b < nmom && mirror[p] < 0; b++)
+      if (!done[b] && reversed(p, b)) mirror[p] = b, done[b] = 1;
+  }
   // tasks: per (p, op, t) the output block phi[p][op][t] (the drivers' layout)
   auto vec = [&](int t) { return v + (size_t)t * nev * K; };
   auto dvec = [&](int j, int t) { return dv + ((size_t)j * nt + t) * nev * K; };
+  auto block = [&](int p, int op, int t) { return (double2*)phi + (((size_t)p * nops + op) * nt + t) * nev * nev; };
   std::vector<ElTask> tasks;
   tasks.reserve((size_t)nmom * nops * nt);
-  for (int p = 0; p < nmom; p++)
+  for (int p = 0; p < nmom; p++) {
+    if (done[p]) continue;
     for (int op = 0; op < nops; op++)
       for (int t = 0; t < nt; t++) {
         ElTask T;
         std::memset(&T, 0, sizeof(T));
         T.p = p;
-        T.out = (double2*)phi + (((size_t)p * nops + op) * nt + t) * nev * nev;
+        T.self = reversed(p, p);
+        T.sign = op < 2 ? 1.0 : -1.0;
+        T.out = block(p, op, t);
+        T.mirror = mirror[p] >= 0 ? block(mirror[p], op, t) : nullptr;
         if (op == 0) {  // <v_r| e^{-ip.x} |v_c>
           T.nterm = 1;
           T.x[0] = vec(t);
@@ -273,12 +378,9 @@ int ctr_elementals(int nev, int nt, int nx, int ny, int nz, const double* evec, 
         }
         tasks.push_back(T);
       }
-  void* d_tasks;
-  CTR_TRY(upload(WS_TASKS, tasks.data(), tasks.size() * sizeof(ElTask), &d_tasks, s));
-  const int ntask = (int)tasks.size();
+  }
   // output tile edge: 50 (250 threads, 5 x 2 outputs each) where it pads Nev least, else 32 (256 threads, 2 x 2)
   const int pad50 = ((nev + 49) / 50) * 50 - nev, pad32 = ((nev + 31) / 32) * 32 - nev;
-  if (nev >= 50 && pad50 <= pad32)
-    return launch_el_gemm<50, 5, 2>((const ElTask*)d_tasks, ntask, nev, K, phase, V, s);
-  return launch_el_gemm<32, 2, 2>((const ElTask*)d_tasks, ntask, nev, K, phase, V, s);
+  if (nev >= 50 && pad50 <= pad32) return launch_el_gemm<50, 5, 2>(tasks, nev, K, phase, V, s);
+  return launch_el_gemm<32, 2, 2>(tasks, nev, K, phase, V, s);
 }

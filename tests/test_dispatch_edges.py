@@ -42,3 +42,19 @@ def test_loop_unity_cluster_sizes(cuda, nt, n):
     # each sum adds at most Nev^2 / 128 + 11 rounded terms in sequence
     terms = np.einsum("tssij,tji->t", np.abs(diag), np.abs(mom))
     assert np.all(np.abs(got - ref) <= 2.0 ** -53 * (n * n / 128 + 16) * terms)
+
+
+@pytest.mark.parametrize("nev", [1, 33, 51])
+def test_elementals_pieces_and_reversed_momenta(cuda, nev):
+    """K long enough for two pieces, tiles with remainders at both tile edges;
+    momenta that are their own reverse (0, and half the lattice), reversed
+    pairs, a pair reversed only modulo the lattice, repeats and one alone."""
+    from oracle import elementals as E
+    nt, nx, ny, nz = 1, 8, 6, 8
+    moms = [(1, 0, 0), (0, 0, 0), (-1, 0, 0), (4, 3, 0), (7, 6, 8), (1, 2, -1), (1, 0, 0), (0, 0, 0)]
+    V, U = synth.make_eigvecs(nt, nev, nx, ny, nz, 700 + nev), synth.make_links(nt, nx, ny, nz, 701)
+    ref = E.elementals(V, moms, U)
+    got = api.elementals(_dev(V, cuda), moms, links=_dev(U, cuda)).cpu().numpy()
+    assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+    plain = api.elementals(_dev(V, cuda), moms).cpu().numpy()
+    assert np.abs(plain[:, 0] - ref[:, 0]).max() <= 1e-12 * np.abs(ref[:, 0]).max()
