@@ -871,7 +871,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
       CTR_TRY(workspace(WS_SPLITTASK).get((size_t)ni * per, &mem));
       uint8_t* lbase = (uint8_t*)mem;
       uint8_t* rbase = lbase + (size_t)ni * (l_b + le_b);
-      std::vector<SliceStackLJob> lj(ni);
+      std::vector<SliceStackLJob> lj;
       std::vector<SliceTaskRJob> rj;
       std::map<const double2*, int> bid;
       std::vector<const double2*> blks;
@@ -883,33 +883,49 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
         }
         return b->second;
       };
-      std::map<std::vector<uintptr_t>, int> rid;
+      std::map<std::vector<uintptr_t>, int> lid, rid;
+      std::vector<uintptr_t> key;
       std::vector<SplitGemmInst> gi(ni);
       std::vector<double2*> outs((size_t)ni * SPLIT_TASK_NB, nullptr);
       for (int i = 0; i < ni; i++) {
         const Piece& pc = all[i0 + i];
         const GridTask& G = grids[pc.g];
-        SliceStackLJob& L = lj[i];
-        std::memset(&L, 0, sizeof(L));
+        // equal left stacks (the same blocks, weights and transposes) are sliced once
+        key.clear();
+        for (int k = 0; k < pc.ns * nterm; k++) key.push_back((uintptr_t)G.A[(size_t)pc.s0 * nterm + k]);
         for (int q = 0; q < nterm; q++) {
-          int ex;
-          std::frexp(G.w[q], &ex);
-          L.w[q] = G.w[q];
-          L.wexp[q] = ex - 1;
+          uint32_t bits;
+          std::memcpy(&bits, &G.w[q], sizeof(bits));
+          key.push_back(bits);
         }
-        for (int sl = 0; sl < pc.ns; sl++)
+        key.push_back((uintptr_t)G.adag);
+        auto lt = lid.find(key);
+        if (lt == lid.end()) {
+          SliceStackLJob L;
+          std::memset(&L, 0, sizeof(L));
           for (int q = 0; q < nterm; q++) {
-            const double2* a = G.A[(size_t)(pc.s0 + sl) * nterm + q];
-            L.a[sl][q] = a;
-            L.bi[sl][q] = block_index(a);
+            int ex;
+            std::frexp(G.w[q], &ex);
+            L.w[q] = G.w[q];
+            L.wexp[q] = ex - 1;
           }
-        L.nslab = pc.ns;
-        L.nterm = nterm;
-        L.dag = G.adag;
-        L.eplus = eplus;
-        L.out = lbase + (size_t)i * (l_b + le_b);
-        L.exps = (int*)(L.out + l_b);
-        std::vector<uintptr_t> key;
+          for (int sl = 0; sl < pc.ns; sl++)
+            for (int q = 0; q < nterm; q++) {
+              const double2* a = G.A[(size_t)(pc.s0 + sl) * nterm + q];
+              L.a[sl][q] = a;
+              L.bi[sl][q] = block_index(a);
+            }
+          L.nslab = pc.ns;
+          L.nterm = nterm;
+          L.dag = G.adag;
+          L.eplus = eplus;
+          L.out = lbase + lj.size() * (l_b + le_b);
+          L.exps = (int*)(L.out + l_b);
+          lt = lid.emplace(key, (int)lj.size()).first;
+          lj.push_back(L);
+        }
+        const SliceStackLJob& L = lj[lt->second];
+        key.clear();
         for (int j = 0; j < nb; j++)
           for (int q = 0; q < nterm; q++) key.push_back((uintptr_t)G.B[j][q]);
         key.push_back((uintptr_t)G.bdag);
@@ -947,8 +963,8 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
       void* d_bexp;
       CTR_TRY(workspace(WS_BLOCKEXP).get(blks.size() * 2 * N * sizeof(int), &d_bexp));
       CTR_TRY(launch_block_exp((const double2* const*)d1[3], (int)blks.size(), N, (int*)d_bexp, stream));
-      CTR_TRY(launch_slice_stack_left((const SliceStackLJob*)d1[0], ni, N, nchunk, mtiles, (const int*)d_bexp,
-                                      stream));
+      CTR_TRY(launch_slice_stack_left((const SliceStackLJob*)d1[0], (int)lj.size(), N, nchunk, mtiles,
+                                      (const int*)d_bexp, stream));
       CTR_TRY(launch_slice_task_right((const SliceTaskRJob*)d1[1], (int)rj.size(), N, nchunk, ntiles,
                                       (const int*)d_bexp, stream));
       SplitGemmBatch B{(const SplitGemmInst*)d_gi, mtiles, ntiles, nchunk, ns * N, nb * N, mtiles * SPLIT_M,
