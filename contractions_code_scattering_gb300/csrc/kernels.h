@@ -62,6 +62,8 @@ __device__ inline double block_sum_256(double v) {
 // that the weights allow the DMMA form.
 int launch_zgemm_f64(const ZTask* d_tasks, int ntask, int N, cudaStream_t s, const ZTask* h_tasks = nullptr);
 int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s);
+// The launch alone, not counted or timed.
+int launch_trace_f64_untimed(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s);
 // loop[t] = sum_s Tr[tau(t,t)_ss Phi(t)] for diag [Nt][4][4][N][N], mom [Nt][N][N].
 int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s);
 int launch_rowsum(const double2* rows, int nrows, const int* off, const int* idx, int nout, int npair,

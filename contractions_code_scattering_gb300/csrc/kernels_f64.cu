@@ -296,10 +296,32 @@ __device__ __forceinline__ float abs_scaled_f32(double v) {
 
 __device__ __forceinline__ float abs1_scaled_f32(double2 v) { return abs_scaled_f32(v.x) + abs_scaled_f32(v.y); }
 
+// Block sums of two FP64 values: lanes 0-15 of each warp carry the first, 16-31
+// the second (5 adds a warp instead of 10: each holds the FP64 pipe for 16
+// clocks), then the warps' sums in order.  Thread k < 2 returns value k.
+template <int TPB>
+__device__ __forceinline__ double block_sum2(double x, double y) {
+  __shared__ double red[TPB / 32][2];
+  const int lane = threadIdx.x & 31;
+  double s = ((lane & 16) ? y : x) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? x : y, 16);
+  for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((lane & 15) == 0) red[threadIdx.x >> 5][lane >> 4] = s;
+  __syncthreads();
+  double v = 0.0;
+  if (threadIdx.x < 2) {
+    v = red[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < TPB / 32; w++) v += red[w][threadIdx.x];
+  }
+  return v;
+}
+
 // out = coef * sum_e X_e * conj(Y_e) over the Nev*Nev elements (mode 0), or
 // coef * sum_ij X_ij * Y_ji = coef * Tr[X Y] (mode 1).  One CTA per task; the
 // reduction tree is fixed, so results are bitwise reproducible.
-__global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restrict__ tasks, int ntask, int N) {
+template <int TPB>
+__global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restrict__ tasks, int ntask, int N) {
+  __shared__ float reda[TPB / 32];
   const int t = blockIdx.x;
   if (t >= ntask) return;
   const TraceTask& T = tasks[t];
@@ -309,7 +331,7 @@ __global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restr
   float abf = 0.f;
   // two FMAs into each accumulator per element (the FP64 pipe is the bound)
   if (T.mode == 0) {
-    for (int e = threadIdx.x; e < n2; e += 256) {
+    for (int e = threadIdx.x; e < n2; e += TPB) {
       double2 x = T.X[e], y = T.Y[e];
       re = fma(x.x, y.x, re);
       re = fma(x.y, y.y, re);
@@ -318,7 +340,7 @@ __global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restr
       if (want_abs) abf = fmaf(abs1_scaled_f32(x), abs1_scaled_f32(y), abf);
     }
   } else {
-    for (int e = threadIdx.x; e < n2; e += 256) {
+    for (int e = threadIdx.x; e < n2; e += TPB) {
       int i = e / N, j = e % N;
       double2 x = T.X[e], y = T.Y[(size_t)j * N + i];
       re = fma(x.x, y.x, re);
@@ -328,15 +350,22 @@ __global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restr
       if (want_abs) abf = fmaf(abs1_scaled_f32(x), abs1_scaled_f32(y), abf);
     }
   }
-  re = block_sum_256(re);
-  im = block_sum_256(im);
-  double ab = 0.0;
-  if (want_abs) ab = block_sum_256((double)abf) * 0x1p-80;  // 2^(-2 TRACE_ABS_SHIFT)
+  if (want_abs) {
+    for (int o = 16; o; o >>= 1) abf += __shfl_xor_sync(0xffffffffu, abf, o);
+    if ((threadIdx.x & 31) == 0) reda[threadIdx.x >> 5] = abf;
+  }
+  const double v = block_sum2<TPB>(re, im);
+  if (threadIdx.x >= 32) return;
+  const double vi = __shfl_sync(0xffffffffu, v, 1);
   if (threadIdx.x == 0) {
-    double2 c = make_double2((double)T.coef[0], (double)T.coef[1]);
-    double2 s = make_double2(re, im);
-    *T.out = cmul(c, s);
-    if (want_abs) *T.absout = sqrt(c.x * c.x + c.y * c.y) * ab;
+    *T.out = cmul(make_double2((double)T.coef[0], (double)T.coef[1]), make_double2(v, vi));
+    if (want_abs) {
+      float ab = reda[0];
+#pragma unroll
+      for (int w = 1; w < TPB / 32; w++) ab += reda[w];
+      // 2^-80 = 2^(-2 TRACE_ABS_SHIFT)
+      *T.absout = (double)sqrtf(T.coef[0] * T.coef[0] + T.coef[1] * T.coef[1]) * ((double)ab * 0x1p-80);
+    }
   }
 }
 
@@ -348,40 +377,39 @@ __global__ void __launch_bounds__(256) trace_f64_kernel(const TraceTask* __restr
 // range of the Nev^2 elements; CTA 0 adds the CTAs' partial sums in rank order
 // through distributed shared memory, so there is one launch, no table to upload
 // and a fixed summation order.
-constexpr int LOOP_TPB = 128;
+constexpr int LOOP_TPB = 256;
 
 __global__ void __launch_bounds__(LOOP_TPB) loop_unity_kernel(const double2* __restrict__ diag,
                                                               const double2* __restrict__ mom, int N, int ncta,
                                                               double2* __restrict__ loop) {
-  __shared__ double red[LOOP_TPB / 32][2];
   __shared__ double part[2];
   const int t = blockIdx.x / ncta, rank = blockIdx.x - t * ncta;
-  const size_t n2 = (size_t)N * N;
+  const unsigned n2 = (unsigned)N * N;  // Nev <= 4096
   const double2* T = diag + (size_t)t * 16 * n2;
   const double2* P = mom + (size_t)t * n2;
-  const size_t e1 = n2 * (rank + 1) / ncta;
+  const unsigned e1 = (unsigned)((unsigned long long)n2 * (rank + 1) / ncta);
+  unsigned e = (unsigned)((unsigned long long)n2 * rank / ncta) + threadIdx.x;
+  unsigned i = e / N, j = e - i * N;
+  const unsigned di = LOOP_TPB / N, dj = LOOP_TPB - di * N;
   double re = 0.0, im = 0.0;
-#pragma unroll 2
-  for (size_t e = n2 * rank / ncta + threadIdx.x; e < e1; e += LOOP_TPB) {
-    const size_t i = e / N, j = e - i * N;
-    const double2 a = T[e], b = T[e + 5 * n2], c = T[e + 10 * n2], d = T[e + 15 * n2], y = P[j * N + i];
+#pragma unroll 4
+  for (; e < e1; e += LOOP_TPB) {
+    const double2 a = T[e], b = T[(size_t)e + 5 * (size_t)n2], c = T[(size_t)e + 10 * (size_t)n2],
+                  d = T[(size_t)e + 15 * (size_t)n2], y = P[(size_t)j * N + i];
     const double xr = (a.x + b.x) + (c.x + d.x), xi = (a.y + b.y) + (c.y + d.y);
     re = fma(xr, y.x, re);
     re = fma(-xi, y.y, re);
     im = fma(xr, y.y, im);
     im = fma(xi, y.x, im);
+    i += di;
+    j += dj;
+    if (j >= (unsigned)N) {
+      j -= N;
+      i++;
+    }
   }
-  // lanes 0-15 take the sum of re, lanes 16-31 that of im
-  const int lane = threadIdx.x & 31;
-  double s = ((lane & 16) ? im : re) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? re : im, 16);
-  for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((lane & 15) == 0) red[threadIdx.x >> 5][lane >> 4] = s;
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    double v = red[0][threadIdx.x];
-    for (int w = 1; w < LOOP_TPB / 32; w++) v += red[w][threadIdx.x];
-    part[threadIdx.x] = v;
-  }
+  const double sum = block_sum2<LOOP_TPB>(re, im);
+  if (threadIdx.x < 2) part[threadIdx.x] = sum;
   if (ncta == 1) {
     if (threadIdx.x < 2) ((double*)(loop + t))[threadIdx.x] = part[threadIdx.x];
     return;
@@ -566,12 +594,22 @@ int launch_zgemm_f64(const ZTask* d_tasks, int ntask, int N, cudaStream_t s, con
   return launch_zgemm_variant(v, d_tasks, ntask, N, s);
 }
 
+// Up to this Nev a trace takes two warps: fewer warps mean fewer cross-lane adds.
+constexpr int TRACE_F64_SMALL = 64;
+
+int launch_trace_f64_untimed(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s) {
+  if (N <= TRACE_F64_SMALL)
+    trace_f64_kernel<64><<<ntask, 64, 0, s>>>(d_tasks, ntask, N);
+  else
+    trace_f64_kernel<256><<<ntask, 256, 0, s>>>(d_tasks, ntask, N);
+  CTR_CUDA(cudaGetLastError());
+  return CTR_OK;
+}
+
 int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s) {
   if (ntask == 0) return CTR_OK;
   TimedLaunch tl(s, "trace_f64");
-  trace_f64_kernel<<<ntask, 256, 0, s>>>(d_tasks, ntask, N);
-  CTR_CUDA(cudaGetLastError());
-  return CTR_OK;
+  return launch_trace_f64_untimed(d_tasks, ntask, N, s);
 }
 
 int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s) {

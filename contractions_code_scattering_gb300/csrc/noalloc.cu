@@ -23,7 +23,6 @@
 namespace ctr {
 
 __global__ void zgemm_f64_kernel(const ZTask* __restrict__ tasks, int ntask, int N, int tiles_per_dim);
-__global__ void trace_f64_kernel(const TraceTask* __restrict__ tasks, int ntask, int N);
 __global__ void rowsum_kernel(const double2* __restrict__ rows, int nrows, const int* __restrict__ off,
                               const int* __restrict__ idx, int nout, int npair, double2* __restrict__ out,
                               size_t out_pair_stride);
@@ -193,8 +192,7 @@ int rho_noalloc(int N, int Nt, int tf, const double* prop_row, const double* mom
     CTR_CUDA(cudaGetLastError());
     zgemm_f64_kernel<<<nprod * tpd * tpd, 256, 0, stream>>>(d_gemm, nprod, N, tpd);
     CTR_CUDA(cudaGetLastError());
-    trace_f64_kernel<<<kRows, 256, 0, stream>>>(d_trace, kRows, N);
-    CTR_CUDA(cudaGetLastError());
+    CTR_TRY(launch_trace_f64_untimed(d_trace, kRows, N, stream));
     rowsum_kernel<<<1, 64, 0, stream>>>(d_rows, kRows, d_csr, d_csr + kOut + 1, kOut, 1,
                                         (double2*)corr + (size_t)ti * kOut, kOut);
     CTR_CUDA(cudaGetLastError());
