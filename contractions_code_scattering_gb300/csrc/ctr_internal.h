@@ -169,6 +169,20 @@ struct GramPlan {
 };
 int trace_gram(int N, const GramPlan& plan, double2* trv, double* tra, cudaStream_t stream);
 
+// Gram products whose every entry is wanted: group g has nblk blocks, each with
+// left blocks left[(g * nblk + b) * mrows + r] and right blocks
+// right[(g * nblk + b) * ncols + c] (null: zeros), and
+//   trv[rowbase[g * mrows + r] + c] = sum_b +-Tr-Had(left, right),
+// - where bit b of negative is set; rows with a negative base are padding.  tra as
+// trace_gram's.
+struct GramRows {
+  int ngroup = 0, nblk = 0, mrows = 0, ncols = 0;
+  unsigned negative = 0;
+  std::vector<const double2*> left, right;
+  std::vector<int> rowbase;
+};
+int gram_rows(int N, const GramRows& plan, double2* trv, double* tra, cudaStream_t stream);
+
 // ------------------------------------------------------------ graph capture
 // A host step that reads device results (e.g. the split engine's refinement
 // list).  Run at once by eager calls; while the thread records a graph, it ends

@@ -22,7 +22,9 @@
 // is one task of the batched GEMM (up to 4 accumulated terms with the gamma_5
 // signs).
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <iterator>
 #include <map>
 #include <tuple>
 #include <utility>
@@ -120,7 +122,8 @@ const float kG5[4] = {(float)G5[0], (float)G5[1], (float)G5[2], (float)G5[3]};
 // extents as even as the batch allows, so that the pairs that share a t_src (the
 // right operands R and Phi(t_src)) and those that share a t_sink (L and
 // Phi(t_sink)) both stack along M: from 7 pairs of 4 slabs up, the padding rows of
-// a 128-row tile are below 2 %.  A list of pairs keeps the list's order.
+// a 128-row tile are below 2 %.  At most hmax sink times a batch.  A list of pairs
+// keeps the list's order.
 struct PairBatch {
   std::vector<int> ent, tf, ti;       // position in the output, time slices
   std::vector<const double2*> T;      // tau(tf, ti)
@@ -129,7 +132,7 @@ struct PairBatch {
 };
 
 std::vector<PairBatch> pair_batches(const double2* tau, size_t blk16, int Nt, int tf_begin, int rows, int batch,
-                                    const std::vector<int>* plist) {
+                                    const std::vector<int>* plist, int hmax = 1 << 30) {
   std::vector<std::vector<std::pair<int, int>>> out;  // (position, pair)
   if (plist) {
     for (size_t i = 0; i < plist->size(); i++) {
@@ -143,6 +146,7 @@ std::vector<PairBatch> pair_batches(const double2* tau, size_t blk16, int Nt, in
       while ((e + 1) * (e + 1) <= batch) e++;
       h = std::min(rows, e >= 16 ? e & ~7 : e);
     }
+    h = std::min(h, hmax);
     const int w = std::min(Nt, std::max(1, batch / h));
     for (int f0 = 0; f0 < rows; f0 += h)
       for (int t0 = 0; t0 < Nt; t0 += w) {
@@ -713,23 +717,25 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
 
 namespace {
 
-// Row sums of batch items whose rows' trace values sit anywhere: row r of item it
-// is trace slot rowslot[it * nrows + r], times rcoef[r] where given; output o sums
-// rows idx[off[o] .. off[o+1]) in that order into out[ent[it] * nout + o]; with
-// trabs, entries whose error estimate exceeds the tolerance append ent * nout + o
-// to the refinement list.
+// Row sums of batch items: row r of item it is trace slot itembase[it] + rowoff[r],
+// conjugated where conj is set, times rcoef[r] where given; output o sums rows
+// idx[off[o] .. off[o+1]) in that order into out[ent[it] * nout + o]; with trabs,
+// entries whose error estimate exceeds the tolerance append ent * nout + o to the
+// refinement list.
 __global__ void rowsum_items_kernel(const double2* __restrict__ trv, const double* __restrict__ trabs,
-                                    const int* __restrict__ rowslot, int nrows, const int* __restrict__ off,
-                                    const int* __restrict__ idx, const float2* __restrict__ rcoef, int nout,
-                                    const int* __restrict__ ent, int nitem, double2* __restrict__ out,
-                                    double eps_over_tol, int* __restrict__ count, int* __restrict__ list) {
+                                    const int* __restrict__ itembase, const int* __restrict__ rowoff, int conj,
+                                    const int* __restrict__ off, const int* __restrict__ idx,
+                                    const float2* __restrict__ rcoef, int nout, const int* __restrict__ ent, int nitem,
+                                    double2* __restrict__ out, double eps_over_tol, int* __restrict__ count,
+                                    int* __restrict__ list) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nitem * nout) return;
-  const int it = g / nout, o = g % nout;
+  const int it = g / nout, o = g % nout, base = itembase[it];
   double re = 0.0, im = 0.0, sc = 0.0;
   for (int k = off[o]; k < off[o + 1]; k++) {
-    const int r = idx[k], j = rowslot[(size_t)it * nrows + r];
+    const int r = idx[k], j = base + rowoff[r];
     double2 v = trv[j];
+    if (conj) v.y = -v.y;
     double a = trabs ? trabs[j] : 0.0;
     if (rcoef) {  // the row's coefficient, applied as the trace kernel applies it
       const double2 c = make_double2((double)rcoef[r].x, (double)rcoef[r].y);
@@ -749,10 +755,11 @@ __global__ void rowsum_items_kernel(const double2* __restrict__ trv, const doubl
 
 // Item tables of one row-sum launch (host), and their device copies.
 struct RowItems {
-  std::vector<int> slot, csr, ent;
-  std::vector<float2> coef;  // per row, or empty
-  int nrows = 0, nout = 0;
-  const int *d_slot = nullptr, *d_csr = nullptr, *d_ent = nullptr;
+  std::vector<int> base, ent;  // per item
+  std::vector<int> off, csr;   // per row; rows of each output
+  std::vector<float2> coef;    // per row, or empty
+  int nout = 0, conj = 0;
+  const int *d_base = nullptr, *d_off = nullptr, *d_csr = nullptr, *d_ent = nullptr;
   const float2* d_coef = nullptr;
 };
 
@@ -760,7 +767,8 @@ struct RowItems {
 int upload_items(const Ctx& c, std::vector<RowItems*> items) {
   std::vector<std::pair<const void*, size_t>> parts;
   for (RowItems* r : items) {
-    parts.push_back({r->slot.data(), r->slot.size() * sizeof(int)});
+    parts.push_back({r->base.data(), r->base.size() * sizeof(int)});
+    parts.push_back({r->off.data(), r->off.size() * sizeof(int)});
     parts.push_back({r->csr.data(), r->csr.size() * sizeof(int)});
     parts.push_back({r->ent.data(), r->ent.size() * sizeof(int)});
     parts.push_back({r->coef.data(), r->coef.size() * sizeof(float2)});
@@ -768,10 +776,11 @@ int upload_items(const Ctx& c, std::vector<RowItems*> items) {
   std::vector<void*> d(parts.size());
   CTR_TRY(upload_group(WS_MISC, parts, d.data(), c.s));
   for (size_t i = 0; i < items.size(); i++) {
-    items[i]->d_slot = (const int*)d[4 * i];
-    items[i]->d_csr = (const int*)d[4 * i + 1];
-    items[i]->d_ent = (const int*)d[4 * i + 2];
-    items[i]->d_coef = items[i]->coef.empty() ? nullptr : (const float2*)d[4 * i + 3];
+    items[i]->d_base = (const int*)d[5 * i];
+    items[i]->d_off = (const int*)d[5 * i + 1];
+    items[i]->d_csr = (const int*)d[5 * i + 2];
+    items[i]->d_ent = (const int*)d[5 * i + 3];
+    items[i]->d_coef = items[i]->coef.empty() ? nullptr : (const float2*)d[5 * i + 4];
   }
   return CTR_OK;
 }
@@ -781,11 +790,102 @@ int rowsum_items(const Ctx& c, const double2* trv, const double* tra, const RowI
   if (r.ent.empty()) return CTR_OK;
   TimedLaunch tl(c.s, "rowsum_items");
   const int n = (int)r.ent.size() * r.nout;
-  rowsum_items_kernel<<<(n + 127) / 128, 128, 0, c.s>>>(trv, rf.on ? tra : nullptr, r.d_slot, r.nrows, r.d_csr,
+  rowsum_items_kernel<<<(n + 127) / 128, 128, 0, c.s>>>(trv, rf.on ? tra : nullptr, r.d_base, r.d_off, r.conj, r.d_csr,
                                                         r.d_csr + r.nout + 1, r.d_coef, r.nout, r.d_ent,
                                                         (int)r.ent.size(), out, rf.eps_over_tol, rf.count, rf.list);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
+}
+
+// ---- sink form of the rho -> pi pi and triangle traces
+// A vertex is one output's sink side: operator `slab`, and for each spin s3 of the
+// closing tau the spin s5 its gamma structure leads to, with coefficient c (g5(s3)
+// included).  The output sum_{s2,s3} c(s3) Tr-Had(Op X_{s5 s2}, tau_{s3 s2}) with
+// X = T G R is
+//   sum_{s1,s2} g5(s1) Tr[Q_{s2 s1} R_{s1 s2}],
+//   (Q_{s2 s1})^dag = H_{s1 s2} = sum_{s3} conj(c(s3)) (Op tau_{s5 s1})^dag tau_{s3 s2},
+// where H does not depend on the momentum set: its products replace the 64 of X
+// per set, and its traces against R, sum_b g5 conj(Tr-Had(H_b, R_b)), are all the
+// entries of one Gram product (rows: pairs of a t_src x vertices; columns: sets).
+struct Vertex {
+  int slab, s5[4];
+  float cre[4], cim[4];
+};
+struct SinkTerm {  // H = sum_k w_k (Op tau_{s5_k s1})^dag tau_{s3_k s2}
+  int slab, n, s3[4], s5[4];
+  float w[4];
+};
+struct SinkPlan {
+  std::vector<SinkTerm> H;
+  std::vector<std::vector<int>> stacks;                     // terms with the same s3 and w: one grid
+  std::vector<std::vector<std::pair<int, float2>>> rows;    // vertex -> (term, coefficient)
+  int products = 0;                                         // block products of the terms, per pair
+};
+
+// False where a vertex's coefficients are not +-1 times one of them.  Two vertices
+// of one operator that differ in the sign of half their spins (gamma_x and gamma_y)
+// share two terms of two spins each, a and b: one is a + b, the other a - b.
+bool sink_plan(const std::vector<Vertex>& V, SinkPlan& P) {
+  std::vector<std::array<int, 4>> sg(V.size());
+  std::map<std::array<int, 5>, std::vector<int>> by;
+  P.rows.resize(V.size());
+  for (size_t v = 0; v < V.size(); v++) {
+    const Vertex& x = V[v];
+    const float n0 = x.cre[0] * x.cre[0] + x.cim[0] * x.cim[0];
+    for (int k = 0; k < 4; k++) {
+      const float re = x.cre[k] * x.cre[0] + x.cim[k] * x.cim[0], im = x.cim[k] * x.cre[0] - x.cre[k] * x.cim[0];
+      if (n0 == 0.f || im != 0.f || (re != n0 && re != -n0)) return false;
+      sg[v][k] = re == n0 ? 1 : -1;
+    }
+    by[{x.slab, x.s5[0], x.s5[1], x.s5[2], x.s5[3]}].push_back((int)v);
+  }
+  auto term = [&](const Vertex& x, const std::array<int, 4>& s, const std::vector<int>& spins) {
+    SinkTerm t;
+    std::memset(&t, 0, sizeof(t));
+    t.slab = x.slab;
+    for (int k : spins) {
+      t.s3[t.n] = k;
+      t.s5[t.n] = x.s5[k];
+      t.w[t.n++] = (float)s[k];
+    }
+    P.H.push_back(t);
+    P.products += 16 * t.n;
+    return (int)P.H.size() - 1;
+  };
+  for (auto& g : by) {
+    std::map<std::array<int, 4>, std::vector<int>> sig;
+    for (int v : g.second) sig[sg[v]].push_back(v);
+    if (sig.size() == 2) {
+      const auto &s1 = sig.begin()->first, &s2 = std::next(sig.begin())->first;
+      std::vector<int> same, diff;
+      for (int k = 0; k < 4; k++) (s1[k] == s2[k] ? same : diff).push_back(k);
+      if (same.size() == 2) {
+        const int a = term(V[g.second[0]], s1, same), b = term(V[g.second[0]], s1, diff);
+        for (auto& e : sig)
+          for (int v : e.second) {
+            const float sb = e.first == s1 ? 1.f : -1.f;
+            P.rows[v].push_back({a, make_float2(V[v].cre[0], V[v].cim[0])});
+            P.rows[v].push_back({b, make_float2(sb * V[v].cre[0], sb * V[v].cim[0])});
+          }
+        continue;
+      }
+    }
+    for (auto& e : sig) {
+      const int h = term(V[e.second[0]], e.first, {0, 1, 2, 3});
+      for (int v : e.second) P.rows[v].push_back({h, make_float2(V[v].cre[0], V[v].cim[0])});
+    }
+  }
+  std::map<std::vector<int>, std::vector<int>> st;
+  for (size_t h = 0; h < P.H.size(); h++) {
+    std::vector<int> key;
+    for (int k = 0; k < P.H[h].n; k++) {
+      key.push_back(P.H[h].s3[k]);
+      key.push_back(P.H[h].w[k] > 0.f ? 1 : -1);
+    }
+    st[key].push_back((int)h);
+  }
+  for (auto& e : st) P.stacks.push_back(e.second);
+  return true;
 }
 
 }  // namespace
@@ -841,7 +941,6 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
     std::vector<TraceTask> tt;
     tt.reserve(ntr);
     RowItems ri;
-    ri.nrows = 16;
     ri.nout = 1;
     for (int k = 0; k < nset; k++)
       for (int i = 0; i < nts; i++) {
@@ -851,12 +950,15 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
           tt.push_back(tr(M[(size_t)cR[k] * Nt + t] + ab * N2, diag + t * blk16 + ab * N2,
                           (double2*)trm + tt.size(), Tb.hf_coef[b][0], Tb.hf_coef[b][1], 0));
           if (tra) tt.back().absout = (double*)tra + (tt.size() - 1);
-          ri.slot.push_back((int)tt.size() - 1);
         }
+        ri.base.push_back((int)tt.size() - 16);
         ri.ent.push_back(k * nts + i);
       }
     ri.csr = {0, 16};
-    for (int b = 0; b < 16; b++) ri.csr.push_back(b);
+    for (int b = 0; b < 16; b++) {
+      ri.csr.push_back(b);
+      ri.off.push_back(b);
+    }
     CTR_TRY(run_traces(c, tt));
     CTR_TRY(upload_items(c, {&ri}));
     CTR_TRY(rowsum_items(c, (double2*)trm, (double*)tra, ri, (double2*)hor_fish, rf));
@@ -939,7 +1041,6 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   std::vector<int> csr_tr = {0, 16, 32};
   for (int k = 0; k < 32; k++) csr_tr.push_back(k);
 
-  const int ngr = rhopi ? (int)grp[0].size() : 0;
   const size_t blk_pair = 16 * ((size_t)nC + nops);
   const size_t tr_pair = (size_t)nset * (uniq.size() + (tri ? 32 : 0));
   const size_t per_pair = blk_pair * N2 * sizeof(double2) + tr_pair * (sizeof(double2) + sizeof(double));
@@ -955,7 +1056,143 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   Refine rf_rp, rf_tr;
   if (rhopi) CTR_TRY(refine_begin(c, (size_t)nset * nd * npairs * 4, WS_REFINE, rf_rp));
   if (tri) CTR_TRY(refine_begin(c, (size_t)nset * npairs * 2, WS_SPLITJOBS3, rf_tr));
-  for (const PairBatch& pb : pair_batches(tau, blk16, Nt, tf_begin, rows, batch, plist)) {
+  // The sink form takes its place where it costs less, per pair: the terms' block
+  // products instead of 64 a set, and its rows to slice for the Gram product (16
+  // blocks a row; a block's slices and its share of that product take about 0.65 of
+  // a block product) instead of a set's and an operator's.  With every output that
+  // is from 11 sets on, for the triangle alone from 2.  Measured, 27 sets at Nev =
+  // 128, Lt = 48, 8 sink times: block products 158 -> 78 ms, slices, Gram products
+  // and sums of the traces 48 -> 26 ms; the call 254 -> 155 ms.
+  SinkPlan sp;
+  bool sink = gram && !fp64_traces_needed;
+  if (sink) {
+    std::vector<Vertex> V;
+    for (int d = 0; d < nd && rhopi; d++)
+      for (int iop = 0; iop < 4; iop++) {
+        Vertex v;
+        std::memset(&v, 0, sizeof(v));
+        for (const Grp& g : grp[d])
+          if (g.iop == iop && g.s2 == 0) {
+            v.slab = g.slab;
+            v.s5[g.s3] = g.s5;
+            v.cre[g.s3] = g.cre;
+            v.cim[g.s3] = g.cim;
+          }
+        V.push_back(v);
+      }
+    for (int ik = 0; ik < 2 && tri; ik++)
+      V.push_back(Vertex{slab_of[5 + ik], {0, 1, 2, 3}, {(float)G5[0], (float)G5[1], (float)G5[2], (float)G5[3]}, {}});
+    sink = sink_plan(V, sp) && sp.products + 10.4 * sp.H.size() < 64.0 * nC + 10.4 * (nC + nops);
+  }
+  const int nH = (int)sp.H.size();
+  const size_t per_pair_sink = 16 * ((size_t)nops + nH) * N2 * sizeof(double2) +
+                               (size_t)nH * nC * (sizeof(double2) + sizeof(double));
+  const int batch_sink = std::max(1, std::min(npairs, (int)(sets_budget() / per_pair_sink)));
+  // 9 sink times of 14 rows fill a 128-row tile of the Gram product
+  for (const PairBatch& pb : sink ? pair_batches(tau, blk16, Nt, tf_begin, rows, batch_sink, plist, 18)
+                                  : std::vector<PairBatch>()) {
+    const int np = (int)pb.ent.size(), ng = (int)pb.by_ti.size();
+    void* mem;
+    CTR_TRY(workspace(WS_SCRATCH).get((size_t)np * per_pair_sink, &mem));
+    double2* bO = (double2*)mem;                      // Op(tf) tau_b, block (b, slab) of pair i
+    double2* bH = bO + (size_t)np * 16 * nops * N2;   // terms, by stack
+    double2* trv = bH + (size_t)np * 16 * nH * N2;
+    double* tra = (rf_rp.on || rf_tr.on) ? (double*)(trv + (size_t)np * nH * nC) : nullptr;
+    auto Oblk = [&](int sl, int i, int b) { return bO + ((size_t)i * 16 * nops + (size_t)b * nops + sl) * N2; };
+    std::vector<GridTask> g0, g1;
+    std::vector<const double2*> hblk((size_t)np * nH * 16);  // [pair][term][s1 * 4 + s2]
+    for (int i = 0; i < np; i++) {
+      for (int jb = 0; jb < 2; jb++) {
+        GridTask go = make_grid(nops, 8, 1, kOne, 0, 0);
+        for (int sl = 0; sl < nops; sl++)
+          go.A[sl] = ops[sl] < 5 ? P5 + ((size_t)pb.tf[i] * 5 + ops[sl]) * N2
+                                 : P2x + ((size_t)pb.tf[i] * 2 + ops[sl] - 5) * N2;
+        for (int j = 0; j < 8; j++) {
+          go.B[j][0] = pb.T[i] + (size_t)(8 * jb + j) * N2;
+          go.C0[j] = Oblk(0, i, 8 * jb + j);
+        }
+        g0.push_back(std::move(go));
+      }
+      double2* next = bH + (size_t)i * 16 * nH * N2;
+      for (const std::vector<int>& st : sp.stacks) {
+        // slab (term, s1), right block s2
+        const SinkTerm& t0 = sp.H[st[0]];
+        const int m = (int)st.size();
+        GridTask gh = make_grid(4 * m, 4, t0.n, t0.w, (1 << t0.n) - 1, 0);
+        for (int u = 0; u < m; u++)
+          for (int s1 = 0; s1 < 4; s1++)
+            for (int k = 0; k < t0.n; k++) {
+              const SinkTerm& t = sp.H[st[u]];
+              gh.A[(size_t)(u * 4 + s1) * t0.n + k] = Oblk(t.slab, i, t.s5[k] * 4 + s1);
+            }
+        for (int j = 0; j < 4; j++) {
+          for (int k = 0; k < t0.n; k++) gh.B[j][k] = pb.T[i] + (size_t)(t0.s3[k] * 4 + j) * N2;
+          gh.C0[j] = next + (size_t)j * 4 * m * N2;
+        }
+        for (int u = 0; u < m; u++)
+          for (int b = 0; b < 16; b++)
+            hblk[((size_t)i * nH + st[u]) * 16 + b] = next + ((size_t)(b % 4) * 4 * m + u * 4 + b / 4) * N2;
+        next += (size_t)16 * m * N2;
+        g1.push_back(std::move(gh));
+      }
+    }
+    GramRows gr;
+    size_t maxm = 0;
+    for (auto& v : pb.by_ti) maxm = std::max(maxm, v.size());
+    gr.ngroup = ng;
+    gr.nblk = 16;
+    gr.mrows = (int)maxm * nH;
+    gr.ncols = nC;
+    for (int b = 0; b < 16; b++)
+      if (G5[b / 4] < 0) gr.negative |= 1u << b;
+    gr.left.assign((size_t)ng * 16 * gr.mrows, nullptr);
+    gr.right.resize((size_t)ng * 16 * nC);
+    gr.rowbase.assign((size_t)ng * gr.mrows, -1);
+    for (int g = 0; g < ng; g++) {
+      const std::vector<int>& mem_i = pb.by_ti[g];
+      for (size_t pp = 0; pp < mem_i.size(); pp++)
+        for (int h = 0; h < nH; h++) {
+          gr.rowbase[(size_t)g * gr.mrows + pp * nH + h] = (mem_i[pp] * nH + h) * nC;
+          for (int b = 0; b < 16; b++)
+            gr.left[((size_t)g * 16 + b) * gr.mrows + pp * nH + h] = hblk[((size_t)mem_i[pp] * nH + h) * 16 + b];
+        }
+      for (int b = 0; b < 16; b++)
+        for (int ci = 0; ci < nC; ci++)
+          gr.right[((size_t)g * 16 + b) * nC + ci] = M[(size_t)ci * Nt + pb.ti[mem_i[0]]] + (size_t)b * N2;
+    }
+    std::vector<RowItems> it(nd + 1);  // polarisations, then the triangle
+    size_t v0 = 0;
+    for (int d = 0; d <= nd; d++) {
+      RowItems& r = it[d];
+      if (d < nd ? !rhopi : !tri) continue;
+      r.nout = d < nd ? 4 : 2;
+      r.conj = 1;
+      r.csr.push_back(0);
+      for (int o = 0; o < r.nout; o++, v0++) {
+        for (auto& e : sp.rows[v0]) {
+          r.off.push_back(e.first * nC);
+          r.coef.push_back(e.second);
+        }
+        r.csr.push_back((int)r.off.size());
+      }
+      for (size_t k = 0; k < r.off.size(); k++) r.csr.push_back((int)k);
+      for (int i = 0; i < np; i++)
+        for (int k = 0; k < nset; k++) {
+          r.base.push_back(i * nH * nC + cR[k]);
+          r.ent.push_back((d < nd ? k * nd + d : k) * npairs + pb.ent[i]);
+        }
+    }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(run_grids(c, g1, WS_TASKS2));
+    CTR_TRY(gram_rows(N, gr, trv, tra, c.s));
+    std::vector<RowItems*> items;
+    for (RowItems& r : it) items.push_back(&r);
+    CTR_TRY(upload_items(c, items));
+    for (int d = 0; d < nd; d++) CTR_TRY(rowsum_items(c, trv, tra, it[d], (double2*)rhopi, rf_rp));
+    CTR_TRY(rowsum_items(c, trv, tra, it[nd], (double2*)tri, rf_tr));
+  }
+  for (const PairBatch& pb : sink ? std::vector<PairBatch>()
+                                  : pair_batches(tau, blk16, Nt, tf_begin, rows, batch, plist)) {
     const int np = (int)pb.ent.size(), ng = (int)pb.by_ti.size();
     void* mem;
     CTR_TRY(workspace(WS_SCRATCH).get((size_t)np * per_pair, &mem));
@@ -1045,15 +1282,14 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
     RowItems it_tr;
     std::vector<RowItems> it_rp(nd);
     for (int d = 0; d < nd && rhopi; d++) {
-      it_rp[d].nrows = ngr;
       it_rp[d].nout = 4;
       it_rp[d].csr = csr_rp[d];
-      it_rp[d].slot.reserve((size_t)np * nset * ngr);
+      it_rp[d].off = uidx[d];
       for (const Grp& g : grp[d]) it_rp[d].coef.push_back(make_float2(g.cre, g.cim));
     }
-    it_tr.nrows = 32;
     it_tr.nout = 2;
     it_tr.csr = csr_tr;
+    for (int r = 0; r < 32; r++) it_tr.off.push_back(r);
     for (int i = 0; i < np; i++) {
       const int pair = pb.ent[i];
       for (int k = 0; k < nset; k++) {
@@ -1068,15 +1304,15 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
             if (gram) gp.tr.push_back({i * 4 + xb % 4, ci * 4 + xb / 4, std::get<0>(u) * 4 + zb / 4, slot, 1.f, 0.f});
           }
           for (int d = 0; d < nd; d++) {
-            for (int g = 0; g < ngr; g++) it_rp[d].slot.push_back(base + uidx[d][g]);
+            it_rp[d].base.push_back(base);
             it_rp[d].ent.push_back((k * nd + d) * npairs + pair);
           }
         }
         if (tri) {
+          it_tr.base.push_back(tp.n);
           for (int ik = 0; ik < 2; ik++)
             for (int b = 0; b < 16; b++) {
               const int slot = tp.add(Xblk(ci, i, b / 4, b % 4), Zblk(slab_of[5 + ik], i, b), (float)G5[b / 4], 0.f, 0);
-              it_tr.slot.push_back(slot);
               if (gram) gp.tr.push_back({i * 4 + b % 4, ci * 4 + b / 4, slab_of[5 + ik] * 4 + b / 4, slot, (float)G5[b / 4], 0.f});
             }
           it_tr.ent.push_back(k * npairs + pair);

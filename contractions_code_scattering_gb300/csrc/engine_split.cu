@@ -1084,4 +1084,70 @@ int trace_gram(int N, const GramPlan& P, double2* trv, double* tra, cudaStream_t
   return CTR_OK;
 }
 
+// Gram products whose every entry is wanted (GramRows): the instances of
+// trace_gram, summed over a group's blocks and pieces.
+int gram_rows(int N, const GramRows& P, double2* trv, double* tra, cudaStream_t stream) {
+  if (P.ngroup == 0) return CTR_OK;
+  if (N > SPLIT_MAXK) return fail(CTR_ERR_UNSUPPORTED, "split engine supports Nev <= %d (got %d)", SPLIT_MAXK, N);
+  const size_t nb = (size_t)P.ngroup * P.nblk;
+  if (P.nblk < 1 || P.nblk > 32 || P.mrows < 1 || P.ncols < 1 || P.left.size() != nb * P.mrows ||
+      P.right.size() != nb * P.ncols || P.rowbase.size() != (size_t)P.ngroup * P.mrows)
+    return fail(CTR_ERR_ARG, "Gram rows: %d groups of %d blocks, %d x %d, do not match their tables", P.ngroup, P.nblk,
+                P.mrows, P.ncols);
+  int* d_err;
+  CTR_TRY(err_flag(&d_err));
+  const int n2 = N * N;
+  const int nchunk = std::min(GRAM_PIECE / SPLIT_K, cdiv(n2, SPLIT_K)), npiece = cdiv(n2, nchunk * SPLIT_K);
+  const int mtiles = cdiv(P.mrows, SPLIT_M), ntiles = cdiv(P.ncols, CfgHP::BN);
+  const int lrows = mtiles * SPLIT_M, rcols = ntiles * CfgHP::BN;
+  const size_t l_b = (size_t)mtiles * nchunk * CfgHP::A_STAGE, r_b = (size_t)ntiles * nchunk * CfgHP::B_STAGE;
+  const size_t p_b = (size_t)lrows * rcols * sizeof(double2);
+  const size_t per_inst = l_b + r_b + p_b + (size_t)(lrows + rcols) * (sizeof(int) + sizeof(float));
+  const size_t per_group = (size_t)P.nblk * npiece * per_inst;
+  const int G = (int)std::max<size_t>(1, std::min<size_t>(P.ngroup, ((size_t)4 << 30) / per_group));
+  for (int g0 = 0; g0 < P.ngroup; g0 += G) {
+    const int ng = std::min(G, P.ngroup - g0), nbl = ng * P.nblk, ni = nbl * npiece;
+    void* mem;
+    CTR_TRY(workspace(WS_GRAM).get((size_t)ni * per_inst + 1024, &mem));
+    uint8_t* lsl = (uint8_t*)mem;
+    uint8_t* rsl = lsl + (size_t)ni * l_b;
+    double2* part = (double2*)(rsl + (size_t)ni * r_b);
+    int* lexp = (int*)(part + (size_t)ni * lrows * rcols);
+    int* rexp = lexp + (size_t)ni * lrows;
+    float* lnorm = (float*)(rexp + (size_t)ni * rcols);
+    float* rnorm = lnorm + (size_t)ni * lrows;
+    std::vector<SplitGemmInst> gi(ni);
+    std::vector<double2*> outs(ni);
+    for (int ip = 0; ip < ni; ip++) {
+      outs[ip] = part + (size_t)ip * lrows * rcols;
+      gi[ip] = SplitGemmInst{lsl + (size_t)ip * l_b, rsl + (size_t)ip * r_b, lexp + (size_t)ip * lrows,
+                             rexp + (size_t)ip * rcols, nullptr, nullptr};
+    }
+    const size_t b0 = (size_t)g0 * P.nblk;
+    void* d[4];
+    CTR_TRY(upload_group(WS_GRAMJOBS,
+                         {{P.left.data() + b0 * P.mrows, (size_t)nbl * P.mrows * sizeof(const double2*)},
+                          {P.right.data() + b0 * P.ncols, (size_t)nbl * P.ncols * sizeof(const double2*)},
+                          {outs.data(), outs.size() * sizeof(double2*)},
+                          {P.rowbase.data() + (size_t)g0 * P.mrows, (size_t)ng * P.mrows * sizeof(int)}},
+                         d, stream));
+    for (int ip = 0; ip < ni; ip++) gi[ip].outs = (double2* const*)d[2] + ip;
+    void* d_gi;
+    CTR_TRY(upload(WS_GEMM_B, gi.data(), gi.size() * sizeof(SplitGemmInst), &d_gi, stream));
+    CTR_TRY(launch_slice_gram(false, (const double2* const*)d[0], nbl, P.mrows, mtiles, n2, npiece, nchunk, lsl, lexp,
+                              lnorm, stream));
+    CTR_TRY(launch_slice_gram(true, (const double2* const*)d[1], nbl, P.ncols, ntiles, n2, npiece, nchunk, rsl, rexp,
+                              rnorm, stream));
+    SplitGemmBatch B{(const SplitGemmInst*)d_gi, mtiles, ntiles, nchunk, P.mrows, P.ncols, lrows, nullptr, 1, rcols, 1};
+    B.order = 0;
+    CTR_TRY(launch_split_gemm(B, ni, d_err, stream, true));
+    CTR_TRY(launch_gram_rows_sum(part, ng, P.nblk, P.negative, npiece, lrows, rcols, P.mrows, P.ncols, lexp, rexp,
+                                 lnorm, rnorm, (const int*)d[3], trv, tra, stream));
+  }
+  if (!capturing())
+    for (int b : P.rowbase)
+      if (b >= 0) g_gram_traces += (double)P.nblk * P.ncols;
+  return CTR_OK;
+}
+
 }  // namespace ctr

@@ -1802,6 +1802,60 @@ __global__ void __launch_bounds__(128) gram_trace_sum_kernel(const GramTrace* __
   if (tra) tra[T.slot] = sqrt(c.x * c.x + c.y * c.y) * ab;
 }
 
+// Values of Gram products whose every entry is wanted: group g's blocks b < nblk
+// (instances (g * nblk + b) * npiece + p) add up, with the sign of bit b of
+// `negative`, into trv[rowbase[g * mrows + r] + c] for c < ncols; rows whose base is
+// negative are skipped.  tra: the same error scale as gram_trace_sum's.  One CTA
+// per (group, row): 32 columns at a time, 8 threads a column in a fixed order.
+__global__ void __launch_bounds__(256) gram_rows_sum_kernel(
+    const double2* __restrict__ part, int nblk, unsigned negative, int npiece, int lrows, int rcols, int mrows,
+    int ncols, const int* __restrict__ lexp, const int* __restrict__ rexp, const float* __restrict__ lnorm,
+    const float* __restrict__ rnorm, const int* __restrict__ rowbase, double2* __restrict__ trv,
+    double* __restrict__ tra) {
+  __shared__ double red[8][3][32];
+  const int g = blockIdx.x / mrows, r = blockIdx.x - g * mrows;
+  const int base = rowbase[blockIdx.x];
+  if (base < 0) return;
+  const int lane = threadIdx.x & 31, ps = threadIdx.x >> 5, np = nblk * npiece;
+  for (int c0 = 0; c0 < ncols; c0 += 32) {
+    const int c = c0 + lane;
+    double re = 0.0, im = 0.0, ab = 0.0;
+    if (c < ncols)
+      for (int q = ps; q < np; q += 8) {
+        const size_t ip = (size_t)g * np + q;
+        const double2 v = part[(ip * lrows + r) * rcols + c];
+        if ((negative >> (q / npiece)) & 1u) {
+          re -= v.x;
+          im -= v.y;
+        } else {
+          re += v.x;
+          im += v.y;
+        }
+        if (tra) {
+          const float nx = lnorm[ip * lrows + r], ny = rnorm[ip * rcols + c];
+          if (nx > 0.f && ny > 0.f)
+            ab += ((double)nx * (double)ny + 8.0) * pow2d(lexp[ip * lrows + r] + rexp[ip * rcols + c]);
+        }
+      }
+    red[ps][0][lane] = re;
+    red[ps][1][lane] = im;
+    red[ps][2][lane] = ab;
+    __syncthreads();
+    if (threadIdx.x < 96) {
+      double v = red[0][ps][lane];
+#pragma unroll
+      for (int w = 1; w < 8; w++) v += red[w][ps][lane];
+      if (c < ncols) {
+        if (ps < 2)
+          ((double*)(trv + base + c))[ps] = v;
+        else if (tra)
+          tra[base + c] = v;
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // --------------------------------------------------------------- launchers
 // Dynamic shared-memory limits are raised once per kernel (before any graph
 // capture, through split_kernels_prepare, or at the first launch).
@@ -1954,6 +2008,17 @@ int launch_slice_gram(bool right, const double2* const* d_blk, int ngroup, int n
     slice_gram_kernel<CfgHP, false><<<(unsigned)(grid * (SPLIT_M / 8)), 256, GRAM_SLICE_SMEM, s>>>(
         d_blk, nrows, ntile, n2, npiece, nchunk, out, exps, norms);
   }
+  CTR_CUDA(cudaGetLastError());
+  return CTR_OK;
+}
+
+int launch_gram_rows_sum(const double2* part, int ngroup, int nblk, unsigned negative, int npiece, int lrows, int rcols,
+                         int mrows, int ncols, const int* lexp, const int* rexp, const float* lnorm,
+                         const float* rnorm, const int* d_rowbase, double2* trv, double* tra, cudaStream_t s) {
+  if (ngroup == 0 || mrows == 0) return CTR_OK;
+  TimedLaunch tl(s, "gram_rows_sum");
+  gram_rows_sum_kernel<<<(unsigned)(ngroup * mrows), 256, 0, s>>>(part, nblk, negative, npiece, lrows, rcols, mrows,
+                                                                  ncols, lexp, rexp, lnorm, rnorm, d_rowbase, trv, tra);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
 }

@@ -227,6 +227,13 @@ int launch_slice_gram(bool right, const double2* const* d_blk, int ngroup, int n
 int launch_gram_trace_sum(const GramTrace* d_tr, int ntr, int g0, const double2* part, int npiece, int lrows, int rcols,
                           const int* lexp, const int* rexp, const float* lnorm, const float* rnorm, double2* trv,
                           double* tra, cudaStream_t s);
+// Every entry of the Gram products of ngroup groups of nblk blocks each:
+// trv[rowbase[g * mrows + r] + c] = sum over b, p of +-partial (r, c) of instance
+// (g * nblk + b) * npiece + p (- where bit b of negative is set; rows with a
+// negative base are skipped), tra likewise the error scales.
+int launch_gram_rows_sum(const double2* part, int ngroup, int nblk, unsigned negative, int npiece, int lrows, int rcols,
+                         int mrows, int ncols, const int* lexp, const int* rexp, const float* lnorm,
+                         const float* rnorm, const int* d_rowbase, double2* trv, double* tra, cudaStream_t s);
 // A bounded wait that runs out (timeout_ns) on an mbarrier nothing arrives at,
 // recording error code 9 in *d_err (the failure-detection check).
 int launch_wait_probe(unsigned long long timeout_ns, int* d_err, cudaStream_t s);

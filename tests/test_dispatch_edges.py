@@ -58,3 +58,33 @@ def test_elementals_pieces_and_reversed_momenta(cuda, nev):
     assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
     plain = api.elementals(_dev(V, cuda), moms).cpu().numpy()
     assert np.abs(plain[:, 0] - ref[:, 0]).max() <= 1e-12 * np.abs(ref[:, 0]).max()
+
+
+@pytest.mark.parametrize("n,rhopi,tri,nset", [(9, True, True, 11), (37, True, False, 12), (20, False, True, 2),
+                                              (8, True, True, 20)])
+def test_momentum_sets_sink_form(cuda, n, rhopi, tri, nset):
+    """rho -> pi pi and triangle over enough sets that the sink operators' products
+    replace the sets' (one Gram product per t_src), at ragged Nev, for the outputs
+    alone and together, repeated sets among them, over a t_sink range."""
+    from tests.test_parity_chains import SPLIT_TOL, ref_rhopi, ref_triangle
+    nt, tr = 4, (1, 4)
+    prop = synth.make_prop(nt, n, seed=800 + n, decay=0.25)
+    moms = [(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0)]
+    phis = synth.make_phi_momenta(nt, n, moms, seed=801 + n)
+    rng = np.random.default_rng(802 + n)
+    mom5 = np.ascontiguousarray(np.stack([synth.make_phi_random(nt, n, rng) for _ in range(5)], axis=1))
+    mom2 = np.ascontiguousarray(np.stack([synth.make_phi_random(nt, n, rng) for _ in range(2)], axis=1))
+    sets = [(k % 5, (k // 5 + k) % 5) for k in range(nset)] + [(0, 0)]
+    tp = _dev(prop, cuda)
+    got = api.run_contract_rhopi_sigmapi_sets(tp[tr[0]:tr[1]].contiguous(), api.prop_diag(tp),
+                                              _dev(np.stack([phis[p] for p in moms], axis=1), cuda), sets,
+                                              _dev(mom5, cuda), _dev(mom2, cuda), engine="split", tf_range=tr,
+                                              rhopi=rhopi, triangle=tri)
+    for k, (a, b) in enumerate(sets):
+        pa, pb = phis[moms[a]], phis[moms[b]]
+        for idir in range(3 if rhopi else 0):
+            ref, ab = ref_rhopi(prop, pa, pb, mom5, idir, range(*tr))
+            P.entrywise(got["rhopi"][k, idir].cpu().numpy(), ref, SPLIT_TOL, ab, "set %d idir %d" % (k, idir))
+        if tri:
+            ref, ab = ref_triangle(prop, pa, pb, mom2, range(*tr))
+            P.entrywise(got["triangle"][k].cpu().numpy(), ref, SPLIT_TOL, ab, "set %d triangle" % k)
