@@ -25,18 +25,21 @@
 // launch.  The profile must have f_k != 0 (the diagonal identity above
 // yields f_k d/df_k).
 //
-// The diagram builders (rho: lib/calculate_rho_core.h; pi pi:
-// lib/calculate_pipi_{square,doubleTriangle,doubleTriangleHor,starfish}_core.h)
-// emit one chain per spin row in the reference's chain order, so the chain
-// values reproduce the reference's rows.
+// The generic chains (ctr_chain_adjoint) run that way.  The diagrams' own gradients
+// (rho: lib/calculate_rho_core.h; pi pi: lib/calculate_pipi_{square,
+// doubleTriangle,doubleTriangleHor,starfish}_core.h) use their spin structure
+// instead of one chain per spin row: a rho trace is Tr[A B] twice, cut at its
+// two pairs of elementals, and the pi pi diagrams are traces of 4x4 spin-block
+// matrices whose co-factors are a few four-term block products a pair (below).
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <utility>
 #include <vector>
 
-#include "kernels.h"
+#include "chains.h"
 
 namespace ctr {
 
@@ -56,18 +59,85 @@ __global__ void apply_profile_kernel(const double2* __restrict__ src, double2* _
   }
 }
 
-// One diagonal reduction d_k = sum_m op(X)[k][m] op(Y)[m][k].
-// mode 0: buf[out * N + k] = Re(w d_k);  mode 1: vals[out] = sum_k d_k.
+// One diagonal reduction d_k = sum_m op(X)[k][m] op(Y)[m][k]: buf[out * N + k] = Re(w d_k)
+// where out >= 0 (w times *wp where wp is set), vals[vout] = sum_k d_k where vout >= 0.
 struct DiagTask {
   const double2* x;
   const double2* y;
+  const double2* wp;
   double wre, wim;
   int xdag, ydag;
-  int mode, out;
+  int out, vout;
 };
 
-// One CTA per task; 32x32 tiles of op(X) (rows k) and op(Y) (columns k) are
-// staged through shared memory with coalesced reads whatever the transposes,
+__device__ __forceinline__ double2 diag_weight(const DiagTask& T) {
+  const double2 w = make_double2(T.wre, T.wim);
+  return T.wp ? cmul(w, *T.wp) : w;
+}
+
+// Nev <= 128.  The FP64 pipe is the bound (4 FMAs an element), so every lane of
+// the working warps has an element: thread t takes k = t mod N and one of P
+// (the largest divisor of DK with P N <= threads) shares of each chunk of DK m's,
+// where 32-wide tiles padded N to a multiple of 32 (Nev = 100: 128).  X and Y go
+// through shared memory in chunks of DK, read along their rows whatever the
+// transposes.  Per task and SM at Nev = 100: see launch_diag.
+constexpr int DIAG_TPB = 320, DK = 12;
+
+__global__ void __launch_bounds__(DIAG_TPB) diag_small_kernel(const DiagTask* __restrict__ tasks, int N, int P,
+                                                              double* __restrict__ buf, double2* __restrict__ vals) {
+  extern __shared__ __align__(16) double2 dsm[];
+  double2* xs = dsm;                 // [N][DK + 1]: op(X)[k][m0 + mm]
+  double2* ys = xs + N * (DK + 1);   // [DK][N + 1]: op(Y)[m0 + mm][k]
+  const DiagTask T = tasks[blockIdx.x];
+  const int k = threadIdx.x % N, part = threadIdx.x / N, share = DK / P;
+  const bool on = part < P;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int m0 = 0; m0 < N; m0 += DK) {
+    const int mn = min(DK, N - m0);
+    for (int e = threadIdx.x; e < N * mn; e += DIAG_TPB) {
+      {
+        const int kk = T.xdag ? e % N : e / mn, mm = T.xdag ? e / N : e % mn;
+        double2 v = T.xdag ? T.x[(size_t)(m0 + mm) * N + kk] : T.x[(size_t)kk * N + m0 + mm];
+        if (T.xdag) v.y = -v.y;
+        xs[kk * (DK + 1) + mm] = v;
+      }
+      {
+        const int kk = T.ydag ? e / mn : e % N, mm = T.ydag ? e % mn : e / N;
+        double2 v = T.ydag ? T.y[(size_t)kk * N + m0 + mm] : T.y[(size_t)(m0 + mm) * N + kk];
+        if (T.ydag) v.y = -v.y;
+        ys[mm * (N + 1) + kk] = v;
+      }
+    }
+    __syncthreads();
+    if (on) {
+      const int hi = min(mn, (part + 1) * share);
+      for (int mm = part * share; mm < hi; mm++) cmac(acc, xs[k * (DK + 1) + mm], ys[mm * (N + 1) + k]);
+    }
+    __syncthreads();
+  }
+  double2* part_sum = dsm;  // [P][N]
+  if (on) part_sum[part * N + k] = acc;
+  __syncthreads();
+  double2 d = make_double2(0.0, 0.0);
+  if (threadIdx.x < N) {
+    d = part_sum[k];
+    for (int q = 1; q < P; q++) {
+      d.x += part_sum[q * N + k].x;
+      d.y += part_sum[q * N + k].y;
+    }
+    if (T.out >= 0) {
+      const double2 w = diag_weight(T);
+      buf[(size_t)T.out * N + k] = w.x * d.x - w.y * d.y;
+    }
+  }
+  if (T.vout >= 0) {
+    const double v = block_sum2<DIAG_TPB>(d.x, d.y);
+    if (threadIdx.x < 2) ((double*)(vals + T.vout))[threadIdx.x] = v;
+  }
+}
+
+// Any Nev.  One CTA per task; 32x32 tiles of op(X) (rows k) and op(Y) (columns k)
+// are staged through shared memory with coalesced reads whatever the transposes,
 // so both operands are read once.
 __global__ void __launch_bounds__(256) diag_reduce_kernel(const DiagTask* __restrict__ tasks, int N,
                                                           double* __restrict__ buf, double2* __restrict__ vals) {
@@ -116,14 +186,14 @@ __global__ void __launch_bounds__(256) diag_reduce_kernel(const DiagTask* __rest
         d.y += part[q][tx].y;
       }
       const int k = k0 + tx;
-      if (T.mode == 0) {
-        if (k < N) buf[(size_t)T.out * N + k] = T.wre * d.x - T.wim * d.y;
-      } else {
-        tot[tx] = k < N ? d : make_double2(0.0, 0.0);
+      if (T.out >= 0 && k < N) {
+        const double2 w = diag_weight(T);
+        buf[(size_t)T.out * N + k] = w.x * d.x - w.y * d.y;
       }
+      tot[tx] = k < N ? d : make_double2(0.0, 0.0);
     }
     __syncthreads();
-    if (T.mode == 1 && threadIdx.x == 0) {
+    if (T.vout >= 0 && threadIdx.x == 0) {
       for (int q = 0; q < 32; q++) {
         vsum.x += tot[q].x;
         vsum.y += tot[q].y;
@@ -131,7 +201,7 @@ __global__ void __launch_bounds__(256) diag_reduce_kernel(const DiagTask* __rest
     }
     __syncthreads();
   }
-  if (T.mode == 1 && threadIdx.x == 0) vals[T.out] = vsum;
+  if (T.vout >= 0 && threadIdx.x == 0) vals[T.vout] = vsum;
 }
 
 // grad[k] += (sum_t buf[t][k]) / f[k], summed in a fixed order.
@@ -142,6 +212,37 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const double* __restri
   for (int t = threadIdx.x; t < ntask; t += 256) s += buf[(size_t)t * N + k];
   s = block_sum_256(s);
   if (threadIdx.x == 0) grad[k] += s / f[k];
+}
+
+// Diagonal reductions of a task list, then grad += (sum of their rows) / f where the
+// list has gradient rows (nrow > 0).
+int launch_diag(const std::vector<DiagTask>& tasks, int nrow, int N, const double* f, double2* vals, double* grad,
+                cudaStream_t s) {
+  if (tasks.empty()) return CTR_OK;
+  void *ddt, *dbuf = nullptr;
+  CTR_TRY(upload(WS_ROWTASKS, tasks.data(), tasks.size() * sizeof(DiagTask), &ddt, s));
+  if (nrow > 0) CTR_TRY(workspace(WS_ROWS).get((size_t)nrow * N * sizeof(double), &dbuf));
+  {
+    TimedLaunch tl(s, "diag_reduce");
+    if (N <= 128) {
+      int P = 1;
+      for (int q : {2, 3, 4, 6, 12})
+        if (q * N <= DIAG_TPB) P = q;
+      const size_t smem = ((size_t)N * (DK + 1) + (size_t)DK * (N + 1)) * sizeof(double2);
+      static_assert((128 * (DK + 1) + DK * 129) * sizeof(double2) <= 56 * 1024, "shared memory of diag_small_kernel");
+      CTR_CUDA(cudaFuncSetAttribute(diag_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 56 * 1024));
+      diag_small_kernel<<<(unsigned)tasks.size(), DIAG_TPB, smem, s>>>((const DiagTask*)ddt, N, P, (double*)dbuf, vals);
+    } else {
+      diag_reduce_kernel<<<(unsigned)tasks.size(), 256, 0, s>>>((const DiagTask*)ddt, N, (double*)dbuf, vals);
+    }
+    CTR_CUDA(cudaGetLastError());
+  }
+  if (nrow > 0) {
+    TimedLaunch tl(s, "grad_reduce");
+    grad_reduce_kernel<<<N, 256, 0, s>>>((const double*)dbuf, nrow, N, f, grad);
+    CTR_CUDA(cudaGetLastError());
+  }
+  return CTR_OK;
 }
 
 // ------------------------------------------------------------- chain program
@@ -319,45 +420,32 @@ int ChainProgram::run(const double* f, double2* values, double* grad, cudaStream
     auto P = [&](int j) { return opnd(c.pre[j - 1], leaf(c.f[0])); };  // P_j, j = 1..n-1
     auto S = [&](int j) { return opnd(c.suf[j - 1], leaf(c.f[n - 1])); };  // S_j, j = 2..n
     auto F = [&](int j) { return leaf(c.f[j - 1]); };
-    auto push = [&](Opnd x, Opnd y, int mode, int out) {
+    auto push = [&](Opnd x, Opnd y, int out, int vout) {
       DiagTask t;
+      std::memset(&t, 0, sizeof(t));
       t.x = x.p;
       t.y = y.p;
       t.xdag = x.dag;
       t.ydag = y.dag;
       t.wre = c.w.x;
       t.wim = c.w.y;
-      t.mode = mode;
       t.out = out;
+      t.vout = vout;
       dtasks.push_back(t);
     };
-    if (c.value_slot >= 0) push(P(n - 1), F(n), 1, c.value_slot);  // Tr = sum diag(P_{n-1} F_n)
+    if (c.value_slot >= 0) push(P(n - 1), F(n), -1, c.value_slot);  // Tr = sum diag(P_{n-1} F_n)
     if (!c.grad) continue;
     for (int j = 1; j <= n; j++) {
       if (c.f[j - 1].kind != CTR_FACTOR_PHI) continue;
       // left D of F_j: diag(S_j P_{j-1}); j = 1: diag(F_1 S_2)
-      if (j == 1) push(F(1), S(2), 0, ngrad++);
-      else push(S(j), P(j - 1), 0, ngrad++);
+      if (j == 1) push(F(1), S(2), ngrad++, -1);
+      else push(S(j), P(j - 1), ngrad++, -1);
       // right D of F_j: diag(S_{j+1} P_j); j = n: diag(P_{n-1} F_n)
-      if (j == n) push(P(n - 1), F(n), 0, ngrad++);
-      else push(S(j + 1), P(j), 0, ngrad++);
+      if (j == n) push(P(n - 1), F(n), ngrad++, -1);
+      else push(S(j + 1), P(j), ngrad++, -1);
     }
   }
-  if (dtasks.empty()) return CTR_OK;
-  void *ddt, *dbuf = nullptr;
-  CTR_TRY(upload(WS_ROWTASKS, dtasks.data(), dtasks.size() * sizeof(DiagTask), &ddt, s));
-  if (ngrad > 0) CTR_TRY(workspace(WS_ROWS).get((size_t)ngrad * N_ * sizeof(double), &dbuf));
-  {
-    TimedLaunch tl(s, "diag_reduce");
-    diag_reduce_kernel<<<(unsigned)dtasks.size(), 256, 0, s>>>((const DiagTask*)ddt, N_, (double*)dbuf, values);
-    CTR_CUDA(cudaGetLastError());
-  }
-  if (ngrad > 0) {
-    TimedLaunch tl(s, "grad_reduce");
-    grad_reduce_kernel<<<N_, 256, 0, s>>>((const double*)dbuf, ngrad, N_, f, grad);
-    CTR_CUDA(cudaGetLastError());
-  }
-  return CTR_OK;
+  return launch_diag(dtasks, ngrad, N_, f, values, grad, s);
 }
 
 // Runs chains through programs of bounded size (node storage <= budget).
@@ -414,32 +502,667 @@ int check_f(int N, const double* f, cudaStream_t s) {
   return CTR_OK;
 }
 
-inline ctr_factor tau(int t1, int t2, int s1, int s2, int dag = 0) {
-  ctr_factor F;
-  F.kind = CTR_FACTOR_TAU;
-  F.dag = dag;
-  F.a = t1;
-  F.b = t2;
-  F.s1 = s1;
-  F.s2 = s2;
-  return F;
-}
-
-inline ctr_factor phi(int t, int op, int dag = 0) {
-  ctr_factor F;
-  F.kind = CTR_FACTOR_PHI;
-  F.dag = dag;
-  F.a = t;
-  F.b = op;
-  F.s1 = 0;
-  F.s2 = 0;
-  return F;
-}
-
 inline double2 cw(double2 w, double re, double im) { return make_double2(w.x * re - w.y * im, w.x * im + w.y * re); }
 
 int check_engine(int engine, int nev) {
   if (engine != CTR_ENGINE_FP64 && engine != CTR_ENGINE_SPLIT) return fail(CTR_ERR_ARG, "unknown engine %d", engine);
+  return CTR_OK;
+}
+
+// ------------------------------------------------------- rho and pi pi gradients
+// Products of a batch in one workspace buffer.
+struct Arena {
+  double2* base = nullptr;
+  size_t N2 = 0, used = 0, cap = 0;
+  double2* take(size_t nblk) {
+    double2* p = base + used;
+    used += nblk * N2;
+    return p;
+  }
+};
+
+// A list of diagonal reductions; add(x, y, w): both diag(x y) and diag(y x).
+struct DiagList {
+  std::vector<DiagTask> t;
+  int nrow = 0;
+  void one(const double2* x, const double2* y, double2 w, const double2* wp, bool row, int vout) {
+    DiagTask d;
+    std::memset(&d, 0, sizeof(d));
+    d.x = x;
+    d.y = y;
+    d.wp = wp;
+    d.wre = w.x;
+    d.wim = w.y;
+    d.out = row ? nrow++ : -1;
+    d.vout = vout;
+    t.push_back(d);
+  }
+  void both(const double2* x, const double2* y, double2 w, const double2* wp = nullptr) {
+    one(x, y, w, wp, true, -1);
+    one(y, x, w, wp, true, -1);
+  }
+  void value(const double2* x, const double2* y, int vout) {
+    one(x, y, make_double2(0.0, 0.0), nullptr, false, vout);
+  }
+};
+
+// out[e] = sum_k coef[k] vals[slot[k]] over k in [off[i], off[i + 1]), e = ent[i].
+__global__ void entry_sum_kernel(const double2* __restrict__ vals, const int* __restrict__ off,
+                                 const int* __restrict__ slot, const float2* __restrict__ coef,
+                                 const int* __restrict__ ent, int n, double2* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double re = 0.0, im = 0.0;
+  for (int k = off[i]; k < off[i + 1]; k++) {
+    const double2 v = cmul(make_double2((double)coef[k].x, (double)coef[k].y), vals[slot[k]]);
+    re += v.x;
+    im += v.y;
+  }
+  out[ent[i]] = make_double2(re, im);
+}
+
+// Pairs (tf * Nt + ti) with a nonzero weight, those of one source time together.
+std::vector<int> weighted_pairs(int Nt, int nout, const double2* w) {
+  std::vector<int> p;
+  for (int ti = 0; ti < Nt; ti++)
+    for (int tf = 0; tf < Nt; tf++) {
+      const double2* wp = w + ((size_t)tf * Nt + ti) * nout;
+      for (int k = 0; k < nout; k++)
+        if (wp[k].x != 0.0 || wp[k].y != 0.0) {
+          p.push_back(tf * Nt + ti);
+          break;
+        }
+    }
+  return p;
+}
+
+// rho (lib/calculate_rho_core.h): a spin row is coef * t, t = Tr[A_cd Bt_ab] with
+// A = tau_cd Phi_L(ti) and Bt = tau_ab^dag Phi_R(tf)^dag, so f_k d/df_k of t is
+// diag(Bt A) at Phi_L's right index and diag(A Bt) at Phi_R's left one.  Cut at the
+// other two indices, conj(t) = Tr[At_ab Bs_cd] with At = tau_ab Phi_L(ti)^dag and Bs =
+// tau_cd^dag Phi_R(tf): diag(Bs At) is Phi_L's left index, diag(At Bs) Phi_R's right one.
+// Per pair and operator that is 64 block products, whatever the number of rows.
+int rho_vjp(const Ctx& c, const double2* prop, const double2* phis, const double* f, const double2* w, double2* corr,
+            double* grad) {
+  const int N = c.N, Nt = c.Nt;
+  const size_t N2 = c.N2, blk16 = 16 * N2;
+  if (corr) CTR_CUDA(cudaMemsetAsync(corr, 0, (size_t)Nt * Nt * 48 * sizeof(double2), c.s));
+  const std::vector<int> pairs = weighted_pairs(Nt, 48, w);
+  if (pairs.empty()) return CTR_OK;
+  const Tables& T = tables();
+  // operators used at the source (L) and at the sink (R)
+  std::vector<int> Ls, Rs, il(5, -1), ir(5, -1);
+  for (int p : pairs)
+    for (int o = 0; o < 48; o++) {
+      const double2 wo = w[(size_t)p * 48 + o];
+      if (wo.x == 0.0 && wo.y == 0.0) continue;
+      for (int is = 0; is < 16; is++) {
+        const int l = T.rho_lprp[o * 16 + is][0], r = T.rho_lprp[o * 16 + is][1];
+        if (il[l] < 0) il[l] = (int)Ls.size(), Ls.push_back(l);
+        if (ir[r] < 0) ir[r] = (int)Rs.size(), Rs.push_back(r);
+      }
+    }
+  const int nL = (int)Ls.size(), nR = (int)Rs.size(), kinds = grad ? 2 : 1;
+  const size_t per_pair = 16 * (size_t)kinds * (nL + nR) * N2 * sizeof(double2);
+  const int batch = std::max(1, std::min((int)pairs.size(), (int)(sets_budget() / per_pair)));
+  for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
+    const int np = (int)pb.ent.size();
+    void* mem;
+    CTR_TRY(workspace(WS_SCRATCH).get((size_t)np * per_pair, &mem));
+    Arena ar;
+    ar.base = (double2*)mem;
+    ar.N2 = N2;
+    // side 0: tau against [Phi_L, Phi_L^dag] per t_src; side 1: tau^dag against [Phi_R^dag, Phi_R] per t_sink
+    std::vector<GridTask> g0;
+    std::vector<double2*> bs[2];
+    for (int side = 0; side < 2; side++) {
+      const auto& groups = side ? pb.by_tf : pb.by_ti;
+      const std::vector<int>& ops = side ? Rs : Ls;
+      const int nr = kinds * (int)ops.size();
+      for (const std::vector<int>& mem_i : groups) {
+        const int m = (int)mem_i.size(), t = side ? pb.tf[mem_i[0]] : pb.ti[mem_i[0]];
+        double2* out = ar.take((size_t)16 * m * nr);
+        bs[side].push_back(out);
+        for (int r0 = 0; r0 < nr; r0 += 8) {
+          GridTask G = make_grid(16 * m, std::min(8, nr - r0), 1, kOne, side, 0);
+          for (int pp = 0; pp < m; pp++)
+            for (int b = 0; b < 16; b++) G.A[pp * 16 + b] = pb.T[mem_i[pp]] + (size_t)b * N2;
+          for (int j = 0; j < G.nb; j++) {
+            const int op = (r0 + j) / kinds, dag = ((r0 + j) % kinds) ^ side;
+            G.B[j][0] = phis + ((size_t)t * 5 + ops[op]) * N2;
+            G.bdag |= dag << (4 * j);
+            G.C0[j] = out + (size_t)(r0 + j) * 16 * m * N2;
+          }
+          g0.push_back(std::move(G));
+        }
+      }
+    }
+    auto blk = [&](int side, int i, int op, int kind, int b) {
+      const int g = side ? pb.gtf[i] : pb.gti[i], pos = side ? pb.ptf[i] : pb.pti[i];
+      const size_t m = side ? pb.by_tf[g].size() : pb.by_ti[g].size();
+      return bs[side][g] + (((size_t)(op * kinds + kind) * m + pos) * 16 + b) * N2;
+    };
+    DiagList dl;
+    std::vector<int> off(1, 0), slot, ent;
+    std::vector<float2> coef;
+    int nval = 0;
+    for (int i = 0; i < np; i++) {
+      const int pr = pairs[pb.ent[i]];
+      std::map<std::array<int, 4>, std::pair<int, double2>> tr;  // (cd, L, ab, R) -> value slot, weight
+      for (int o = 0; o < 48; o++) {
+        const double2 wo = w[(size_t)pr * 48 + o];
+        if (wo.x == 0.0 && wo.y == 0.0) continue;
+        for (int is = 0; is < 16; is++) {
+          const int r = o * 16 + is;
+          const int16_t* sp = T.rho_spin[r];
+          const std::array<int, 4> key = {sp[2] * 4 + sp[3], T.rho_lprp[r][0], sp[0] * 4 + sp[1], T.rho_lprp[r][1]};
+          auto it = tr.emplace(key, std::make_pair(nval, make_double2(0.0, 0.0))).first;
+          if (it->second.first == nval) nval++;
+          const double2 x = cw(wo, T.rho_coef[r][0], T.rho_coef[r][1]);
+          it->second.second.x += x.x;
+          it->second.second.y += x.y;
+          slot.push_back(it->second.first);
+          coef.push_back(make_float2(T.rho_coef[r][0], T.rho_coef[r][1]));
+        }
+        off.push_back((int)slot.size());
+        ent.push_back(pr * 48 + o);
+      }
+      for (const auto& e : tr) {
+        const double2* A = blk(0, i, il[e.first[1]], 0, e.first[0]);
+        const double2* Bt = blk(1, i, ir[e.first[3]], 0, e.first[2]);
+        const double2 wt = e.second.second;
+        dl.one(A, Bt, wt, nullptr, grad != nullptr, corr ? e.second.first : -1);
+        if (!grad) continue;
+        dl.one(Bt, A, wt, nullptr, true, -1);
+        dl.both(blk(0, i, il[e.first[1]], 1, e.first[2]), blk(1, i, ir[e.first[3]], 1, e.first[0]),
+                make_double2(wt.x, -wt.y));
+      }
+    }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    void* dv = nullptr;
+    if (corr) CTR_TRY(workspace(WS_ROWABS).get((size_t)std::max(1, nval) * sizeof(double2), &dv));
+    CTR_TRY(launch_diag(dl.t, dl.nrow, N, f, (double2*)dv, grad, c.s));
+    if (corr) {
+      void* d[4];
+      CTR_TRY(upload_group(WS_MISC, {{off.data(), off.size() * sizeof(int)}, {slot.data(), slot.size() * sizeof(int)},
+                                     {coef.data(), coef.size() * sizeof(float2)}, {ent.data(), ent.size() * sizeof(int)}},
+                           d, c.s));
+      TimedLaunch tl(c.s, "entry_sum");
+      const int n = (int)ent.size();
+      entry_sum_kernel<<<(n + 127) / 128, 128, 0, c.s>>>((const double2*)dv, (const int*)d[0], (const int*)d[1],
+                                                         (const float2*)d[2], (const int*)d[3], n, corr);
+      CTR_CUDA(cudaGetLastError());
+    }
+  }
+  return CTR_OK;
+}
+
+// out = sum_k w_k in_k (added to out where add is set), one CTA column per block.
+struct CombTask {
+  double2* out;
+  int first, n, add, pad;
+};
+struct CombIn {
+  const double2* in;
+  double2 w;
+};
+__global__ void __launch_bounds__(256) combine_blocks_kernel(const CombTask* __restrict__ tasks,
+                                                             const CombIn* __restrict__ in, int n2) {
+  const CombTask T = tasks[blockIdx.x];
+  for (int e = threadIdx.x; e < n2; e += 256) {
+    double2 v = T.add ? T.out[e] : make_double2(0.0, 0.0);
+    for (int k = 0; k < T.n; k++) cmac(v, in[T.first + k].w, in[T.first + k].in[e]);
+    T.out[e] = v;
+  }
+}
+
+struct CombList {
+  std::vector<CombTask> t;
+  std::vector<CombIn> in;
+  void begin(double2* out, bool add) { t.push_back(CombTask{out, (int)in.size(), 0, add ? 1 : 0, 0}); }
+  void term(const double2* x, double2 w) {
+    in.push_back(CombIn{x, w});
+    t.back().n++;
+  }
+  int run(int n2, cudaStream_t s) {
+    if (t.empty()) return CTR_OK;
+    void* d[2];
+    CTR_TRY(upload_group(WS_TASKS2, {{t.data(), t.size() * sizeof(CombTask)}, {in.data(), in.size() * sizeof(CombIn)}},
+                         d, s));
+    TimedLaunch tl(s, "combine_blocks");
+    combine_blocks_kernel<<<(unsigned)t.size(), 256, 0, s>>>((const CombTask*)d[0], (const CombIn*)d[1], n2);
+    CTR_CUDA(cudaGetLastError());
+    return CTR_OK;
+  }
+};
+
+// Per pair: vals [64] = 16 each of square, double triangle, horizontal double triangle
+// and 4 x 4 of the twin traces (P4, P1), (P3, P2), (P3, P1), (P4, P2); corr [5] the
+// weighted slots; twin weights wk [4]: star = t0 t1, fish = t2 t3, so d(star) = t1 dt0 + t0 dt1.
+__global__ void pipi_vjp_combine_kernel(const double2* __restrict__ vals, const int* __restrict__ ent,
+                                        const double2* __restrict__ wsf, int npair, double wsq, double wdt, double wst,
+                                        double wfi, double wdh, double2* __restrict__ corr, double2* __restrict__ wk) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= npair) return;
+  const double2* v = vals + (size_t)p * 64;
+  double2 a[3], t[4];
+  for (int g = 0; g < 3; g++) {
+    a[g] = make_double2(0.0, 0.0);
+    for (int b = 0; b < 16; b++) {
+      // the 4x4 block matrices carry gamma_5 on the first index of square and double triangle
+      const double sg = g < 2 && b >= 8 ? -1.0 : 1.0;
+      a[g].x += sg * v[g * 16 + b].x;
+      a[g].y += sg * v[g * 16 + b].y;
+    }
+  }
+  for (int k = 0; k < 4; k++) {
+    t[k] = make_double2(0.0, 0.0);
+    for (int b = 0; b < 4; b++) {
+      t[k].x += v[48 + k * 4 + b].x;
+      t[k].y += v[48 + k * 4 + b].y;
+    }
+  }
+  if (corr) {
+    const double2 st = cmul(t[0], t[1]), fi = cmul(t[2], t[3]);
+    double2* o = corr + (size_t)ent[p] * 5;
+    o[0] = make_double2(wsq * a[0].x, wsq * a[0].y);
+    o[1] = make_double2(wdt * a[1].x, wdt * a[1].y);
+    o[2] = make_double2(wst * st.x, wst * st.y);
+    o[3] = make_double2(wfi * fi.x, wfi * fi.y);
+    o[4] = make_double2(wdh * a[2].x, wdh * a[2].y);
+  }
+  const double2 ws = wsf[2 * p], wf = wsf[2 * p + 1];
+  wk[4 * p] = cmul(ws, t[1]);
+  wk[4 * p + 1] = cmul(ws, t[0]);
+  wk[4 * p + 2] = cmul(wf, t[3]);
+  wk[4 * p + 3] = cmul(wf, t[2]);
+}
+
+// pi pi.  Per pair, T = tau(tf, ti) as a 4x4 block matrix, W = T^dag L:
+//   square = Tr[Rsq J], double triangle = Tr[Rdt J],  J = W G T G,
+//   w_sq square + w_dt double triangle = Tr[L K],     K = G T G (w_sq Rsq + w_dt Rdt) T^dag,
+// so J (weighted, summed per t_src) is the co-factor of R = Phi tau(ti,ti) Phi and K
+// (summed per t_sink) that of L: what remains is a product of two elementals and two
+// block matrices per time slice.  The horizontal double triangle is Tr[P3 Pm1 P4 Pm2],
+// Pm_q = T P_q T^dag, cut at P3 and P4 as (P3 Pm1)(P4 Pm2) and (Pm1 P4)(Pm2 P3), and
+// Tr[P1 N1], N1 = sum T^dag (P4 Pm2 P3) T at P1.  The star / fish twins are
+// Tr[P_x sum_c Pm_cc(y)] = Tr[P_y sum tau^dag P_x tau].  About 700 block products a pair
+// where one chain per spin row took 6 000 and 14 000 diagonals.
+int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>& el, const int32_t* q, const double* f,
+             const double2* w, double2* corr, double* grad) {
+  const int N = c.N, Nt = c.Nt;
+  const size_t N2 = c.N2, blk16 = 16 * N2;
+  if (corr) CTR_CUDA(cudaMemsetAsync(corr, 0, (size_t)Nt * Nt * 5 * sizeof(double2), c.s));
+  const std::vector<int> pairs = weighted_pairs(Nt, 5, w);
+  if (pairs.empty()) return CTR_OK;
+  // isospin weights of the correlator slots (lib/contract_kernels_pipi.cu:288-303, :463-478)
+  const double wsq = iso == 1 ? -2.0 : -1.0 / 3.0, wdt = iso == 1 ? 2.0 : -1.0 / 3.0;
+  const double wst = iso == 1 ? -1.0 : 1.0, wfi = 1.0, wdh = iso == 1 ? 0.0 : -5.0 / 3.0;
+  const bool g = grad != nullptr, hor = iso == 0;
+  auto P = [&](int k, int t) { return el[q[k]].p + (size_t)t * el[q[k]].stride; };  // k = 0..3: P1..P4
+  enum { P1 = 0, P2 = 1, P3 = 2, P4 = 3 };
+  // tau(t, t) [t][16]
+  void* dmem;
+  CTR_TRY(workspace(WS_ADJ_DIAG).get((size_t)Nt * blk16 * sizeof(double2), &dmem));
+  double2* diag = (double2*)dmem;
+  for (int t = 0; t < Nt; t++)
+    CTR_CUDA(cudaMemcpyAsync(diag + (size_t)t * blk16, prop + ((size_t)t * Nt + t) * blk16, blk16 * sizeof(double2),
+                             cudaMemcpyDeviceToDevice, c.s));
+  Combos cb(Nt);
+  const int cL = cb.use(q[P3], q[P4]), cSq = cb.use(q[P2], q[P1]), cDt = cb.use(q[P1], q[P2]);
+  std::vector<char> on_tf(Nt, 0), on_ti(Nt, 0);
+  for (int p : pairs) {
+    on_tf[p / Nt] = on_ti[p % Nt] = 1;
+    cb.need[cL][p / Nt] = cb.need[cSq][p % Nt] = cb.need[cDt][p % Nt] = 1;
+  }
+  std::vector<const double2*> M;
+  CTR_TRY(per_t_products(c, diag, el, WS_RPHI, cb.list, cb.need, M));
+  // co-factors per time slice: K [tf][16], Jsq, Jdt [ti][16] (block (row, column) of the co-factor)
+  double2 *Ks = nullptr, *Js = nullptr, *Jd = nullptr;
+  if (g) {
+    void* am;
+    CTR_TRY(workspace(WS_ADJ_SUM).get(3 * (size_t)Nt * blk16 * sizeof(double2), &am));
+    CTR_CUDA(cudaMemsetAsync(am, 0, 3 * (size_t)Nt * blk16 * sizeof(double2), c.s));
+    Ks = (double2*)am;
+    Js = Ks + (size_t)Nt * blk16;
+    Jd = Js + (size_t)Nt * blk16;
+  }
+  const size_t blocks = 32 + 32 + (hor ? 32 : 8)          // W, J; V; Pm
+                        + (hor ? 32 : 0)                  // X1, X2
+                        + (g ? 48 + 32 + 8 : 0)           // Rw, S, K; U; O
+                        + (g && hor ? 32 + 32 + 32 + 8 : 0);  // Y; Z; Q; N
+  const size_t per_pair = blocks * N2 * sizeof(double2);
+  const int batch = std::max(1, std::min((int)pairs.size(), (int)(sets_budget() / per_pair)));
+  for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
+    const int np = (int)pb.ent.size();
+    void* mem;
+    CTR_TRY(workspace(WS_SCRATCH).get((size_t)np * per_pair, &mem));
+    Arena ar;
+    ar.base = (double2*)mem;
+    ar.N2 = N2;
+    auto each = [&](size_t n) {
+      std::vector<double2*> v(np);
+      for (int i = 0; i < np; i++) v[i] = ar.take(n);
+      return v;
+    };
+    std::vector<double2*> bW, bV;
+    for (const auto& m : pb.by_tf) bW.push_back(ar.take(16 * m.size()));
+    for (const auto& m : pb.by_ti) bV.push_back(ar.take(32 * m.size()));
+    auto Wb = [&](int i, int b, int a) {
+      const int h = pb.gtf[i];
+      return bW[h] + ((size_t)a * 4 * pb.by_tf[h].size() + pb.ptf[i] * 4 + b) * N2;
+    };
+    auto Vb = [&](int y, int i, int b) {
+      const int h = pb.gti[i];
+      return bV[h] + ((size_t)y * 16 * pb.by_ti[h].size() + pb.pti[i] * 16 + b) * N2;
+    };
+    const std::vector<double2*> bJ = each(16), bP = each(hor ? 32 : 8), bX = each(hor ? 32 : 0),
+                                bR = each(g ? 16 : 0), bS = each(g ? 16 : 0), bK = each(g ? 16 : 0),
+                                bU = each(g ? 32 : 0), bO = each(g ? 8 : 0), bY = each(g && hor ? 32 : 0),
+                                bZ = each(g && hor ? 32 : 0), bQ = each(g && hor ? 32 : 0),
+                                bN = each(g && hor ? 8 : 0);
+    // blocks (row, column) of the stacked outputs: right block (column) major
+    auto rc = [&](double2* b, int r, int col) { return b + (size_t)(col * 4 + r) * N2; };
+    // Pm(y): hor: block (a, c) at [c][y * 4 + a]; else the diagonal blocks a at [a][y]
+    auto Pm = [&](int y, int i, int a, int c2) {
+      return hor ? bP[i] + (size_t)(c2 * 8 + y * 4 + a) * N2 : bP[i] + (size_t)(a * 2 + y) * N2;
+    };
+    std::vector<GridTask> g0, g1, g2, g3, g4, g5;
+    CombList comb;
+    for (size_t h = 0; h < pb.by_tf.size(); h++) {
+      const std::vector<int>& mi = pb.by_tf[h];
+      const int m = (int)mi.size(), tf = pb.tf[mi[0]];
+      // W = T^dag L: slab (pair, row b), right block a
+      GridTask G = make_grid(4 * m, 4, 4, kOne, 0xF, 0);
+      for (int pp = 0; pp < m; pp++)
+        for (int b = 0; b < 4; b++)
+          for (int k = 0; k < 4; k++) G.A[(size_t)(pp * 4 + b) * 4 + k] = pb.T[mi[pp]] + (size_t)(k * 4 + b) * N2;
+      for (int j = 0; j < 4; j++) {
+        for (int k = 0; k < 4; k++) G.B[j][k] = M[(size_t)cL * Nt + tf] + (size_t)(k * 4 + j) * N2;
+        G.C0[j] = bW[h] + (size_t)j * 4 * m * N2;
+      }
+      g0.push_back(std::move(G));
+    }
+    for (size_t h = 0; h < pb.by_ti.size(); h++) {
+      const std::vector<int>& mi = pb.by_ti[h];
+      const int m = (int)mi.size(), ti = pb.ti[mi[0]];
+      // V(y) = tau_b P_y(ti): slab (pair, block b), right block y
+      GridTask G = make_grid(16 * m, 2, 1, kOne, 0, 0);
+      for (int pp = 0; pp < m; pp++)
+        for (int b = 0; b < 16; b++) G.A[pp * 16 + b] = pb.T[mi[pp]] + (size_t)b * N2;
+      for (int y = 0; y < 2; y++) {
+        G.B[y][0] = P(P1 + y, ti);
+        G.C0[y] = bV[h] + (size_t)y * 16 * m * N2;
+      }
+      g0.push_back(std::move(G));
+    }
+    for (int i = 0; i < np; i++) {
+      const int tf = pb.tf[i], ti = pb.ti[i];
+      const double2* T = pb.T[i];
+      const double2* wp = w + (size_t)pairs[pb.ent[i]] * 5;
+      {  // J = W G T (the trailing G is a sign of its column): slab b, right block d
+        GridTask G = make_grid(4, 4, 4, kG5, 0, 0);
+        for (int b = 0; b < 4; b++)
+          for (int k = 0; k < 4; k++) G.A[b * 4 + k] = Wb(i, b, k);
+        for (int j = 0; j < 4; j++) {
+          for (int k = 0; k < 4; k++) G.B[j][k] = T + (size_t)(k * 4 + j) * N2;
+          G.C0[j] = rc(bJ[i], 0, j);
+        }
+        g1.push_back(std::move(G));
+      }
+      if (hor) {  // Pm(y) = V(y) T^dag: slab (y, a), right block c
+        GridTask G = make_grid(8, 4, 4, kOne, 0, 0xFFFF);
+        for (int y = 0; y < 2; y++)
+          for (int a = 0; a < 4; a++)
+            for (int k = 0; k < 4; k++) G.A[(size_t)(y * 4 + a) * 4 + k] = Vb(y, i, a * 4 + k);
+        for (int j = 0; j < 4; j++) {
+          for (int k = 0; k < 4; k++) G.B[j][k] = T + (size_t)(j * 4 + k) * N2;
+          G.C0[j] = bP[i] + (size_t)j * 8 * N2;
+        }
+        g1.push_back(std::move(G));
+        for (int y = 0; y < 2; y++) {
+          // X(1) = P3 Pm(1), X(2) = P4 Pm(2): block (a, c) at [a * 4 + c]
+          for (int jb = 0; jb < 2; jb++) {
+            GridTask H = make_grid(1, 8, 1, kOne, 0, 0);
+            H.A[0] = P(P3 + y, tf);
+            for (int j = 0; j < 8; j++) {
+              const int b = 8 * jb + j;
+              H.B[j][0] = Pm(y, i, b / 4, b % 4);
+              H.C0[j] = bX[i] + (size_t)(y * 16 + b) * N2;
+            }
+            g2.push_back(std::move(H));
+          }
+          if (!g) continue;
+          // Y(1) = Pm(1) P4, Y(2) = Pm(2) P3; Z(1) = X(2) P3, Z(2) = X(1) P4
+          GridTask Y = make_grid(16, 1, 1, kOne, 0, 0), Z = make_grid(16, 1, 1, kOne, 0, 0);
+          for (int b = 0; b < 16; b++) {
+            Y.A[b] = Pm(y, i, b / 4, b % 4);
+            Z.A[b] = bX[i] + (size_t)((1 - y) * 16 + b) * N2;
+          }
+          Y.B[0][0] = P(y ? P3 : P4, tf);
+          Z.B[0][0] = P(y ? P4 : P3, tf);
+          Y.C0[0] = bY[i] + (size_t)y * 16 * N2;
+          Z.C0[0] = bZ[i] + (size_t)y * 16 * N2;
+          g2.push_back(std::move(Y));
+          g3.push_back(std::move(Z));
+        }
+        if (g) {
+          // Q(h)_{b u} = sum_v tau_vb^dag Z(h)_{v u}: slab b, right block (h, u)
+          GridTask Q = make_grid(4, 8, 4, kOne, 0xF, 0);
+          for (int b = 0; b < 4; b++)
+            for (int v = 0; v < 4; v++) Q.A[b * 4 + v] = T + (size_t)(v * 4 + b) * N2;
+          for (int j = 0; j < 8; j++) {
+            for (int v = 0; v < 4; v++) Q.B[j][v] = bZ[i] + (size_t)((j / 4) * 16 + v * 4 + j % 4) * N2;
+            Q.C0[j] = bQ[i] + (size_t)j * 4 * N2;
+          }
+          g4.push_back(std::move(Q));
+          // N(h) = sum_u N(h)_u, N(h)_u = sum_b Q(h)_{b u} tau_ub: slab h
+          for (int u = 0; u < 4; u++) {
+            GridTask G = make_grid(2, 1, 4, kOne, 0, 0);
+            for (int h = 0; h < 2; h++)
+              for (int b = 0; b < 4; b++) G.A[h * 4 + b] = bQ[i] + (size_t)((h * 4 + u) * 4 + b) * N2;
+            for (int b = 0; b < 4; b++) G.B[0][b] = T + (size_t)(u * 4 + b) * N2;
+            G.C0[0] = bN[i] + (size_t)u * 2 * N2;
+            g5.push_back(std::move(G));
+          }
+        }
+      } else {  // the diagonal blocks Pm(y)_aa alone: slab y
+        for (int a = 0; a < 4; a++) {
+          GridTask G = make_grid(2, 1, 4, kOne, 0, 0xF);
+          for (int y = 0; y < 2; y++)
+            for (int k = 0; k < 4; k++) G.A[y * 4 + k] = Vb(y, i, a * 4 + k);
+          for (int k = 0; k < 4; k++) G.B[0][k] = T + (size_t)(a * 4 + k) * N2;
+          G.C0[0] = Pm(0, i, a, a);
+          g1.push_back(std::move(G));
+        }
+      }
+      if (!g) continue;
+      // Rw = w_sq Rsq + w_dt Rdt, S = T G Rw, K = S T^dag (the leading G is a sign of its row)
+      const double2 a = make_double2(wp[0].x * wsq, wp[0].y * wsq), b = make_double2(wp[1].x * wdt, wp[1].y * wdt);
+      for (int k = 0; k < 16; k++) {
+        comb.begin(bR[i] + (size_t)k * N2, false);
+        comb.term(M[(size_t)cSq * Nt + ti] + (size_t)k * N2, a);
+        comb.term(M[(size_t)cDt * Nt + ti] + (size_t)k * N2, b);
+      }
+      GridTask S = make_grid(4, 4, 4, kG5, 0, 0), K = make_grid(4, 4, 4, kOne, 0, 0xFFFF);
+      for (int r = 0; r < 4; r++)
+        for (int k = 0; k < 4; k++) {
+          S.A[r * 4 + k] = T + (size_t)(r * 4 + k) * N2;
+          K.A[r * 4 + k] = rc(bS[i], r, k);
+        }
+      for (int j = 0; j < 4; j++) {
+        for (int k = 0; k < 4; k++) {
+          S.B[j][k] = bR[i] + (size_t)(k * 4 + j) * N2;
+          K.B[j][k] = T + (size_t)(j * 4 + k) * N2;
+        }
+        S.C0[j] = rc(bS[i], 0, j);
+        K.C0[j] = rc(bK[i], 0, j);
+      }
+      g0.push_back(std::move(S));
+      g1.push_back(std::move(K));
+      // U(x) = P_x tau_b (x = P3, P4): slab x, right block b; O(x)_a = sum_b tau_ab^dag U(x)_ab: right block x
+      for (int jb = 0; jb < 2; jb++) {
+        GridTask U = make_grid(2, 8, 1, kOne, 0, 0);
+        U.A[0] = P(P3, tf);
+        U.A[1] = P(P4, tf);
+        for (int j = 0; j < 8; j++) {
+          U.B[j][0] = T + (size_t)(8 * jb + j) * N2;
+          U.C0[j] = bU[i] + (size_t)(8 * jb + j) * 2 * N2;
+        }
+        g0.push_back(std::move(U));
+      }
+      for (int r = 0; r < 4; r++) {
+        GridTask O = make_grid(1, 2, 4, kOne, 0xF, 0);
+        for (int k = 0; k < 4; k++) O.A[k] = T + (size_t)(r * 4 + k) * N2;
+        for (int x = 0; x < 2; x++) {
+          for (int k = 0; k < 4; k++) O.B[x][k] = bU[i] + (size_t)((r * 4 + k) * 2 + x) * N2;
+          O.C0[x] = bO[i] + (size_t)(x * 4 + r) * N2;
+        }
+        g1.push_back(std::move(O));
+      }
+    }
+    CTR_TRY(comb.run((int)N2, c.s));
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(run_grids(c, g1, WS_TASKS));
+    CTR_TRY(run_grids(c, g2, WS_TASKS));
+    CTR_TRY(run_grids(c, g3, WS_TASKS));
+    CTR_TRY(run_grids(c, g4, WS_TASKS));
+    CTR_TRY(run_grids(c, g5, WS_TASKS));
+    // ---- values: 64 traces a pair, then the correlators and the twins' weights
+    static const int tx[4] = {P4, P3, P3, P4}, ty[4] = {0, 1, 0, 1};  // twins (P4, P1), (P3, P2), (P3, P1), (P4, P2)
+    void *dv, *dw[2];
+    CTR_TRY(workspace(WS_ROWABS).get((size_t)np * 68 * sizeof(double2), &dv));
+    double2* vals = (double2*)dv;
+    double2* wk = vals + (size_t)np * 64;
+    if (!hor) CTR_CUDA(cudaMemsetAsync(vals, 0, (size_t)np * 64 * sizeof(double2), c.s));
+    DiagList dv_l, dg;
+    std::vector<int> ent(np);
+    std::vector<double2> wsf((size_t)np * 2);
+    for (int i = 0; i < np; i++) {
+      const int v0 = i * 64, ti = pb.ti[i], tf = pb.tf[i];
+      ent[i] = pairs[pb.ent[i]];
+      const double2* wp = w + (size_t)ent[i] * 5;
+      wsf[2 * i] = make_double2(wp[2].x * wst, wp[2].y * wst);
+      wsf[2 * i + 1] = make_double2(wp[3].x * wfi, wp[3].y * wfi);
+      for (int b = 0; b < 16; b++) {
+        // Tr[R_{a b} J_{b a}] g5(a)
+        dv_l.value(M[(size_t)cSq * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + b);
+        dv_l.value(M[(size_t)cDt * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + 16 + b);
+        if (hor)
+          dv_l.value(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + (b % 4) * 4 + b / 4) * N2, v0 + 32 + b);
+      }
+      for (int k = 0; k < 4; k++)
+        for (int a = 0; a < 4; a++) dv_l.value(P(tx[k], tf), Pm(ty[k], i, a, a), v0 + 48 + k * 4 + a);
+      if (!g) continue;
+      if (hor) {
+        const double2 wh = make_double2(wp[4].x * wdh, wp[4].y * wdh);
+        for (int b = 0; b < 16; b++) {
+          const int bt = (b % 4) * 4 + b / 4;
+          dg.both(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + bt) * N2, wh);
+          dg.both(bY[i] + (size_t)b * N2, bY[i] + (size_t)(16 + bt) * N2, wh);
+        }
+        for (int y = 0; y < 2; y++)
+          for (int u = 0; u < 4; u++) dg.both(P(P1 + y, ti), bN[i] + (size_t)(u * 2 + y) * N2, wh);
+      }
+      for (int k = 0; k < 4; k++)
+        for (int a = 0; a < 4; a++) {
+          const double2* wkp = wk + 4 * (size_t)i + k;
+          dg.both(P(tx[k], tf), Pm(ty[k], i, a, a), make_double2(1.0, 0.0), wkp);
+          dg.both(P(P1 + ty[k], ti), bO[i] + (size_t)((tx[k] - P3) * 4 + a) * N2, make_double2(1.0, 0.0), wkp);
+        }
+    }
+    CTR_TRY(launch_diag(dv_l.t, 0, N, f, vals, nullptr, c.s));
+    CTR_TRY(upload_group(WS_MISC, {{ent.data(), ent.size() * sizeof(int)}, {wsf.data(), wsf.size() * sizeof(double2)}},
+                         dw, c.s));
+    {
+      TimedLaunch tl(c.s, "pipi_combine");
+      pipi_vjp_combine_kernel<<<(np + 127) / 128, 128, 0, c.s>>>(vals, (const int*)dw[0], (const double2*)dw[1], np, wsq,
+                                                                 wdt, wst, wfi, wdh, corr, wk);
+      CTR_CUDA(cudaGetLastError());
+    }
+    CTR_TRY(launch_diag(dg.t, dg.nrow, N, f, nullptr, grad, c.s));
+    if (!g) continue;
+    // ---- co-factors of the batch, summed per time slice
+    CombList sum;
+    for (const std::vector<int>& mi : pb.by_tf)
+      for (int b = 0; b < 16; b++) {
+        sum.begin(Ks + (size_t)pb.tf[mi[0]] * blk16 + (size_t)b * N2, true);
+        for (int i : mi) sum.term(rc(bK[i], b / 4, b % 4), make_double2(1.0, 0.0));
+      }
+    for (const std::vector<int>& mi : pb.by_ti)
+      for (int k = 0; k < 2; k++)
+        for (int b = 0; b < 16; b++) {
+          sum.begin((k ? Jd : Js) + (size_t)pb.ti[mi[0]] * blk16 + (size_t)b * N2, true);
+          for (int i : mi) {
+            const double2 wv = w[(size_t)pairs[pb.ent[i]] * 5 + k];
+            const double sc = k ? wdt : wsq;
+            sum.term(rc(bJ[i], b / 4, b % 4), make_double2(wv.x * sc, wv.y * sc));
+          }
+        }
+    CTR_TRY(sum.run((int)N2, c.s));
+  }
+  if (!g) return CTR_OK;
+  // ---- per time slice: Tr[Pa tau_ab Pb F_ba] with co-factor F = K (L at the sink times) and Jsq, Jdt (R at the
+  // source times): (tau Pb)(F Pa) holds the right indices, (Pa tau)(Pb F) the left ones
+  struct Slice {
+    int t, a, b;
+    const double2* F;
+    bool row_sign;  // gamma_5 on F's row (K) or its column (J)
+  };
+  std::vector<Slice> sl;
+  for (int t = 0; t < Nt; t++) {
+    if (on_tf[t]) sl.push_back({t, P3, P4, Ks + (size_t)t * blk16, true});
+    if (on_ti[t]) {
+      sl.push_back({t, P2, P1, Js + (size_t)t * blk16, false});
+      sl.push_back({t, P1, P2, Jd + (size_t)t * blk16, false});
+    }
+  }
+  const size_t per_sl = 64 * N2 * sizeof(double2);
+  const size_t chunk = std::max<size_t>(1, std::min(sl.size(), sets_budget() / per_sl));
+  for (size_t s0 = 0; s0 < sl.size(); s0 += chunk) {
+    const size_t ns = std::min(chunk, sl.size() - s0);
+    void* mem;
+    CTR_TRY(workspace(WS_SCRATCH).get(ns * per_sl, &mem));
+    std::vector<GridTask> g0;
+    DiagList dl;
+    for (size_t k = 0; k < ns; k++) {
+      const Slice& S = sl[s0 + k];
+      const double2* D = diag + (size_t)S.t * blk16;
+      double2* o = (double2*)mem + k * 64 * N2;  // tau Pb, F Pa, Pa tau, Pb F
+      GridTask A = make_grid(16, 1, 1, kOne, 0, 0), B = make_grid(16, 1, 1, kOne, 0, 0);
+      for (int b = 0; b < 16; b++) {
+        A.A[b] = D + (size_t)b * N2;
+        B.A[b] = S.F + (size_t)b * N2;
+      }
+      A.B[0][0] = P(S.b, S.t);
+      B.B[0][0] = P(S.a, S.t);
+      A.C0[0] = o;
+      B.C0[0] = o + blk16;
+      g0.push_back(std::move(A));
+      g0.push_back(std::move(B));
+      for (int jb = 0; jb < 2; jb++) {
+        GridTask C = make_grid(1, 8, 1, kOne, 0, 0), E = make_grid(1, 8, 1, kOne, 0, 0);
+        C.A[0] = P(S.a, S.t);
+        E.A[0] = P(S.b, S.t);
+        for (int j = 0; j < 8; j++) {
+          C.B[j][0] = D + (size_t)(8 * jb + j) * N2;
+          E.B[j][0] = S.F + (size_t)(8 * jb + j) * N2;
+          C.C0[j] = o + 2 * blk16 + (size_t)(8 * jb + j) * N2;
+          E.C0[j] = o + 3 * blk16 + (size_t)(8 * jb + j) * N2;
+        }
+        g0.push_back(std::move(C));
+        g0.push_back(std::move(E));
+      }
+      for (int b = 0; b < 16; b++) {
+        const int bt = (b % 4) * 4 + b / 4;  // tau_ab against F_ba
+        const double2 sg = make_double2((double)G5[S.row_sign ? b % 4 : b / 4], 0.0);
+        dl.both(o + (size_t)b * N2, o + blk16 + (size_t)bt * N2, sg);
+        dl.both(o + 2 * blk16 + (size_t)b * N2, o + 3 * blk16 + (size_t)bt * N2, sg);
+      }
+    }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(launch_diag(dl.t, dl.nrow, N, f, nullptr, grad, c.s));
+  }
   return CTR_OK;
 }
 
@@ -510,60 +1233,10 @@ int ctr_rho_profile_vjp(int engine, int nev, int nt, const double* prop, const d
   std::vector<double> hw((size_t)nt * nt * 48 * 2);
   CTR_CUDA(cudaMemcpyAsync(hw.data(), w, hw.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
   CTR_CUDA(cudaStreamSynchronize(s));
-  std::vector<int> pairs;
-  for (int p = 0; p < nt * nt; p++) {
-    bool any = false;
-    for (int k = 0; k < 96; k++) any = any || hw[(size_t)p * 96 + k] != 0.0;
-    if (any) pairs.push_back(p);
-  }
   double2* phis;
   CTR_TRY(profiled(nev, (long long)nt * 5, mom5, f, WS_PHI, &phis, s));
-  const Tables& T = tables();
-  void* dvals = nullptr;
-  const size_t nval = std::max<size_t>(1, pairs.size() * 768);
-  if (corr) {
-    CTR_TRY(workspace(WS_TASKS2).get(nval * sizeof(double2), &dvals));
-    CTR_CUDA(cudaMemsetAsync(dvals, 0, nval * sizeof(double2), s));
-  }
-  ChainRunner R(nev, nt, 5, (const double2*)prop, phis, f, (double2*)dvals, grad, s, engine);
-  // lib/calculate_rho_core.h: coef * Tr[tau_{s3s4} Phi_lp(ti) (Phi_rp(tf) tau_{s1s2})^dagger]
-  for (size_t q = 0; q < pairs.size(); q++) {
-    const int tf = pairs[q] / nt, ti = pairs[q] % nt;
-    for (int o = 0; o < 48; o++) {
-      const size_t wi = ((size_t)pairs[q] * 48 + o) * 2;
-      const double2 wo = make_double2(hw[wi], hw[wi + 1]);
-      if (wo.x == 0.0 && wo.y == 0.0) continue;
-      for (int is = 0; is < 16; is++) {
-        const int r = o * 16 + is;
-        const int s1 = T.rho_spin[r][0], s2 = T.rho_spin[r][1], s3 = T.rho_spin[r][2], s4 = T.rho_spin[r][3];
-        const int lp = T.rho_lprp[r][0], rp = T.rho_lprp[r][1];
-        const ctr_factor ch[4] = {tau(tf, ti, s3, s4), phi(ti, lp), tau(tf, ti, s1, s2, 1), phi(tf, rp, 1)};
-        CTR_TRY(R.add(ch, 4, cw(wo, T.rho_coef[r][0], T.rho_coef[r][1]), corr ? (int)(q * 768 + r) : -1,
-                      grad != nullptr));
-      }
-    }
-    CTR_TRY(R.end_group());
-  }
-  CTR_TRY(R.flush());
-  if (corr) {
-    // corr[tf][ti][o] = sum of the 16 coefficient-weighted spin rows (lib/contract_kernels_rho.cu:108-116)
-    std::vector<double2> rv(pairs.size() * 768);
-    if (!rv.empty()) {
-      CTR_CUDA(cudaMemcpyAsync(rv.data(), dvals, rv.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-      CTR_CUDA(cudaStreamSynchronize(s));
-    }
-    std::vector<double2> hc((size_t)nt * nt * 48, make_double2(0.0, 0.0));
-    for (size_t q = 0; q < pairs.size(); q++)
-      for (int r = 0; r < 768; r++) {
-        const double2 v = cmul(make_double2(T.rho_coef[r][0], T.rho_coef[r][1]), rv[q * 768 + r]);
-        double2& c = hc[(size_t)pairs[q] * 48 + r / 16];
-        c.x += v.x;
-        c.y += v.y;
-      }
-    CTR_CUDA(cudaMemcpyAsync(corr, hc.data(), hc.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
-    CTR_CUDA(cudaStreamSynchronize(s));
-  }
-  return CTR_OK;
+  return rho_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, (const double2*)prop, phis, f, (const double2*)hw.data(),
+                 (double2*)corr, grad);
 }
 
 int ctr_pipi_profile_vjp(int engine, int nev, int nt, int isospin, const double* prop, const double* p1,
@@ -576,159 +1249,23 @@ int ctr_pipi_profile_vjp(int engine, int nev, int nt, int isospin, const double*
     return fail(CTR_ERR_ARG, "ctr_pipi_profile_vjp: bad arguments");
   if (isospin != 0 && isospin != 1) return fail(CTR_ERR_ARG, "isospin must be 0 (I=0) or 1 (I=1)");
   CTR_TRY(check_f(nev, f, s));
-  const size_t N2 = (size_t)nev * nev;
   std::vector<double> hw((size_t)nt * nt * 5 * 2);
   CTR_CUDA(cudaMemcpyAsync(hw.data(), w, hw.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  // elementals [t][4] = P1..P4 (profiled)
-  void* raw;
-  CTR_TRY(workspace(WS_MISC).get((size_t)nt * 4 * N2 * sizeof(double2), &raw));
-  const double* ps[4] = {p1, p2, p3, p4};
-  for (int t = 0; t < nt; t++)
-    for (int k = 0; k < 4; k++)
-      CTR_CUDA(cudaMemcpyAsync((double2*)raw + ((size_t)t * 4 + k) * N2, (const double2*)ps[k] + (size_t)t * N2,
-                               N2 * sizeof(double2), cudaMemcpyDeviceToDevice, s));
-  double2* phis;
-  CTR_TRY(profiled(nev, (long long)nt * 4, (const double*)raw, f, WS_PHI, &phis, s));
-  const Tables& T = tables();
-  enum { P1 = 0, P2 = 1, P3 = 2, P4 = 3 };
-  // isospin weights of the correlator slots (lib/contract_kernels_pipi.cu:288-303, :463-478)
-  const double wsq = isospin == 1 ? -2.0 : -1.0 / 3.0, wdt = isospin == 1 ? 2.0 : -1.0 / 3.0;
-  const double wstar = isospin == 1 ? -1.0 : 1.0, wfish = 1.0, wdth = isospin == 1 ? 0.0 : -5.0 / 3.0;
-
-  std::vector<int> pairs;
-  for (int p = 0; p < nt * nt; p++) {
-    bool any = false;
-    for (int k = 0; k < 10; k++) any = any || hw[(size_t)p * 10 + k] != 0.0;
-    if (any) pairs.push_back(p);
+  CTR_CUDA(cudaStreamSynchronize(s));
+  // the distinct elementals, profiled: [elemental][t]
+  int32_t set[4];
+  std::vector<Elem> el = elems(nev, {p1, p2, p3, p4}, set);
+  const size_t n1 = (size_t)nt * nev * nev;
+  void* mem;
+  CTR_TRY(workspace(WS_PHI).get(el.size() * n1 * sizeof(double2), &mem));
+  for (size_t k = 0; k < el.size(); k++) {
+    TimedLaunch tl(s, "apply_profile");
+    apply_profile_kernel<<<1024, 256, 0, s>>>(el[k].p, (double2*)mem + k * n1, f, nev, nt);
+    CTR_CUDA(cudaGetLastError());
+    el[k].p = (const double2*)mem + k * n1;
   }
-  // star / fish are products of two spin-summed traces: their values come first
-  // (lib/calculate_pipi_starfish_core.h: tr = Tr[Pa(tf) tau_{s1s2} Pb(ti) tau_{s1s2}^dagger])
-  auto sf_chain = [&](int tf, int ti, int is, int a, int b, ctr_factor* ch) {
-    const int s1 = is / 4, s2 = is % 4;
-    ch[0] = phi(tf, a);
-    ch[1] = tau(tf, ti, s1, s2);
-    ch[2] = phi(ti, b);
-    ch[3] = tau(tf, ti, s1, s2, 1);
-  };
-  // [pair][4 traces: star tr1 (P4,P1), star tr2 (P3,P2), fish tr1 (P3,P1), fish tr2 (P4,P2)][16]
-  const int sfa[4] = {P4, P3, P3, P4}, sfb[4] = {P1, P2, P1, P2};
-  std::vector<double2> sfv(pairs.size() * 64, make_double2(0.0, 0.0));
-  {
-    void* dv;
-    CTR_TRY(workspace(WS_TASKS2).get(std::max<size_t>(1, sfv.size()) * sizeof(double2), &dv));
-    ChainRunner R(nev, nt, 4, (const double2*)prop, phis, f, (double2*)dv, nullptr, s, engine);
-    for (size_t q = 0; q < pairs.size(); q++) {
-      const int tf = pairs[q] / nt, ti = pairs[q] % nt;
-      for (int k = 0; k < 4; k++)
-        for (int is = 0; is < 16; is++) {
-          ctr_factor ch[4];
-          sf_chain(tf, ti, is, sfa[k], sfb[k], ch);
-          CTR_TRY(R.add(ch, 4, make_double2(0.0, 0.0), (int)(q * 64 + k * 16 + is), false));
-        }
-      CTR_TRY(R.end_group());
-    }
-    CTR_TRY(R.flush());
-    if (!sfv.empty()) {
-      CTR_CUDA(cudaMemcpyAsync(sfv.data(), dv, sfv.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-      CTR_CUDA(cudaStreamSynchronize(s));
-    }
-  }
-  void* dvals = nullptr;
-  if (corr) {
-    // per-chain values: 256 square + 256 dT + 256 dTH rows per pair
-    CTR_TRY(workspace(WS_TASKS2).get(std::max<size_t>(1, pairs.size() * 768) * sizeof(double2), &dvals));
-    CTR_CUDA(cudaMemsetAsync(dvals, 0, std::max<size_t>(1, pairs.size() * 768) * sizeof(double2), s));
-  }
-  const bool g = grad != nullptr;
-  ChainRunner R(nev, nt, 4, (const double2*)prop, phis, f, (double2*)dvals, grad, s, engine);
-  for (size_t q = 0; q < pairs.size(); q++) {
-    const int tf = pairs[q] / nt, ti = pairs[q] % nt;
-    const double* wp = &hw[(size_t)pairs[q] * 10];
-    const double2 w_sq = make_double2(wp[0] * wsq, wp[1] * wsq), w_dt = make_double2(wp[2] * wdt, wp[3] * wdt);
-    const double2 w_st = make_double2(wp[4] * wstar, wp[5] * wstar), w_fi = make_double2(wp[6] * wfish, wp[7] * wfish);
-    const double2 w_dh = make_double2(wp[8] * wdth, wp[9] * wdth);
-    for (int bx = 0; bx < 256; bx++) {
-      const int16_t* sq = T.sq_spin[bx];
-      // lib/calculate_pipi_square_core.h
-      const ctr_factor c_sq[8] = {phi(tf, P3),          tau(tf, tf, sq[2], sq[3]), phi(tf, P4),
-                                  tau(tf, ti, sq[4], sq[5]), phi(ti, P2),           tau(ti, ti, sq[0], sq[1]),
-                                  phi(ti, P1),          tau(tf, ti, sq[2], sq[1], 1)};
-      CTR_TRY(R.add(c_sq, 8, cw(w_sq, T.sq_coef[bx][0], T.sq_coef[bx][1]), corr ? (int)(q * 768 + bx) : -1, g));
-      const int16_t* dt = T.dt_spin[bx];
-      // lib/calculate_pipi_doubleTriangle_core.h
-      const ctr_factor c_dt[8] = {phi(tf, P3),          tau(tf, tf, dt[4], dt[5]), phi(tf, P4),
-                                  tau(tf, ti, dt[0], dt[1]), phi(ti, P1),           tau(ti, ti, dt[2], dt[3]),
-                                  phi(ti, P2),          tau(tf, ti, dt[4], dt[3], 1)};
-      CTR_TRY(R.add(c_dt, 8, cw(w_dt, T.dt_coef[bx][0], T.dt_coef[bx][1]), corr ? (int)(q * 768 + 256 + bx) : -1,
-                    g));
-      if (isospin == 0) {
-        const int16_t* dh = T.dth_spin[bx];
-        // lib/calculate_pipi_doubleTriangleHor_core.h (all blocks tau(tf, ti))
-        const ctr_factor c_dh[8] = {phi(tf, P3),          tau(tf, ti, dh[0], dh[1]),    phi(ti, P1),
-                                    tau(tf, ti, dh[2], dh[1], 1), phi(tf, P4),         tau(tf, ti, dh[2], dh[3]),
-                                    phi(ti, P2),          tau(tf, ti, dh[0], dh[3], 1)};
-        CTR_TRY(R.add(c_dh, 8, cw(w_dh, T.dth_coef[bx][0], T.dth_coef[bx][1]),
-                      corr ? (int)(q * 768 + 512 + bx) : -1, g));
-      }
-    }
-    // star = tr1 * tr2 (sums over 16 spins): d(star) = tr2 d(tr1) + tr1 d(tr2); fish likewise
-    double2 sum[4];
-    for (int k = 0; k < 4; k++) {
-      sum[k] = make_double2(0.0, 0.0);
-      for (int is = 0; is < 16; is++) {
-        sum[k].x += sfv[q * 64 + k * 16 + is].x;
-        sum[k].y += sfv[q * 64 + k * 16 + is].y;
-      }
-    }
-    const double2 wk[4] = {cmul(w_st, sum[1]), cmul(w_st, sum[0]), cmul(w_fi, sum[3]), cmul(w_fi, sum[2])};
-    for (int k = 0; k < 4 && g; k++) {
-      if (wk[k].x == 0.0 && wk[k].y == 0.0) continue;
-      for (int is = 0; is < 16; is++) {
-        ctr_factor ch[4];
-        sf_chain(tf, ti, is, sfa[k], sfb[k], ch);
-        CTR_TRY(R.add(ch, 4, wk[k], -1, true));
-      }
-    }
-    CTR_TRY(R.end_group());
-  }
-  CTR_TRY(R.flush());
-  if (corr) {
-    // corr[tf][ti][5] for the pairs with nonzero weight (zero elsewhere), isospin-weighted
-    std::vector<double2> rv(pairs.size() * 768);
-    if (!rv.empty()) {
-      CTR_CUDA(cudaMemcpyAsync(rv.data(), dvals, rv.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-      CTR_CUDA(cudaStreamSynchronize(s));
-    }
-    std::vector<double2> hc((size_t)nt * nt * 5, make_double2(0.0, 0.0));
-    for (size_t q = 0; q < pairs.size(); q++) {
-      double2 a[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-      for (int d = 0; d < 3; d++)
-        for (int bx = 0; bx < 256; bx++) {
-          const float* cf = d == 0 ? T.sq_coef[bx] : d == 1 ? T.dt_coef[bx] : T.dth_coef[bx];
-          const double2 v = cmul(make_double2(cf[0], cf[1]), rv[q * 768 + d * 256 + bx]);
-          a[d].x += v.x;
-          a[d].y += v.y;
-        }
-      double2 sum[4];
-      for (int k = 0; k < 4; k++) {
-        sum[k] = make_double2(0.0, 0.0);
-        for (int is = 0; is < 16; is++) {
-          sum[k].x += sfv[q * 64 + k * 16 + is].x;
-          sum[k].y += sfv[q * 64 + k * 16 + is].y;
-        }
-      }
-      const double2 st = cmul(sum[0], sum[1]), fi = cmul(sum[2], sum[3]);
-      double2* c = &hc[(size_t)pairs[q] * 5];
-      c[0] = make_double2(wsq * a[0].x, wsq * a[0].y);
-      c[1] = make_double2(wdt * a[1].x, wdt * a[1].y);
-      c[2] = make_double2(wstar * st.x, wstar * st.y);
-      c[3] = make_double2(wfish * fi.x, wfish * fi.y);
-      c[4] = make_double2(wdth * a[2].x, wdth * a[2].y);
-    }
-    CTR_CUDA(cudaMemcpyAsync(corr, hc.data(), hc.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
-    CTR_CUDA(cudaStreamSynchronize(s));
-  }
-  return CTR_OK;
+  return pipi_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, isospin, (const double2*)prop, el, set, f,
+                  (const double2*)hw.data(), (double2*)corr, grad);
 }
 
 }  // extern "C"

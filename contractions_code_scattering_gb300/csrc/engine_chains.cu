@@ -29,20 +29,9 @@
 #include <tuple>
 #include <utility>
 
-#include "kernels.h"
+#include "chains.h"
 
 namespace ctr {
-
-namespace {
-
-constexpr int G5[4] = {1, 1, -1, -1};  // gamma_5 = diag(1,1,-1,-1) of the table basis
-
-struct Ctx {
-  int N, Nt;
-  size_t N2;
-  cudaStream_t s;
-  int engine = CTR_ENGINE_FP64;
-};
 
 // Stage = one launch of the batched GEMM; stages run in order on the stream.
 int run_stage(const Ctx& c, const std::vector<ZTask>& tasks, int slot) {
@@ -83,7 +72,7 @@ int run_grids(const Ctx& c, const std::vector<GridTask>& g, int slot) {
   return run_stage(c, t, slot);
 }
 
-inline TraceTask tr(const double2* X, const double2* Y, double2* out, float cre, float cim, int mode) {
+static inline TraceTask tr(const double2* X, const double2* Y, double2* out, float cre, float cim, int mode) {
   TraceTask t{};
   t.X = X;
   t.Y = Y;
@@ -93,13 +82,6 @@ inline TraceTask tr(const double2* X, const double2* Y, double2* out, float cre,
   t.mode = mode;
   return t;
 }
-
-// Elemental of a call: Phi(t) = p + t * stride (an [Nt][N][N] array, or one momentum
-// of an [Nt][nphi][N][N] array).
-struct Elem {
-  const double2* p;
-  size_t stride;
-};
 
 GridTask make_grid(int nslab, int nb, int nterm, const float* w, int adag, int bdag) {
   GridTask G;
@@ -115,24 +97,8 @@ GridTask make_grid(int nslab, int nb, int nterm, const float* w, int adag, int b
   return G;
 }
 
-const float kOne[4] = {1.f, 1.f, 1.f, 1.f};
-const float kG5[4] = {(float)G5[0], (float)G5[1], (float)G5[2], (float)G5[3]};
-
-// The pairs of one call in batches.  All pairs: tiles of t_sink x t_src, both
-// extents as even as the batch allows, so that the pairs that share a t_src (the
-// right operands R and Phi(t_src)) and those that share a t_sink (L and
-// Phi(t_sink)) both stack along M: from 7 pairs of 4 slabs up, the padding rows of
-// a 128-row tile are below 2 %.  At most hmax sink times a batch.  A list of pairs
-// keeps the list's order.
-struct PairBatch {
-  std::vector<int> ent, tf, ti;       // position in the output, time slices
-  std::vector<const double2*> T;      // tau(tf, ti)
-  std::vector<std::vector<int>> by_ti, by_tf;  // groups of batch indices
-  std::vector<int> gti, pti, gtf, ptf;         // group and position of each pair
-};
-
 std::vector<PairBatch> pair_batches(const double2* tau, size_t blk16, int Nt, int tf_begin, int rows, int batch,
-                                    const std::vector<int>* plist, int hmax = 1 << 30) {
+                                    const std::vector<int>* plist, int hmax) {
   std::vector<std::vector<std::pair<int, int>>> out;  // (position, pair)
   if (plist) {
     for (size_t i = 0; i < plist->size(); i++) {
@@ -181,6 +147,8 @@ std::vector<PairBatch> pair_batches(const double2* tau, size_t blk16, int Nt, in
   }
   return res;
 }
+
+namespace {
 
 // ---- per-entry refinement of split-engine chains
 // A chain entry's rounding error is estimated as REFINE_EPS_CHAIN times the sum
@@ -310,6 +278,8 @@ __global__ void pipi_combine_sets_kernel(const double2* __restrict__ trv, const 
   }
 }
 
+}  // namespace
+
 // Scratch budget of a set batch: 16 GB, or an eighth of the device's memory where less.
 size_t sets_budget() {
   static size_t b = 0;
@@ -380,33 +350,14 @@ int per_t_products(const Ctx& c, const double2* diag, const std::vector<Elem>& e
   return run_grids(c, g1, WS_TASKS2);
 }
 
-// Distinct pairs of elementals, and the time slices each is needed at.
-struct Combos {
-  std::vector<std::pair<int, int>> list;
-  std::vector<std::vector<char>> need;
-  std::map<std::pair<int, int>, int> at;
-  int Nt;
-  explicit Combos(int nt) : Nt(nt) {}
-  int use(int a, int b) {
-    auto it = at.emplace(std::make_pair(a, b), (int)list.size()).first;
-    if (it->second == (int)list.size()) {
-      list.push_back({a, b});
-      need.emplace_back(Nt, 0);
-    }
-    return it->second;
-  }
-};
-
 // Distinct values in ascending order, and the index of each of 0 .. n - 1.
-std::vector<int> index_of(std::vector<int>& v, int n) {
+static std::vector<int> index_of(std::vector<int>& v, int n) {
   std::sort(v.begin(), v.end());
   v.erase(std::unique(v.begin(), v.end()), v.end());
   std::vector<int> ix(n, -1);
   for (size_t a = 0; a < v.size(); a++) ix[v[a]] = (int)a;
   return ix;
 }
-
-}  // namespace
 
 // ------------------------------------------------------------------ pi pi
 // Every momentum set (P1..P4 = el[sets[4k ..]]) of one call; with plist, the listed
@@ -1396,7 +1347,7 @@ namespace ctr {
 
 // One call's own elementals, [nt][nev][nev] each; set[k]: the first of them with
 // the k-th one's address.
-static std::vector<Elem> elems(int nev, const std::vector<const double*>& p, int32_t* set) {
+std::vector<Elem> elems(int nev, const std::vector<const double*>& p, int32_t* set) {
   std::vector<Elem> el;
   for (size_t k = 0; k < p.size(); k++) {
     size_t j = 0;

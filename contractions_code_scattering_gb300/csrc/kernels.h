@@ -58,6 +58,26 @@ __device__ inline double block_sum_256(double v) {
   return r;  // valid in thread 0
 }
 
+// Block sums of two FP64 values: lanes 0-15 of each warp carry the first, 16-31
+// the second (5 adds a warp instead of 10: each holds the FP64 pipe for 16
+// clocks), then the warps' sums in order.  Thread k < 2 returns value k.
+template <int TPB>
+__device__ __forceinline__ double block_sum2(double x, double y) {
+  __shared__ double red[TPB / 32][2];
+  const int lane = threadIdx.x & 31;
+  double s = ((lane & 16) ? y : x) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? x : y, 16);
+  for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((lane & 15) == 0) red[threadIdx.x >> 5][lane >> 4] = s;
+  __syncthreads();
+  double v = 0.0;
+  if (threadIdx.x < 2) {
+    v = red[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < TPB / 32; w++) v += red[w][threadIdx.x];
+  }
+  return v;
+}
+
 // h_tasks: the same tasks on the host (optional); it lets the launcher check
 // that the weights allow the DMMA form.
 int launch_zgemm_f64(const ZTask* d_tasks, int ntask, int N, cudaStream_t s, const ZTask* h_tasks = nullptr);

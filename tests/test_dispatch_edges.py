@@ -88,3 +88,54 @@ def test_momentum_sets_sink_form(cuda, n, rhopi, tri, nset):
         if tri:
             ref, ab = ref_triangle(prop, pa, pb, mom2, range(*tr))
             P.entrywise(got["triangle"][k].cpu().numpy(), ref, SPLIT_TOL, ab, "set %d triangle" % k)
+
+
+@pytest.mark.parametrize("engine,tol", [("fp64", 1e-11), ("split", 1e-8)])
+@pytest.mark.parametrize("n,iso", [(1, 0), (33, 1), (7, 0), (129, 0)])
+def test_profile_gradients_block_form(cuda, n, iso, engine, tol):
+    """rho and pi pi profile gradients for arbitrary complex weights -- several t_sink
+    a t_src and the reverse, pairs on the time diagonal, single slots, outputs of
+    every operator pair -- with four different elementals, against autograd; Nev
+    129 takes the tiled diagonal kernel (FP64 engine only)."""
+    from contractions_code_scattering_gb300 import adjoint
+    from oracle import torch_ref as R
+    if n > 128 and engine == "split":
+        pytest.skip("the split engine takes Nev <= 128")
+    nt = 2 if n > 128 else 4
+    prop = synth.make_prop(nt, n, seed=900 + n)
+    rng = np.random.default_rng(901 + n)
+    mom5 = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(5)], axis=1)
+    ps = [synth.make_phi_random(nt, n, rng) for _ in range(4)]
+    f = adjoint.default_profile(n, seed=902)
+    z = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+    wr, wp = np.zeros((nt, nt, 48), complex), np.zeros((nt, nt, 5), complex)
+    if n <= 33:
+        wr[0, 1], wr[2, 1, 5], wr[1, 1, 47], wr[1, 0, 3:9] = z(48), z(), z(), z(6)
+        wp[0, 1], wp[3, 1], wp[2, 2], wp[0, 2, 4], wp[1, 3, 2] = z(5), z(5), z(5), z(), z()
+    else:
+        wr[0, 1, :2], wp[0, 1] = z(2), z(5)
+    dp, df = _dev(prop, cuda), _dev(f, cuda)
+    rho, gr = api.rho_profile_vjp(dp, _dev(mom5, cuda), df, _dev(wr, cuda), engine=engine)
+    pipi, gp = api.pipi_profile_vjp(dp, *[_dev(p, cuda) for p in ps], df, _dev(wp, cuda), iso, engine=engine)
+    ft = torch.tensor(f, requires_grad=True)
+    tp = torch.from_numpy(prop)
+    m5 = R.profiled(ft, torch.from_numpy(np.ascontiguousarray(mom5)))
+    pr = tuple(R.profiled(ft, torch.from_numpy(p)) for p in ps)
+    ref_r, ref_p, lr, lp = np.zeros_like(wr), np.zeros_like(wp), 0.0, 0.0
+    for tf in range(nt):
+        for ti in range(nt):
+            on = np.flatnonzero(wr[tf, ti])
+            if len(on):
+                v = R.rho_pair(tp, m5, tf, ti, [int(o) for o in on])
+                ref_r[tf, ti, on] = v.detach().numpy()
+                lr = lr + (torch.from_numpy(wr[tf, ti, on]) * v).real.sum()
+            if wp[tf, ti].any():
+                v = R.pipi_pair(tp, pr, tf, ti, iso)
+                ref_p[tf, ti] = v.detach().numpy()
+                lp = lp + (torch.from_numpy(wp[tf, ti]) * v).real.sum()
+    for got, ref, loss, g in ((rho, ref_r, lr, gr), (pipi, ref_p, lp, gp)):
+        got, g = got.cpu().numpy(), g.cpu().numpy()
+        assert np.all(got[ref == 0] == 0)
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+        want = torch.autograd.grad(loss, ft, retain_graph=True)[0].numpy()
+        assert np.abs(g - want).max() <= tol * np.abs(want).max()
