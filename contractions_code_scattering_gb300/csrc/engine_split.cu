@@ -6,6 +6,7 @@
 #include <cstring>
 #include <map>
 #include <tuple>
+#include <unordered_map>
 
 #include "kernels.h"
 #include "split.h"
@@ -24,6 +25,55 @@ int err_flag(int** out) {
   *out = g_err_dev;
   return CTR_OK;
 }
+
+// Index of each distinct pointer in order of first use: open addressing over a
+// power-of-two table (a launch of 1024 pairs looks up ~10^5 block pointers; an
+// ordered map took longer than the launch's kernels).
+class PtrIndex {
+ public:
+  int of(const void* p) {
+    if (2 * (n_ + 1) > slot_.size()) grow();
+    size_t h = hash(p) & (slot_.size() - 1);
+    while (slot_[h].p) {
+      if (slot_[h].p == p) return slot_[h].i;
+      h = (h + 1) & (slot_.size() - 1);
+    }
+    slot_[h] = Slot{p, (int)n_};
+    return (int)n_++;
+  }
+
+ private:
+  struct Slot {
+    const void* p = nullptr;
+    int i = 0;
+  };
+  static size_t hash(const void* p) { return (size_t)(((uintptr_t)p >> 4) * 0x9E3779B97F4A7C15ull >> 20); }
+  void grow() {
+    std::vector<Slot> old(std::max<size_t>(64, 2 * slot_.size()));
+    old.swap(slot_);
+    for (const Slot& s : old)
+      if (s.p) {
+        size_t h = hash(s.p) & (slot_.size() - 1);
+        while (slot_[h].p) h = (h + 1) & (slot_.size() - 1);
+        slot_[h] = s;
+      }
+  }
+  std::vector<Slot> slot_;
+  size_t n_ = 0;
+};
+
+// Hash of an operand list (its block pointers, weights and transposes).
+struct KeyHash {
+  size_t operator()(const std::vector<uintptr_t>& v) const {
+    uint64_t h = v.size();
+    for (uintptr_t x : v) {
+      h = (h ^ x) * 0x9E3779B97F4A7C15ull;
+      h ^= h >> 29;
+    }
+    return (size_t)h;
+  }
+};
+using KeyMap = std::unordered_map<std::vector<uintptr_t>, int, KeyHash>;
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -721,18 +771,15 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
       uint8_t* rbase = lbase + (size_t)ni * (l_b + le_b);   // <= ni x (right slices + column exponents)
       std::vector<SliceTaskLJob> lj;
       std::vector<SliceTaskRJob> rj;
-      std::map<const double2*, int> bid;          // distinct blocks -> exponent table index
+      PtrIndex bid;  // distinct blocks -> exponent table index
       std::vector<const double2*> blks;
       auto block_index = [&](const double2* p) {
-        auto b = bid.find(p);
-        if (b == bid.end()) {
-          b = bid.emplace(p, (int)blks.size()).first;
-          blks.push_back(p);
-        }
-        return b->second;
+        const int b = bid.of(p);
+        if (b == (int)blks.size()) blks.push_back(p);
+        return b;
       };
-      std::map<int, int> lid;                     // instances of one left group share its slices
-      std::map<std::vector<uintptr_t>, int> rid;  // identical right sides are sliced once
+      std::map<int, int> lid;  // instances of one left group share its slices
+      KeyMap rid;              // identical right sides are sliced once
       std::vector<SplitGemmInst> gi(ni);
       std::vector<double2*> outs((size_t)ni * SPLIT_TASK_NB, nullptr);
       for (int i = 0; i < ni; i++) {
@@ -873,17 +920,14 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
       uint8_t* rbase = lbase + (size_t)ni * (l_b + le_b);
       std::vector<SliceStackLJob> lj;
       std::vector<SliceTaskRJob> rj;
-      std::map<const double2*, int> bid;
+      PtrIndex bid;
       std::vector<const double2*> blks;
       auto block_index = [&](const double2* p) {
-        auto b = bid.find(p);
-        if (b == bid.end()) {
-          b = bid.emplace(p, (int)blks.size()).first;
-          blks.push_back(p);
-        }
-        return b->second;
+        const int b = bid.of(p);
+        if (b == (int)blks.size()) blks.push_back(p);
+        return b;
       };
-      std::map<std::vector<uintptr_t>, int> lid, rid;
+      KeyMap lid, rid;
       std::vector<uintptr_t> key;
       std::vector<SplitGemmInst> gi(ni);
       std::vector<double2*> outs((size_t)ni * SPLIT_TASK_NB, nullptr);

@@ -240,24 +240,36 @@ struct Staging {
 };
 static Staging g_stage[WS_COUNT];
 
-int upload(int slot, const void* host, size_t bytes, void** dev, cudaStream_t stream) {
-  if (g_cap) return capture_upload(host, bytes, dev);
+// The slot's staging buffer, free to be filled with `bytes`.
+static int stage_open(int slot, size_t bytes) {
   Staging& s = g_stage[slot];
   if (s.done) CTR_CUDA(cudaEventSynchronize(s.done));  // the previous upload from this buffer was consumed
   if (bytes > s.bytes) {
     if (s.host) CTR_CUDA(cudaFreeHost(s.host));
     s.host = nullptr;
+    s.bytes = 0;
     size_t nb = bytes < 4096 ? 4096 : bytes * 2;
     CTR_CUDA(cudaHostAlloc(&s.host, nb, cudaHostAllocMapped));
     CTR_CUDA(cudaHostGetDevicePointer(&s.host_dev, s.host, 0));
     s.bytes = nb;
   }
   if (!s.done) CTR_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
-  std::memcpy(s.host, host, bytes);
+  return CTR_OK;
+}
+
+static int stage_send(int slot, size_t bytes, void** dev, cudaStream_t stream) {
+  Staging& s = g_stage[slot];
   CTR_TRY(g_ws[slot].get(bytes, dev));
   CTR_TRY(launch_stage_copy(*dev, s.host_dev, bytes, stream));
   CTR_CUDA(cudaEventRecord(s.done, stream));
   return CTR_OK;
+}
+
+int upload(int slot, const void* host, size_t bytes, void** dev, cudaStream_t stream) {
+  if (g_cap) return capture_upload(host, bytes, dev);
+  CTR_TRY(stage_open(slot, bytes));
+  std::memcpy(g_stage[slot].host, host, bytes);
+  return stage_send(slot, bytes, dev, stream);
 }
 
 int upload_group(int slot, const std::vector<std::pair<const void*, size_t>>& parts, void** devs,
@@ -268,11 +280,20 @@ int upload_group(int slot, const std::vector<std::pair<const void*, size_t>>& pa
     off[i] = total;
     total += (parts[i].second + 255) & ~(size_t)255;
   }
-  std::vector<uint8_t> packed(std::max<size_t>(total, 1));
-  for (size_t i = 0; i < parts.size(); i++)
-    if (parts[i].second) std::memcpy(packed.data() + off[i], parts[i].first, parts[i].second);
+  auto pack = [&](uint8_t* to) {
+    for (size_t i = 0; i < parts.size(); i++)
+      if (parts[i].second) std::memcpy(to + off[i], parts[i].first, parts[i].second);
+  };
   void* d;
-  CTR_TRY(upload(slot, packed.data(), total, &d, stream));
+  if (g_cap) {
+    std::vector<uint8_t> packed(std::max<size_t>(total, 1));
+    pack(packed.data());
+    CTR_TRY(upload(slot, packed.data(), total, &d, stream));
+  } else {  // straight into the staging buffer
+    CTR_TRY(stage_open(slot, total));
+    pack((uint8_t*)g_stage[slot].host);
+    CTR_TRY(stage_send(slot, total, &d, stream));
+  }
   for (size_t i = 0; i < parts.size(); i++) devs[i] = (uint8_t*)d + off[i];
   return CTR_OK;
 }
