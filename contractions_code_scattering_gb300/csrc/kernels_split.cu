@@ -754,7 +754,7 @@ constexpr int NSTAGE = 3;
 constexpr uint32_t TMEM_COLS = 512;  // (re, im) x NL levels x BN columns fit in 512 for both configurations
 constexpr uint64_t WAIT_NS = 2000000000ull;  // 2 s per wait
 
-constexpr int GEMM_SMEM_TAIL = 1024;  // barriers, TMEM slot, column exponents and output pointers
+constexpr int GEMM_SMEM_TAIL = 2048;  // barriers, TMEM slot, column exponents and output pointers
 
 template <class C>
 constexpr size_t gemm_smem_bytes() {
@@ -811,6 +811,12 @@ template <class C>
 constexpr int tmem_groups() { return C::NL - 1; }
 __host__ __device__ constexpr int level_group(int l) { return l <= 1 ? 0 : l - 1; }
 
+// A descriptor moved on by `units` of 16 bytes: one 32-bit add, since the address
+// field cannot carry out of the low word (shared addresses are below 2^18).
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t units) {
+  return (desc & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)desc + units);
+}
+
 // The MMAs of one slice pair (i, j) of one K chunk into its level accumulator.
 // adesc / bdesc describe sub-tile (slice 0, re) of the stage; the other
 // sub-tiles are constant byte offsets (added as offset >> 4 to the
@@ -823,18 +829,18 @@ __device__ __forceinline__ void issue_pair(uint32_t tbase, uint64_t adesc, uint6
   constexpr int lvl = (I + J) < C::NL - 1 ? (I + J) : C::NL - 1;
   // in i-major order the first pair of level l is (0, l)
   const uint32_t accum = (!first_chunk || !(I == 0 && J <= C::NL - 1)) ? 1u : 0u;
-  const uint64_t ar = adesc + (uint64_t)(((I * 2 + 0) * C::A_SUB) >> 4);
-  const uint64_t ai = adesc + (uint64_t)(((I * 2 + 1) * C::A_SUB) >> 4);
+  const uint64_t ar = desc_at(adesc, ((I * 2 + 0) * C::A_SUB) >> 4);
+  const uint64_t ai = desc_at(adesc, ((I * 2 + 1) * C::A_SUB) >> 4);
   if constexpr (C::PACK) {
     // planes -Yi, Yr, Yi of slice j are adjacent along N (row groups 256 B apart)
-    const uint64_t b_nr = bdesc + (uint64_t)(((J * 3 + 0) * C::B_SUB) >> 4);  // [-Yi | Yr]
-    const uint64_t b_ri = bdesc + (uint64_t)(((J * 3 + 1) * C::B_SUB) >> 4);  // [Yr | Yi]
+    const uint64_t b_nr = desc_at(bdesc, ((J * 3 + 0) * C::B_SUB) >> 4);  // [-Yi | Yr]
+    const uint64_t b_ri = desc_at(bdesc, ((J * 3 + 1) * C::B_SUB) >> 4);  // [Yr | Yi]
     const uint32_t d = tbase + (uint32_t)C::acc_col(0, lvl);
     umma_f16(d, ar, b_ri, id_wide, accum);  // [Re | Im] += Xr [Yr | Yi]
     umma_f16(d, ai, b_nr, id_wide, 1u);     // [Re | Im] += Xi [-Yi | Yr]
   } else {
-    const uint64_t br = bdesc + (uint64_t)(((J * 2 + 0) * C::B_SUB) >> 4);
-    const uint64_t bi = bdesc + (uint64_t)(((J * 2 + 1) * C::B_SUB) >> 4);
+    const uint64_t br = desc_at(bdesc, ((J * 2 + 0) * C::B_SUB) >> 4);
+    const uint64_t bi = desc_at(bdesc, ((J * 2 + 1) * C::B_SUB) >> 4);
     const uint32_t dre = tbase + (uint32_t)C::acc_col(0, lvl);
     const uint32_t dim = tbase + (uint32_t)C::acc_col(1, lvl);
     umma_f16(dre, ar, br, id_pos, accum);  // Re += Xr Yr
@@ -925,13 +931,13 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   uint64_t* tempty = tfull + 1;  // one per hand-back group
   uint64_t* drainb = tempty + tmem_groups<C>();
   uint32_t* tslot = (uint32_t*)(drainb + 1);
-  int* sexp = (int*)(tslot + 4);  // C::BN column exponents of the current tile
-  // complex128 output: destination of row 0 of each column of the current tile
-  double2** colp = (double2**)(smem + NSTAGE * (C::A_STAGE + C::B_STAGE) + 512);
-  static_assert(512 + 8 * C::BN <= GEMM_SMEM_TAIL && 16 * 8 + 16 + 4 * C::BN <= 512, "GEMM shared-memory tail");
+  int* sexp = (int*)(tslot + 4);  // C::BN column exponents, of the even and of the odd tiles
+  // complex128 output: destination of row 0 of each column, of the even and of the odd tiles
+  double2** colp = (double2**)(smem + NSTAGE * (C::A_STAGE + C::B_STAGE) + 768);
+  static_assert(768 + 2 * 8 * 48 <= GEMM_SMEM_TAIL && 12 * 8 + 16 + 2 * 4 * C::BN <= 768, "GEMM shared-memory tail");
 
   volatile int* status = (volatile int*)(tslot + 1);  // block-uniform decisions
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; s++) {
@@ -954,7 +960,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = *tslot;
+  const uint32_t tbase = __shfl_sync(0xffffffffu, *tslot, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -980,85 +986,142 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t g_chunk = 0, local = 0;
-      bool ok = true;
-      const uint64_t adesc0 = sdesc_kmajor_noswz(smem_u32(sA), 128, 256);
-      const uint64_t bdesc0 = sdesc_kmajor_noswz(smem_u32(sB), 128, 256);
-      for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x, local++) {
-        for (int kc = 0; kc < g.nchunk; kc++, g_chunk++) {
-          const int s = g_chunk % NSTAGE;
-          if (!mbar_wait(&full[s], (g_chunk / NSTAGE) & 1, WAIT_NS, err)) {
-            atomicExch(err, 2);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t ad = adesc0 + (uint64_t)((s * C::A_STAGE) >> 4);
-          const uint64_t bd = bdesc0 + (uint64_t)((s * C::B_STAGE) >> 4);
-          if (kc == 0) {
-            // first chunk: each group of levels once the epilogue handed it back
-            for (int grp = 0; grp < tmem_groups<C>() && ok; grp++) {
-              if (local > 0 && !mbar_wait(&tempty[grp], (local - 1) & 1, 2 * WAIT_NS, err)) {
-                atomicExch(err, 4);
-                ok = false;
+    // The whole warp walks the tiles and waits; one elected lane issues.  Loop
+    // and descriptor arithmetic is then uniform over the warp and stays off the
+    // issuing thread's path.  With a single-lane branch around the whole loop and
+    // 64-bit descriptor adds an MMA of the complex128 form took 71 clocks in tiles
+    // of 7 K chunks and 63 in tiles of 25 (the pipe: 56), as the issuing thread
+    // shares its scheduler with four storing epilogue warps; 65 and 60 now.
+    uint32_t g_chunk = 0, local = 0;
+    bool ok = true;
+    const uint64_t adesc0 = sdesc_kmajor_noswz(smem_u32(sA), 128, 256);
+    const uint64_t bdesc0 = sdesc_kmajor_noswz(smem_u32(sB), 128, 256);
+    for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x, local++) {
+      for (int kc = 0; kc < g.nchunk; kc++, g_chunk++) {
+        const int s = g_chunk % NSTAGE;
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (g_chunk / NSTAGE) & 1, WAIT_NS, err));
+        if (!ok) {
+          if (lane == 0) atomicExch(err, 2);
+          break;
+        }
+        tc_fence_after();
+        const uint64_t ad = desc_at(adesc0, (s * C::A_STAGE) >> 4);
+        const uint64_t bd = desc_at(bdesc0, (s * C::B_STAGE) >> 4);
+        if (kc == 0) {
+          // first chunk: each group of levels once the epilogue handed it back
+          for (int grp = 0; grp < tmem_groups<C>(); grp++) {
+            if (local > 0) {
+              ok = __all_sync(0xffffffffu, mbar_wait(&tempty[grp], (local - 1) & 1, 2 * WAIT_NS, err));
+              if (!ok) {
+                if (lane == 0) atomicExch(err, 4);
                 break;
               }
-              tc_fence_after();
-              issue_group<C>(grp, tbase, ad, bd, true);
             }
-            if (!ok) break;
-          } else {
-            issue_chunk<C>(tbase, ad, bd, false);
+            tc_fence_after();
+            if (elect_one()) issue_group<C>(grp, tbase, ad, bd, true);
+            __syncwarp();
           }
-          umma_commit(&empty[s]);  // stage s free once these MMAs have read it
+          if (!ok) break;
+        } else {
+          if (elect_one()) issue_chunk<C>(tbase, ad, bd, false);
+          __syncwarp();
         }
-        if (ok) umma_commit(tfull);
+        if (elect_one()) umma_commit(&empty[s]);  // stage s free once these MMAs have read it
+        __syncwarp();
       }
-      // wait for every issued MMA before the accumulators are released
-      umma_commit(drainb);
-      if (!mbar_wait(drainb, 0, WAIT_NS)) atomicExch(err, 5);
+      if (ok && elect_one()) umma_commit(tfull);
+      __syncwarp();
     }
+    // wait for every issued MMA before the accumulators are released
+    if (elect_one()) umma_commit(drainb);
+    __syncwarp();
+    if (!mbar_wait(drainb, 0, WAIT_NS) && lane == 0) atomicExch(err, 5);
+    __syncwarp();
   } else {
     // epilogue: warp w drains TMEM lane quadrant w % 4; the EPI_WARPS / 4
-    // warps of a quadrant split the tile's columns between them
+    // warps of a quadrant split the tile between them.  Float-float output: a
+    // quarter of the columns each, a thread holds one row (column-major stores,
+    // 512 contiguous bytes a warp).  Complex128 output: half the rows and half the
+    // columns each, loaded as 16 x 256-bit fragments, in which 4 lanes hold 8
+    // consecutive columns of a row: a warp's 32-byte stores fill 8 whole 128-byte
+    // lines.  With a row a lane every store touched 32 lines, 16 bytes of each, and
+    // the stores of a tile took 12 400 clocks (7 K chunks of MMAs: 16 500); they take
+    // 7 200 now (Nev = 100).
     constexpr int EPH = C::EPI_WARPS / 4, CPW = C::BN / EPH;
     const int q = warp & 3, half = (warp - 2) / 4;
     const int et = threadIdx.x - 64;  // 0 .. 32 * EPI_WARPS - 1 within the epilogue group
-    const int row = q * 32 + lane;
-    const uint32_t tl = tbase + ((uint32_t)(q * 32) << 16);
+    const int row = C::INT_OUT ? q * 32 + (half & 1) * 16 + (lane >> 2) : q * 32 + lane;
+    const uint32_t tl = tbase + ((uint32_t)(q * 32 + (C::INT_OUT ? (half & 1) * 16 : 0)) << 16);
+    // Complex128 output: a tile's scale exponents and output pointers are fetched
+    // while the tile before it drains (the instance's pointers) and stores (what
+    // they point to), so that no tile waits for them (3 500 clocks before).  The
+    // float-float epilogue has no registers to spare for that: fetched ahead, its
+    // spills cost 4 % of the launch.
+    int nmt = 0, nnt = 0, mexp = 0, mrow0 = 0, mrow1 = 0;
+    double2* mptr = nullptr;
+    float4* nout = nullptr;
+    const int *nlexp = nullptr, *nrexp = nullptr;
+    double2* const* nouts = nullptr;
+    auto fetch_instance = [&](int tile) {
+      if (tile >= ntiles_total) return;
+      int inst;
+      tile_coords(g, tile, inst, nmt, nnt);
+      const SplitGemmInst* I = &g.inst[inst];
+      nlexp = I->lexp;
+      nrexp = I->rexp;
+      if constexpr (C::INT_OUT)
+        nouts = I->outs;
+      else
+        nout = I->out;
+    };
+    auto fetch_scales = [&](int tile) {
+      if (tile >= ntiles_total) return;
+      if (et < C::BN) {
+        const int gcol = nnt * C::BN + et;
+        mexp = nrexp[gcol];
+        if constexpr (C::INT_OUT) mptr = gcol < g.ncols ? nouts[gcol / g.blkn] + (gcol % g.blkn) : nullptr;
+      }
+      mrow0 = nlexp[nmt * SPLIT_M + row];
+      if constexpr (C::INT_OUT) mrow1 = nlexp[nmt * SPLIT_M + row + 8];
+    };
+    if constexpr (C::INT_OUT) {
+      fetch_instance(blockIdx.x);
+      fetch_scales(blockIdx.x);
+    }
     uint32_t local = 0;
     for (int tile = blockIdx.x; tile < ntiles_total; tile += gridDim.x, local++) {
-      int inst, mt, nt;
-      tile_coords(g, tile, inst, mt, nt);
-      const SplitGemmInst* I = &g.inst[inst];
-      // stage this tile's column exponents; the barrier also keeps the previous
-      // tile's values until every epilogue thread has used them
-      epi_bar<32 * C::EPI_WARPS>();
+      if constexpr (!C::INT_OUT) {
+        fetch_instance(tile);
+        fetch_scales(tile);
+      }
+      const int mt = nmt, nt = nnt, erow0 = mrow0, erow1 = mrow1;
+      float4* const out_ff = nout;
+      // this tile's half of the tables; the other half was last read before the
+      // previous tile's barrier
+      int* const sx = sexp + (local & 1) * C::BN;
+      double2** const cp = colp + (local & 1) * C::BN;
+      volatile int* const failed = status + 1 + (local & 1);
       if (et < C::BN) {
-        sexp[et] = I->rexp[nt * C::BN + et];
-        if constexpr (C::INT_OUT) {
-          const int gcol = nt * C::BN + et;
-          colp[et] = gcol < g.ncols ? I->outs[gcol / g.blkn] + (gcol % g.blkn) : nullptr;
-        }
+        sx[et] = mexp;
+        if constexpr (C::INT_OUT) cp[et] = mptr;
       }
       const int grow = mt * SPLIT_M + row;
       const bool rvalid = grow < g.mrows;
-      const int erow = I->lexp[grow];
       // one thread waits for the accumulators; the outcome is shared so that
       // all epilogue threads leave the loop together
       if (et == 0) {
         const bool done = mbar_wait(tfull, local & 1, 4 * WAIT_NS, err);
         if (!done) atomicExch(err, 3);
-        status[1] = done ? 0 : 1;
+        *failed = done ? 0 : 1;
       }
       epi_bar<32 * C::EPI_WARPS>();
-      if (status[1]) break;
+      if (*failed) break;
       tc_fence_after();
+      if constexpr (C::INT_OUT) fetch_instance(tile + gridDim.x);
       // Each warp drains its CPW columns into registers and hands TMEM back to
       // the MMA warp before it writes anything to global memory, so the next
       // tile's MMAs run while this tile's products are stored.
-      const int cbase = half * CPW;
+      const int cbase = C::INT_OUT ? (half >> 1) * 2 * CPW : half * CPW;
       // hand TMEM group grp back to the MMA warp (after this warp's loads of it)
       auto hand_back = [&](int grp) {
         tc_fence_before();
@@ -1082,12 +1145,13 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         };
         // (each group goes back as soon as its last load has landed, before
         // that load's values are folded in: the MMA warp waits on the loads only)
+        static_assert(!C::INT_OUT || (CPW == 12 && EPH == 4), "16 x 24 fragments of a warp");
         long long acc[2][CPW];
 #pragma unroll
         for (int part = 0; part < 2; part++) {  // group 0: levels 0 and 1
           float v0[CPW], v1[CPW];
-          tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, 0) + cbase), v0);
-          tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, 1) + cbase), v1);
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 0) + cbase), v0);
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 1) + cbase), v1);
           tmem_ld_wait();
           if (part == 1) hand_back(0);
 #pragma unroll
@@ -1098,21 +1162,30 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
 #pragma unroll
           for (int part = 0; part < 2; part++) {
             float v[CPW];
-            tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, l) + cbase), v);
+            tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, l) + cbase), v);
             tmem_ld_wait();
             if (part == 1) hand_back(l - 1);
 #pragma unroll
             for (int c = 0; c < CPW; c++) acc[part][c] += level_units(v[c], l);
           }
         }
-        if (rvalid) {
-          const int erow = I->lexp[grow];
+        fetch_scales(tile + gridDim.x);
 #pragma unroll
-          for (int c = 0; c < CPW; c++) {
-            double2* dst = colp[cbase + c];
-            if (!dst) continue;
-            const int e = erow + sexp[cbase + c] - 54;
-            dst[(size_t)grow * g.blkn] = make_double2(i2d_scaled(acc[0][c], e), i2d_scaled(acc[1][c], e));
+        for (int c = 0; c < CPW; c += 2) {
+          // two adjacent columns of row grow + 8 h
+          const int col = cbase + (c >> 2) * 8 + 2 * (lane & 3), h = (c >> 1) & 1;
+          if (grow + 8 * h >= g.mrows) continue;
+          double2 *p0 = cp[col], *p1 = cp[col + 1];
+          if (!p0) continue;
+          const int e0 = (h ? erow1 : erow0) + sx[col] - 54, e1 = (h ? erow1 : erow0) + sx[col + 1] - 54;
+          const double2 z0 = make_double2(i2d_scaled(acc[0][c], e0), i2d_scaled(acc[1][c], e0));
+          const double2 z1 = make_double2(i2d_scaled(acc[0][c + 1], e1), i2d_scaled(acc[1][c + 1], e1));
+          const size_t off = (size_t)(grow + 8 * h) * g.blkn;
+          if (p1 == p0 + 1 && ((uintptr_t)(p0 + off) & 31) == 0) {
+            st_global_v4f64(p0 + off, z0, z1);
+          } else {
+            p0[off] = z0;
+            if (p1) p1[off] = z1;
           }
         }
       } else {
@@ -1182,7 +1255,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
           }
         }
         if (rvalid && !g.levels) {
-          float4* outp = I->out;
+          float4* outp = out_ff;
 #pragma unroll
           for (int c = 0; c < CPW; c++) {
             const int gcol = nt * C::BN + cbase + c;
@@ -1191,7 +1264,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
             // scale stays well inside FP32's normal range; below 2^-100 the
             // product is written as NaN, which flags the entries that use it for
             // recomputation in FP64 range
-            const int ex = erow + sexp[cbase + c];
+            const int ex = erow0 + sx[cbase + c];
             const float sc = ex < FF_MIN_EXP ? __int_as_float(0x7fc00000) : pow2f(ex);
             outp[(size_t)gcol * ldo + grow] =
                 make_float4(s[0][c] * sc, e[0][c] * sc, s[1][c] * sc, e[1][c] * sc);

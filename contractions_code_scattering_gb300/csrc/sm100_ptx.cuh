@@ -111,6 +111,17 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
       : "memory");
 }
 
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 // Arrive on the mbarrier once every previously issued tcgen05.mma of this thread completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -152,6 +163,27 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
                : "memory");
 #pragma unroll
   for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 lanes x 256 bit (8 columns a step): v[4 s + 2 h + c] is row lane / 4 + 8 h, column
+// 8 s + 2 (lane % 4) + c of the 16 x 24 (16 x 8 S) elements at taddr.
+__device__ __forceinline__ void tmem_ld_16x24(uint32_t taddr, float* v) {
+  uint32_t r[12];
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11])
+               : "r"(taddr + 16)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 12; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 32-byte global store (p 32-byte aligned).
+__device__ __forceinline__ void st_global_v4f64(double2* p, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
