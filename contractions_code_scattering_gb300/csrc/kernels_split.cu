@@ -47,34 +47,34 @@ __device__ __forceinline__ int f64_exp_bound(double x) {
   return be == 0 ? -30000 : be - 1022;
 }
 
-// f64_fixed of x * (+-2^k) without the FP64 product: a power-of-two factor
-// only moves the exponent (and flips the sign when `flip`).  A product that
-// would leave the normal range (|x 2^k| < 2^-1022) gives 0, as the subnormal
-// FP64 product does in f64_fixed; the sign is the product's in every case.
-__device__ __forceinline__ uint64_t f64_fixed_pow2(double x, int k, bool flip, int E, bool& neg) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  neg = ((b >> 63) != 0) != flip;
-  const int be = (int)((b >> 52) & 0x7FF);
-  if (be == 0 || be + k <= 0) return 0;
-  const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-  const int sh = be + k - 1012 - E;
-  if (sh >= 0) return m << sh;
-  if (sh <= -64) return 0;
-  return m >> (-sh);
+// x >> t, 0 for t > 31 (as unsigned).
+__device__ __forceinline__ uint32_t shr_clamp(uint32_t x, uint32_t t) {
+  uint32_t r;
+  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(t));
+  return r;
 }
 
-// 63-bit fixed-point magnitude of x / 2^E (|x| < 2^E) and its sign.
-__device__ __forceinline__ uint64_t f64_fixed(double x, int E, bool& neg) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  neg = (b >> 63) != 0;
-  const int be = (int)((b >> 52) & 0x7FF);
-  if (be == 0) return 0;
-  const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-  const int sh = be - 1012 - E;  // <= 10 because |x| < 2^E
-  if (sh >= 0) return m << sh;
-  if (sh <= -64) return 0;
-  return m >> (-sh);
+// 63-bit fixed-point magnitude of x (+-2^k) / 2^E (|x 2^k| < 2^E) and its sign: a
+// power-of-two factor only moves the exponent (and flips the sign when `flip`).
+// A product that would leave the normal range (|x 2^k| < 2^-1022) gives 0; the sign
+// is the product's in every case.  The significand sits at the top of 64 bits and
+// moves right by t >= 1 in 32-bit shifts that clamp, without a case for the
+// direction or for an empty result: the slicers are bound by these integer
+// operations (the ALU pipe 75 % busy).  With 64-bit variable shifts, a sign per
+// digit and an index division per element, stacked left operands took 6.06 ms
+// and right ones 6.44 ms of a 19-set pi pi call (2 t_sink rows, Nev = 100); 5.12
+// and 5.85 ms now.
+__device__ __forceinline__ uint64_t f64_fixed_pow2(double x, int k, bool flip, int E, bool& neg) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  neg = ((int)hi < 0) != flip;
+  const int be = (int)((hi >> 20) & 0x7FF);
+  const uint32_t mh = __funnelshift_l(lo, (hi & 0xFFFFFu) | 0x100000u, 11), ml = lo << 11;
+  const uint32_t t = be <= max(0, -k) ? 64u : (uint32_t)(1023 + E - k - be);
+  const uint32_t rl = t < 32 ? __funnelshift_r(ml, mh, t) : shr_clamp(mh, t - 32);
+  return ((uint64_t)shr_clamp(mh, t) << 32) | rl;
 }
+
+__device__ __forceinline__ uint64_t f64_fixed(double x, int E, bool& neg) { return f64_fixed_pow2(x, 0, false, E, neg); }
 
 // Balanced digits of the magnitude U (63-bit fixed point, U < 2^63).  Digit s
 // sits at bit slice_shift(s) = 55 - 9s.  Adding 256 at every digit position
@@ -116,9 +116,11 @@ __device__ __forceinline__ __nv_bfloat16 slice_bf16(uint64_t W, int s, bool neg)
 // The value of slice_bf16 before its conversion to BF16 (exact in BF16).
 __device__ __forceinline__ float slice_f32(uint64_t W, int s, bool neg) { return __uint_as_float(slice_bits(W, s, neg)); }
 
-// Two slices of adjacent k as one packed BF16 pair (k in the low half).
+// Two slices of adjacent k as one packed BF16 pair (k in the low half), the signs
+// put on the pair.
 __device__ __forceinline__ uint32_t slice_pair(uint64_t W0, bool n0, uint64_t W1, bool n1, int s) {
-  return __byte_perm(slice_bits(W0, s, n0), slice_bits(W1, s, n1), 0x7632);
+  const uint32_t signs = (n0 ? 0x8000u : 0u) | (n1 ? 0x80000000u : 0u);
+  return __byte_perm(slice_bits(W0, s, false), slice_bits(W1, s, false), 0x7632) ^ signs;
 }
 
 // BF16 bits of -x for BF16 bits x (one value, or a packed pair).
@@ -478,15 +480,6 @@ __device__ __forceinline__ void weighted_fixed(double2 x, int wexp, bool wneg, b
   Ui = f64_fixed_pow2(x.y, wexp, wneg != dag, E, ni);
 }
 
-// Element (k, n) of a right task operand before its conjugation (applied as a
-// sign by the slicer).
-__device__ __forceinline__ double2 task_right_raw(const SliceTaskRJob& J, int nev, int k, int n) {
-  const int q = k / nev, i = k - q * nev, jb = n / nev, c = n - jb * nev;
-  if (q >= J.nterm || jb >= J.nb) return make_double2(0.0, 0.0);
-  const double2* B = J.b[jb][q];
-  return ((J.dag >> (4 * jb + q)) & 1) ? B[(size_t)c * nev + i] : B[(size_t)i * nev + c];
-}
-
 // Task-form slicing runs in two launches: the exponent bounds of every distinct
 // block of the launch (one read of each block), then one CTA per (operand tile,
 // K chunk), which combines the bounds of its operand's blocks into the row or
@@ -623,35 +616,48 @@ __global__ void __launch_bounds__(256) slice_stack_left_kernel(const SliceStackL
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[g] = E;
   }
+  // a thread's k pair is the same for its 4 rows: one division each for its two
+  // k's and its rows
   constexpr int PER = SPLIT_M * SPLIT_K / 2 / 256;
+  const int kp = threadIdx.x & 7;
+  int kq[2], kj[2];
+  bool kv[2], kdag[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int k = kc * SPLIT_K + 2 * kp + h;
+    kv[h] = k < K;
+    kq[h] = kv[h] ? k / nev : 0;
+    kj[h] = k - kq[h] * nev;
+    kdag[h] = (J.dag >> kq[h]) & 1;
+  }
   double2 v[PER][2];
 #pragma unroll
   for (int u = 0; u < PER; u++) {
-    const int e = threadIdx.x + u * 256;
-    const int rr = e >> 3, g = mt * SPLIT_M + rr;
+    const int g = mt * SPLIT_M + (threadIdx.x >> 3) + 32 * u, sl = g / nev, r = g - sl * nev;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int k = kc * SPLIT_K + 2 * (e & 7) + h;
       v[u][h] = make_double2(0.0, 0.0);
-      if (k < K && g < rows) {
-        const int sl = g / nev, r = g - sl * nev, q = k / nev, j = k - q * nev;
-        v[u][h] = ((J.dag >> q) & 1) ? J.a[sl][q][(size_t)j * nev + r] : J.a[sl][q][(size_t)r * nev + j];
-      }
+      if (kv[h] && g < rows) v[u][h] = J.a[sl][kq[h]][kdag[h] ? (size_t)kj[h] * nev + r : (size_t)r * nev + kj[h]];
     }
+  }
+  int wexp[2];
+  bool wneg[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    wexp[h] = J.wexp[kq[h]];
+    wneg[h] = J.w[kq[h]] < 0.f;
   }
   __syncthreads();
   uint8_t* d0 = J.out + ((size_t)mt * nchunk + kc) * C::A_STAGE;
 #pragma unroll
   for (int u = 0; u < PER; u++) {
-    const int e = threadIdx.x + u * 256;
-    const int rr = e >> 3, kp = e & 7;
+    const int rr = (threadIdx.x >> 3) + 32 * u;
     const int E = sexp[rr];
     uint64_t Ur[2], Ui[2];
     bool nr[2], ni[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int q = min((kc * SPLIT_K + 2 * kp + h) / nev, J.nterm - 1);
-      weighted_fixed(v[u][h], J.wexp[q], J.w[q] < 0.f, (J.dag >> q) & 1, E, Ur[h], nr[h], Ui[h], ni[h]);
+      weighted_fixed(v[u][h], wexp[h], wneg[h], kdag[h], E, Ur[h], nr[h], Ui[h], ni[h]);
       Ur[h] = round_fixed<C::NS>(Ur[h]);
       Ui[h] = round_fixed<C::NS>(Ui[h]);
     }
@@ -693,33 +699,45 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[n] = E;  // exps sized ntiles * BN (padding columns get 0)
   }
+  // a thread's k pair is the same for its columns (as in slice_stack_left)
   constexpr int PER = C::BN * SPLIT_K / 2 / 128;
   static_assert(C::BN * SPLIT_K / 2 % 128 == 0, "column pairs a thread");
+  const int kp = threadIdx.x & 7;
+  int kq[2], kj[2];
+  bool kv[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int k = kc * SPLIT_K + 2 * kp + h;
+    kv[h] = k < K;
+    kq[h] = kv[h] ? k / nev : 0;
+    kj[h] = k - kq[h] * nev;
+  }
   double2 v[PER][2];
+  bool dag[PER][2];
 #pragma unroll
   for (int u = 0; u < PER; u++) {
-    const int e = threadIdx.x + u * 128;
-    const int n = nt * C::BN + (e >> 3);
+    const int n = nt * C::BN + (threadIdx.x >> 3) + 16 * u, jb = n / nev, c = n - jb * nev;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int k = kc * SPLIT_K + 2 * (e & 7) + h;
-      v[u][h] = (n < ncols && k < K) ? task_right_raw(J, nev, k, n) : make_double2(0.0, 0.0);
+      v[u][h] = make_double2(0.0, 0.0);
+      dag[u][h] = false;
+      if (kv[h] && n < ncols) {
+        dag[u][h] = (J.dag >> (4 * jb + kq[h])) & 1;
+        v[u][h] = J.b[jb][kq[h]][dag[u][h] ? (size_t)c * nev + kj[h] : (size_t)kj[h] * nev + c];
+      }
     }
   }
   __syncthreads();
   uint8_t* d0 = J.out + ((size_t)nt * nchunk + kc) * C::B_STAGE;
 #pragma unroll
   for (int u = 0; u < PER; u++) {
-    const int e = threadIdx.x + u * 128;
-    const int nn = e >> 3, kp = e & 7, n = nt * C::BN + nn;
-    const int jb = min(n / nev, J.nb - 1);
+    const int nn = (threadIdx.x >> 3) + 16 * u;
     const int E = sexp[nn];
     uint64_t Ur[2], Ui[2];
     bool nr[2], ni[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int q = min((kc * SPLIT_K + 2 * kp + h) / nev, J.nterm - 1);
-      weighted_fixed(v[u][h], 0, false, (J.dag >> (4 * jb + q)) & 1, E, Ur[h], nr[h], Ui[h], ni[h]);
+      weighted_fixed(v[u][h], 0, false, dag[u][h], E, Ur[h], nr[h], Ui[h], ni[h]);
       Ur[h] = round_fixed<C::NS>(Ur[h]);
       Ui[h] = round_fixed<C::NS>(Ui[h]);
     }
