@@ -354,15 +354,20 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
 // FP64 pipe is the bound: summing the four spin blocks first takes 6 adds + 4
 // FMAs an element where four traces take 16 FMAs (10.7 against 17 us of the pipe
 // at Nev = 100, Lt = 64).  One cluster of up to 8 CTAs a time slice, each over a
-// range of the Nev^2 elements; CTA 0 adds the CTAs' partial sums in rank order
-// through distributed shared memory, so there is one launch, no table to upload
-// and a fixed summation order.
+// range of the Nev^2 elements, which write their partial sums into CTA 0's shared
+// memory; CTA 0 adds them in rank order.  One launch, no table to upload and a
+// fixed summation order.  (Two plain launches take 20.5 us a call at Nev = 100,
+// Lt = 64, but 17.5 against 15 us where the call is bound by the host.)
 constexpr int LOOP_TPB = 256;
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __global__ void __launch_bounds__(LOOP_TPB) loop_unity_kernel(const double2* __restrict__ diag,
                                                               const double2* __restrict__ mom, int N, int ncta,
                                                               double2* __restrict__ loop) {
-  __shared__ double part[2];
+  __shared__ double part[16];  // in CTA 0: the CTAs' partial sums
+  if (ncta > 1) cluster_arrive();
   const int t = blockIdx.x / ncta, rank = blockIdx.x - t * ncta;
   const unsigned n2 = (unsigned)N * N;  // Nev <= 4096
   const double2* T = diag + (size_t)t * 16 * n2;
@@ -389,19 +394,25 @@ __global__ void __launch_bounds__(LOOP_TPB) loop_unity_kernel(const double2* __r
     }
   }
   const double sum = block_sum2<LOOP_TPB>(re, im);
-  if (threadIdx.x < 2) part[threadIdx.x] = sum;
   if (ncta == 1) {
-    if (threadIdx.x < 2) ((double*)(loop + t))[threadIdx.x] = part[threadIdx.x];
+    if (threadIdx.x < 2) ((double*)(loop + t))[threadIdx.x] = sum;
     return;
   }
-  auto cl = cooperative_groups::this_cluster();
-  cl.sync();
-  if (rank == 0 && threadIdx.x < 2) {
+  if (threadIdx.x >= 32) {  // the other warps only count in the cluster's barriers
+    cluster_wait();
+    cluster_arrive();
+    return;
+  }
+  cluster_wait();  // every CTA of the cluster runs
+  if (threadIdx.x < 2) cooperative_groups::this_cluster().map_shared_rank(part, 0)[2 * rank + threadIdx.x] = sum;
+  cluster_arrive();
+  if (rank) return;
+  cluster_wait();
+  if (threadIdx.x < 2) {
     double v = part[threadIdx.x];
-    for (int r = 1; r < ncta; r++) v += cl.map_shared_rank(part, r)[threadIdx.x];
+    for (int r = 1; r < ncta; r++) v += part[2 * r + threadIdx.x];
     ((double*)(loop + t))[threadIdx.x] = v;
   }
-  cl.sync();  // the other CTAs' partial sums stay in place until they are read
 }
 
 // ------------------------------------------------------------- row sums
@@ -596,15 +607,17 @@ int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, do
   int dev = 0, nsm = 0;
   CTR_CUDA(cudaGetDevice(&dev));
   CTR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  // CTAs a time slice (at most 8, the portable cluster size, and no less than a
-  // CTA's worth of elements each): the split whose most loaded SM has the least
-  // work, ceil(Nt c / SMs) / c, the smaller one of equals.  At Lt = 64 that is 7
-  // (448 CTAs, at most 3 an SM); 8 would put 4 on some.
+  // CTAs a time slice, a CTA's worth of elements each at least: the split whose most
+  // loaded SM has the least work, ceil(Nt c / SMs) / c.  Among equals up to 4 the
+  // larger (more warps an SM); 8 only where it is better.  Clusters of 5 to 8 pack
+  // unevenly into the GPCs: at Nev = 100, Lt = 64, 1 to 8 CTAs take 51, 32, 27, 21.9,
+  // 27, 22.5, 24.6 and 22.6 us, at Lt = 96 three take 26.7, four 28.8, eight 30.7.
   int best = 1;
-  const long long most = std::min<long long>(8, ((long long)N * N + LOOP_TPB - 1) / LOOP_TPB);
-  for (int c = 2; c <= most; c++) {
+  const long long most = ((long long)N * N + LOOP_TPB - 1) / LOOP_TPB;
+  for (int c : {2, 3, 4, 8}) {
+    if (c > most) break;
     const long long a = ((long long)Nt * c + nsm - 1) / nsm * best, b = ((long long)Nt * best + nsm - 1) / nsm * c;
-    if (a < b) best = c;
+    if (a < b || (a == b && c <= 4)) best = c;
   }
   TimedLaunch tl(s, "loop_unity");
   cudaLaunchConfig_t cfg = {};
