@@ -92,12 +92,9 @@ enum {
   WS_REFINE,        // refinement list / patches of the split engine
   WS_SPLITTASK,     // sliced operands of split-engine task stages
   WS_SPLITJOBS,     // their job / instance / pointer tables
-  WS_SPLITJOBS2,
   WS_SPLITJOBS3,
   WS_RPHI,          // per-time-slice products of a recomputation call
-  WS_SPLITJOBS4,    // distinct blocks of a task launch
   WS_BLOCKEXP,      // their row / column exponent bounds
-  WS_TRACEGROUPS,   // grouped closing traces of a two-sided call
   WS_GRAM,          // sliced operands and partial products of Gram traces
   WS_GRAMJOBS,      // their block, instance and pointer tables
   WS_GRAMTRACES,    // their trace lists
@@ -224,6 +221,19 @@ int upload(int slot, const void* host, size_t bytes, void** dev, cudaStream_t st
 // device address of parts[i] (256-byte aligned inside the slot).
 int upload_group(int slot, const std::vector<std::pair<const void*, size_t>>& parts, void** devs,
                  cudaStream_t stream);
+// One upload of `bytes` whose host contents are written by fill(host, dev), which is
+// given their device address (tables that point into one another).
+int upload_build(int slot, size_t bytes, const std::function<void(uint8_t*, uint8_t*)>& fill, void** dev,
+                 cudaStream_t stream);
+// Parts of one upload_build: reserve the sizes, then place the parts.
+struct UploadParts {
+  size_t total = 0;
+  size_t reserve(size_t bytes) {
+    const size_t o = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return o;
+  }
+};
 // dst (device) <- src (device-accessible, e.g. mapped pinned host memory), by a kernel.
 int launch_stage_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 // dst <- src for any alignment (a kernel; dst may be mapped pinned host memory).

@@ -581,6 +581,10 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
         }
       }
     }
+    // the block products run while the host lists the traces
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(run_grids(c, g1, WS_TASKS2));
+    CTR_TRY(run_grids(c, g2, WS_GEMM_A));
     // traces: values (and error scales) after the products in the same buffer
     const size_t ntr = (size_t)np * tr_pair;
     double2* trv = base + used;
@@ -621,9 +625,6 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       tp.tt[k].out = trv + k;
       if (tra) tp.tt[k].absout = tra + k;
     }
-    CTR_TRY(run_grids(c, g0, WS_TASKS));
-    CTR_TRY(run_grids(c, g1, WS_TASKS2));
-    CTR_TRY(run_grids(c, g2, WS_GEMM_A));
     CTR_TRY(run_traces(c, tp.tt));
     void* d[2];
     CTR_TRY(upload_group(WS_MISC, {{slots.data(), slots.size() * sizeof(int)}, {ent.data(), ent.size() * sizeof(int)}},
@@ -1087,6 +1088,8 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
         g1.push_back(std::move(gh));
       }
     }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(run_grids(c, g1, WS_TASKS2));
     GramRows gr;
     size_t maxm = 0;
     for (auto& v : pb.by_ti) maxm = std::max(maxm, v.size());
@@ -1133,8 +1136,6 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
           r.ent.push_back((d < nd ? k * nd + d : k) * npairs + pb.ent[i]);
         }
     }
-    CTR_TRY(run_grids(c, g0, WS_TASKS));
-    CTR_TRY(run_grids(c, g1, WS_TASKS2));
     CTR_TRY(gram_rows(N, gr, trv, tra, c.s));
     std::vector<RowItems*> items;
     for (RowItems& r : it) items.push_back(&r);
@@ -1199,6 +1200,7 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
         }
         g0.push_back(std::move(gz));
       }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));  // while the host lists the traces
     // traces
     const size_t ntr = (size_t)np * tr_pair;
     double2* trv = base + used;
@@ -1274,7 +1276,6 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
       tp.tt[k].out = trv + k;
       if (tra) tp.tt[k].absout = tra + k;
     }
-    CTR_TRY(run_grids(c, g0, WS_TASKS));
     if (gram) {
       // 0: the FP64 trace kernel, 1: Gram products on the tensor cores
       int form = 1;

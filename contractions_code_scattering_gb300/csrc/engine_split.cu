@@ -247,28 +247,23 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
     p += align256((size_t)Nt * F.mtiles * SPLIT_M * 4);
     F.rexp = (int*)p;
   }
+  std::vector<SliceLeftJob> phi_lj(Nt);
+  std::vector<SliceRightJob> phi_rj(Nt);
   {
-    std::vector<SliceLeftJob> lj(Nt);
-    std::vector<SliceRightJob> rj(Nt);
     for (int t = 0; t < Nt; t++) {
-      SliceLeftJob& L = lj[t];
+      SliceLeftJob& L = phi_lj[t];
       std::memset(&L, 0, sizeof(L));
       for (int k = 0; k < nR; k++) L.blk[k] = ph + ((size_t)t * nphi + Rl[k]) * N2;
       L.rows = nR * N;
       L.out = F.left + (size_t)t * F.mtiles * nchunk * SPLIT_A_STAGE;
       L.exps = F.lexp + (size_t)t * F.mtiles * SPLIT_M;
-      SliceRightJob& R = rj[t];
+      SliceRightJob& R = phi_rj[t];
       std::memset(&R, 0, sizeof(R));
       for (int k = 0; k < nL; k++) R.blk[k] = ph + ((size_t)t * nphi + Ll[k]) * N2;
       R.cols = nL * N;
       R.out = F.right + (size_t)t * F.ntiles * nchunk * SPLIT_B_STAGE;
       R.exps = F.rexp + (size_t)t * F.ntiles * SPLIT_N;
     }
-    void *dl, *dr;
-    CTR_TRY(upload(WS_TASKS, lj.data(), lj.size() * sizeof(SliceLeftJob), &dl, stream));
-    CTR_TRY(launch_slice_left((const SliceLeftJob*)dl, Nt, N, nchunk, F.mtiles, stream, 1));
-    CTR_TRY(upload(WS_TASKS2, rj.data(), rj.size() * sizeof(SliceRightJob), &dr, stream));
-    CTR_TRY(launch_slice_right((const SliceRightJob*)dr, Nt, N, nchunk, F.ntiles, stream, 1));
   }
 
   // ---- per (t_sink, t_src) pair buffers
@@ -294,8 +289,6 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
   }
   std::vector<int> csr(off);
   csr.insert(csr.end(), ord.begin(), ord.end());
-  void* d_csr;
-  CTR_TRY(upload(WS_MISC, csr.data(), csr.size() * sizeof(int), &d_csr, stream));
   // refinement list: one slot per output entry of the call, plus the counter
   void* d_ref;
   const size_t nentries = (size_t)npairs_total * nout;
@@ -329,11 +322,20 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
   build_trace_groups(trow.data(), ntr, 2, 2, 4, tquads);
   tgroups.insert(tgroups.end(), tquads.begin(), tquads.end());
   const int ngroups = (int)(tgroups.size() - tquads.size()), nquads = (int)tquads.size();
-  void *d_trow, *d_tix, *d_rcoef, *d_tgroups;
-  CTR_TRY(upload(WS_SPLITJOBS, trow.data(), trow.size() * sizeof(TraceRow), &d_trow, stream));
-  CTR_TRY(upload(WS_TRACEGROUPS, tgroups.data(), tgroups.size() * sizeof(TraceGroup), &d_tgroups, stream));
-  CTR_TRY(upload(WS_SPLITJOBS2, tix.data(), tix.size() * sizeof(int), &d_tix, stream));
-  CTR_TRY(upload(WS_SPLITJOBS3, coef.data(), coef.size() * sizeof(float), &d_rcoef, stream));
+  // every table of the call in one staging copy (a small call is bound by its launches)
+  void* dc[7];
+  CTR_TRY(upload_group(WS_MISC,
+                       {{phi_lj.data(), phi_lj.size() * sizeof(SliceLeftJob)},
+                        {phi_rj.data(), phi_rj.size() * sizeof(SliceRightJob)},
+                        {csr.data(), csr.size() * sizeof(int)},
+                        {trow.data(), trow.size() * sizeof(TraceRow)},
+                        {tgroups.data(), tgroups.size() * sizeof(TraceGroup)},
+                        {tix.data(), tix.size() * sizeof(int)},
+                        {coef.data(), coef.size() * sizeof(float)}},
+                       dc, stream));
+  void *d_csr = dc[2], *d_trow = dc[3], *d_tgroups = dc[4], *d_tix = dc[5], *d_rcoef = dc[6];
+  CTR_TRY(launch_slice_left((const SliceLeftJob*)dc[0], Nt, N, nchunk, F.mtiles, stream, 1));
+  CTR_TRY(launch_slice_right((const SliceRightJob*)dc[1], Nt, N, nchunk, F.ntiles, stream, 1));
 
   std::vector<SliceLeftJob> lj;
   std::vector<SliceRightJob> rj;
@@ -386,14 +388,16 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
       abase[q] = A;
       bbase[q] = B;
     }
-    void* d4[4];
+    void* d5[5];
+    abase.insert(abase.end(), bbase.begin(), bbase.end());
     CTR_TRY(upload_group(WS_TASKS,
                          {{lj.data(), lj.size() * sizeof(SliceLeftJob)},
                           {rj.data(), rj.size() * sizeof(SliceRightJob)},
                           {ga.data(), ga.size() * sizeof(SplitGemmInst)},
-                          {gb.data(), gb.size() * sizeof(SplitGemmInst)}},
-                         d4, stream));
-    void *d_lj = d4[0], *d_rj = d4[1], *d_ga = d4[2], *d_gb = d4[3], *d_tt;
+                          {gb.data(), gb.size() * sizeof(SplitGemmInst)},
+                          {abase.data(), abase.size() * sizeof(const float4*)}},
+                         d5, stream));
+    void *d_lj = d5[0], *d_rj = d5[1], *d_ga = d5[2], *d_gb = d5[3], *d_tt = d5[4];
     // slicer form (autotuned; all three write the same bytes, so candidates re-run)
     auto slice_tau = [&](int form) {
       CTR_TRY(launch_slice_left((const SliceLeftJob*)d_lj, np, N, nchunk, mtT, stream, form));
@@ -419,8 +423,6 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
       G->order = order;
       CTR_TRY(launch_split_gemm(*G, np, d_err, stream));
     }
-    abase.insert(abase.end(), bbase.begin(), bbase.end());
-    CTR_TRY(upload(WS_ROWTASKS, abase.data(), abase.size() * sizeof(const float4*), &d_tt, stream));
     // candidates: the TRACE_VARIANTS per-trace kernels, the grouped one, then
     // the two quad-group kernels
     auto traces = [&](int variant) {
@@ -698,6 +700,37 @@ extern "C" int ctr_split_levels(int nev, const double* x, const double* y, float
 
 namespace ctr {
 
+// The tables of one task or grid launch: left and right jobs, output pointer lists
+// (SPLIT_TASK_NB an instance), distinct blocks, and the instances, whose outs point
+// into the uploaded lists.
+template <class LeftJob>
+static int upload_stage(const std::vector<LeftJob>& lj, const std::vector<SliceTaskRJob>& rj,
+                        const std::vector<double2*>& outs, const std::vector<const double2*>& blks,
+                        std::vector<SplitGemmInst>& gi, void** d_lj, void** d_rj, void** d_blk, void** d_gi,
+                        cudaStream_t stream) {
+  UploadParts up;
+  const size_t ol = up.reserve(lj.size() * sizeof(LeftJob)), orr = up.reserve(rj.size() * sizeof(SliceTaskRJob)),
+               oo = up.reserve(outs.size() * sizeof(double2*)), ob = up.reserve(blks.size() * sizeof(const double2*)),
+               og = up.reserve(gi.size() * sizeof(SplitGemmInst));
+  void* d;
+  CTR_TRY(upload_build(WS_SPLITJOBS, up.total,
+                       [&](uint8_t* to, uint8_t* dev) {
+                         for (size_t i = 0; i < gi.size(); i++)
+                           gi[i].outs = (double2* const*)(dev + oo) + i * SPLIT_TASK_NB;
+                         std::memcpy(to + ol, lj.data(), lj.size() * sizeof(LeftJob));
+                         std::memcpy(to + orr, rj.data(), rj.size() * sizeof(SliceTaskRJob));
+                         std::memcpy(to + oo, outs.data(), outs.size() * sizeof(double2*));
+                         std::memcpy(to + ob, blks.data(), blks.size() * sizeof(const double2*));
+                         std::memcpy(to + og, gi.data(), gi.size() * sizeof(SplitGemmInst));
+                       },
+                       &d, stream));
+  *d_lj = (uint8_t*)d + ol;
+  *d_rj = (uint8_t*)d + orr;
+  *d_blk = (uint8_t*)d + ob;
+  *d_gi = (uint8_t*)d + og;
+  return CTR_OK;
+}
+
 // Split-engine execution of a stage of FP64-engine GEMM tasks, on the
 // high-precision configuration (6 slices, 5 levels, tiles of 128 x 48).  Tasks
 // with the same left side (A pointers, transposes, weights) share one sliced
@@ -836,18 +869,9 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
         const SliceTaskRJob& Ru = rj[it->second];
         gi[i] = SplitGemmInst{L.out, Ru.out, L.exps, Ru.exps, nullptr, nullptr};
       }
-      // the launch's tables in two staging copies (the instances need the
-      // device address of their output pointer lists)
-      void* d1[4];
-      CTR_TRY(upload_group(WS_SPLITJOBS,
-                           {{lj.data(), lj.size() * sizeof(SliceTaskLJob)},
-                            {rj.data(), rj.size() * sizeof(SliceTaskRJob)},
-                            {outs.data(), outs.size() * sizeof(double2*)},
-                            {blks.data(), blks.size() * sizeof(const double2*)}},
-                           d1, stream));
-      void *d_lj = d1[0], *d_rj = d1[1], *d_outs = d1[2], *d_blk = d1[3], *d_gi;
-      for (int i = 0; i < ni; i++) gi[i].outs = (double2* const*)d_outs + (size_t)i * SPLIT_TASK_NB;
-      CTR_TRY(upload(WS_GEMM_B, gi.data(), gi.size() * sizeof(SplitGemmInst), &d_gi, stream));
+      // the launch's tables in one staging copy (the instances point at their output lists)
+      void *d_lj, *d_rj, *d_blk, *d_gi;
+      CTR_TRY(upload_stage(lj, rj, outs, blks, gi, &d_lj, &d_rj, &d_blk, &d_gi, stream));
       // exponent bounds of every distinct block once, then the slices
       void* d_bexp;
       CTR_TRY(workspace(WS_BLOCKEXP).get(blks.size() * 2 * N * sizeof(int), &d_bexp));
@@ -994,22 +1018,14 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
         for (int j = 0; j < nb; j++) outs[(size_t)i * SPLIT_TASK_NB + j] = G.C0[j] + (size_t)pc.s0 * N2;
         gi[i] = SplitGemmInst{L.out, rj[it->second].out, L.exps, rj[it->second].exps, nullptr, nullptr};
       }
-      void* d1[4];
-      CTR_TRY(upload_group(WS_SPLITJOBS,
-                           {{lj.data(), lj.size() * sizeof(SliceStackLJob)},
-                            {rj.data(), rj.size() * sizeof(SliceTaskRJob)},
-                            {outs.data(), outs.size() * sizeof(double2*)},
-                            {blks.data(), blks.size() * sizeof(const double2*)}},
-                           d1, stream));
-      for (int i = 0; i < ni; i++) gi[i].outs = (double2* const*)d1[2] + (size_t)i * SPLIT_TASK_NB;
-      void* d_gi;
-      CTR_TRY(upload(WS_GEMM_B, gi.data(), gi.size() * sizeof(SplitGemmInst), &d_gi, stream));
+      void *d_lj, *d_rj, *d_blk, *d_gi;
+      CTR_TRY(upload_stage(lj, rj, outs, blks, gi, &d_lj, &d_rj, &d_blk, &d_gi, stream));
       void* d_bexp;
       CTR_TRY(workspace(WS_BLOCKEXP).get(blks.size() * 2 * N * sizeof(int), &d_bexp));
-      CTR_TRY(launch_block_exp((const double2* const*)d1[3], (int)blks.size(), N, (int*)d_bexp, stream));
-      CTR_TRY(launch_slice_stack_left((const SliceStackLJob*)d1[0], (int)lj.size(), N, nchunk, mtiles,
+      CTR_TRY(launch_block_exp((const double2* const*)d_blk, (int)blks.size(), N, (int*)d_bexp, stream));
+      CTR_TRY(launch_slice_stack_left((const SliceStackLJob*)d_lj, (int)lj.size(), N, nchunk, mtiles,
                                       (const int*)d_bexp, stream));
-      CTR_TRY(launch_slice_task_right((const SliceTaskRJob*)d1[1], (int)rj.size(), N, nchunk, ntiles,
+      CTR_TRY(launch_slice_task_right((const SliceTaskRJob*)d_rj, (int)rj.size(), N, nchunk, ntiles,
                                       (const int*)d_bexp, stream));
       SplitGemmBatch B{(const SplitGemmInst*)d_gi, mtiles, ntiles, nchunk, ns * N, nb * N, mtiles * SPLIT_M,
                        nullptr, 1, N, 1};

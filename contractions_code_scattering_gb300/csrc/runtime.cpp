@@ -104,7 +104,8 @@ static int capture_workspace(int slot, size_t need, void** out) {
   return CTR_OK;
 }
 
-static int capture_upload(const void* host, size_t bytes, void** dev) {
+// Space for a table in the recording's arena, and its one-time copy.
+static int capture_reserve(size_t bytes, void** dev) {
   ctr_graph& g = *g_cap;
   const size_t nb = (bytes + 255) & ~(size_t)255;
   if (g.arena_used + nb > g.arena_cap) {
@@ -115,19 +116,27 @@ static int capture_upload(const void* host, size_t bytes, void** dev) {
     g.arena_used = 0;
     g.arena_cap = cap;
   }
-  void* dst = g.arena + g.arena_used;
+  *dev = g.arena + g.arena_used;
   g.arena_used += nb;
-  if (bytes) {
-    RelaxedCapture rc;
-    cudaError_t e = cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, g.setup);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g.setup);
-    if (e != cudaSuccess) {
-      g.error = CTR_ERR_CUDA;
-      return cuda_fail(e, "table copy while recording", __FILE__, __LINE__);
-    }
-  }
-  *dev = dst;
   return CTR_OK;
+}
+
+static int capture_copy(void* dev, const void* host, size_t bytes) {
+  ctr_graph& g = *g_cap;
+  if (!bytes) return CTR_OK;
+  RelaxedCapture rc;
+  cudaError_t e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, g.setup);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g.setup);
+  if (e != cudaSuccess) {
+    g.error = CTR_ERR_CUDA;
+    return cuda_fail(e, "table copy while recording", __FILE__, __LINE__);
+  }
+  return CTR_OK;
+}
+
+static int capture_upload(const void* host, size_t bytes, void** dev) {
+  CTR_TRY(capture_reserve(bytes, dev));
+  return capture_copy(*dev, host, bytes);
 }
 
 static int close_segment(ctr_graph& g) {
@@ -257,43 +266,44 @@ static int stage_open(int slot, size_t bytes) {
   return CTR_OK;
 }
 
-static int stage_send(int slot, size_t bytes, void** dev, cudaStream_t stream) {
+static int stage_send(int slot, size_t bytes, void* dev, cudaStream_t stream) {
   Staging& s = g_stage[slot];
-  CTR_TRY(g_ws[slot].get(bytes, dev));
-  CTR_TRY(launch_stage_copy(*dev, s.host_dev, bytes, stream));
+  CTR_TRY(launch_stage_copy(dev, s.host_dev, bytes, stream));
   CTR_CUDA(cudaEventRecord(s.done, stream));
   return CTR_OK;
 }
 
 int upload(int slot, const void* host, size_t bytes, void** dev, cudaStream_t stream) {
   if (g_cap) return capture_upload(host, bytes, dev);
+  return upload_build(slot, bytes, [&](uint8_t* to, uint8_t*) { std::memcpy(to, host, bytes); }, dev, stream);
+}
+
+int upload_build(int slot, size_t bytes, const std::function<void(uint8_t*, uint8_t*)>& fill, void** dev,
+                 cudaStream_t stream) {
+  if (g_cap) {
+    std::vector<uint8_t> packed(std::max<size_t>(bytes, 1));
+    CTR_TRY(capture_reserve(bytes, dev));
+    fill(packed.data(), (uint8_t*)*dev);
+    return capture_copy(*dev, packed.data(), bytes);
+  }
   CTR_TRY(stage_open(slot, bytes));
-  std::memcpy(g_stage[slot].host, host, bytes);
-  return stage_send(slot, bytes, dev, stream);
+  CTR_TRY(g_ws[slot].get(bytes, dev));
+  fill((uint8_t*)g_stage[slot].host, (uint8_t*)*dev);
+  return stage_send(slot, bytes, *dev, stream);
 }
 
 int upload_group(int slot, const std::vector<std::pair<const void*, size_t>>& parts, void** devs,
                  cudaStream_t stream) {
-  std::vector<size_t> off(parts.size());
-  size_t total = 0;
-  for (size_t i = 0; i < parts.size(); i++) {
-    off[i] = total;
-    total += (parts[i].second + 255) & ~(size_t)255;
-  }
-  auto pack = [&](uint8_t* to) {
-    for (size_t i = 0; i < parts.size(); i++)
-      if (parts[i].second) std::memcpy(to + off[i], parts[i].first, parts[i].second);
-  };
+  UploadParts up;
+  std::vector<size_t> off;
+  for (auto& p : parts) off.push_back(up.reserve(p.second));
   void* d;
-  if (g_cap) {
-    std::vector<uint8_t> packed(std::max<size_t>(total, 1));
-    pack(packed.data());
-    CTR_TRY(upload(slot, packed.data(), total, &d, stream));
-  } else {  // straight into the staging buffer
-    CTR_TRY(stage_open(slot, total));
-    pack((uint8_t*)g_stage[slot].host);
-    CTR_TRY(stage_send(slot, total, &d, stream));
-  }
+  CTR_TRY(upload_build(slot, up.total,
+                       [&](uint8_t* to, uint8_t*) {
+                         for (size_t i = 0; i < parts.size(); i++)
+                           if (parts[i].second) std::memcpy(to + off[i], parts[i].first, parts[i].second);
+                       },
+                       &d, stream));
   for (size_t i = 0; i < parts.size(); i++) devs[i] = (uint8_t*)d + off[i];
   return CTR_OK;
 }
