@@ -2354,8 +2354,10 @@ int launch_trace_quads(const TraceGroup* d_groups, int ngroups, const TraceRow* 
 }
 
 // Covers the traces of one component by quads (2 A and 2 B blocks at most): for
-// each A block in turn, while it has traces left, the other A block with the most
-// B blocks in common (two are enough), and two B blocks, common ones first.
+// each A block in turn, while it has traces left, another A block with two B blocks
+// in common (one, where none has two), and two B blocks, common ones first.  Looked
+// for among the A blocks of its own B blocks: a sparse table of 512 + 512 blocks
+// costs its traces, not all pairs of its blocks.
 static void cover_quads(const TraceRow* rows, const std::vector<int>& comp, const std::function<void(int)>& add,
                         const std::function<void()>& flush) {
   std::map<int, int> ia, ib;
@@ -2365,16 +2367,18 @@ static void cover_quads(const TraceRow* rows, const std::vector<int>& comp, cons
   }
   const int na = (int)ia.size(), nb = (int)ib.size(), nw = (nb + 63) / 64;
   std::vector<uint64_t> left((size_t)na * nw, 0);         // B blocks of each A block's traces still to cover
-  std::vector<int> trace((size_t)na * nb, -1);
+  std::vector<int> trace((size_t)na * nb, -1), shared(na, 0);
+  std::vector<std::vector<int>> whose(nb);  // the A blocks of each B block's traces
   for (int r : comp) {
     const int a = ia[rows[r].aoff], b = ib[rows[r].boff];
     left[(size_t)a * nw + b / 64] |= 1ull << (b % 64);
     trace[(size_t)a * nb + b] = r;
+    whose[b].push_back(a);
   }
+  auto has = [&](int a, int b) { return (left[(size_t)a * nw + b / 64] >> (b % 64)) & 1ull; };
   auto take = [&](int a, int b) {
-    uint64_t& w = left[(size_t)a * nw + b / 64];
-    if (!((w >> (b % 64)) & 1ull)) return;
-    w &= ~(1ull << (b % 64));
+    if (!has(a, b)) return;
+    left[(size_t)a * nw + b / 64] &= ~(1ull << (b % 64));
     add(trace[(size_t)a * nb + b]);
   };
   // up to two B blocks of x (and of y, where given), appended to bs
@@ -2389,12 +2393,19 @@ static void cover_quads(const TraceRow* rows, const std::vector<int>& comp, cons
   for (int a = 0; a < na; a++) {
     const uint64_t* la = &left[(size_t)a * nw];
     for (;;) {
-      int bs[2], best = -1, common = 0;
+      int bs[2], best = -1;
       if (pick(la, nullptr, bs, 0) == 0) break;
-      for (int a2 = a + 1; a2 < na && common < 2; a2++) {
-        const int n = pick(la, &left[(size_t)a2 * nw], bs, 0);
-        if (n > common) common = n, best = a2;
+      std::vector<int> seen;
+      for (int b = 0; b < nb && (best < 0 || shared[best] < 2); b++) {
+        if (!has(a, b)) continue;
+        for (int a2 : whose[b]) {
+          if (a2 <= a || !has(a2, b)) continue;
+          seen.push_back(a2);
+          if (++shared[a2] == 2 || best < 0) best = a2;
+          if (shared[a2] == 2) break;
+        }
       }
+      for (int a2 : seen) shared[a2] = 0;
       int n = best >= 0 ? pick(la, &left[(size_t)best * nw], bs, 0) : 0;
       n = pick(la, nullptr, bs, n);
       for (int k = 0; k < n; k++) {

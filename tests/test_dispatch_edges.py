@@ -29,6 +29,29 @@ def test_quad_traces_one_warp_or_one_block_a_group(cuda, n):
                 "sigma Nev=%d" % n)
 
 
+@pytest.mark.parametrize("n,nrows", [(7, 9), (20, 300), (65, 900)])
+def test_quad_traces_cover_large_components(cuda, n, nrows):
+    """Random tables whose traces link many blocks, sparse to dense: every trace is
+    in one quad, whatever blocks it shares.  One row an output, so a trace may cancel:
+    2^-40 of its products' Frobenius norms (the float-float products carry 2^-44 of
+    their rows' and columns' largest entries), beside the engine's 1e-9."""
+    nt, nphi = 2, 3
+    rng = np.random.default_rng(800 + nrows)
+    prop = synth.make_prop(nt, n, seed=801 + n)
+    phi = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(nphi)], axis=1)
+    rows = np.concatenate([rng.integers(0, 4, (nrows, 4)), rng.integers(0, nphi, (nrows, 2))], axis=1).astype(np.int16)
+    coef = rng.integers(1, 3, (nrows, 2)).astype(np.float32)
+    oi = np.arange(nrows, dtype=np.int32)
+    got = api.twosided(_dev(prop, cuda), _dev(phi, cuda), rows, coef, oi, nrows, engine="split").cpu().numpy()
+    want = np.stack([O.twosided_rows(prop[tf], phi, rows, coef, tf, 0, nt) for tf in range(nt)])
+    a, b, c, d, L, R = rows.T
+    norm = lambda x: np.linalg.norm(x, axis=(-2, -1))
+    ab = np.abs(coef[:, 0] + 1j * coef[:, 1]) * np.array(
+        [[norm(prop[tf, ti, c, d] @ phi[ti, L]) * norm(phi[tf, R] @ prop[tf, ti, a, b]) for ti in range(nt)]
+         for tf in range(nt)])
+    P.entrywise(got, want, 1e-9, ab, "random table of %d rows, Nev=%d" % (nrows, n), floor=2.0 ** -40)
+
+
 @pytest.mark.parametrize("nt,n", [(1, 1), (5, 11), (3, 12), (22, 37), (64, 100), (200, 9)])
 def test_loop_unity_cluster_sizes(cuda, nt, n):
     """One CTA a time slice up to a cluster of 8, ragged element ranges; per
