@@ -13,7 +13,7 @@
 //    NSLICE = 5 the residual is <= 2^-45 of 2^E and unbiased.
 //  * MMA.  Slice pairs (i,j) with i+j <= 4 (15 pairs) are multiplied with
 //    tcgen05.mma kind::f16 (BF16 in, FP32 accumulate in TMEM); the complex
-//    product takes 4 real MMAs per pair (the -Xi*Yi term uses the A-negate bit).
+//    product takes 2 MMAs per pair (Xr and Xi with packed planes of Y).
 //    Pairs accumulate in four levels, i+j = 0, 1, 2 and >= 3.  Levels 0-2 hold
 //    integer multiples of 2^-16, 2^-25, 2^-34 below 2^24 units (level 0 for any
 //    data with K <= 128, levels 1-2 for non-adversarial data), which the FP32
@@ -836,53 +836,53 @@ __device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t units) {
   return (desc & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)desc + units);
 }
 
-// The MMAs of one slice pair (i, j) of one K chunk into its level accumulator.
-// adesc / bdesc describe sub-tile (slice 0, re) of the stage; the other
-// sub-tiles are constant byte offsets (added as offset >> 4 to the
-// start-address field, which cannot carry: shared addresses are < 2^18).
-template <class C, int I, int J>
-__device__ __forceinline__ void issue_pair(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first_chunk) {
-  constexpr uint32_t id_pos = idesc_bf16_f32(SPLIT_M, C::BN, false);
-  constexpr uint32_t id_neg = idesc_bf16_f32(SPLIT_M, C::BN, true);
-  constexpr uint32_t id_wide = idesc_bf16_f32(SPLIT_M, 2 * C::BN, false);
-  constexpr int lvl = (I + J) < C::NL - 1 ? (I + J) : C::NL - 1;
-  // in i-major order the first pair of level l is (0, l)
-  const uint32_t accum = (!first_chunk || !(I == 0 && J <= C::NL - 1)) ? 1u : 0u;
-  const uint64_t ar = desc_at(adesc, ((I * 2 + 0) * C::A_SUB) >> 4);
-  const uint64_t ai = desc_at(adesc, ((I * 2 + 1) * C::A_SUB) >> 4);
-  if constexpr (C::PACK) {
-    // planes -Yi, Yr, Yi of slice j are adjacent along N (row groups 256 B apart)
-    const uint64_t b_nr = desc_at(bdesc, ((J * 3 + 0) * C::B_SUB) >> 4);  // [-Yi | Yr]
-    const uint64_t b_ri = desc_at(bdesc, ((J * 3 + 1) * C::B_SUB) >> 4);  // [Yr | Yi]
-    const uint32_t d = tbase + (uint32_t)C::acc_col(0, lvl);
-    umma_f16(d, ar, b_ri, id_wide, accum);  // [Re | Im] += Xr [Yr | Yi]
-    umma_f16(d, ai, b_nr, id_wide, 1u);     // [Re | Im] += Xi [-Yi | Yr]
-  } else {
-    const uint64_t br = desc_at(bdesc, ((J * 2 + 0) * C::B_SUB) >> 4);
-    const uint64_t bi = desc_at(bdesc, ((J * 2 + 1) * C::B_SUB) >> 4);
-    const uint32_t dre = tbase + (uint32_t)C::acc_col(0, lvl);
-    const uint32_t dim = tbase + (uint32_t)C::acc_col(1, lvl);
-    umma_f16(dre, ar, br, id_pos, accum);  // Re += Xr Yr
-    umma_f16(dre, ai, bi, id_neg, 1u);     // Re -= Xi Yi
-    umma_f16(dim, ar, bi, id_pos, accum);  // Im += Xr Yi
-    umma_f16(dim, ai, br, id_pos, 1u);     // Im += Xi Yr
+// Slice pair (i, j), i + j < NS, falls in hand-back group G (G < 0: any).
+template <class C, int G>
+__host__ __device__ constexpr bool pair_in_group(int i, int j) {
+  return i + j < C::NS && (G < 0 || level_group(i + j < C::NL - 1 ? i + j : C::NL - 1) == G);
+}
+
+// The MMAs of plane P (0 Re, 1 Im) of left slice I with the right slices J, J + 1, ...
+// of group G.  They read one left sub-tile (4 KB, more than the right one's 3 KB
+// of the complex128 form), which the first leaves in the collector buffer and the
+// others take from there: shared memory feeds the MMAs 12 left sub-tiles a K chunk
+// instead of 42.  Issued alone, an MMA of the complex128 form takes 48.3 clocks
+// (56.0 bound by 7 KB of operand reads before); its launches at Nev = 100 (pi pi
+// sets) 66.9 -> 60.7 ms, the standard form's (64 clocks either way, less shared
+// memory traffic beside the copies) 9.75 -> 9.52 ms.
+template <class C, int G, int I, int P, int J, bool FILLED>
+__device__ __forceinline__ void issue_row(uint32_t tbase, uint64_t a, uint64_t bdesc, bool first_chunk) {
+  constexpr auto next = [](int j) {
+    while (j < C::NS && !pair_in_group<C, G>(I, j)) j++;
+    return j;
+  };
+  constexpr int j = next(J);
+  if constexpr (j < C::NS) {
+    constexpr bool more = next(j + 1) < C::NS;
+    constexpr int lvl = (I + j) < C::NL - 1 ? (I + j) : C::NL - 1;
+    constexpr Collect op = FILLED ? (more ? Collect::use : Collect::lastuse) : (more ? Collect::fill : Collect::discard);
+    // planes -Yi, Yr, Yi of slice j are adjacent along N (row groups 256 B apart):
+    // [Re | Im] += Xr [Yr | Yi] and Xi [-Yi | Yr]
+    const uint64_t b = desc_at(bdesc, ((j * 3 + (P ? 0 : 1)) * C::B_SUB) >> 4);
+    // the first MMA of level l in a tile is Xr of pair (0, l)
+    const uint32_t accum = (!first_chunk || !(I == 0 && P == 0 && j <= C::NL - 1)) ? 1u : 0u;
+    umma_f16<op>(tbase + (uint32_t)C::acc_col(0, lvl), a, b, idesc_bf16_f32(SPLIT_M, 2 * C::BN, false), accum);
+    issue_row<C, G, I, P, j + 1, true>(tbase, a, bdesc, first_chunk);
   }
 }
 
-// The slice pairs (i, j), i + j < NS, whose level falls in hand-back group G
-// (G < 0: all pairs), in i-major order.  Every level accumulator sees its
-// pairs in the same order whatever the grouping, so the FP32 last level sums
-// them in the same order and the results do not depend on it.
-template <class C, int G, int I = 0, int J = 0>
+// The slice pairs of hand-back group G (G < 0: all), in order of (left slice,
+// plane, right slice).  Every level accumulator sees its MMAs in the same order
+// whatever the grouping, so the FP32 last level sums them in the same order and
+// the results do not depend on it.  adesc / bdesc describe sub-tile (slice 0,
+// plane 0) of the stage; the others are constant byte offsets.
+template <class C, int G, int I = 0>
 __device__ __forceinline__ void issue_pairs(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first_chunk) {
+  static_assert(C::PACK, "packed complex operands");
   if constexpr (I < C::NS) {
-    if constexpr (I + J < C::NS) {
-      constexpr int lvl = (I + J) < C::NL - 1 ? (I + J) : C::NL - 1;
-      if constexpr (G < 0 || level_group(lvl) == G) issue_pair<C, I, J>(tbase, adesc, bdesc, first_chunk);
-      issue_pairs<C, G, I, J + 1>(tbase, adesc, bdesc, first_chunk);
-    } else {
-      issue_pairs<C, G, I + 1, 0>(tbase, adesc, bdesc, first_chunk);
-    }
+    issue_row<C, G, I, 0, 0, false>(tbase, desc_at(adesc, ((I * 2 + 0) * C::A_SUB) >> 4), bdesc, first_chunk);
+    issue_row<C, G, I, 1, 0, false>(tbase, desc_at(adesc, ((I * 2 + 1) * C::A_SUB) >> 4), bdesc, first_chunk);
+    issue_pairs<C, G, I + 1>(tbase, adesc, bdesc, first_chunk);
   }
 }
 
@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
     // and descriptor arithmetic is then uniform over the warp and stays off the
     // issuing thread's path.  With a single-lane branch around the whole loop and
     // 64-bit descriptor adds an MMA of the complex128 form took 71 clocks in tiles
-    // of 7 K chunks and 63 in tiles of 25 (the pipe: 56), as the issuing thread
+    // of 7 K chunks and 63 in tiles of 25 (alone: 56, see issue_row), as the issuing thread
     // shares its scheduler with four storing epilogue warps; 65 and 60 now.
     uint32_t g_chunk = 0, local = 0;
     bool ok = true;

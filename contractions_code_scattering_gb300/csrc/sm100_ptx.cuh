@@ -100,15 +100,30 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// What an MMA does with the collector buffer for its A operand: leave it alone
+// (discard), keep A there (fill), or take A from there (use; lastuse gives it up).
+enum class Collect { discard, fill, use, lastuse };
+
 // D[tmem] (+)= A[smem] * B[smem], kind::f16 (bf16 inputs, f32 accumulation).
+template <Collect OP>
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+#define CTR_UMMA_F16(COLLECTOR)                                                              \
+  asm volatile(                                                                              \
+      "{\n\t.reg .pred p;\n\t"                                                              \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                            \
+      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" COLLECTOR " [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem), \
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                    \
+      : "memory")
+  if constexpr (OP == Collect::fill)
+    CTR_UMMA_F16("fill");
+  else if constexpr (OP == Collect::use)
+    CTR_UMMA_F16("use");
+  else if constexpr (OP == Collect::lastuse)
+    CTR_UMMA_F16("lastuse");
+  else
+    CTR_UMMA_F16("discard");
+#undef CTR_UMMA_F16
 }
 
 // True in one lane of a converged warp.
