@@ -1005,56 +1005,62 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       }
     }
   } else if (warp == 1) {
-    // The whole warp walks the tiles and waits; one elected lane issues.  Loop
-    // and descriptor arithmetic is then uniform over the warp and stays off the
-    // issuing thread's path.  With a single-lane branch around the whole loop and
-    // 64-bit descriptor adds an MMA of the complex128 form took 71 clocks in tiles
-    // of 7 K chunks and 63 in tiles of 25 (alone: 56, see issue_row), as the issuing thread
-    // shares its scheduler with four storing epilogue warps; 65 and 60 now.
-    uint32_t g_chunk = 0, local = 0;
-    bool ok = true;
-    const uint64_t adesc0 = sdesc_kmajor_noswz(smem_u32(sA), 128, 256);
-    const uint64_t bdesc0 = sdesc_kmajor_noswz(smem_u32(sB), 128, 256);
-    for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x, local++) {
-      for (int kc = 0; kc < g.nchunk; kc++, g_chunk++) {
-        const int s = g_chunk % NSTAGE;
-        ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (g_chunk / NSTAGE) & 1, WAIT_NS, err));
-        if (!ok) {
-          if (lane == 0) atomicExch(err, 2);
-          break;
+    // One elected thread walks the tiles, waits and issues: an MMA is handed over
+    // in about the time one takes, so whatever lies between the last MMA of a chunk
+    // and the first of the next is a gap of the tensor pipe.  With a whole warp that
+    // waits, votes and elects a lane for each chunk an MMA took 55.0 clocks in the
+    // complex128 form and 71.1 in the standard one (schedule and copies alone, no
+    // epilogue); 50.0 and 64.0 in one thread, of which the pipe needs 48 and 64.
+    if (elect_one()) {
+      uint32_t local = 0, st = 0, ph = 0;
+      bool ok = true;
+      const uint64_t adesc0 = sdesc_kmajor_noswz(smem_u32(sA), 128, 256);
+      const uint64_t bdesc0 = sdesc_kmajor_noswz(smem_u32(sB), 128, 256);
+      auto wait_full = [&](uint32_t s, uint32_t parity) {
+        ok = mbar_wait(&full[s], parity, WAIT_NS, err);
+        if (!ok) atomicExch(err, 2);
+        tc_fence_after();
+        return ok;
+      };
+      auto wait_group = [&](int grp) {
+        if (local > 0) {
+          ok = mbar_wait(&tempty[grp], (local - 1) & 1, 2 * WAIT_NS, err);
+          if (!ok) atomicExch(err, 4);
         }
         tc_fence_after();
-        const uint64_t ad = desc_at(adesc0, (s * C::A_STAGE) >> 4);
-        const uint64_t bd = desc_at(bdesc0, (s * C::B_STAGE) >> 4);
-        if (kc == 0) {
-          // first chunk: each group of levels once the epilogue handed it back
+        return ok;
+      };
+      auto adesc = [&](uint32_t s) { return desc_at(adesc0, (s * C::A_STAGE) >> 4); };
+      auto bdesc = [&](uint32_t s) { return desc_at(bdesc0, (s * C::B_STAGE) >> 4); };
+      auto next = [&]() {
+        if (++st == NSTAGE) st = 0, ph ^= 1;
+      };
+      for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x, local++) {
+        // first chunk: each group of levels once the epilogue handed it back
+        if (!wait_full(st, ph)) break;
+        if (local == 0) {
+          issue_chunk<C>(tbase, adesc(st), bdesc(st), true);
+        } else {
           for (int grp = 0; grp < tmem_groups<C>(); grp++) {
-            if (local > 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(&tempty[grp], (local - 1) & 1, 2 * WAIT_NS, err));
-              if (!ok) {
-                if (lane == 0) atomicExch(err, 4);
-                break;
-              }
-            }
-            tc_fence_after();
-            if (elect_one()) issue_group<C>(grp, tbase, ad, bd, true);
-            __syncwarp();
+            if (!wait_group(grp)) break;
+            issue_group<C>(grp, tbase, adesc(st), bdesc(st), true);
           }
           if (!ok) break;
-        } else {
-          if (elect_one()) issue_chunk<C>(tbase, ad, bd, false);
-          __syncwarp();
         }
-        if (elect_one()) umma_commit(&empty[s]);  // stage s free once these MMAs have read it
-        __syncwarp();
+        umma_commit(&empty[st]);
+        next();
+        int kc = 1;
+        for (; kc < g.nchunk && ok; kc++, next()) {
+          if (!wait_full(st, ph)) break;
+          issue_chunk<C>(tbase, adesc(st), bdesc(st), false);
+          umma_commit(&empty[st]);  // stage st free once these MMAs have read it
+        }
+        if (ok) umma_commit(tfull);
       }
-      if (ok && elect_one()) umma_commit(tfull);
-      __syncwarp();
+      // wait for every issued MMA before the accumulators are released
+      umma_commit(drainb);
+      if (!mbar_wait(drainb, 0, WAIT_NS)) atomicExch(err, 5);
     }
-    // wait for every issued MMA before the accumulators are released
-    if (elect_one()) umma_commit(drainb);
-    __syncwarp();
-    if (!mbar_wait(drainb, 0, WAIT_NS) && lane == 0) atomicExch(err, 5);
     __syncwarp();
   } else {
     // epilogue: warp w drains TMEM lane quadrant w % 4; the EPI_WARPS / 4
