@@ -763,9 +763,9 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
 // of 128 x SPLIT_N.  Warp 0: TMEM allocation and the bulk-copy producer, which
 // runs ahead across tile boundaries through an NSTAGE ring; warp 1: MMA issue;
 // warps 2 .. 2 + EPI_WARPS - 1: epilogue (TMEM lanes 32*(warp%4) .. +31).  The
-// MMA warp and the epilogue hand the TMEM accumulators back and forth with two
-// mbarriers (tmem_full after the last MMA of a tile, tmem_empty once the
-// epilogue holds them in registers, before its global stores).
+// MMA warp and the epilogue hand the TMEM accumulators back and forth with
+// mbarriers (tfull after the last MMA of a tile, tempty once the epilogue holds
+// them in registers, before its global stores), in groups of levels.
 // Threads of a GEMM CTA: producer and MMA warps plus C::EPI_WARPS epilogue warps.
 template <class C>
 constexpr int gemm_threads() { return 64 + 32 * C::EPI_WARPS; }
@@ -821,14 +821,19 @@ __device__ __forceinline__ double pow2d(int e) {
 template <int NTHR>
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(NTHR) : "memory"); }
 
-// TMEM hand-back groups: the epilogue drains the level accumulators in groups,
-// levels {0, 1} first, then each further level on its own, and hands every
-// group back as soon as it holds it in registers.  The first K chunk of the
-// next tile issues its MMAs group by group, each after that group's hand-back,
-// so the MMAs of the early levels run while later levels are still drained.
+// TMEM hand-over groups: the epilogue drains the level accumulators in groups, the
+// last level first, then levels {0, 1}, then each further level on its own, and
+// hands every group back as soon as it holds it in registers.  The last level has
+// half of the MMAs (complex128: 22 of 42 a K chunk, standard: 18 of 30).  It goes
+// first at both ends: in a tile's last chunk its MMAs come before the others', and
+// it is drained beside those; the last-level MMAs of the next tile's first two
+// chunks (2.1 and 2.3 K clocks) run while the other levels are drained.  From the
+// MMA warp's last issue to its next 1 300 -> 250 clocks, to the end of the first
+// two chunks 6 500 -> 5 300 (complex128, Nev = 100).
 template <class C>
 constexpr int tmem_groups() { return C::NL - 1; }
-__host__ __device__ constexpr int level_group(int l) { return l <= 1 ? 0 : l - 1; }
+template <class C>
+__host__ __device__ constexpr int level_group(int l) { return l == C::NL - 1 ? 0 : (l <= 1 ? 1 : l); }
 
 // A descriptor moved on by `units` of 16 bytes: one 32-bit add, since the address
 // field cannot carry out of the low word (shared addresses are below 2^18).
@@ -836,10 +841,13 @@ __device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t units) {
   return (desc & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)desc + units);
 }
 
-// Slice pair (i, j), i + j < NS, falls in hand-back group G (G < 0: any).
+// Slice pair (i, j), i + j < NS, falls in hand-back group G (ALL: any, REST: any but
+// the first).
+constexpr int GROUP_ALL = -1, GROUP_REST = -2;
 template <class C, int G>
 __host__ __device__ constexpr bool pair_in_group(int i, int j) {
-  return i + j < C::NS && (G < 0 || level_group(i + j < C::NL - 1 ? i + j : C::NL - 1) == G);
+  const int grp = level_group<C>(i + j < C::NL - 1 ? i + j : C::NL - 1);
+  return i + j < C::NS && (G == GROUP_ALL || grp == G || (G == GROUP_REST && grp > 0));
 }
 
 // The MMAs of plane P (0 Re, 1 Im) of left slice I with the right slices J, J + 1, ...
@@ -871,8 +879,7 @@ __device__ __forceinline__ void issue_row(uint32_t tbase, uint64_t a, uint64_t b
   }
 }
 
-// The slice pairs of hand-back group G (G < 0: all), in order of (left slice,
-// plane, right slice).  Every level accumulator sees its MMAs in the same order
+// The slice pairs of group G in order of (left slice, plane, right slice).  Every level accumulator sees its MMAs in the same order
 // whatever the grouping, so the FP32 last level sums them in the same order and
 // the results do not depend on it.  adesc / bdesc describe sub-tile (slice 0,
 // plane 0) of the stage; the others are constant byte offsets.
@@ -890,7 +897,7 @@ __device__ __forceinline__ void issue_pairs(uint32_t tbase, uint64_t adesc, uint
 // level accumulators.
 template <class C>
 __device__ __forceinline__ void issue_chunk(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first_chunk) {
-  issue_pairs<C, -1>(tbase, adesc, bdesc, first_chunk);
+  issue_pairs<C, GROUP_ALL>(tbase, adesc, bdesc, first_chunk);
 }
 
 // The MMAs of hand-back group g (runtime index) of one K chunk.
@@ -946,14 +953,14 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   uint8_t* sB = smem + NSTAGE * C::A_STAGE;
   uint64_t* full = (uint64_t*)(smem + NSTAGE * (C::A_STAGE + C::B_STAGE));
   uint64_t* empty = full + NSTAGE;
-  uint64_t* tfull = empty + NSTAGE;
-  uint64_t* tempty = tfull + 1;  // one per hand-back group
+  uint64_t* tfull = empty + NSTAGE;  // the last level, every level
+  uint64_t* tempty = tfull + 2;  // one per hand-back group
   uint64_t* drainb = tempty + tmem_groups<C>();
   uint32_t* tslot = (uint32_t*)(drainb + 1);
   int* sexp = (int*)(tslot + 4);  // C::BN column exponents, of the even and of the odd tiles
   // complex128 output: destination of row 0 of each column, of the even and of the odd tiles
   double2** colp = (double2**)(smem + NSTAGE * (C::A_STAGE + C::B_STAGE) + 768);
-  static_assert(768 + 2 * 8 * 48 <= GEMM_SMEM_TAIL && 12 * 8 + 16 + 2 * 4 * C::BN <= 768, "GEMM shared-memory tail");
+  static_assert(768 + 2 * 8 * 48 <= GEMM_SMEM_TAIL && 13 * 8 + 16 + 2 * 4 * C::BN <= 768, "GEMM shared-memory tail");
 
   volatile int* status = (volatile int*)(tslot + 1);  // block-uniform decisions
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -963,7 +970,8 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(tfull, 1);
+    mbar_init(&tfull[0], 1);
+    mbar_init(&tfull[1], 1);
     for (int g = 0; g < tmem_groups<C>(); g++) mbar_init(&tempty[g], C::EPI_WARPS);  // one arrival per epilogue warp
     mbar_init(drainb, 1);
     fence_mbar_init();
@@ -981,6 +989,10 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   tc_fence_after();
   const uint32_t tbase = __shfl_sync(0xffffffffu, *tslot, 0);
 
+  // The last level is handed over ahead of the others from 4 chunks a tile (Nev > 48;
+  // Nev = 57 741 -> 704 us, Nev = 100 9.25 -> 8.98 ms); shorter tiles are bound by their
+  // epilogue, which the second wait only lengthens (Nev = 32 223 -> 242 us).
+  const bool early = g.nchunk >= 4;
   if (warp == 0) {
     if (lane == 0) {
       uint32_t g_chunk = 0;
@@ -1036,26 +1048,44 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         if (++st == NSTAGE) st = 0, ph ^= 1;
       };
       for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x, local++) {
-        // first chunk: each group of levels once the epilogue handed it back
-        if (!wait_full(st, ph)) break;
-        if (local == 0) {
-          issue_chunk<C>(tbase, adesc(st), bdesc(st), true);
-        } else {
-          for (int grp = 0; grp < tmem_groups<C>(); grp++) {
-            if (!wait_group(grp)) break;
-            issue_group<C>(grp, tbase, adesc(st), bdesc(st), true);
-          }
-          if (!ok) break;
+        // The first two chunks: their last-level MMAs once the epilogue handed that
+        // level back, then, chunk by chunk, the other groups as they come back.  (Two
+        // stages hold chunks of this tile by then, and the third one's copy is not
+        // held up.)  The CTA's first tile has nothing to wait for but its chunks.
+        const int pre = min(local == 0 ? 1 : 2, g.nchunk);
+        if (!wait_group(0)) break;
+        uint32_t s = st, p = ph;
+        for (int c = 0; c < pre; c++) {
+          if (!wait_full(s, p)) break;
+          issue_group<C>(0, tbase, adesc(s), bdesc(s), c == 0);
+          if (++s == NSTAGE) s = 0, p ^= 1;
         }
-        umma_commit(&empty[st]);
+        if (!ok) break;
+        for (int grp = 1; grp < tmem_groups<C>(); grp++) {
+          if (!wait_group(grp)) break;
+          issue_group<C>(grp, tbase, adesc(st), bdesc(st), true);
+        }
+        if (!ok) break;
+        umma_commit(&empty[st]);  // stage st free once these MMAs have read it
         next();
-        int kc = 1;
-        for (; kc < g.nchunk && ok; kc++, next()) {
-          if (!wait_full(st, ph)) break;
-          issue_chunk<C>(tbase, adesc(st), bdesc(st), false);
-          umma_commit(&empty[st]);  // stage st free once these MMAs have read it
+        if (pre > 1) {
+          issue_pairs<C, GROUP_REST>(tbase, adesc(st), bdesc(st), false);
+          umma_commit(&empty[st]);
+          next();
         }
-        if (ok) umma_commit(tfull);
+        for (int kc = pre; kc < g.nchunk; kc++, next()) {
+          if (!wait_full(st, ph)) break;
+          if (!early || kc + 1 < g.nchunk) {
+            issue_chunk<C>(tbase, adesc(st), bdesc(st), false);
+          } else {
+            // the last chunk: the last level first, drained beside the others' MMAs
+            issue_pairs<C, 0>(tbase, adesc(st), bdesc(st), false);
+            umma_commit(&tfull[0]);
+            issue_pairs<C, GROUP_REST>(tbase, adesc(st), bdesc(st), false);
+          }
+          umma_commit(&empty[st]);
+        }
+        if (ok) umma_commit(&tfull[early ? 1 : 0]);
       }
       // wait for every issued MMA before the accumulators are released
       umma_commit(drainb);
@@ -1132,10 +1162,10 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       }
       const int grow = mt * SPLIT_M + row;
       const bool rvalid = grow < g.mrows;
-      // one thread waits for the accumulators; the outcome is shared so that
-      // all epilogue threads leave the loop together
+      // one thread waits for the last level; the outcome is shared so that all
+      // epilogue threads leave the loop together
       if (et == 0) {
-        const bool done = mbar_wait(tfull, local & 1, 4 * WAIT_NS, err);
+        const bool done = mbar_wait(&tfull[0], local & 1, 4 * WAIT_NS, err);
         if (!done) atomicExch(err, 3);
         *failed = done ? 0 : 1;
       }
@@ -1152,6 +1182,14 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[grp]);
+      };
+      // the other levels, by each warp for itself (it carries on after a failure, which
+      // the wait above finds at the next tile)
+      auto wait_rest = [&]() {
+        if (!early) return;
+        if (!mbar_wait(&tfull[1], local & 1, 4 * WAIT_NS, err)) atomicExch(err, 3);
+        __syncwarp();
+        tc_fence_after();
       };
       if constexpr (C::INT_OUT) {
         // complex128 output: the exact levels and the last one summed exactly
@@ -1172,24 +1210,37 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         // that load's values are folded in: the MMA warp waits on the loads only)
         static_assert(!C::INT_OUT || (CPW == 12 && EPH == 4), "16 x 24 fragments of a warp");
         long long acc[2][CPW];
+        {  // group 0: the last level
+          float v0[CPW], v1[CPW];
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(0, C::NL - 1) + cbase), v0);
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(1, C::NL - 1) + cbase), v1);
+          tmem_ld_wait();
+          hand_back(0);
 #pragma unroll
-        for (int part = 0; part < 2; part++) {  // group 0: levels 0 and 1
+          for (int c = 0; c < CPW; c++) {
+            acc[0][c] = level_units(v0[c], C::NL - 1);
+            acc[1][c] = level_units(v1[c], C::NL - 1);
+          }
+        }
+        wait_rest();
+#pragma unroll
+        for (int part = 0; part < 2; part++) {  // group 1: levels 0 and 1
           float v0[CPW], v1[CPW];
           tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 0) + cbase), v0);
           tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 1) + cbase), v1);
           tmem_ld_wait();
-          if (part == 1) hand_back(0);
+          if (part == 1) hand_back(1);
 #pragma unroll
-          for (int c = 0; c < CPW; c++) acc[part][c] = level_units(v0[c], 0) + level_units(v1[c], 1);
+          for (int c = 0; c < CPW; c++) acc[part][c] += level_units(v0[c], 0) + level_units(v1[c], 1);
         }
 #pragma unroll
-        for (int l = 2; l < C::NL; l++) {  // group l - 1: level l
+        for (int l = 2; l < C::NL - 1; l++) {  // group l: level l
 #pragma unroll
           for (int part = 0; part < 2; part++) {
             float v[CPW];
             tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, l) + cbase), v);
             tmem_ld_wait();
-            if (part == 1) hand_back(l - 1);
+            if (part == 1) hand_back(l);
 #pragma unroll
             for (int c = 0; c < CPW; c++) acc[part][c] += level_units(v[c], l);
           }
@@ -1222,6 +1273,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         if (g.levels) {
           // raw level values for the exactness tests, read before any hand-back
           // (the loads are warp-collective; rows past the end store nothing)
+          wait_rest();
 #pragma unroll 1
           for (int pl = 0; pl < 2 * C::NL; pl++) {
             const int part = pl / C::NL, l = pl % C::NL;
@@ -1241,40 +1293,44 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         // (each group goes back as soon as its last load has landed, before
         // that load's values are folded in: the MMA warp waits on the loads only)
         float s[2][CPW], e[2][CPW];
+        // group 0: the last level
+        tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(0, C::NL - 1) + cbase), e[0]);
+        tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(1, C::NL - 1) + cbase), e[1]);
+        tmem_ld_wait();
+        hand_back(0);
+        wait_rest();
 #pragma unroll
-        for (int part = 0; part < 2; part++) {  // group 0: levels 0 and 1
+        for (int part = 0; part < 2; part++) {  // group 1: levels 0 and 1
+          float v[CPW];
           tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, 0) + cbase), s[part]);
-          tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, 1) + cbase), e[part]);
+          tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, 1) + cbase), v);
           tmem_ld_wait();
-          if (part == 1) hand_back(0);
+          if (part == 1) hand_back(1);
 #pragma unroll
           for (int c = 0; c < CPW; c++) {
             float t, d;
-            two_sum(s[part][c], e[part][c], t, d);
+            two_sum(s[part][c], v[c], t, d);
             s[part][c] = t;
-            e[part][c] = 0.f + d;
+            e[part][c] += d;
           }
         }
 #pragma unroll
-        for (int l = 2; l < C::NL; l++) {  // group l - 1: level l
+        for (int l = 2; l < C::NL - 1; l++) {  // group l: level l
 #pragma unroll
           for (int part = 0; part < 2; part++) {
             float v[CPW];
             tmem_ld_cols<CPW>(tl + (uint32_t)(C::acc_col(part, l) + cbase), v);
             tmem_ld_wait();
-            if (part == 1) hand_back(l - 1);
+            if (part == 1) hand_back(l);
 #pragma unroll
             for (int c = 0; c < CPW; c++) {
-              if (l < C::NL - 1) {
-                float t, d;
-                two_sum(s[part][c], v[c], t, d);
+              float t, d;
+              two_sum(s[part][c], v[c], t, d);
+              if (l < C::NL - 2) {
                 s[part][c] = t;
                 e[part][c] += d;
               } else {
-                float h, lw;
-                fast_two_sum(s[part][c], e[part][c] + v[c], h, lw);
-                s[part][c] = h;
-                e[part][c] = lw;
+                fast_two_sum(t, e[part][c] + d, s[part][c], e[part][c]);
               }
             }
           }
