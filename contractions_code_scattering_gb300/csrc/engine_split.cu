@@ -208,18 +208,20 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
   }
   // distinct source blocks (c,d), source elementals L, sink blocks (a,b), sink elementals R
   std::vector<int> cdl, Ll, abl, Rl;
-  auto idx = [](std::vector<int>& v, int x) {
-    auto it = std::find(v.begin(), v.end(), x);
-    if (it != v.end()) return (int)(it - v.begin());
-    v.push_back(x);
-    return (int)v.size() - 1;
+  std::vector<int> cdx(16, -1), Lx(nphi, -1), abx(16, -1), Rx(nphi, -1);
+  auto idx = [](std::vector<int>& v, std::vector<int>& at, int x) {
+    if (at[x] < 0) {
+      at[x] = (int)v.size();
+      v.push_back(x);
+    }
+    return at[x];
   };
   std::vector<int> ia(nrows), il(nrows), ib(nrows), ir(nrows);
   for (int r = 0; r < nrows; r++) {
-    ia[r] = idx(cdl, rows[r].c * 4 + rows[r].d);
-    il[r] = idx(Ll, rows[r].L);
-    ib[r] = idx(abl, rows[r].a * 4 + rows[r].b);
-    ir[r] = idx(Rl, rows[r].R);
+    ia[r] = idx(cdl, cdx, rows[r].c * 4 + rows[r].d);
+    il[r] = idx(Ll, Lx, rows[r].L);
+    ib[r] = idx(abl, abx, rows[r].a * 4 + rows[r].b);
+    ir[r] = idx(Rl, Rx, rows[r].R);
   }
   if ((int)Ll.size() > SPLIT_MAXBLK || (int)Rl.size() > SPLIT_MAXBLK)
     return fail(CTR_ERR_ARG, "too many distinct elementals (max %d)", SPLIT_MAXBLK);
@@ -303,37 +305,22 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
   std::vector<TraceRow> trow;
   std::vector<int> tix(nrows);
   {
-    std::map<std::pair<int, int>, int> seen;
+    std::vector<int> seen((size_t)nL * ncd * nR * nab, -1);
     for (int r = 0; r < nrows; r++) {
-      const int aoff = (il[r] * N) * ldA + ia[r] * N, boff = (ib[r] * N) * ldB + ir[r] * N;
-      auto it = seen.find({aoff, boff});
-      if (it == seen.end()) {
-        it = seen.emplace(std::make_pair(aoff, boff), (int)trow.size()).first;
-        trow.push_back(TraceRow{aoff, boff, {1.f, 0.f}});
+      int& t = seen[((size_t)(il[r] * ncd + ia[r]) * nab + ib[r]) * nR + ir[r]];
+      if (t < 0) {
+        t = (int)trow.size();
+        trow.push_back(TraceRow{(il[r] * N) * ldA + ia[r] * N, (ib[r] * N) * ldB + ir[r] * N, {1.f, 0.f}});
       }
-      tix[r] = it->second;
+      tix[r] = t;
     }
   }
   const int ntr = (int)trow.size();
-  // the same traces in groups that share their product blocks (trace_groups)
-  // (trace_groups), and in quad groups of at most 2 + 2 blocks (trace_quads)
-  std::vector<TraceGroup> tgroups, tquads;
-  const int tg_maxcols = build_trace_groups(trow.data(), ntr, TG_MAXA, TG_MAXB, TG_MAXT, tgroups);
-  build_trace_groups(trow.data(), ntr, 2, 2, 4, tquads);
-  tgroups.insert(tgroups.end(), tquads.begin(), tquads.end());
-  const int ngroups = (int)(tgroups.size() - tquads.size()), nquads = (int)tquads.size();
-  // every table of the call in one staging copy (a small call is bound by its launches)
-  void* dc[7];
+  void* dc[2];
   CTR_TRY(upload_group(WS_MISC,
                        {{phi_lj.data(), phi_lj.size() * sizeof(SliceLeftJob)},
-                        {phi_rj.data(), phi_rj.size() * sizeof(SliceRightJob)},
-                        {csr.data(), csr.size() * sizeof(int)},
-                        {trow.data(), trow.size() * sizeof(TraceRow)},
-                        {tgroups.data(), tgroups.size() * sizeof(TraceGroup)},
-                        {tix.data(), tix.size() * sizeof(int)},
-                        {coef.data(), coef.size() * sizeof(float)}},
+                        {phi_rj.data(), phi_rj.size() * sizeof(SliceRightJob)}},
                        dc, stream));
-  void *d_csr = dc[2], *d_trow = dc[3], *d_tgroups = dc[4], *d_tix = dc[5], *d_rcoef = dc[6];
   CTR_TRY(launch_slice_left((const SliceLeftJob*)dc[0], Nt, N, nchunk, F.mtiles, stream, 1));
   CTR_TRY(launch_slice_right((const SliceRightJob*)dc[1], Nt, N, nchunk, F.ntiles, stream, 1));
 
@@ -343,6 +330,30 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
   std::vector<const float4*> abase, bbase;
   char shape[160];
   snprintf(shape, sizeof(shape), "nev=%d,ncd=%d,nab=%d,nL=%d,nR=%d,ntr=%d", N, ncd, nab, nL, nR, ntr);
+  // The traces in quad groups of at most 2 + 2 product blocks (trace_quads) and, where
+  // they may be asked for, in groups that share more (trace_groups), with the rows'
+  // tables.  Built when the first batch's products are launched: the host takes
+  // 0.2 ms for the 624 traces of rho, as long as those products at Nev = 32, Lt = 16.
+  std::vector<TraceGroup> tgroups, tquads;
+  int tg_maxcols = 0, ngroups = 0, nquads = 0;
+  void* dt[5] = {};
+  auto trace_tables = [&]() -> int {
+    if (dt[0]) return CTR_OK;
+    int v;
+    if (tune_mode() > 0 || tune_forced("trace_rows") == TRACE_VARIANTS ||
+        (tune_lookup(tune_key("trace_rows", shape), &v) && v == TRACE_VARIANTS))
+      tg_maxcols = build_trace_groups(trow.data(), ntr, TG_MAXA, TG_MAXB, TG_MAXT, tgroups);
+    build_trace_groups(trow.data(), ntr, 2, 2, 4, tquads);
+    ngroups = (int)tgroups.size(), nquads = (int)tquads.size();
+    tgroups.insert(tgroups.end(), tquads.begin(), tquads.end());
+    return upload_group(WS_TASKS2,
+                        {{csr.data(), csr.size() * sizeof(int)},
+                         {trow.data(), trow.size() * sizeof(TraceRow)},
+                         {tgroups.data(), tgroups.size() * sizeof(TraceGroup)},
+                         {tix.data(), tix.size() * sizeof(int)},
+                         {coef.data(), coef.size() * sizeof(float)}},
+                        dt, stream);
+  };
   // one batch of pairs [p0, p0 + np): slice tau, both GEMMs, traces, per-entry sums
   auto run_batch = [&](int p0, int np) -> int {
     void *mem, *rowbuf, *absbuf;
@@ -423,6 +434,8 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
       G->order = order;
       CTR_TRY(launch_split_gemm(*G, np, d_err, stream));
     }
+    CTR_TRY(trace_tables());
+    void *d_csr = dt[0], *d_trow = dt[1], *d_tgroups = dt[2], *d_tix = dt[3], *d_rcoef = dt[4];
     // candidates: the TRACE_VARIANTS per-trace kernels, the grouped one, then
     // the two quad-group kernels
     auto traces = [&](int variant) {
