@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <map>
 #include <tuple>
+#include <unordered_map>
 
 #include "kernels.h"
 
@@ -71,13 +72,28 @@ int twosided_fp64(int N, int Nt, int tf_begin, int tf_end, const double* prop_ro
   int batch = (int)std::max<size_t>(1, budget / per_pair);
   batch = std::min(batch, npairs_total);
 
-  // CSR of output rows (constant for all batches)
-  std::vector<int> csr(P.off);
-  csr.insert(csr.end(), P.idx.begin(), P.idx.end());
-  void* d_csr;
-  CTR_TRY(upload(WS_MISC, csr.data(), csr.size() * sizeof(int), &d_csr, stream));
-  const int* d_off = (const int*)d_csr;
-  const int* d_idx = d_off + (nout + 1);
+  // each distinct (A block, B block) trace once (144 of rho's 768 rows repeat one)
+  std::vector<int> tix(nrows), ta, tb;
+  {
+    std::unordered_map<long long, int> seen;
+    for (int r = 0; r < nrows; r++) {
+      const auto it = seen.emplace((long long)P.rowA[r] * nB + P.rowB[r], (int)ta.size());
+      if (it.second) {
+        ta.push_back(P.rowA[r]);
+        tb.push_back(P.rowB[r]);
+      }
+      tix[r] = it.first->second;
+    }
+  }
+  const int ntr = (int)ta.size();
+  // CSR of output rows, their traces and coefficients (constant for all batches)
+  void* dc[4];
+  CTR_TRY(upload_group(WS_MISC,
+                       {{P.off.data(), P.off.size() * sizeof(int)},
+                        {P.idx.data(), P.idx.size() * sizeof(int)},
+                        {tix.data(), tix.size() * sizeof(int)},
+                        {coef.data(), coef.size() * sizeof(float)}},
+                       dc, stream));
 
   const double2* tau = (const double2*)prop_rows;
   const double2* ph = (const double2*)phi;
@@ -87,7 +103,7 @@ int twosided_fp64(int N, int Nt, int tf_begin, int tf_end, const double* prop_ro
     const int np = std::min(batch, npairs_total - p0);
     void *scratch, *rowbuf;
     CTR_TRY(workspace(WS_SCRATCH).get((size_t)np * per_pair, &scratch));
-    CTR_TRY(workspace(WS_ROWS).get((size_t)np * nrows * sizeof(double2), &rowbuf));
+    CTR_TRY(workspace(WS_ROWS).get((size_t)np * ntr * sizeof(double2), &rowbuf));
     double2* S = (double2*)scratch;
     double2* R = (double2*)rowbuf;
     gt.clear();
@@ -120,14 +136,12 @@ int twosided_fp64(int N, int Nt, int tf_begin, int tf_end, const double* prop_ro
         z.nterm = 1;
         gt.push_back(z);
       }
-      for (int r = 0; r < nrows; r++) {
+      for (int k = 0; k < ntr; k++) {
         TraceTask t{};
-        t.X = SA + (size_t)P.rowA[r] * N2;
-        t.Y = SB + (size_t)P.rowB[r] * N2;
-        t.out = R + (size_t)q * nrows + r;
-        t.coef[0] = coef[2 * r];
-        t.coef[1] = coef[2 * r + 1];
-        t.mode = 0;
+        t.X = SA + (size_t)ta[k] * N2;
+        t.Y = SB + (size_t)tb[k] * N2;
+        t.out = R + (size_t)q * ntr + k;
+        t.mode = 2;
         tt.push_back(t);
       }
     }
@@ -137,7 +151,8 @@ int twosided_fp64(int N, int Nt, int tf_begin, int tf_end, const double* prop_ro
     // The trace tasks live behind the GEMM tasks in a second upload slot.
     CTR_TRY(upload(WS_ROWTASKS, tt.data(), tt.size() * sizeof(TraceTask), &d_tt, stream));
     CTR_TRY(launch_trace_f64((const TraceTask*)d_tt, (int)tt.size(), N, stream));
-    CTR_TRY(launch_rowsum(R, nrows, d_off, d_idx, nout, np, (double2*)out + (size_t)p0 * nout, nout, stream));
+    CTR_TRY(launch_rowsum_coef(R, ntr, (const int*)dc[0], (const int*)dc[1], (const int*)dc[2], (const float*)dc[3], nout,
+                               np, (double2*)out + (size_t)p0 * nout, stream));
   }
   return CTR_OK;
 }

@@ -28,7 +28,7 @@ struct TraceTask {
   double2* out;
   double* absout;
   float coef[2];
-  int mode;
+  int mode;  // bit 0: Y transposed (no conjugate); bit 1: the trace without its coefficient
   int pad;
 };
 
@@ -86,8 +86,8 @@ int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s)
 int launch_trace_f64_untimed(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s);
 // loop[t] = sum_s Tr[tau(t,t)_ss Phi(t)] for diag [Nt][4][4][N][N], mom [Nt][N][N].
 int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s);
-int launch_rowsum(const double2* rows, int nrows, const int* off, const int* idx, int nout, int npair,
-                  double2* out, size_t out_pair_stride, cudaStream_t s);
+int launch_rowsum_coef(const double2* tr, int ntr, const int* off, const int* idx, const int* tix, const float* coef,
+                       int nout, int npair, double2* out, cudaStream_t s);
 int launch_source_average(int Nt, int ncorr, const double2* corr, double scale, double2* avg, cudaStream_t s);
 // Row sums as launch_rowsum (out stride nout) plus per-entry refinement flags:
 // entries with eps_over_tol * sum(rabs) > |out| append (pair_base + p) * nout + o to list.

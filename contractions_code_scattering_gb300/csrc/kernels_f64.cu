@@ -81,16 +81,21 @@ __global__ void __launch_bounds__(256) zgemm_f64_kernel(const ZTask* __restrict_
       }
       __syncthreads();
     }
-    const double2 w = make_double2((double)T.wre[q], (double)T.wim[q]);
-    for (int a = 0; a < 2; a++)
-      for (int b = 0; b < 2; b++) {
-        if (q == 0 && w.x == 1.0 && w.y == 0.0) acc[a][b] = part[a][b];
-        else {
+    // a branch around the weights, which the barrier keeps one: predicated off, their
+    // operations still take the FP64 pipe, 6 % of a product at Nev = 32
+    if (q == 0 && T.wre[q] == 1.f && T.wim[q] == 0.f) {
+      for (int a = 0; a < 2; a++)
+        for (int b = 0; b < 2; b++) acc[a][b] = part[a][b];
+    } else {
+      __syncwarp();
+      const double2 w = make_double2((double)T.wre[q], (double)T.wim[q]);
+      for (int a = 0; a < 2; a++)
+        for (int b = 0; b < 2; b++) {
           double2 t = cmul(w, part[a][b]);
           acc[a][b].x += t.x;
           acc[a][b].y += t.y;
         }
-      }
+    }
   }
   for (int a = 0; a < 2; a++)
     for (int b = 0; b < 2; b++) {
@@ -170,18 +175,23 @@ __global__ void __launch_bounds__((T / TM) * (T / TN), 2) zgemm_f64_tile_kernel(
       }
       __syncthreads();
     }
-    const double2 w = make_double2((double)Tk.wre[q], (double)Tk.wim[q]);
+    if (q == 0 && Tk.wre[q] == 1.f && Tk.wim[q] == 0.f) {  // a branch, as in zgemm_f64_kernel
 #pragma unroll
-    for (int a = 0; a < TM; a++)
+      for (int a = 0; a < TM; a++)
 #pragma unroll
-      for (int b = 0; b < TN; b++) {
-        if (q == 0 && w.x == 1.0 && w.y == 0.0) acc[a][b] = part[a][b];
-        else {
+        for (int b = 0; b < TN; b++) acc[a][b] = part[a][b];
+    } else {
+      __syncwarp(__activemask());
+      const double2 w = make_double2((double)Tk.wre[q], (double)Tk.wim[q]);
+#pragma unroll
+      for (int a = 0; a < TM; a++)
+#pragma unroll
+        for (int b = 0; b < TN; b++) {
           const double2 t = cmul(w, part[a][b]);
           acc[a][b].x += t.x;
           acc[a][b].y += t.y;
         }
-      }
+    }
   }
 #pragma unroll
   for (int a = 0; a < TM; a++)
@@ -310,7 +320,7 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
   double re = 0.0, im = 0.0;
   float abf = 0.f;
   // two FMAs into each accumulator per element (the FP64 pipe is the bound)
-  if (T.mode == 0) {
+  if ((T.mode & 1) == 0) {
     for (int e = threadIdx.x; e < n2; e += TPB) {
       double2 x = T.X[e], y = T.Y[e];
       re = fma(x.x, y.x, re);
@@ -338,7 +348,8 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
   if (threadIdx.x >= 32) return;
   const double vi = __shfl_sync(0xffffffffu, v, 1);
   if (threadIdx.x == 0) {
-    *T.out = cmul(make_double2((double)T.coef[0], (double)T.coef[1]), make_double2(v, vi));
+    const double2 z = make_double2(v, vi);
+    *T.out = T.mode & 2 ? z : cmul(make_double2((double)T.coef[0], (double)T.coef[1]), z);
     if (want_abs) {
       float ab = reda[0];
 #pragma unroll
@@ -432,6 +443,24 @@ __global__ void rowsum_kernel(const double2* __restrict__ rows, int nrows, const
   out[(size_t)p * out_pair_stride + o] = make_double2(re, im);
 }
 
+// out[p][o] = sum of coef_r tr[p][tix[r]] over the rows r of output o, in row order.
+__global__ void rowsum_coef_kernel(const double2* __restrict__ tr, int ntr, const int* __restrict__ off,
+                                   const int* __restrict__ idx, const int* __restrict__ tix,
+                                   const float* __restrict__ coef, int nout, int npair, double2* __restrict__ out) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= npair * nout) return;
+  const int p = g / nout, o = g % nout, k1 = off[o + 1];
+  double re = 0.0, im = 0.0;
+#pragma unroll 4
+  for (int k = off[o]; k < k1; k++) {
+    const int r = idx[k];
+    const double2 v = cmul(make_double2(coef[2 * r], coef[2 * r + 1]), tr[(size_t)p * ntr + tix[r]]);
+    re += v.x;
+    im += v.y;
+  }
+  out[g] = make_double2(re, im);
+}
+
 __global__ void rowsum_refine_kernel(const double2* __restrict__ rows, const double* __restrict__ rabs, int nrows,
                                      const int* __restrict__ off, const int* __restrict__ idx, int nout, int npair,
                                      double2* __restrict__ out, double eps_over_tol, int* __restrict__ count,
@@ -466,9 +495,10 @@ __global__ void rowsum_coef_refine_kernel(const double2* __restrict__ tr, const 
                                           int* __restrict__ count, int* __restrict__ list, int pair_base) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= npair * nout) return;
-  const int p = g / nout, o = g % nout;
+  const int p = g / nout, o = g % nout, k1 = off[o + 1];
   double re = 0.0, im = 0.0, sc = 0.0;
-  for (int k = off[o]; k < off[o + 1]; k++) {
+#pragma unroll 4  // three dependent loads a row: 20 us for rho's 768 rows, one after another
+  for (int k = off[o]; k < k1; k++) {
     const int r = idx[k];
     const size_t t = (size_t)p * ntr + tix[r];
     const double cr = coef[2 * r], ci = coef[2 * r + 1];
@@ -634,12 +664,12 @@ int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, do
   return CTR_OK;
 }
 
-int launch_rowsum(const double2* rows, int nrows, const int* off, const int* idx, int nout, int npair,
-                  double2* out, size_t out_pair_stride, cudaStream_t s) {
-  int n = npair * nout;
+int launch_rowsum_coef(const double2* tr, int ntr, const int* off, const int* idx, const int* tix, const float* coef,
+                       int nout, int npair, double2* out, cudaStream_t s) {
+  const int n = npair * nout;
   if (n == 0) return CTR_OK;
   TimedLaunch tl(s, "rowsum");
-  rowsum_kernel<<<(n + 255) / 256, 256, 0, s>>>(rows, nrows, off, idx, nout, npair, out, out_pair_stride);
+  rowsum_coef_kernel<<<(n + 63) / 64, 64, 0, s>>>(tr, ntr, off, idx, tix, coef, nout, npair, out);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
 }
@@ -671,7 +701,7 @@ int launch_rowsum_coef_refine(const double2* tr, const double* trabs, int ntr, c
   const int n = npair * nout;
   if (n == 0) return CTR_OK;
   TimedLaunch tl(s, "rowsum_refine");
-  rowsum_coef_refine_kernel<<<(n + 255) / 256, 256, 0, s>>>(tr, trabs, ntr, off, idx, tix, coef, nout, npair, out,
+  rowsum_coef_refine_kernel<<<(n + 63) / 64, 64, 0, s>>>(tr, trabs, ntr, off, idx, tix, coef, nout, npair, out,
                                                              eps_over_tol, count, list, pair_base);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
