@@ -32,7 +32,6 @@
 // two pairs of elementals, and the pi pi diagrams are traces of 4x4 spin-block
 // matrices whose co-factors are a few four-term block products a pair (below).
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -214,6 +213,13 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const double* __restri
   if (threadIdx.x == 0) grad[k] += s / f[k];
 }
 
+int launch_grad_reduce(const double* buf, int nrow, int N, const double* f, double* grad, cudaStream_t s) {
+  TimedLaunch tl(s, "grad_reduce");
+  grad_reduce_kernel<<<N, 256, 0, s>>>(buf, nrow, N, f, grad);
+  CTR_CUDA(cudaGetLastError());
+  return CTR_OK;
+}
+
 // Diagonal reductions of a task list, then grad += (sum of their rows) / f where the
 // list has gradient rows (nrow > 0).
 int launch_diag(const std::vector<DiagTask>& tasks, int nrow, int N, const double* f, double2* vals, double* grad,
@@ -237,13 +243,202 @@ int launch_diag(const std::vector<DiagTask>& tasks, int nrow, int N, const doubl
     }
     CTR_CUDA(cudaGetLastError());
   }
-  if (nrow > 0) {
-    TimedLaunch tl(s, "grad_reduce");
-    grad_reduce_kernel<<<N, 256, 0, s>>>((const double*)dbuf, nrow, N, f, grad);
-    CTR_CUDA(cudaGetLastError());
-  }
+  if (nrow > 0) CTR_TRY(launch_grad_reduce((const double*)dbuf, nrow, N, f, grad, s));
   return CTR_OK;
 }
+
+// Sums over pairs of blocks.  A group's elementwise products
+//   S[k][m] = sum_j i^u_j X_j[k][m] Y_j[m][k]   (X_j, Y_j conjugated where bit 2 of u_j is set)
+// hold all that its traces' value and gradient need: their sum over the first nval
+// terms is the value, and the row and column sums of Re(w S) are the terms of
+// f_k d/df_k at the two indices the traces are cut at.  So a term takes 4 FMAs an
+// element, where a diagonal of X Y and one of Y X took 8 in two passes over its
+// blocks.  One CTA a group and tile of S, which stays in registers over the terms;
+// the tile's edge is Nev / ceil(Nev / 32), so that no lane of the FP64 pipe, the
+// bound, works on padding.  Nev = 100, rho at 512 pairs and pi pi at 64: 60 000 terms
+// in 4.7 ms (4.1 ms of FMAs) where the diagonals took 10.9.
+struct PairTerm {
+  const double2* x;
+  const double2* y;
+  int unit;  // u_j
+  int pad;
+};
+struct PairGroup {
+  int first, n;     // terms
+  int nval;         // terms of the value, 0: none wanted
+  int row;          // first gradient row (2 nt rows), -1: none wanted
+  double scale;     // of S
+  double wre, wim;  // weight, times *wp where wp is set
+  const double2* wp;
+};
+__device__ __forceinline__ double flip_sign(double v, int mask) {
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
+}
+
+constexpr int PS_T = 32, PS_J = 4, PS_TPB = PS_T * PS_T / PS_J;
+
+__global__ void __launch_bounds__(PS_TPB) pair_sums_kernel(const PairGroup* __restrict__ groups,
+                                                           const PairTerm* __restrict__ terms, int N, int T, int nt,
+                                                           double* __restrict__ buf, double2* __restrict__ part) {
+  __shared__ double2 ys[2][PS_T * (PS_T + 1)];  // Y's tile, transposed
+  __shared__ double red[PS_TPB / 32][2];
+  const PairGroup G = groups[blockIdx.x / (nt * nt)];
+  const int tile = blockIdx.x % (nt * nt), tk = tile / nt, tm = tile % nt, k0 = tk * T, m0 = tm * T;
+  const int nk = min(T, N - k0), nm = min(T, N - m0);
+  // element e of the tile: row e / T, column e % T of X's and of Y's tile
+  int xo[PS_J], yo[PS_J], rd[PS_J], wr[PS_J];
+#pragma unroll
+  for (int j = 0; j < PS_J; j++) {
+    const int e = threadIdx.x + j * (int)blockDim.x, r = e / T, q = e - r * T;
+    xo[j] = r < nk && q < nm ? (k0 + r) * N + m0 + q : -1;
+    yo[j] = r < nm && q < nk ? (m0 + r) * N + k0 + q : -1;
+    rd[j] = r < T ? r * (T + 1) + q : 0;
+    wr[j] = r < T ? q * (T + 1) + r : -1;
+  }
+  double2 x[PS_J], y[PS_J], S[PS_J];
+  double2 v = make_double2(0.0, 0.0);
+  int unit = 0;
+#pragma unroll
+  for (int j = 0; j < PS_J; j++) S[j] = make_double2(0.0, 0.0);
+  auto load = [&](int i) {
+    const PairTerm P = terms[G.first + i];
+    unit = P.unit;
+#pragma unroll
+    for (int j = 0; j < PS_J; j++) {
+      x[j] = xo[j] >= 0 ? P.x[xo[j]] : make_double2(0.0, 0.0);
+      y[j] = yo[j] >= 0 ? P.y[yo[j]] : make_double2(0.0, 0.0);
+    }
+  };
+  load(0);
+  for (int i = 0; i < G.n; i++) {
+    double2* const Y = ys[i & 1];
+    double2 a[PS_J];
+    // a = i^u x, signs as integer operations (a negation of a double takes the FP64 pipe)
+    const int conj = unit & 4 ? 1 << 31 : 0, neg = unit & 2 ? 1 << 31 : 0;
+    const bool swap = unit & 1;
+    const int sx = swap ? neg ^ conj ^ (1 << 31) : neg, sy = swap ? neg : neg ^ conj;
+#pragma unroll
+    for (int j = 0; j < PS_J; j++) {
+      if (wr[j] >= 0) Y[wr[j]] = make_double2(y[j].x, flip_sign(y[j].y, conj));
+      a[j].x = flip_sign(swap ? x[j].y : x[j].x, sx);
+      a[j].y = flip_sign(swap ? x[j].x : x[j].y, sy);
+    }
+    if (i + 1 < G.n) load(i + 1);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PS_J; j++) cmac(S[j], a[j], Y[rd[j]]);
+    if (i + 1 == G.nval) {
+#pragma unroll
+      for (int j = 0; j < PS_J; j++) {
+        v.x += S[j].x;
+        v.y += S[j].y;
+      }
+    }
+  }
+  if (G.nval > 0) {
+    for (int o = 16; o; o >>= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = v.x, red[threadIdx.x >> 5][1] = v.y;
+  }
+  __syncthreads();
+  if (G.nval > 0 && threadIdx.x == 0) {
+    double2 z = make_double2(red[0][0], red[0][1]);
+    for (int w = 1; w < (int)blockDim.x / 32; w++) {
+      z.x += red[w][0];
+      z.y += red[w][1];
+    }
+    part[blockIdx.x] = make_double2(G.scale * z.x, G.scale * z.y);
+  }
+  if (G.row < 0) return;
+  double2 w = make_double2(G.scale * G.wre, G.scale * G.wim);
+  if (G.wp) w = cmul(w, *G.wp);
+  double* const R = (double*)ys[0];
+#pragma unroll
+  for (int j = 0; j < PS_J; j++)
+    if (wr[j] >= 0) R[rd[j]] = w.x * S[j].x - w.y * S[j].y;
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * T; t += blockDim.x) {
+    double s = 0.0;
+    if (t < T) {
+      if (t >= nk) continue;
+      for (int q = 0; q < nm; q++) s += R[t * (T + 1) + q];
+      buf[(size_t)(G.row + tm) * N + k0 + t] = s;
+    } else {
+      if (t - T >= nm) continue;
+      for (int r = 0; r < nk; r++) s += R[r * (T + 1) + t - T];
+      buf[(size_t)(G.row + nt + tk) * N + m0 + t - T] = s;
+    }
+  }
+}
+
+// out[ent[g]] = sum of the group's tiles' parts.
+__global__ void pair_value_kernel(const double2* __restrict__ part, int ntile, const int* __restrict__ ent, int n,
+                                  double2* __restrict__ out) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n) return;
+  double2 z = part[(size_t)g * ntile];
+  for (int t = 1; t < ntile; t++) {
+    z.x += part[(size_t)g * ntile + t].x;
+    z.y += part[(size_t)g * ntile + t].y;
+  }
+  out[ent[g]] = z;
+}
+
+// Power u of i with c = |c| i^u, -1 where there is none.
+int unit_of(float re, float im) {
+  if (im == 0.f) return re > 0.f ? 0 : 2;
+  if (re == 0.f) return im > 0.f ? 1 : 3;
+  return -1;
+}
+
+// A list of groups; run: values to out[ent[g]] (one entry a group, where ent is not
+// empty) and grad += (gradient terms) / f where grad is set.
+struct PairList {
+  std::vector<PairGroup> g;
+  std::vector<PairTerm> t;
+  std::vector<int> ent;
+  void begin(double2 w, const double2* wp = nullptr, double scale = 1.0) {
+    g.push_back({(int)t.size(), 0, 0, -1, scale, w.x, w.y, wp});
+  }
+  void term(const double2* x, const double2* y, int unit = 0) {
+    t.push_back({x, y, unit, 0});
+    g.back().n++;
+  }
+  int run(int N, const double* f, double2* out, double* grad, cudaStream_t s) {
+    if (g.empty()) return CTR_OK;
+    const int nt = (N + PS_T - 1) / PS_T, T = (N + nt - 1) / nt;
+    const long long grid = (long long)g.size() * nt * nt;
+    if (grid > 0x7fffffffLL) return fail(CTR_ERR_ARG, "profile gradient: too many groups (%zu)", g.size());
+    if (grad)
+      for (size_t k = 0; k < g.size(); k++) g[k].row = (int)k * 2 * nt;
+    void *d[3], *dbuf = nullptr, *dpart = nullptr;
+    CTR_TRY(upload_group(WS_ROWTASKS,
+                         {{g.data(), g.size() * sizeof(PairGroup)},
+                          {t.data(), t.size() * sizeof(PairTerm)},
+                          {ent.data(), ent.size() * sizeof(int)}},
+                         d, s));
+    const int nrow = grad ? (int)g.size() * 2 * nt : 0;
+    if (grad) CTR_TRY(workspace(WS_ROWS).get((size_t)nrow * N * sizeof(double), &dbuf));
+    if (!ent.empty()) CTR_TRY(workspace(WS_ROWABS).get((size_t)grid * sizeof(double2), &dpart));
+    {
+      TimedLaunch tl(s, "pair_sums");
+      const int tpb = std::max(32, (T * T + PS_J * 32 - 1) / (PS_J * 32) * 32);
+      pair_sums_kernel<<<(unsigned)grid, tpb, 0, s>>>((const PairGroup*)d[0], (const PairTerm*)d[1], N, T, nt,
+                                                      (double*)dbuf, (double2*)dpart);
+      CTR_CUDA(cudaGetLastError());
+    }
+    if (!ent.empty()) {
+      TimedLaunch tl(s, "pair_value");
+      const int n = (int)ent.size();
+      pair_value_kernel<<<(n + 63) / 64, 64, 0, s>>>((const double2*)dpart, nt * nt, (const int*)d[2], n, out);
+      CTR_CUDA(cudaGetLastError());
+    }
+    if (grad) CTR_TRY(launch_grad_reduce((const double*)dbuf, nrow, N, f, grad, s));
+    return CTR_OK;
+  }
+};
 
 // ------------------------------------------------------------- chain program
 inline int64_t factor_key(const ctr_factor& F) {
@@ -502,8 +697,6 @@ int check_f(int N, const double* f, cudaStream_t s) {
   return CTR_OK;
 }
 
-inline double2 cw(double2 w, double re, double im) { return make_double2(w.x * re - w.y * im, w.x * im + w.y * re); }
-
 int check_engine(int engine, int nev) {
   if (engine != CTR_ENGINE_FP64 && engine != CTR_ENGINE_SPLIT) return fail(CTR_ERR_ARG, "unknown engine %d", engine);
   return CTR_OK;
@@ -520,46 +713,6 @@ struct Arena {
     return p;
   }
 };
-
-// A list of diagonal reductions; add(x, y, w): both diag(x y) and diag(y x).
-struct DiagList {
-  std::vector<DiagTask> t;
-  int nrow = 0;
-  void one(const double2* x, const double2* y, double2 w, const double2* wp, bool row, int vout) {
-    DiagTask d;
-    std::memset(&d, 0, sizeof(d));
-    d.x = x;
-    d.y = y;
-    d.wp = wp;
-    d.wre = w.x;
-    d.wim = w.y;
-    d.out = row ? nrow++ : -1;
-    d.vout = vout;
-    t.push_back(d);
-  }
-  void both(const double2* x, const double2* y, double2 w, const double2* wp = nullptr) {
-    one(x, y, w, wp, true, -1);
-    one(y, x, w, wp, true, -1);
-  }
-  void value(const double2* x, const double2* y, int vout) {
-    one(x, y, make_double2(0.0, 0.0), nullptr, false, vout);
-  }
-};
-
-// out[e] = sum_k coef[k] vals[slot[k]] over k in [off[i], off[i + 1]), e = ent[i].
-__global__ void entry_sum_kernel(const double2* __restrict__ vals, const int* __restrict__ off,
-                                 const int* __restrict__ slot, const float2* __restrict__ coef,
-                                 const int* __restrict__ ent, int n, double2* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double re = 0.0, im = 0.0;
-  for (int k = off[i]; k < off[i + 1]; k++) {
-    const double2 v = cmul(make_double2((double)coef[k].x, (double)coef[k].y), vals[slot[k]]);
-    re += v.x;
-    im += v.y;
-  }
-  out[ent[i]] = make_double2(re, im);
-}
 
 // Pairs (tf * Nt + ti) with a nonzero weight, those of one source time together.
 std::vector<int> weighted_pairs(int Nt, int nout, const double2* w) {
@@ -642,57 +795,33 @@ int rho_vjp(const Ctx& c, const double2* prop, const double2* phis, const double
       const size_t m = side ? pb.by_tf[g].size() : pb.by_ti[g].size();
       return bs[side][g] + (((size_t)(op * kinds + kind) * m + pos) * 16 + b) * N2;
     };
-    DiagList dl;
-    std::vector<int> off(1, 0), slot, ent;
-    std::vector<float2> coef;
-    int nval = 0;
+    // an output's 16 rows: its value, and f d/df at Phi_L's right and Phi_R's left index,
+    // from the first cut; the other two indices from the second one's conjugates
+    PairList pl;
     for (int i = 0; i < np; i++) {
       const int pr = pairs[pb.ent[i]];
-      std::map<std::array<int, 4>, std::pair<int, double2>> tr;  // (cd, L, ab, R) -> value slot, weight
       for (int o = 0; o < 48; o++) {
         const double2 wo = w[(size_t)pr * 48 + o];
         if (wo.x == 0.0 && wo.y == 0.0) continue;
-        for (int is = 0; is < 16; is++) {
-          const int r = o * 16 + is;
-          const int16_t* sp = T.rho_spin[r];
-          const std::array<int, 4> key = {sp[2] * 4 + sp[3], T.rho_lprp[r][0], sp[0] * 4 + sp[1], T.rho_lprp[r][1]};
-          auto it = tr.emplace(key, std::make_pair(nval, make_double2(0.0, 0.0))).first;
-          if (it->second.first == nval) nval++;
-          const double2 x = cw(wo, T.rho_coef[r][0], T.rho_coef[r][1]);
-          it->second.second.x += x.x;
-          it->second.second.y += x.y;
-          slot.push_back(it->second.first);
-          coef.push_back(make_float2(T.rho_coef[r][0], T.rho_coef[r][1]));
+        // the rows' coefficients are one magnitude, a power of two, times powers of i
+        auto mag = [&](int r) { return std::max(std::fabs(T.rho_coef[r][0]), std::fabs(T.rho_coef[r][1])); };
+        pl.begin(wo, nullptr, mag(o * 16));
+        for (int kind = 0; kind < kinds; kind++)
+          for (int is = 0; is < 16; is++) {
+            const int r = o * 16 + is, u = unit_of(T.rho_coef[r][0], T.rho_coef[r][1]);
+            if (u < 0 || mag(r) != mag(o * 16)) return fail(CTR_ERR_ARG, "rho row %d: unexpected coefficient", r);
+            const int16_t* sp = T.rho_spin[r];
+            const int cd = sp[2] * 4 + sp[3], ab = sp[0] * 4 + sp[1], l = il[T.rho_lprp[r][0]], q = ir[T.rho_lprp[r][1]];
+            pl.term(blk(0, i, l, kind, kind ? ab : cd), blk(1, i, q, kind, kind ? cd : ab), u + 4 * kind);
+          }
+        if (corr) {
+          pl.g.back().nval = 16;
+          pl.ent.push_back(pr * 48 + o);
         }
-        off.push_back((int)slot.size());
-        ent.push_back(pr * 48 + o);
-      }
-      for (const auto& e : tr) {
-        const double2* A = blk(0, i, il[e.first[1]], 0, e.first[0]);
-        const double2* Bt = blk(1, i, ir[e.first[3]], 0, e.first[2]);
-        const double2 wt = e.second.second;
-        dl.one(A, Bt, wt, nullptr, grad != nullptr, corr ? e.second.first : -1);
-        if (!grad) continue;
-        dl.one(Bt, A, wt, nullptr, true, -1);
-        dl.both(blk(0, i, il[e.first[1]], 1, e.first[2]), blk(1, i, ir[e.first[3]], 1, e.first[0]),
-                make_double2(wt.x, -wt.y));
       }
     }
     CTR_TRY(run_grids(c, g0, WS_TASKS));
-    void* dv = nullptr;
-    if (corr) CTR_TRY(workspace(WS_ROWABS).get((size_t)std::max(1, nval) * sizeof(double2), &dv));
-    CTR_TRY(launch_diag(dl.t, dl.nrow, N, f, (double2*)dv, grad, c.s));
-    if (corr) {
-      void* d[4];
-      CTR_TRY(upload_group(WS_MISC, {{off.data(), off.size() * sizeof(int)}, {slot.data(), slot.size() * sizeof(int)},
-                                     {coef.data(), coef.size() * sizeof(float2)}, {ent.data(), ent.size() * sizeof(int)}},
-                           d, c.s));
-      TimedLaunch tl(c.s, "entry_sum");
-      const int n = (int)ent.size();
-      entry_sum_kernel<<<(n + 127) / 128, 128, 0, c.s>>>((const double2*)dv, (const int*)d[0], (const int*)d[1],
-                                                         (const float2*)d[2], (const int*)d[3], n, corr);
-      CTR_CUDA(cudaGetLastError());
-    }
+    CTR_TRY(pl.run(N, f, corr, grad, c.s));
   }
   return CTR_OK;
 }
@@ -1035,7 +1164,17 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
     double2* vals = (double2*)dv;
     double2* wk = vals + (size_t)np * 64;
     if (!hor) CTR_CUDA(cudaMemsetAsync(vals, 0, (size_t)np * 64 * sizeof(double2), c.s));
-    DiagList dv_l, dg;
+    std::vector<DiagTask> vt;
+    PairList pl;
+    auto value = [&](const double2* x, const double2* y, int slot) {
+      DiagTask d;
+      std::memset(&d, 0, sizeof(d));
+      d.x = x;
+      d.y = y;
+      d.out = -1;
+      d.vout = slot;
+      vt.push_back(d);
+    };
     std::vector<int> ent(np);
     std::vector<double2> wsf((size_t)np * 2);
     for (int i = 0; i < np; i++) {
@@ -1046,32 +1185,33 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
       wsf[2 * i + 1] = make_double2(wp[3].x * wfi, wp[3].y * wfi);
       for (int b = 0; b < 16; b++) {
         // Tr[R_{a b} J_{b a}] g5(a)
-        dv_l.value(M[(size_t)cSq * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + b);
-        dv_l.value(M[(size_t)cDt * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + 16 + b);
+        value(M[(size_t)cSq * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + b);
+        value(M[(size_t)cDt * Nt + ti] + (size_t)b * N2, rc(bJ[i], b % 4, b / 4), v0 + 16 + b);
         if (hor)
-          dv_l.value(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + (b % 4) * 4 + b / 4) * N2, v0 + 32 + b);
+          value(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + (b % 4) * 4 + b / 4) * N2, v0 + 32 + b);
       }
       for (int k = 0; k < 4; k++)
-        for (int a = 0; a < 4; a++) dv_l.value(P(tx[k], tf), Pm(ty[k], i, a, a), v0 + 48 + k * 4 + a);
+        for (int a = 0; a < 4; a++) value(P(tx[k], tf), Pm(ty[k], i, a, a), v0 + 48 + k * 4 + a);
       if (!g) continue;
       if (hor) {
-        const double2 wh = make_double2(wp[4].x * wdh, wp[4].y * wdh);
+        pl.begin(make_double2(wp[4].x * wdh, wp[4].y * wdh));
         for (int b = 0; b < 16; b++) {
           const int bt = (b % 4) * 4 + b / 4;
-          dg.both(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + bt) * N2, wh);
-          dg.both(bY[i] + (size_t)b * N2, bY[i] + (size_t)(16 + bt) * N2, wh);
+          pl.term(bX[i] + (size_t)b * N2, bX[i] + (size_t)(16 + bt) * N2);
+          pl.term(bY[i] + (size_t)b * N2, bY[i] + (size_t)(16 + bt) * N2);
         }
         for (int y = 0; y < 2; y++)
-          for (int u = 0; u < 4; u++) dg.both(P(P1 + y, ti), bN[i] + (size_t)(u * 2 + y) * N2, wh);
+          for (int u = 0; u < 4; u++) pl.term(P(P1 + y, ti), bN[i] + (size_t)(u * 2 + y) * N2);
       }
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < 4; k++) {
+        pl.begin(make_double2(1.0, 0.0), wk + 4 * (size_t)i + k);
         for (int a = 0; a < 4; a++) {
-          const double2* wkp = wk + 4 * (size_t)i + k;
-          dg.both(P(tx[k], tf), Pm(ty[k], i, a, a), make_double2(1.0, 0.0), wkp);
-          dg.both(P(P1 + ty[k], ti), bO[i] + (size_t)((tx[k] - P3) * 4 + a) * N2, make_double2(1.0, 0.0), wkp);
+          pl.term(P(tx[k], tf), Pm(ty[k], i, a, a));
+          pl.term(P(P1 + ty[k], ti), bO[i] + (size_t)((tx[k] - P3) * 4 + a) * N2);
         }
+      }
     }
-    CTR_TRY(launch_diag(dv_l.t, 0, N, f, vals, nullptr, c.s));
+    CTR_TRY(launch_diag(vt, 0, N, f, vals, nullptr, c.s));
     CTR_TRY(upload_group(WS_MISC, {{ent.data(), ent.size() * sizeof(int)}, {wsf.data(), wsf.size() * sizeof(double2)}},
                          dw, c.s));
     {
@@ -1080,7 +1220,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
                                                                  wdt, wst, wfi, wdh, corr, wk);
       CTR_CUDA(cudaGetLastError());
     }
-    CTR_TRY(launch_diag(dg.t, dg.nrow, N, f, nullptr, grad, c.s));
+    CTR_TRY(pl.run(N, f, nullptr, grad, c.s));
     if (!g) continue;
     // ---- co-factors of the batch, summed per time slice
     CombList sum;
@@ -1124,7 +1264,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
     void* mem;
     CTR_TRY(workspace(WS_SCRATCH).get(ns * per_sl, &mem));
     std::vector<GridTask> g0;
-    DiagList dl;
+    PairList pl;
     for (size_t k = 0; k < ns; k++) {
       const Slice& S = sl[s0 + k];
       const double2* D = diag + (size_t)S.t * blk16;
@@ -1153,15 +1293,16 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
         g0.push_back(std::move(C));
         g0.push_back(std::move(E));
       }
+      pl.begin(make_double2(1.0, 0.0));
       for (int b = 0; b < 16; b++) {
         const int bt = (b % 4) * 4 + b / 4;  // tau_ab against F_ba
-        const double2 sg = make_double2((double)G5[S.row_sign ? b % 4 : b / 4], 0.0);
-        dl.both(o + (size_t)b * N2, o + blk16 + (size_t)bt * N2, sg);
-        dl.both(o + 2 * blk16 + (size_t)b * N2, o + 3 * blk16 + (size_t)bt * N2, sg);
+        const int u = G5[S.row_sign ? b % 4 : b / 4] < 0 ? 2 : 0;
+        pl.term(o + (size_t)b * N2, o + blk16 + (size_t)bt * N2, u);
+        pl.term(o + 2 * blk16 + (size_t)b * N2, o + 3 * blk16 + (size_t)bt * N2, u);
       }
     }
     CTR_TRY(run_grids(c, g0, WS_TASKS));
-    CTR_TRY(launch_diag(dl.t, dl.nrow, N, f, nullptr, grad, c.s));
+    CTR_TRY(pl.run(N, f, nullptr, grad, c.s));
   }
   return CTR_OK;
 }

@@ -162,3 +162,26 @@ def test_profile_gradients_block_form(cuda, n, iso, engine, tol):
         assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
         want = torch.autograd.grad(loss, ft, retain_graph=True)[0].numpy()
         assert np.abs(g - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n", [1, 31, 64, 65])
+def test_profile_sums_tile_edges(cuda, n):
+    """The gradients' sums over pairs of blocks take tiles of Nev / ceil(Nev / 32): one
+    and several tiles, whole and ragged, against autograd; 1e-11 as for the block form."""
+    from contractions_code_scattering_gb300 import adjoint
+    from oracle import torch_ref as R
+    nt, on = 2, [0, 9, 47]
+    prop = synth.make_prop(nt, n, seed=950 + n)
+    rng = np.random.default_rng(951 + n)
+    mom5 = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(5)], axis=1)
+    f = adjoint.default_profile(n, seed=952)
+    w = np.zeros((nt, nt, 48), complex)
+    w[1, 0, on] = rng.normal(size=3) + 1j * rng.normal(size=3)
+    got, g = api.rho_profile_vjp(_dev(prop, cuda), _dev(mom5, cuda), _dev(f, cuda), _dev(w, cuda), engine="fp64")
+    ft = torch.tensor(f, requires_grad=True)
+    v = R.rho_pair(torch.from_numpy(prop), R.profiled(ft, torch.from_numpy(np.ascontiguousarray(mom5))), 1, 0, on)
+    loss = (torch.from_numpy(w[1, 0, on]) * v).real.sum()
+    want = torch.autograd.grad(loss, ft)[0].numpy()
+    ref = v.detach().numpy()
+    assert np.abs(got.cpu().numpy()[1, 0, on] - ref).max() <= 1e-11 * np.abs(ref).max()
+    assert np.abs(g.cpu().numpy() - want).max() <= 1e-11 * np.abs(want).max()
