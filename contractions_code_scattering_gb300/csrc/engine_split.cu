@@ -420,6 +420,7 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
     // tile walk of each GEMM (autotuned; idempotent, so candidates re-run on the same data)
     SplitGemmBatch GA{(const SplitGemmInst*)d_ga, mtT, F.ntiles, nchunk, ncd * N, nL * N, ldA};
     SplitGemmBatch GB{(const SplitGemmInst*)d_gb, F.mtiles, ntT, nchunk, nR * N, nab * N, ldB};
+    GA.step = GB.step = split_tail_step(N);
     for (SplitGemmBatch* G : {&GA, &GB}) {
       char gshape[96];
       snprintf(gshape, sizeof(gshape), "std,m=%d,n=%d,k=%d", G->mtiles, G->ntiles, G->nchunk);
@@ -630,6 +631,7 @@ int zgemm_split_batched(int N, int nb, const double* const* x, const double* con
   CTR_TRY(launch_slice_right((const SliceRightJob*)dr, nb, N, nchunk, nt, stream, 1));
   CTR_TRY(upload(WS_GEMM_A, gi.data(), nb * sizeof(SplitGemmInst), &dg, stream));
   SplitGemmBatch G{(const SplitGemmInst*)dg, 1, nt, nchunk, N, N, ldo};
+  G.step = split_tail_step(N);
   CTR_TRY(launch_split_gemm(G, nb, d_err, stream));
   for (int b = 0; b < nb; b++) {
     TimedLaunch tl(stream, "ff_to_f64");
@@ -672,6 +674,7 @@ int split_levels(int N, const double* x, const double* y, float* levels, cudaStr
   CTR_TRY(launch_slice_right((const SliceRightJob*)dr, 1, N, nchunk, nt, stream));
   CTR_TRY(upload(WS_GEMM_A, &gi, sizeof(gi), &dg, stream));
   SplitGemmBatch G{(const SplitGemmInst*)dg, 1, nt, nchunk, N, N, SPLIT_M, levels};
+  G.step = split_tail_step(N);
   return launch_split_gemm(G, 1, d_err, stream);
 }
 
@@ -894,6 +897,7 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
       CTR_TRY(launch_slice_task_right((const SliceTaskRJob*)d_rj, (int)rj.size(), N, nchunk, ntiles,
                                       (const int*)d_bexp, stream));
       SplitGemmBatch G{(const SplitGemmInst*)d_gi, 1, ntiles, nchunk, N, nb * N, SPLIT_M, nullptr, 1, N, 1};
+      G.step = split_tail_step(K);
       CTR_TRY(launch_split_gemm(G, ni, d_err, stream));
       if (!capturing()) g_split_products += (double)ni * nb * nterm;
     }
@@ -1042,6 +1046,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
                                       (const int*)d_bexp, stream));
       SplitGemmBatch B{(const SplitGemmInst*)d_gi, mtiles, ntiles, nchunk, ns * N, nb * N, mtiles * SPLIT_M,
                        nullptr, 1, N, 1};
+      B.step = split_tail_step(K);
       // persistent tile walk (N tiles or M tiles innermost), autotuned per tile shape
       // by re-launching the GEMM on the same operands (it rewrites the same outputs)
       char gshape[96];

@@ -31,6 +31,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <type_traits>
 
 #include "kernels.h"
 #include "sm100_ptx.cuh"
@@ -137,6 +138,38 @@ __device__ __forceinline__ uint32_t core_offset(int row, int k) {
   return (uint32_t)((row >> 3) * 256 + ((k >> 3) & 1) * 128 + (row & 7) * 16 + (k & 7) * 2);
 }
 
+// One k (or pair of adjacent k) of a row or column in the last chunk of a packed
+// tail (split_tail_step): digit(s) gives its slice s, put(sub-tile, column, digit)
+// stores it.  k >= 16 / step is past the valid ones.
+template <int NS, class Digit, class Put>
+__device__ __forceinline__ void tail_left(int step, int k, Digit digit, Put put) {
+  const int lg = step == 4 ? 2 : 1, w = SPLIT_K >> lg;
+  if (k >= w) return;
+#pragma unroll
+  for (int s = 0; s < 8; s++)
+    if (s < NS)
+      put(s >> lg, (s & (step - 1)) * w + k, digit(s));
+    else if (s < ((NS + step - 1) & ~(step - 1)))
+      put(s >> lg, (s & (step - 1)) * w + k, decltype(digit(0)){});
+}
+template <int NS, class Digit, class Put>
+__device__ __forceinline__ void tail_right(int step, int k, Digit digit, Put put) {
+  const int w = step == 4 ? 4 : 8;
+  if (k >= w) return;
+#pragma unroll
+  for (int s = 0; s < NS; s++) {
+    const auto d = digit(s);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (q < step && s + q < NS) put(s + q, q * w + k, d);
+  }
+#pragma unroll
+  for (int q = 1; q < 4; q++)
+#pragma unroll
+    for (int m = 0; m < q; m++)
+      if (q < step) put(m, q * w + k, decltype(digit(0)){});
+}
+
 // Left operand: one M tile (128 stacked rows) of one operand instance.
 // Row r of the stack is row (r % nev) of block blk[r / nev]; element k of it
 // is blk[r/nev][(r%nev)*nev + k].  Output: [nchunk][SPLIT_A_STAGE] bytes and
@@ -170,6 +203,7 @@ __global__ void __launch_bounds__(256) slice_left_kernel(const SliceLeftJob* __r
   __syncthreads();
   uint8_t* dst_tile = J.out + (size_t)mt * nchunk * SPLIT_A_STAGE;
   constexpr int PER = SPLIT_M * SPLIT_K / 256;
+  const int step = split_tail_step(nev);
   for (int kc = 0; kc < nchunk; kc++) {
     // 128 rows x 16 k: 16 consecutive threads read one row segment (coalesced);
     // a thread's 8 loads are issued before any of them is sliced
@@ -188,6 +222,16 @@ __global__ void __launch_bounds__(256) slice_left_kernel(const SliceLeftJob* __r
       const int E = sexp[rr];
       bool nr, ni;
       const uint64_t Ur = round_fixed(f64_fixed(v.x, E, nr)), Ui = round_fixed(f64_fixed(v.y, E, ni));
+      if (step > 1 && kc == nchunk - 1) {
+        tail_left<SPLIT_NSLICE>(
+            step, kk, [&](int s) { return make_uint2(slice_bits(Ur, s, nr), slice_bits(Ui, s, ni)); },
+            [&](int sub, int col, uint2 d) {
+              uint8_t* t = stage + sub * 2 * SPLIT_A_SUB + core_offset(rr, col);
+              *(uint16_t*)t = (uint16_t)(d.x >> 16);
+              *(uint16_t*)(t + SPLIT_A_SUB) = (uint16_t)(d.y >> 16);
+            });
+        continue;
+      }
       const uint32_t off = core_offset(rr, kk);
 #pragma unroll
       for (int s = 0; s < SPLIT_NSLICE; s++) {
@@ -241,6 +285,7 @@ __global__ void __launch_bounds__(256) slice_right_kernel(const SliceRightJob* _
   __syncthreads();
   uint8_t* dst_tile = J.out + (size_t)nt * nchunk * SPLIT_B_STAGE;
   constexpr int PER = SPLIT_N * SPLIT_K / 256;
+  const int step = split_tail_step(nev);
   for (int kc = 0; kc < nchunk; kc++) {
     double2 vv[PER];
 #pragma unroll
@@ -257,6 +302,17 @@ __global__ void __launch_bounds__(256) slice_right_kernel(const SliceRightJob* _
       const int E = sexp[nn];
       bool nr, ni;
       const uint64_t Ur = round_fixed(f64_fixed(v.x, E, nr)), Ui = round_fixed(f64_fixed(v.y, E, ni));
+      if (step > 1 && kc == nchunk - 1) {
+        tail_right<SPLIT_NSLICE>(
+            step, kk, [&](int s) { return make_uint2(slice_bits(Ur, s, nr), slice_bits(Ui, s, ni)); },
+            [&](int sub, int col, uint2 d) {
+              uint8_t* t = stage + sub * 3 * SPLIT_B_SUB + core_offset(nn, col);
+              *(uint16_t*)t = (uint16_t)((d.y >> 16) ^ 0x8000u);
+              *(uint16_t*)(t + SPLIT_B_SUB) = (uint16_t)(d.x >> 16);
+              *(uint16_t*)(t + 2 * SPLIT_B_SUB) = (uint16_t)(d.y >> 16);
+            });
+        continue;
+      }
       const uint32_t off = core_offset(nn, kk);
 #pragma unroll
       for (int s = 0; s < SPLIT_NSLICE; s++) {
@@ -340,7 +396,7 @@ __global__ void __launch_bounds__(256) slice_left_staged_kernel(const SliceLeftJ
   static_assert(SLQ * SPLIT_K == 2 * 256, "two adjacent k per thread");
   const int rr = threadIdx.x >> 3, kk = (threadIdx.x & 7) * 2;
   const uint32_t off = core_offset(rr, kk);  // k and k + 1 are adjacent
-  const int E = sexp[rr];
+  const int E = sexp[rr], step = split_tail_step(nev);
   for (int kc = 0; kc < nchunk; kc++) {
     const int k = kc * SPLIT_K + kk;
     const double2 v0 = k < nev ? data[rr * nev + k] : make_double2(0.0, 0.0);
@@ -348,7 +404,21 @@ __global__ void __launch_bounds__(256) slice_left_staged_kernel(const SliceLeftJ
     bool nr0, ni0, nr1, ni1;
     const uint64_t Ur0 = round_fixed(f64_fixed(v0.x, E, nr0)), Ui0 = round_fixed(f64_fixed(v0.y, E, ni0));
     const uint64_t Ur1 = round_fixed(f64_fixed(v1.x, E, nr1)), Ui1 = round_fixed(f64_fixed(v1.y, E, ni1));
+    const bool tail = step > 1 && kc == nchunk - 1;
+    if (tail) {
+      constexpr int SUB = DIRECT ? SPLIT_A_SUB : 1024;
+      uint8_t* const t0 = DIRECT ? dst_tile + (size_t)kc * SPLIT_A_STAGE : stage;
+      tail_left<SPLIT_NSLICE>(
+          step, kk,
+          [&](int s) { return make_uint2(slice_pair(Ur0, nr0, Ur1, nr1, s), slice_pair(Ui0, ni0, Ui1, ni1, s)); },
+          [&](int sub, int col, uint2 d) {
+            uint8_t* t = t0 + sub * 2 * SUB + core_offset(rr, col);
+            *(uint32_t*)t = d.x;
+            *(uint32_t*)(t + SUB) = d.y;
+          });
+    }
     if constexpr (DIRECT) {
+      if (tail) break;
       uint8_t* d = dst_tile + (size_t)kc * SPLIT_A_STAGE + off;
 #pragma unroll
       for (int sl = 0; sl < SPLIT_NSLICE; sl++) {
@@ -358,6 +428,7 @@ __global__ void __launch_bounds__(256) slice_left_staged_kernel(const SliceLeftJ
     } else {
 #pragma unroll
       for (int sl = 0; sl < SPLIT_NSLICE; sl++) {
+        if (tail) break;
         *(uint32_t*)(stage + (sl * 2 + 0) * 1024 + off) = slice_pair(Ur0, nr0, Ur1, nr1, sl);
         *(uint32_t*)(stage + (sl * 2 + 1) * 1024 + off) = slice_pair(Ui0, ni0, Ui1, ni1, sl);
       }
@@ -426,7 +497,7 @@ __global__ void __launch_bounds__(256) slice_right_staged_kernel(const SliceRigh
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nn = (warp & 3) * 8 + (lane & 7), kk = ((warp >> 2) * 4 + (lane >> 3)) * 2;
   const uint32_t off = core_offset(nn, kk);  // k and k + 1 are adjacent
-  const int E = sexp[nn];
+  const int E = sexp[nn], step = split_tail_step(nev);
   for (int kc = 0; kc < nchunk; kc++) {
     const int k = kc * SPLIT_K + kk;
     const double2 v0 = k < nev ? data[k * SLQ + nn] : make_double2(0.0, 0.0);
@@ -434,7 +505,22 @@ __global__ void __launch_bounds__(256) slice_right_staged_kernel(const SliceRigh
     bool nr0, ni0, nr1, ni1;
     const uint64_t Ur0 = round_fixed(f64_fixed(v0.x, E, nr0)), Ui0 = round_fixed(f64_fixed(v0.y, E, ni0));
     const uint64_t Ur1 = round_fixed(f64_fixed(v1.x, E, nr1)), Ui1 = round_fixed(f64_fixed(v1.y, E, ni1));
+    const bool tail = step > 1 && kc == nchunk - 1;
+    if (tail) {
+      constexpr int SUB = DIRECT ? SPLIT_B_SUB : 1024;
+      uint8_t* const t0 = DIRECT ? dst_tile + (size_t)kc * SPLIT_B_STAGE : stage;
+      tail_right<SPLIT_NSLICE>(
+          step, kk,
+          [&](int s) { return make_uint2(slice_pair(Ur0, nr0, Ur1, nr1, s), slice_pair(Ui0, ni0, Ui1, ni1, s)); },
+          [&](int sub, int col, uint2 d) {
+            uint8_t* t = t0 + sub * 3 * SUB + core_offset(nn, col);
+            *(uint32_t*)t = d.y ^ BF16X2_SIGNS;
+            *(uint32_t*)(t + SUB) = d.x;
+            *(uint32_t*)(t + 2 * SUB) = d.y;
+          });
+    }
     if constexpr (DIRECT) {
+      if (tail) break;
       uint8_t* d = dst_tile + (size_t)kc * SPLIT_B_STAGE + off;
 #pragma unroll
       for (int sl = 0; sl < SPLIT_NSLICE; sl++) {
@@ -446,6 +532,7 @@ __global__ void __launch_bounds__(256) slice_right_staged_kernel(const SliceRigh
     } else {
 #pragma unroll
       for (int sl = 0; sl < SPLIT_NSLICE; sl++) {
+        if (tail) break;
         // planes -im, re, im (packed complex MMAs)
         const uint32_t pi = slice_pair(Ui0, ni0, Ui1, ni1, sl);
         *(uint32_t*)(stage + (sl * 3 + 0) * 1024 + off) = pi ^ BF16X2_SIGNS;
@@ -541,7 +628,7 @@ __global__ void __launch_bounds__(256) slice_task_left_kernel(const SliceTaskLJo
   uint8_t* stage = sm + 512;
   const SliceTaskLJob& J = jobs[blockIdx.x / nchunk];
   const int kc = blockIdx.x % nchunk;
-  const int K = J.nterm * nev;
+  const int K = J.nterm * nev, step = split_tail_step(K);
   if (threadIdx.x < SPLIT_M) {
     // row r over all K: the row (column, for a conjugate-transposed term) bounds of
     // the terms' blocks, shifted by the weights' exponents
@@ -577,6 +664,16 @@ __global__ void __launch_bounds__(256) slice_task_left_kernel(const SliceTaskLJo
     weighted_fixed(v[u], J.wexp[q], J.w[q] < 0.f, (J.dag >> q) & 1, E, Ur, nr, Ui, ni);
     Ur = round_fixed<C::NS>(Ur);
     Ui = round_fixed<C::NS>(Ui);
+    if (step > 1 && kc == nchunk - 1) {
+      tail_left<C::NS>(
+          step, kk, [&](int s) { return make_uint2(slice_bits(Ur, s, nr), slice_bits(Ui, s, ni)); },
+          [&](int sub, int col, uint2 d) {
+            uint8_t* t = stage + sub * 2 * C::A_SUB + core_offset(rr, col);
+            *(uint16_t*)t = (uint16_t)(d.x >> 16);
+            *(uint16_t*)(t + C::A_SUB) = (uint16_t)(d.y >> 16);
+          });
+      continue;
+    }
     const uint32_t off = core_offset(rr, kk);
 #pragma unroll
     for (int s = 0; s < C::NS; s++) {
@@ -650,6 +747,8 @@ __global__ void __launch_bounds__(256) slice_stack_left_kernel(const SliceStackL
   }
   __syncthreads();
   uint8_t* d0 = J.out + ((size_t)mt * nchunk + kc) * C::A_STAGE;
+  const int step = split_tail_step(K);
+  const bool tail = step > 1 && kc == nchunk - 1;
 #pragma unroll
   for (int u = 0; u < PER; u++) {
     const int rr = (threadIdx.x >> 3) + 32 * u;
@@ -661,6 +760,17 @@ __global__ void __launch_bounds__(256) slice_stack_left_kernel(const SliceStackL
       weighted_fixed(v[u][h], wexp[h], wneg[h], kdag[h], E, Ur[h], nr[h], Ui[h], ni[h]);
       Ur[h] = round_fixed<C::NS>(Ur[h]);
       Ui[h] = round_fixed<C::NS>(Ui[h]);
+    }
+    if (tail) {
+      tail_left<C::NS>(
+          step, 2 * kp,
+          [&](int s) { return make_uint2(slice_pair(Ur[0], nr[0], Ur[1], nr[1], s), slice_pair(Ui[0], ni[0], Ui[1], ni[1], s)); },
+          [&](int sub, int col, uint2 w) {
+            uint8_t* t = d0 + sub * 2 * C::A_SUB + core_offset(rr, col);
+            *(uint32_t*)t = w.x;
+            *(uint32_t*)(t + C::A_SUB) = w.y;
+          });
+      continue;
     }
     uint8_t* d = d0 + core_offset(rr, 2 * kp);
 #pragma unroll
@@ -730,6 +840,8 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
   }
   __syncthreads();
   uint8_t* d0 = J.out + ((size_t)nt * nchunk + kc) * C::B_STAGE;
+  const int step = split_tail_step(K);
+  const bool tail = step > 1 && kc == nchunk - 1;
 #pragma unroll
   for (int u = 0; u < PER; u++) {
     const int nn = (threadIdx.x >> 3) + 16 * u;
@@ -741,6 +853,18 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
       weighted_fixed(v[u][h], 0, false, dag[u][h], E, Ur[h], nr[h], Ui[h], ni[h]);
       Ur[h] = round_fixed<C::NS>(Ur[h]);
       Ui[h] = round_fixed<C::NS>(Ui[h]);
+    }
+    if (tail) {
+      tail_right<C::NS>(
+          step, 2 * kp,
+          [&](int s) { return make_uint2(slice_pair(Ur[0], nr[0], Ur[1], nr[1], s), slice_pair(Ui[0], ni[0], Ui[1], ni[1], s)); },
+          [&](int sub, int col, uint2 w) {
+            uint8_t* t = d0 + sub * 3 * C::B_SUB + core_offset(nn, col);
+            *(uint32_t*)t = w.y ^ BF16X2_SIGNS;
+            *(uint32_t*)(t + C::B_SUB) = w.x;
+            *(uint32_t*)(t + 2 * C::B_SUB) = w.y;
+          });
+      continue;
     }
     uint8_t* d = d0 + core_offset(nn, 2 * kp);
 #pragma unroll
@@ -882,14 +1006,17 @@ __device__ __forceinline__ void issue_row(uint32_t tbase, uint64_t a, uint64_t b
 // The slice pairs of group G in order of (left slice, plane, right slice).  Every level accumulator sees its MMAs in the same order
 // whatever the grouping, so the FP32 last level sums them in the same order and
 // the results do not depend on it.  adesc / bdesc describe sub-tile (slice 0,
-// plane 0) of the stage; the others are constant byte offsets.
-template <class C, int G, int I = 0>
+// plane 0) of the stage; the others are constant byte offsets.  STEP > 1: the last
+// chunk of a packed tail, whose MMA of left sub-tile I / STEP and right sub-tile J
+// sums the pairs (I + q, J - q).
+template <class C, int G, int STEP = 1, int I = 0>
 __device__ __forceinline__ void issue_pairs(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first_chunk) {
   static_assert(C::PACK, "packed complex operands");
   if constexpr (I < C::NS) {
-    issue_row<C, G, I, 0, 0, false>(tbase, desc_at(adesc, ((I * 2 + 0) * C::A_SUB) >> 4), bdesc, first_chunk);
-    issue_row<C, G, I, 1, 0, false>(tbase, desc_at(adesc, ((I * 2 + 1) * C::A_SUB) >> 4), bdesc, first_chunk);
-    issue_pairs<C, G, I + 1>(tbase, adesc, bdesc, first_chunk);
+    constexpr int a = I / STEP * 2 * C::A_SUB;
+    issue_row<C, G, I, 0, 0, false>(tbase, desc_at(adesc, a >> 4), bdesc, first_chunk);
+    issue_row<C, G, I, 1, 0, false>(tbase, desc_at(adesc, (a + C::A_SUB) >> 4), bdesc, first_chunk);
+    issue_pairs<C, G, STEP, I + STEP>(tbase, adesc, bdesc, first_chunk);
   }
 }
 
@@ -997,6 +1124,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
     if (lane == 0) {
       uint32_t g_chunk = 0;
       bool ok = true;
+      const uint32_t alast = g.step > 1 ? (C::NS + g.step - 1) / g.step * 2 * C::A_SUB : C::A_STAGE;
       for (int tile = blockIdx.x; tile < ntiles_total && ok; tile += gridDim.x) {
         int inst, mt, nt;
         tile_coords(g, tile, inst, mt, nt);
@@ -1010,8 +1138,9 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&full[s], C::A_STAGE + C::B_STAGE);
-          bulk_g2s(sA + s * C::A_STAGE, gA + (size_t)kc * C::A_STAGE, C::A_STAGE, &full[s]);
+          const uint32_t abytes = kc == g.nchunk - 1 ? alast : C::A_STAGE;
+          mbar_arrive_expect_tx(&full[s], abytes + C::B_STAGE);
+          bulk_g2s(sA + s * C::A_STAGE, gA + (size_t)kc * C::A_STAGE, abytes, &full[s]);
           bulk_g2s(sB + s * C::B_STAGE, gB + (size_t)kc * C::B_STAGE, C::B_STAGE, &full[s]);
         }
       }
@@ -1079,9 +1208,17 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
             issue_chunk<C>(tbase, adesc(st), bdesc(st), false);
           } else {
             // the last chunk: the last level first, drained beside the others' MMAs
-            issue_pairs<C, 0>(tbase, adesc(st), bdesc(st), false);
-            umma_commit(&tfull[0]);
-            issue_pairs<C, GROUP_REST>(tbase, adesc(st), bdesc(st), false);
+            auto last = [&](auto step) {
+              issue_pairs<C, 0, step.value>(tbase, adesc(st), bdesc(st), false);
+              umma_commit(&tfull[0]);
+              issue_pairs<C, GROUP_REST, step.value>(tbase, adesc(st), bdesc(st), false);
+            };
+            if (g.step == 4)
+              last(std::integral_constant<int, 4>());
+            else if (g.step == 2)
+              last(std::integral_constant<int, 2>());
+            else
+              last(std::integral_constant<int, 1>());
           }
           umma_commit(&empty[st]);
         }
@@ -2305,7 +2442,11 @@ static int launch_split_gemm_cfg(const SplitGemmBatch& g, int ninst, int* d_err,
   split_gemm_kernel<C><<<grid, gemm_threads<C>(), smem, s>>>(g, (int)total, d_err);
   CTR_CUDA(cudaGetLastError());
   // slice pairs i + j < NS, each two packed MMAs of M x 2BN x 16: 8 M BN 16 flops
-  if (!capturing()) *flops += (double)total * (C::NS * (C::NS + 1) / 2) * 8.0 * SPLIT_M * C::BN * SPLIT_K * g.nchunk;
+  constexpr int pairs = C::NS * (C::NS + 1) / 2;
+  int last = pairs;
+  if (g.step > 1)
+    for (int i = last = 0; i < C::NS; i += g.step) last += C::NS - i;
+  if (!capturing()) *flops += (double)total * 8.0 * SPLIT_M * C::BN * SPLIT_K * ((double)pairs * (g.nchunk - 1) + last);
   return CTR_OK;
 }
 

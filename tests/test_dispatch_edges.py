@@ -185,3 +185,27 @@ def test_profile_sums_tile_edges(cuda, n):
     ref = v.detach().numpy()
     assert np.abs(got.cpu().numpy()[1, 0, on] - ref).max() <= 1e-11 * np.abs(ref).max()
     assert np.abs(g.cpu().numpy() - want).max() <= 1e-11 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n", [48, 49, 52, 53, 56, 57, 72])
+def test_packed_tail_chunks(cuda, n):
+    """Nev whose last chunk of 16 k holds 1 to 4, 5 to 8 or more valid ones (4, 2 and
+    1 slice pairs an MMA): standard products to 1e-11 of their largest entry (45-bit
+    operands), complex128 ones (one and four terms) through the triangle."""
+    from tests.test_parity_chains import SPLIT_TOL, ref_triangle
+    rng = np.random.default_rng(970 + n)
+    x, y = (rng.normal(size=(2, n, n)) + 1j * rng.normal(size=(2, n, n)) for _ in range(2))
+    got = api.zgemm_batched(_dev(x, cuda), _dev(y, cuda), engine="split").cpu().numpy()
+    ref = x @ y
+    assert np.abs(got - ref).max() <= 1e-11 * np.abs(ref).max()
+    nt = 2
+    prop = synth.make_prop(nt, n, seed=971 + n)
+    pa, pb = synth.make_phi_random(nt, n, rng), synth.make_phi_random(nt, n, rng)
+    mom2 = np.ascontiguousarray(np.stack([synth.make_phi_random(nt, n, rng) for _ in range(2)], axis=1))
+    tp = _dev(prop, cuda)
+    got = api.run_contract_rhopi_sigmapi_sets(tp, api.prop_diag(tp), _dev(np.stack([pa, pb], axis=1), cuda), [(0, 1)],
+                                              _dev(np.zeros((nt, 5, n, n), complex), cuda), _dev(mom2, cuda),
+                                              engine="split", tf_range=(0, nt), rhopi=False, triangle=True)
+    tri = got["triangle"][0].cpu().numpy()
+    want, ab = ref_triangle(prop, pa, pb, mom2)
+    P.entrywise(tri, want, SPLIT_TOL, ab, "triangle Nev=%d" % n)
