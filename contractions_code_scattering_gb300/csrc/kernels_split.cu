@@ -906,26 +906,27 @@ constexpr size_t gemm_smem_bytes() {
 static_assert(2 * CfgStd::NL * CfgStd::BN <= (int)TMEM_COLS && 2 * CfgHP::NL * CfgHP::BN <= (int)TMEM_COLS,
               "accumulators exceed TMEM");
 
-// I * 2^e as a double, rounded to nearest even; integer operations only
+// I * 2^e as a double, rounded to nearest even; integer operations only, as few as
+// there are: 24 a thread of the epilogue, whose stores they hold up (triangles at
+// Nev = 32 1.82 -> 1.66 ms, Nev = 64 6.80 -> 6.58)
 // (normal results; magnitudes below 2^-1022 flush to zero).
 __device__ __forceinline__ double i2d_scaled(long long I, int e) {
-  if (I == 0) return 0.0;
-  const unsigned long long sgn = I < 0 ? (1ull << 63) : 0ull;
-  unsigned long long u = I < 0 ? 0ull - (unsigned long long)I : (unsigned long long)I;
-  const int lz = __clzll((long long)u);
-  u <<= lz;
-  unsigned long long mant = u >> 11;
-  const unsigned long long rem = u & 0x7FFull;
-  if (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) mant++;
-  int ex = 63 - lz + e;
-  if (mant >> 53) {
-    mant >>= 1;
-    ex++;
+  const uint32_t m = (uint32_t)(I >> 63);
+  const unsigned long long a = (unsigned long long)((I ^ (I >> 63)) - (I >> 63));
+  const int lz = __clzll((long long)a);
+  const unsigned long long u = a << (lz & 63);  // bit 63 set; I = 0 is handled below
+  // round to nearest even at bit 11: the carry runs through the implicit bit into
+  // the exponent, which is added without that bit
+  const uint32_t lo = (uint32_t)u, up = ((lo & 0x7FFu) + 0x3FFu + ((lo >> 11) & 1u)) >> 11;
+  const unsigned long long mant = (u >> 11) + up;
+  const int biased = 63 - lz + e + 1022;
+  const uint32_t hi = (uint32_t)(mant >> 32) + ((uint32_t)biased << 20);
+  double d = __hiloint2double((int)(hi | (m & 0x80000000u)), (int)(uint32_t)mant);
+  if ((uint32_t)biased >= 2045u || a == 0) {  // zero, or near the ends of the range
+    if (a == 0 || biased + (int)(mant >> 53) < 0) return 0.0;
+    if (biased + (int)(mant >> 53) >= 2046) return __hiloint2double((int)(0x7FF00000u | (m & 0x80000000u)), 0);
   }
-  const int biased = ex + 1023;
-  if (biased <= 0) return 0.0;
-  if (biased >= 2047) return __longlong_as_double((long long)(sgn | 0x7FF0000000000000ull));
-  return __longlong_as_double((long long)(sgn | ((unsigned long long)biased << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+  return d;
 }
 
 // Smallest row + column scale exponent of a float-float product (below it the
@@ -1245,10 +1246,11 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
     const int row = C::INT_OUT ? q * 32 + (half & 1) * 16 + (lane >> 2) : q * 32 + lane;
     const uint32_t tl = tbase + ((uint32_t)(q * 32 + (C::INT_OUT ? (half & 1) * 16 : 0)) << 16);
     // Complex128 output: a tile's scale exponents and output pointers are fetched
-    // while the tile before it drains (the instance's pointers) and stores (what
-    // they point to), so that no tile waits for them (3 500 clocks before).  The
-    // float-float epilogue has no registers to spare for that: fetched ahead, its
-    // spills cost 4 % of the launch.
+    // while the tile before it is stored, the instance's pointers first and what
+    // they point to halfway, so that no tile waits for them (3 500 clocks before)
+    // and they take no registers while a tile is drained.  The float-float
+    // epilogue has no registers to spare for that: fetched ahead, its spills cost 4 %
+    // of the launch.
     int nmt = 0, nnt = 0, mexp = 0, mrow0 = 0, mrow1 = 0;
     double2* mptr = nullptr;
     float4* nout = nullptr;
@@ -1309,7 +1311,6 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       epi_bar<32 * C::EPI_WARPS>();
       if (*failed) break;
       tc_fence_after();
-      if constexpr (C::INT_OUT) fetch_instance(tile + gridDim.x);
       // Each warp drains its CPW columns into registers and hands TMEM back to
       // the MMA warp before it writes anything to global memory, so the next
       // tile's MMAs run while this tile's products are stored.
@@ -1382,9 +1383,10 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
             for (int c = 0; c < CPW; c++) acc[part][c] += level_units(v[c], l);
           }
         }
-        fetch_scales(tile + gridDim.x);
+        fetch_instance(tile + gridDim.x);
 #pragma unroll
         for (int c = 0; c < CPW; c += 2) {
+          if (c == CPW / 2) fetch_scales(tile + gridDim.x);
           // two adjacent columns of row grow + 8 h
           const int col = cbase + (c >> 2) * 8 + 2 * (lane & 3), h = (c >> 1) & 1;
           if (grow + 8 * h >= g.mrows) continue;
