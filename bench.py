@@ -615,7 +615,11 @@ def roofline(engine, report, steps, nt, nev, nmom):
         return None
     pk = measured_peaks()
     peak = pk.get("bf16_tflops", 1924.8)
-    mma_flops = steps * prods * 8.0 * n3 * 15 * (112.0 / 100.0)
+    # executed K: whole chunks of 16 and, in the last one, the MMAs of its packed slice pairs (of 15)
+    chunks, tail = (nev + 15) // 16, nev % 16
+    step = 1 if chunks < 4 or tail == 0 or tail > 8 else (2 if tail > 4 else 4)
+    k_exec = 16.0 * (chunks - 1) + 16.0 * sum(range(5, 0, -step)) / 15.0
+    mma_flops = steps * prods * 8.0 * n3 * 15 * (k_exec / nev)
     achieved = mma_flops / launches / (ms / launches / 1e3) / 1e12
     # DRAM traffic per launch: the ncu capture of one launch at Nt=8 (64 pairs, 7 momenta, Nev=100)
     # read 0.390 GB and wrote 1.093 GB, i.e. 23.2 MB per (t_sink, t_src) pair; scaled by the
@@ -627,8 +631,8 @@ def roofline(engine, report, steps, nt, nev, nmom):
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at Nt=8, scaled "
                               "by pairs per launch (the split_gemm rho Nt=8 ncu summary under profiles/)",
             "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)" if "bf16_tflops" in pk else "fallback 1924.8",
-            "fp64_equivalent_tflops": achieved / 15 / 1.12,
-            "algorithmic": "15 bf16 slice-pair products x 8*Nev^3 flops (K padded 100->112) per block product"}
+            "fp64_equivalent_tflops": achieved / 15 * nev / k_exec,
+            "algorithmic": "15 bf16 slice-pair products x 8*Nev^2*K flops per block product, K as executed (%.1f)" % k_exec}
 
 
 # ------------------------------------------------------- other workloads
@@ -1188,8 +1192,10 @@ def run_elementals(args):
     step = lambda: api.elementals(V, moms, links=U, out=out)
     t, launches, kern = _timed(step, args.steps, args.warmup)
     K = 3 * L ** 3
-    # 10 products X^dag diag(phase) Y of nev x nev over K per (t, p): 8 nev^2 K flops each
-    flops = 10 * 8.0 * nev * nev * K * nt * len(moms)
+    # products X^dag diag(phase) Y of nev x nev over K, 8 nev^2 K flops each: 10 per (t, +-p), the other of
+    # the two being its mirror, and 7 at p = 0
+    pairs = sum(1 for p in moms if p > tuple(-x for x in p))
+    flops = (10 * pairs + 7) * 8.0 * nev * nev * K * nt
     peak = fp64_peak_tflops()
     achieved = flops / (kern["el_gemm"]["ms"] / 1e3 / args.steps) / 1e12
     # parity on a sample: t = 0, two momenta, against the numpy restatement; and the
@@ -1207,7 +1213,7 @@ def run_elementals(args):
             "roofline": {"kernel": "el_gemm", "bound": "fp64 pipe", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": "measured in bench.py: cuBLAS DGEMM 8192^3",
-                         "algorithmic": "10 products of 8 nev^2 (3 L^3) flops per (t, p)"},
+                         "algorithmic": "10 products of 8 nev^2 (3 L^3) flops per (t, +-p), 7 per (t, 0)"},
             "vs_restatement": _errs(got, ref),
             "cpu_baseline": {"value": 2 * 5 / tcpu, "unit": "elementals/s", "cores": os.cpu_count(), "kind": "port",
                              "sample": "t = 0, 2 momenta, 5 operators (numpy restatement)"}}

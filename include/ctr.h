@@ -111,7 +111,8 @@ int ctr_pipi(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin,
  * elemental; set s contracts with P1..P4 = phi[:, sets[4s + k]] (k = 0..3, host array
  * [nset][4]).  corr [nset][tf_end-tf_begin][Nt][5], each set's entries as ctr_pipi gives them.
  * Block products and traces that several sets share (e.g. Phi(q) tau, tau Phi(q) tau^dag for the
- * sets (p, -p) and (-p, p)) are computed once; every stage of a pair batch is one launch. */
+ * sets (p, -p) and (-p, p), L T and T^dag L of sets with the same sink pair) are computed once
+ * per batch of (t_sink, t_src) pairs. */
 int ctr_pipi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin, const double* prop_rows,
                   const double* prop_diag, const double* phi, int nphi, int nset, const int32_t* sets, double* corr,
                   void* stream);
@@ -122,13 +123,14 @@ int ctr_pipi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, int iso
  * P1 = phi[:, sets[2s]], P2 = phi[:, sets[2s + 1]] (phi [Nt][nphi][N][N], sets host [nset][2]);
  * the sink operators mom5_p1p2 [Nt][5][N][N] (rho) and mom2_p1p2 [Nt][2][N][N] (sigma) are
  * the same for every set.  Both families contract X = tau(tf,ti) G R(ti),
- * R = Phi_P2 taud Phi_P1: X is computed once per set and pair and multiplied by all the
- * sink operators the outputs need in one stacked launch.  Outputs (each may be NULL; then
+ * R = Phi_P2 taud Phi_P1, with Op(tf)^dag tau_b, which all sets share.  Outputs (each may be NULL; then
  * its operands may be NULL too): rhopi [nset][3][tf_end-tf_begin][Nt][4] (idir 0..2, as
  * ctr_rhopi), triangle [nset][tf_end-tf_begin][Nt][2] and hor_fish [nset][Nt] (as ctr_sigmapi).
  * On the split engine the rho -> pi pi and triangle traces of a pair run as Gram products
  * on the tensor cores (the tuning knob "chains.trace_form" = 1, the default; each entry
- * within the engine's per-entry tolerance); with the knob forced to 0 they run as FP64
+ * within the engine's per-entry tolerance): X of every set against the sink operators'
+ * tau, or, where many sets make it cheaper, the sides that do not depend on the set
+ * against every set's R; with the knob forced to 0 they run as FP64
  * traces and every set's entries are bitwise those of its own ctr_rhopi / ctr_sigmapi. */
 int ctr_rhopi_sigmapi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, const double* prop_rows,
                            const double* prop_diag, const double* phi, int nphi, const double* mom5_p1p2,
@@ -328,7 +330,8 @@ int ctr_split_available(void);
  * traces (|z|_1 = |Re z| + |Im z|); entries whose estimate exceeds rel_tol * |entry|
  * -- those with heavy cancellation -- are recomputed (two-sided form: their spin rows
  * on the high-precision split configuration; chains: their (t_sink, t_src) pairs on
- * the FP64 engine) and patched in.  rel_tol = 0 disables the check.  Default 1e-9. */
+ * the FP64 engine, those of Gram products only where FP64 traces flag them too) and
+ * patched in.  rel_tol = 0 disables the check.  Default 1e-9. */
 int ctr_split_set_refine(double rel_tol);
 /* Number of entries the last split call recomputed. */
 long long ctr_split_refined(void);

@@ -209,3 +209,32 @@ def test_packed_tail_chunks(cuda, n):
     tri = got["triangle"][0].cpu().numpy()
     want, ab = ref_triangle(prop, pa, pb, mom2)
     P.entrywise(tri, want, SPLIT_TOL, ab, "triangle Nev=%d" % n)
+
+
+@pytest.mark.parametrize("tol", [1e-12, 1e-14])
+def test_set_recomputation_in_two_steps(cuda, tol):
+    """Set calls recompute flagged units with FP64 traces on the split engine, and what
+    is still flagged on the FP64 engine: tolerances that flag some and most entries,
+    against the FP64 engine's set call, per entry as the engine's default asks."""
+    from contractions_code_scattering_gb300._lib import check, lib
+    nt, n, tr = 4, 21, (1, 4)
+    prop = synth.make_prop(nt, n, seed=990, decay=0.25)
+    rng = np.random.default_rng(991)
+    phi = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(5)], axis=1)
+    mom5 = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(5)], axis=1)
+    mom2 = np.stack([synth.make_phi_random(nt, n, rng) for _ in range(2)], axis=1)
+    sets = [(a, b) for a in range(5) for b in range(5)]
+    tp = _dev(prop, cuda)
+    run = lambda engine: api.run_contract_rhopi_sigmapi_sets(
+        tp[tr[0]:tr[1]].contiguous(), api.prop_diag(tp), _dev(phi, cuda), sets, _dev(mom5, cuda), _dev(mom2, cuda),
+        engine=engine, tf_range=tr, rhopi=True, triangle=True)
+    ref = run("fp64")
+    check(lib().ctr_split_set_refine(tol))
+    try:
+        got = run("split")
+        assert lib().ctr_split_refined() > 0
+    finally:
+        check(lib().ctr_split_set_refine(1e-9))
+    for k in ("rhopi", "triangle"):
+        want = ref[k].cpu().numpy()
+        P.entrywise(got[k].cpu().numpy(), want, 1e-9, np.abs(want), k)
