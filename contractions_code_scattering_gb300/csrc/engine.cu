@@ -75,14 +75,19 @@ int twosided_fp64(int N, int Nt, int tf_begin, int tf_end, const double* prop_ro
   // each distinct (A block, B block) trace once (144 of rho's 768 rows repeat one)
   std::vector<int> tix(nrows), ta, tb;
   {
-    std::unordered_map<long long, int> seen;
+    // (a flat table where the blocks are few: hashing rho's 768 rows takes 40 us)
+    const long long cells = (long long)nA * nB;
+    std::vector<int> flat(cells <= (1 << 20) ? cells : 0, -1);
+    std::unordered_map<long long, int> sparse;
     for (int r = 0; r < nrows; r++) {
-      const auto it = seen.emplace((long long)P.rowA[r] * nB + P.rowB[r], (int)ta.size());
-      if (it.second) {
+      const long long key = (long long)P.rowA[r] * nB + P.rowB[r];
+      int& t = flat.empty() ? sparse.emplace(key, -1).first->second : flat[key];
+      if (t < 0) {
+        t = (int)ta.size();
         ta.push_back(P.rowA[r]);
         tb.push_back(P.rowB[r]);
       }
-      tix[r] = it.first->second;
+      tix[r] = t;
     }
   }
   const int ntr = (int)ta.size();
