@@ -90,7 +90,6 @@ enum {
   WS_MISC,          // small tables (CSR of output rows)
   WS_ROWABS,        // per-row error scales of the split engine
   WS_REFINE,        // refinement list / patches of the split engine
-  WS_REFINE2,       // the same of a recomputation that is itself checked
   WS_SPLITTASK,     // sliced operands of split-engine task stages
   WS_SPLITJOBS,     // their job / instance / pointer tables
   WS_SPLITJOBS3,

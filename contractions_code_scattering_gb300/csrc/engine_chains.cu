@@ -1006,9 +1006,8 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   const bool fp64_traces_needed = !gram ||
                                   !tune_peek("chains.trace_form", trace_shape, 2, 1, &known_form) || known_form == 0;
   Refine rf_rp, rf_tr;
-  const int slot_rp = rerun ? WS_REFINE2 : WS_REFINE, slot_tr = rerun ? WS_REFINE2 : WS_SPLITJOBS3;  // (a rerun has one output)
-  if (rhopi) CTR_TRY(refine_begin(c, (size_t)nset * nd * npairs * 4, slot_rp, rf_rp));
-  if (tri) CTR_TRY(refine_begin(c, (size_t)nset * npairs * 2, slot_tr, rf_tr));
+  if (rhopi) CTR_TRY(refine_begin(c, (size_t)nset * nd * npairs * 4, WS_REFINE, rf_rp));
+  if (tri) CTR_TRY(refine_begin(c, (size_t)nset * npairs * 2, WS_SPLITJOBS3, rf_tr));
   // The sink form takes its place where it costs less, per pair: the terms' block
   // products instead of 64 a set, and its rows to slice for the Gram product (16
   // blocks a row; a block's slices and its share of that product take about 0.65 of
@@ -1293,37 +1292,38 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
     for (const RowItems& r : it_rp) CTR_TRY(rowsum_items(c, trv, tra, r, (double2*)rhopi, rf_rp));
     if (tri) CTR_TRY(rowsum_items(c, trv, tra, it_tr, (double2*)tri, rf_tr));
   }
-  // Flagged units.  The Gram products' error scales are bounds by the blocks' norms, and
-  // the sink form's traces are larger terms than X's: they flag two to four times
-  // the units that the FP64 traces' own scales flag.  Those units first run with X
-  // and FP64 traces on this engine, and what is still flagged on the FP64 engine
-  // (2 ms a unit at Nev = 128).
-  const bool again = gram;
-  const std::vector<int> pos = plist ? *plist : std::vector<int>();
-  auto rerun_units = [=](const std::vector<int>& units, bool rp, double2* out, cudaStream_t ls) -> int {
-    const long long counted = g_refined_last;
-    for (size_t u0 = 0, u1; u0 < units.size(); u0 = u1) {  // units = (set [* nd + d]) * npairs + pair
-      const int kd = units[u0] / npairs, k = rp ? kd / nd : kd;
-      std::vector<int> pl, dirs;
-      for (u1 = u0; u1 < units.size() && units[u1] / npairs == kd; u1++)
-        pl.push_back(pos.empty() ? units[u1] % npairs : pos[units[u1] % npairs]);
-      if (rp) dirs.push_back(idirs[kd % nd]);
-      CTR_TRY(rhopi_sigmapi_core(N, Nt, tf_begin, tf_end, prop_rows, prop_diag, elc, mom5, mom2, 1, sc.data() + 2 * k,
-                                 dirs, rp ? (double*)(out + u0 * 4) : nullptr, rp ? nullptr : (double*)(out + u0 * 2),
-                                 nullptr, ls, again ? CTR_ENGINE_SPLIT : CTR_ENGINE_FP64, false, &pl, nullptr));
-    }
-    g_refined_last = counted;
-    return CTR_OK;
-  };
   if (rhopi)
-    CTR_TRY(refine_end(c, rf_rp, 4, slot_rp, (double2*)rhopi,
-                       [=](const std::vector<int>& units, double2* out, cudaStream_t ls) {
-                         return rerun_units(units, true, out, ls);
+    CTR_TRY(refine_end(c, rf_rp, 4, WS_REFINE, (double2*)rhopi,
+                       [=](const std::vector<int>& units, double2* out, cudaStream_t ls) -> int {
+                         size_t u0 = 0;  // units = (set * nd + d) * npairs + pair
+                         while (u0 < units.size()) {
+                           const int kd = units[u0] / npairs;
+                           std::vector<int> pl;
+                           size_t u1 = u0;
+                           while (u1 < units.size() && units[u1] / npairs == kd) pl.push_back(units[u1++] % npairs);
+                           CTR_TRY(rhopi_sigmapi_core(N, Nt, tf_begin, tf_end, prop_rows, prop_diag, elc, mom5, mom2,
+                                                      1, sc.data() + 2 * (kd / nd), {idirs[kd % nd]},
+                                                      (double*)(out + u0 * 4), nullptr, nullptr, ls, CTR_ENGINE_FP64,
+                                                      false, &pl, nullptr));
+                           u0 = u1;
+                         }
+                         return CTR_OK;
                        }));
   if (tri)
-    CTR_TRY(refine_end(c, rf_tr, 2, slot_tr, (double2*)tri,
-                       [=](const std::vector<int>& units, double2* out, cudaStream_t ls) {
-                         return rerun_units(units, false, out, ls);
+    CTR_TRY(refine_end(c, rf_tr, 2, WS_SPLITJOBS3, (double2*)tri,
+                       [=](const std::vector<int>& units, double2* out, cudaStream_t ls) -> int {
+                         size_t u0 = 0;  // units = set * npairs + pair
+                         while (u0 < units.size()) {
+                           const int k = units[u0] / npairs;
+                           std::vector<int> pl;
+                           size_t u1 = u0;
+                           while (u1 < units.size() && units[u1] / npairs == k) pl.push_back(units[u1++] % npairs);
+                           CTR_TRY(rhopi_sigmapi_core(N, Nt, tf_begin, tf_end, prop_rows, prop_diag, elc, mom5, mom2,
+                                                      1, sc.data() + 2 * k, {}, nullptr, (double*)(out + u0 * 2),
+                                                      nullptr, ls, CTR_ENGINE_FP64, false, &pl, nullptr));
+                           u0 = u1;
+                         }
+                         return CTR_OK;
                        }));
   return CTR_OK;
 }

@@ -330,8 +330,7 @@ int ctr_split_available(void);
  * traces (|z|_1 = |Re z| + |Im z|); entries whose estimate exceeds rel_tol * |entry|
  * -- those with heavy cancellation -- are recomputed (two-sided form: their spin rows
  * on the high-precision split configuration; chains: their (t_sink, t_src) pairs on
- * the FP64 engine, those of Gram products only where FP64 traces flag them too) and
- * patched in.  rel_tol = 0 disables the check.  Default 1e-9. */
+ * the FP64 engine) and patched in.  rel_tol = 0 disables the check.  Default 1e-9. */
 int ctr_split_set_refine(double rel_tol);
 /* Number of entries the last split call recomputed. */
 long long ctr_split_refined(void);

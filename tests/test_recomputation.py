@@ -1,0 +1,38 @@
+"""The split engine's recomputation: what its error scales have to flag, and that
+flagged units get the FP64 engine's values."""
+import numpy as np
+import pytest
+import torch
+
+from contractions_code_scattering_gb300 import api, synth
+from contractions_code_scattering_gb300._lib import check, lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a, cuda):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+
+@pytest.mark.parametrize("tol", [1e-12, 1e-14])
+def test_flagged_set_units_take_fp64_values(cuda, tol):
+    """rho -> pi pi / sigma -> pi pi set calls: every recomputed entry is bitwise the FP64
+    engine's (at these tolerances some, and most, of the units are recomputed)."""
+    nt, n, tr = 4, 21, (1, 4)
+    prop = synth.make_prop(nt, n, seed=990, decay=0.25)
+    rng = np.random.default_rng(991)
+    phi, mom5, mom2 = (np.stack([synth.make_phi_random(nt, n, rng) for _ in range(k)], axis=1) for k in (5, 5, 2))
+    sets = [(a, b) for a in range(5) for b in range(5)]
+    tp = _dev(prop, cuda)
+    run = lambda engine: api.run_contract_rhopi_sigmapi_sets(
+        tp[tr[0]:tr[1]].contiguous(), api.prop_diag(tp), _dev(phi, cuda), sets, _dev(mom5, cuda), _dev(mom2, cuda),
+        engine=engine, tf_range=tr, rhopi=True, triangle=True)
+    ref = run("fp64")
+    check(lib().ctr_split_set_refine(tol))
+    try:
+        got = run("split")
+        refined = lib().ctr_split_refined()
+    finally:
+        check(lib().ctr_split_set_refine(1e-9))
+    same = sum(int((got[k] == ref[k]).sum()) for k in ("rhopi", "triangle", "hor_fish"))
+    assert refined > 0 and same >= refined
