@@ -12,8 +12,7 @@
 //   square(tf,ti) = Tr[G S W],  S = T G Rsq,  W = T^dag L,  Rsq = Phi2 taud Phi1
 //   dtri(tf,ti)   = Tr[G S W],  S = T G Rdt,                Rdt = Phi1 taud Phi2
 //   dtri_hor      = Tr[Phi3 Pm(1) Phi4 Pm(2)],  Pm(q) = T Phi_q T^dag
-//   star / fish   = products of twin traces Tr[Phi_x(tf) sum_cc Pm(y)_cc]
-//                 = sum_b Tr[(tau_b Phi_y(ti)) (tau_b^dag Phi_x(tf))]
+//   star / fish   = products of twin traces sum_b Tr[(tau_b Phi_y(ti)) (tau_b^dag Phi_x(tf))]
 //   rho->pipi     = sum c * Tr[Phi_ip (T G R)_{s5 s2} tau_{s3 s2}^dag]
 //   sigma->pipi triangle = sum g5(s1) Tr[Phi_ik (T G R)_{s1 s5} tau_{s1 s5}^dag]
 // with T = tau(tf,ti) as a 4x4 block matrix.  S depends on the source side only
@@ -426,7 +425,10 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       }
   int nF = 0;
   for (auto& v : FK) nF += (int)v.size();
-  // star / fish twin traces (sink elemental, source elemental): (4, 1), (3, 2), (3, 1), (4, 2) of every set
+  // star / fish twin traces (sink elemental, source elemental): (4, 1), (3, 2), (3, 1), (4, 2)
+  // of every set, a term for each of tau's 16 blocks.  (I = 0 has Tr[Phi_x Pm(y)_cc] for
+  // less, 151 instead of 165 ms for 19 sets at Nev = 100 and 4 sink times, but a Pm that
+  // cancels in its spin sum takes the traces' error scales down with it.)
   std::map<std::pair<int, int>, int> twk;
   std::vector<std::pair<int, int>> TW;
   std::vector<int> twin(4 * nset);
@@ -439,9 +441,9 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       twin[4 * k + h] = it->second;
     }
   }
-  const int nTW = (int)TW.size(), ntw = iso == 0 ? 4 : 16;  // traces a twin
-  const size_t blk_pair = 16 * (size_t)(nCR + nCL + nW + (iso == 0 ? nW + nF : nU));
-  const size_t tr_pair = (size_t)nset * (iso == 0 ? 48 : 32) + (size_t)ntw * nTW;
+  const int nTW = (int)TW.size();
+  const size_t blk_pair = 16 * (size_t)(nCR + nCL + nW + nU + (iso == 0 ? nW + nF : 0));
+  const size_t tr_pair = (size_t)nset * (iso == 0 ? 48 : 32) + 16 * (size_t)nTW;
   const size_t per_pair = blk_pair * N2 * sizeof(double2) + tr_pair * (sizeof(double2) + sizeof(double));
   const int batch = std::max(1, std::min(npairs, (int)(sets_budget() / std::max<size_t>(per_pair, 1))));
   Refine rf;
@@ -457,7 +459,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       used += nblk * N2;
       return p;
     };
-    std::vector<double2*> bS((size_t)ng * nCR), bV(ng), bW((size_t)nh * nCL), bY(nh, nullptr), bP(np, nullptr);
+    std::vector<double2*> bS((size_t)ng * nCR), bV(ng), bW((size_t)nh * nCL), bY(nh), bP(np, nullptr);
     std::vector<std::vector<double2*>> bF(np, std::vector<double2*>(nW, nullptr));
     for (int g = 0; g < ng; g++) {
       const size_t m = pb.by_ti[g].size();
@@ -467,7 +469,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
     for (int h = 0; h < nh; h++) {
       const size_t m = pb.by_tf[h].size();
       for (int ci = 0; ci < nCL; ci++) bW[(size_t)h * nCL + ci] = alloc(16 * m);
-      if (iso != 0) bY[h] = alloc(16 * (size_t)nU * m);
+      bY[h] = alloc(16 * (size_t)nU * m);
     }
     for (int i = 0; i < np && iso == 0; i++) {
       bP[i] = alloc(16 * (size_t)nW);
@@ -543,7 +545,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
         g0.push_back(std::move(G));
       }
       // Y(q) = tau_b^dag Phi_q(tf): slab (pair, block b), right block q
-      for (int q0 = 0; q0 < nU && iso != 0; q0 += 8) {
+      for (int q0 = 0; q0 < nU; q0 += 8) {
         GridTask G = make_grid(16 * m, std::min(8, nU - q0), 1, kOne, 1, 0);
         for (int pp = 0; pp < m; pp++)
           for (int b = 0; b < 16; b++) G.A[pp * 16 + b] = pb.T[mem_i[pp]] + b * N2;
@@ -593,13 +595,12 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       return fail(CTR_ERR_ALLOC, "pi pi: batch arena overflow");
     TracePlan tp;
     tp.tt.reserve(ntr);
-    std::vector<int> slots, ent, tws((size_t)ntw * nTW);
+    std::vector<int> slots, ent, tws(16 * (size_t)nTW);
     slots.reserve((size_t)np * nset * 112);
     for (int i = 0; i < np; i++) {
       for (int t = 0; t < nTW; t++)
-        for (int b = 0; b < ntw; b++)
-          tws[t * ntw + b] = iso == 0 ? tp.add(P(TW[t].first, pb.tf[i]), Pblk(iw[TW[t].second], i, b, b), 1.f, 0.f, 1)
-                                      : tp.add(Vblk(iw[TW[t].second], i, b), Yblk(iu[TW[t].first], i, b), 1.f, 0.f, 1);
+        for (int b = 0; b < 16; b++)
+          tws[t * 16 + b] = tp.add(Vblk(iw[TW[t].second], i, b), Yblk(iu[TW[t].first], i, b), 1.f, 0.f, 1);
       for (int k = 0; k < nset; k++) {
         const int* q = sets + 4 * k;
         for (int cr : {cSq[k], cDt[k]})
@@ -617,7 +618,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
           slots.push_back(tp.add(Fb, Gb, 1.f, 0.f, 1));
         }
         for (int h = 0; h < 4; h++)
-          for (int b = 0; b < 16; b++) slots.push_back(b < ntw ? tws[twin[4 * k + h] * ntw + b] : -1);
+          for (int b = 0; b < 16; b++) slots.push_back(tws[twin[4 * k + h] * 16 + b]);
         ent.push_back(k * npairs + pb.ent[i]);
       }
     }

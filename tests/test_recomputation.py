@@ -36,3 +36,31 @@ def test_flagged_set_units_take_fp64_values(cuda, tol):
         check(lib().ctr_split_set_refine(1e-9))
     same = sum(int((got[k] == ref[k]).sum()) for k in ("rhopi", "triangle", "hor_fish"))
     assert refined > 0 and same >= refined
+
+
+@pytest.mark.parametrize("sets_call", [False, True])
+def test_cancelling_twins_are_flagged(cuda, sets_call):
+    """I = 0 star and fish where tau Phi tau^dagger cancels over its spin sum: with
+    tau_{a1} = tau_{a0} S, tau_{a3} = tau_{a2} S and S Phi S = -Phi up to 1e-8 of Phi,
+    the twin traces are 1e-8 of their terms, so both have to be recomputed."""
+    nt, n = 2, 20
+    prop = synth.make_prop(nt, n, seed=995)
+    rng = np.random.default_rng(996)
+    s = np.where(np.arange(n) < n // 2, 1.0, -1.0)
+    prop[..., 1, :, :], prop[..., 3, :, :] = prop[..., 0, :, :] * s, prop[..., 2, :, :] * s
+    odd = s[:, None] * s[None, :] < 0
+    src = [synth.make_phi_random(nt, n, rng) * np.where(odd, 1.0, 1e-8) for _ in range(2)]
+    snk = [synth.make_phi_random(nt, n, rng) for _ in range(2)]
+    ps = [_dev(p, cuda) for p in src + snk]
+    tp = _dev(prop, cuda)
+    diag = api.prop_diag(_dev(synth.make_prop(nt, n, seed=997), cuda))
+
+    def run(engine):
+        if sets_call:
+            return api.run_contract_pipi_sets(tp, diag, torch.stack(ps, dim=1).contiguous(), [(0, 1, 2, 3)], 0,
+                                              engine=engine, tf_range=(0, nt))[0]
+        return api.run_contract_pipi(tp, diag, *ps, 0, engine=engine, tf_range=(0, nt))
+
+    ref, got = run("fp64"), run("split")
+    assert lib().ctr_split_refined() == got.numel()
+    assert torch.equal(got, ref)
