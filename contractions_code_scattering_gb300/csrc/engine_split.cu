@@ -805,7 +805,6 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
   for (auto& bk : buckets) {
     const int nterm = bk.first.first, nb = bk.first.second;
     const int K = nterm * N, nchunk = cdiv(K, SPLIT_K), ntiles = cdiv(nb * N, CfgHP::BN);
-    const int eplus = K > 128 ? 1 : 0;
     const size_t l_b = align256((size_t)nchunk * CfgHP::A_STAGE);
     const size_t r_b = align256((size_t)ntiles * nchunk * CfgHP::B_STAGE);
     const size_t le_b = align256(SPLIT_M * 4), re_b = align256((size_t)ntiles * CfgHP::BN * 4);
@@ -849,7 +848,6 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
           }
           L.nterm = nterm;
           L.dag = k.dag;
-          L.eplus = eplus;
           L.out = p;
           L.exps = (int*)(p + l_b);
           lt = lid.emplace(in.g, (int)lj.size()).first;
@@ -860,7 +858,6 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
         std::memset(&R, 0, sizeof(R));
         R.nb = in.nb;
         R.nterm = nterm;
-        R.eplus = eplus;
         std::vector<uintptr_t> key;
         for (int j = 0; j < in.nb; j++) {
           const ZTask& z = tasks[groups[in.g][in.t0 + j]];
@@ -947,7 +944,6 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
     const int nterm = std::get<0>(bk.first), nb = std::get<1>(bk.first), ns = std::get<2>(bk.first);
     const int K = nterm * N, nchunk = cdiv(K, SPLIT_K), ntiles = cdiv(nb * N, CfgHP::BN),
               mtiles = cdiv(ns * N, SPLIT_M);
-    const int eplus = K > 128 ? 1 : 0;
     const size_t l_b = align256((size_t)mtiles * nchunk * CfgHP::A_STAGE), le_b = align256((size_t)mtiles * SPLIT_M * 4);
     const size_t r_b = align256((size_t)ntiles * nchunk * CfgHP::B_STAGE), re_b = align256((size_t)ntiles * CfgHP::BN * 4);
     const size_t per = l_b + le_b + r_b + re_b;  // one left and at most one distinct right per piece
@@ -1003,7 +999,6 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
           L.nslab = pc.ns;
           L.nterm = nterm;
           L.dag = G.adag;
-          L.eplus = eplus;
           L.out = lbase + lj.size() * (l_b + le_b);
           L.exps = (int*)(L.out + l_b);
           lt = lid.emplace(key, (int)lj.size()).first;
@@ -1020,7 +1015,6 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
           std::memset(&R, 0, sizeof(R));
           R.nb = nb;
           R.nterm = nterm;
-          R.eplus = eplus;
           R.dag = G.bdag;
           for (int j = 0; j < nb; j++)
             for (int q = 0; q < nterm; q++) {

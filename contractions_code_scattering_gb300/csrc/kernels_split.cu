@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(256) slice_task_left_kernel(const SliceTaskLJo
         const int b = bexp[((size_t)J.bi[q] * 2 + ((J.dag >> q) & 1)) * nev + r];
         if (b > -30000) e = max(e, b + J.wexp[q]);
       }
-    const int E = (e < -1000 ? 0 : e) + J.eplus;
+    const int E = e < -1000 ? 0 : e;
     sexp[r] = E;
     if (kc == 0) J.exps[r] = E;
   }
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(256) slice_stack_left_kernel(const SliceStackL
         if (b > -30000) e = max(e, b + J.wexp[q]);
       }
     }
-    const int E = (e < -1000 ? 0 : e) + J.eplus;
+    const int E = e < -1000 ? 0 : e;
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[g] = E;
   }
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
         e = max(e, bexp[((size_t)J.bi[jb][q] * 2 + (dag ? 0 : 1)) * nev + c]);
       }
     }
-    const int E = (e < -1000 ? 0 : e) + J.eplus;
+    const int E = e < -1000 ? 0 : e;
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[n] = E;  // exps sized ntiles * BN (padding columns get 0)
   }
@@ -967,12 +967,12 @@ __device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t units) {
 }
 
 // Slice pair (i, j), i + j < NS, falls in hand-back group G (ALL: any, REST: any but
-// the first).
-constexpr int GROUP_ALL = -1, GROUP_REST = -2;
+// the first, NOT01: any but the first two).
+constexpr int GROUP_ALL = -1, GROUP_REST = -2, GROUP_NOT01 = -3;
 template <class C, int G>
 __host__ __device__ constexpr bool pair_in_group(int i, int j) {
   const int grp = level_group<C>(i + j < C::NL - 1 ? i + j : C::NL - 1);
-  return i + j < C::NS && (G == GROUP_ALL || grp == G || (G == GROUP_REST && grp > 0));
+  return i + j < C::NS && (G == GROUP_ALL || grp == G || (G == GROUP_REST && grp > 0) || (G == GROUP_NOT01 && grp > 1));
 }
 
 // The MMAs of plane P (0 Re, 1 Im) of left slice I with the right slices J, J + 1, ...
@@ -1121,6 +1121,15 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   // Nev = 57 741 -> 704 us, Nev = 100 9.25 -> 8.98 ms); shorter tiles are bound by their
   // epilogue, which the second wait only lengthens (Nev = 32 223 -> 242 us).
   const bool early = g.nchunk >= 4;
+  // The pieces of a tile of more than 128 k, 4 to 8 chunks each, at whose ends levels 0 and 1
+  // and the last level are drained into the epilogue's 64-bit sums.  Level 0 then stays
+  // below 2^24 units, where FP32 sums are exact, for any data and with operands at full
+  // scale: halved instead (the digits of both then reach 512 k), products of four terms
+  // lost two bits.  The last level, truncated by the tensor core at each MMA, gets an error
+  // that grows with the chunks summed.  Error of a four-term product of Gaussian blocks,
+  // largest entries 1: 4.8e-15 -> 8e-16 at Nev = 100 (one term 8e-16); the drains cost 1.5 to
+  // 4 % of a call (pi pi sets 166 -> 173 ms, profile 25.6 -> 26.1).
+  const uint32_t pieces = C::LONG ? (g.nchunk + 7) / 8 : 1;
   if (warp == 0) {
     if (lane == 0) {
       uint32_t g_chunk = 0;
@@ -1164,9 +1173,9 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         tc_fence_after();
         return ok;
       };
-      auto wait_group = [&](int grp) {
-        if (local > 0) {
-          ok = mbar_wait(&tempty[grp], (local - 1) & 1, 2 * WAIT_NS, err);
+      auto wait_group = [&](int grp, uint32_t drains) {
+        if (drains > 0) {
+          ok = mbar_wait(&tempty[grp], (drains - 1) & 1, 2 * WAIT_NS, err);
           if (!ok) atomicExch(err, 4);
         }
         tc_fence_after();
@@ -1183,7 +1192,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         // stages hold chunks of this tile by then, and the third one's copy is not
         // held up.)  The CTA's first tile has nothing to wait for but its chunks.
         const int pre = min(local == 0 ? 1 : 2, g.nchunk);
-        if (!wait_group(0)) break;
+        if (!wait_group(0, local * pieces)) break;
         uint32_t s = st, p = ph;
         for (int c = 0; c < pre; c++) {
           if (!wait_full(s, p)) break;
@@ -1192,7 +1201,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
         }
         if (!ok) break;
         for (int grp = 1; grp < tmem_groups<C>(); grp++) {
-          if (!wait_group(grp)) break;
+          if (!wait_group(grp, grp <= 1 ? local * pieces : local)) break;
           issue_group<C>(grp, tbase, adesc(st), bdesc(st), true);
         }
         if (!ok) break;
@@ -1203,9 +1212,28 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
           umma_commit(&empty[st]);
           next();
         }
+        uint32_t piece = 1;  // the next one, which starts at chunk `cut`
+        int cut = g.nchunk / pieces;
         for (int kc = pre; kc < g.nchunk; kc++, next()) {
           if (!wait_full(st, ph)) break;
-          if (!early || kc + 1 < g.nchunk) {
+          if (C::LONG && piece < pieces && kc + 1 == cut) {
+            // a piece's last chunk: levels 0 and 1 first, then the last level, drained beside
+            // the MMAs of the others and of the next chunk
+            issue_pairs<C, 1>(tbase, adesc(st), bdesc(st), false);
+            umma_commit(&tfull[0]);
+            issue_pairs<C, 0>(tbase, adesc(st), bdesc(st), false);
+            umma_commit(&tfull[1]);
+            issue_pairs<C, GROUP_NOT01>(tbase, adesc(st), bdesc(st), false);
+          } else if (C::LONG && piece < pieces && kc == cut) {
+            // the next piece's first chunk: they start again at zero
+            issue_pairs<C, GROUP_NOT01>(tbase, adesc(st), bdesc(st), false);
+            if (!wait_group(1, local * pieces + piece)) break;
+            issue_pairs<C, 1>(tbase, adesc(st), bdesc(st), true);
+            if (!wait_group(0, local * pieces + piece)) break;
+            issue_pairs<C, 0>(tbase, adesc(st), bdesc(st), true);
+            piece++;
+            cut = g.nchunk * piece / pieces;
+          } else if (!early || kc + 1 < g.nchunk) {
             issue_chunk<C>(tbase, adesc(st), bdesc(st), false);
           } else {
             // the last chunk: the last level first, drained beside the others' MMAs
@@ -1304,7 +1332,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       // one thread waits for the last level; the outcome is shared so that all
       // epilogue threads leave the loop together
       if (et == 0) {
-        const bool done = mbar_wait(&tfull[0], local & 1, 4 * WAIT_NS, err);
+        const bool done = mbar_wait(&tfull[0], (local * pieces) & 1, 4 * WAIT_NS, err);
         if (!done) atomicExch(err, 3);
         *failed = done ? 0 : 1;
       }
@@ -1325,44 +1353,32 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
       // the wait above finds at the next tile)
       auto wait_rest = [&]() {
         if (!early) return;
-        if (!mbar_wait(&tfull[1], local & 1, 4 * WAIT_NS, err)) atomicExch(err, 3);
+        if (!mbar_wait(&tfull[1], (local * pieces + pieces - 1) & 1, 4 * WAIT_NS, err)) atomicExch(err, 3);
         __syncwarp();
         tc_fence_after();
       };
       if constexpr (C::INT_OUT) {
         // complex128 output: the exact levels and the last one summed exactly
-        // in 64-bit integers (units 2^-54 of the row/column scale; level 0 is
-        // below 2^8, so no overflow), then rounded once to double.
+        // in 64-bit integers (units 2^-54 of the row/column scale, 2^-52 above 128
+        // k; a product is below 2 K, so no overflow), then rounded once to double.
         // Level l < NL-1 holds integer multiples of 2^-(16+9l) (products of
         // digits d_i 2^(-8-9i) with i+j = l), at most 2^28 of them, so one
         // FP32 -> int32 conversion of v 2^(16+9l) is exact; the last level is
-        // rounded to 2^-54 (|v| < 2^-24 there, so it fits an int32 as well;
+        // rounded to a unit (|v| < 2^-24 there, so it fits an int32 as well;
         // 64-bit conversions would go through GB300's slow FP64 pipe).
         // Integer sums do not depend on the order of the levels.
+        constexpr int UNIT = C::LONG ? 52 : 54;
         auto level_units = [](float v, int l) -> long long {
-          if (l < C::NL - 1) return (long long)__float2int_rn(v * __int_as_float((127 + 16 + 9 * l) << 23)) << (38 - 9 * l);
+          if (l < C::NL - 1)
+            return (long long)__float2int_rn(v * __int_as_float((127 + 16 + 9 * l) << 23)) << (UNIT - 16 - 9 * l);
           // the last level holds pairs i+j >= NL-1: |v| 2^54 <= 5 K 2^16 2^-52 2^54 < 2^30
-          return (long long)__float2int_rn(v * __int_as_float((127 + 54) << 23));
+          return (long long)__float2int_rn(v * __int_as_float((127 + UNIT) << 23));
         };
         // (each group goes back as soon as its last load has landed, before
         // that load's values are folded in: the MMA warp waits on the loads only)
         static_assert(!C::INT_OUT || (CPW == 12 && EPH == 4), "16 x 24 fragments of a warp");
         long long acc[2][CPW];
-        {  // group 0: the last level
-          float v0[CPW], v1[CPW];
-          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(0, C::NL - 1) + cbase), v0);
-          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(1, C::NL - 1) + cbase), v1);
-          tmem_ld_wait();
-          hand_back(0);
-#pragma unroll
-          for (int c = 0; c < CPW; c++) {
-            acc[0][c] = level_units(v0[c], C::NL - 1);
-            acc[1][c] = level_units(v1[c], C::NL - 1);
-          }
-        }
-        wait_rest();
-#pragma unroll
-        for (int part = 0; part < 2; part++) {  // group 1: levels 0 and 1
+        auto add_levels01 = [&](int part) {
           float v0[CPW], v1[CPW];
           tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 0) + cbase), v0);
           tmem_ld_16x24(tl + (uint32_t)(C::acc_col(part, 1) + cbase), v1);
@@ -1370,7 +1386,41 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
           if (part == 1) hand_back(1);
 #pragma unroll
           for (int c = 0; c < CPW; c++) acc[part][c] += level_units(v0[c], 0) + level_units(v1[c], 1);
+        };
+        auto add_last = [&]() {
+          float v0[CPW], v1[CPW];
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(0, C::NL - 1) + cbase), v0);
+          tmem_ld_16x24(tl + (uint32_t)(C::acc_col(1, C::NL - 1) + cbase), v1);
+          tmem_ld_wait();
+          hand_back(0);
+#pragma unroll
+          for (int c = 0; c < CPW; c++) {
+            acc[0][c] = (C::LONG ? acc[0][c] : 0) + level_units(v0[c], C::NL - 1);
+            acc[1][c] = (C::LONG ? acc[1][c] : 0) + level_units(v1[c], C::NL - 1);
+          }
+        };
+        if constexpr (C::LONG) {
+          // the pieces before the tile's last one: levels 0 and 1, then the last level
+#pragma unroll
+          for (int c = 0; c < CPW; c++) acc[0][c] = acc[1][c] = 0;
+          auto wait_piece = [&](int which, uint32_t n) {
+            if (!mbar_wait(&tfull[which], (local * pieces + n) & 1, 4 * WAIT_NS, err)) atomicExch(err, 3);
+            __syncwarp();
+            tc_fence_after();
+          };
+#pragma unroll 1
+          for (uint32_t n = 0; n + 1 < pieces; n++) {
+            add_levels01(0);
+            add_levels01(1);
+            wait_piece(1, n);
+            add_last();
+            wait_piece(0, n + 1);
+          }
         }
+        add_last();  // group 0
+        wait_rest();
+#pragma unroll
+        for (int part = 0; part < 2; part++) add_levels01(part);  // group 1
 #pragma unroll
         for (int l = 2; l < C::NL - 1; l++) {  // group l: level l
 #pragma unroll
@@ -1392,7 +1442,7 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
           if (grow + 8 * h >= g.mrows) continue;
           double2 *p0 = cp[col], *p1 = cp[col + 1];
           if (!p0) continue;
-          const int e0 = (h ? erow1 : erow0) + sx[col] - 54, e1 = (h ? erow1 : erow0) + sx[col + 1] - 54;
+          const int e0 = (h ? erow1 : erow0) + sx[col] - UNIT, e1 = (h ? erow1 : erow0) + sx[col + 1] - UNIT;
           const double2 z0 = make_double2(i2d_scaled(acc[0][c], e0), i2d_scaled(acc[1][c], e0));
           const double2 z1 = make_double2(i2d_scaled(acc[0][c + 1], e1), i2d_scaled(acc[1][c + 1], e1));
           const size_t off = (size_t)(grow + 8 * h) * g.blkn;
@@ -2162,7 +2212,7 @@ static int ensure_smem(K kernel, size_t smem, bool& done) {
 }
 static bool g_attr_sls = false, g_attr_srs = false, g_attr_tg = false, g_attr_sld = false, g_attr_srd = false;
 static bool g_attr_sl = false, g_attr_sr = false, g_attr_tl = false, g_attr_std = false,
-            g_attr_hp = false;
+            g_attr_hp = false, g_attr_hpl = false;
 static int g_nsm = 0;
 
 template <class C>
@@ -2171,6 +2221,8 @@ template <>
 bool& gemm_attr_flag<CfgStd>() { return g_attr_std; }
 template <>
 bool& gemm_attr_flag<CfgHP>() { return g_attr_hp; }
+template <>
+bool& gemm_attr_flag<CfgHPLong>() { return g_attr_hpl; }
 
 static int sm_count(int* out) {
   if (!g_nsm) {
@@ -2195,6 +2247,7 @@ int split_kernels_prepare() {
   CTR_TRY(ensure_smem(slice_task_left_kernel<CfgHP>, 512 + CfgHP::A_STAGE, g_attr_tl));
   CTR_TRY(ensure_smem(split_gemm_kernel<CfgStd>, gemm_smem_bytes<CfgStd>(), g_attr_std));
   CTR_TRY(ensure_smem(split_gemm_kernel<CfgHP>, gemm_smem_bytes<CfgHP>(), g_attr_hp));
+  CTR_TRY(ensure_smem(split_gemm_kernel<CfgHPLong>, gemm_smem_bytes<CfgHPLong>(), g_attr_hpl));
   return CTR_OK;
 }
 
@@ -2456,6 +2509,9 @@ int launch_split_gemm(const SplitGemmBatch& g, int ninst, int* d_err, cudaStream
   if (ninst == 0) return CTR_OK;
   if (g.hp) {
     if (g.out_mode != 1 || g.levels) return fail(CTR_ERR_ARG, "split GEMM: the high-precision tiles write complex128");
+    // (Gram products halve their leading digits instead: their pieces' errors are far below their scales)
+    if (!gram && g.nchunk > 8)
+      return launch_split_gemm_cfg<CfgHPLong>(g, ninst, d_err, s, "split_gemm_hp", &g_split_mma_flops);
     return gram ? launch_split_gemm_cfg<CfgHP>(g, ninst, d_err, s, "gram_gemm", &g_gram_mma_flops)
                 : launch_split_gemm_cfg<CfgHP>(g, ninst, d_err, s, "split_gemm_hp", &g_split_mma_flops);
   }

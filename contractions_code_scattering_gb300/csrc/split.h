@@ -37,9 +37,10 @@ constexpr int SPLIT_MAXBLK = 32;
 // width 2 BN per slice pair, Xr [Yr | Yi] and Xi [-Yi | Yr], into one [Re | Im]
 // accumulator per level (instead of four MMAs of width BN); the left operand
 // tile is then read from shared memory half as often per flop.
-template <int NS_, int NL_, int BN_, bool PACK_, bool INT_OUT_>
+template <int NS_, int NL_, int BN_, bool PACK_, bool INT_OUT_, bool LONG_ = false>
 struct SplitCfg {
   static constexpr int NS = NS_, NL = NL_, BN = BN_;
+  static constexpr bool LONG = LONG_;  // K above 128: levels 0 and 1 drained piece by piece
   static constexpr bool PACK = PACK_;
   static constexpr bool INT_OUT = INT_OUT_;  // epilogue: complex128 via exact integer sums (else float-float)
   static constexpr int EPI_WARPS = 16;             // 4 per TMEM lane quadrant, splitting the columns
@@ -54,6 +55,7 @@ struct SplitCfg {
 };
 using CfgStd = SplitCfg<SPLIT_NSLICE, 4, SPLIT_N, true, false>;
 using CfgHP = SplitCfg<6, 5, 48, true, true>;
+using CfgHPLong = SplitCfg<6, 5, 48, true, true, true>;  // CfgHP's operands, any number of chunks
 static_assert(CfgStd::B_STAGE == SPLIT_B_STAGE && CfgStd::A_STAGE == SPLIT_A_STAGE, "standard stage sizes");
 static_assert(CfgStd::BN % (CfgStd::EPI_CW * (CfgStd::EPI_WARPS / 4)) == 0 &&
                   CfgHP::BN % (CfgHP::EPI_CW * (CfgHP::EPI_WARPS / 4)) == 0,
@@ -108,7 +110,7 @@ struct SplitGemmBatch {
                      // [8][ncols][ldo] of instance 0 instead of the ff output
   int out_mode;      // 0: float-float column-major, 1: complex128 row-major blocks
   int blkn;          // out_mode 1: columns (and row stride) of one output block
-  int hp;            // 0: CfgStd operands and tiles, 1: CfgHP (out_mode 1 only)
+  int hp;            // 0: CfgStd operands and tiles, 1: CfgHP's (out_mode 1 only)
   int order;         // persistent tile walk: 0 N tiles innermost, 1 M tiles innermost
   int step;          // split_tail_step(K) of operands sliced that way, 0 or 1 otherwise
 };
@@ -117,8 +119,6 @@ struct SplitGemmBatch {
 // concatenated along K (term q occupies k in [q N, (q+1) N)).  Left: rows of
 // the A side with the weights applied; right: up to SPLIT_TASK_NB output blocks
 // stacked along N.  dag bit q (left) / bit 4j+q (right): conjugate transpose.
-// eplus = 1 halves the leading digit (|d_0| <= 128) so that level 0 stays
-// exact for K <= 512.
 // The scale exponents come from per-block tables: bi indexes a table of
 // [2][nev] ints per distinct block of the launch (row-wise and column-wise
 // exponent bounds, launch_block_exp); wexp is the exponent of the power-of-two
@@ -128,14 +128,14 @@ struct SliceTaskLJob {
   const double2* a[4];
   float w[4];
   int bi[4], wexp[4];
-  int nterm, dag, eplus, pad;
+  int nterm, dag;
   uint8_t* out;  // [nchunk][CfgHP::A_STAGE]
   int* exps;     // [SPLIT_M]
 };
 struct SliceTaskRJob {
   const double2* b[SPLIT_TASK_NB][4];
   int bi[SPLIT_TASK_NB][4];
-  int nb, nterm, dag, eplus;
+  int nb, nterm, dag;
   uint8_t* out;  // [ntiles][nchunk][CfgHP::B_STAGE]
   int* exps;     // [ntiles * CfgHP::BN]
 };
@@ -150,7 +150,7 @@ struct SliceStackLJob {
   int bi[SPLIT_STACK][4];
   float w[4];
   int wexp[4];
-  int nslab, nterm, dag, eplus;
+  int nslab, nterm, dag;
   uint8_t* out;  // [mtiles][nchunk][CfgHP::A_STAGE]
   int* exps;     // [mtiles * SPLIT_M]
 };
