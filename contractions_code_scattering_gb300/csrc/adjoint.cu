@@ -757,7 +757,7 @@ int rho_vjp(const Ctx& c, const double2* prop, const double2* phis, const double
     }
   const int nL = (int)Ls.size(), nR = (int)Rs.size(), kinds = grad ? 2 : 1;
   const size_t per_pair = 16 * (size_t)kinds * (nL + nR) * N2 * sizeof(double2);
-  const int batch = std::max(1, std::min((int)pairs.size(), (int)(sets_budget() / per_pair)));
+  const int batch = (int)std::max<size_t>(1, std::min(pairs.size(), CHAIN_BUDGET / per_pair));
   for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
     const int np = (int)pb.ent.size();
     void* mem;
@@ -930,13 +930,6 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
   const bool g = grad != nullptr, hor = iso == 0;
   auto P = [&](int k, int t) { return el[q[k]].p + (size_t)t * el[q[k]].stride; };  // k = 0..3: P1..P4
   enum { P1 = 0, P2 = 1, P3 = 2, P4 = 3 };
-  // tau(t, t) [t][16]
-  void* dmem;
-  CTR_TRY(workspace(WS_ADJ_DIAG).get((size_t)Nt * blk16 * sizeof(double2), &dmem));
-  double2* diag = (double2*)dmem;
-  for (int t = 0; t < Nt; t++)
-    CTR_CUDA(cudaMemcpyAsync(diag + (size_t)t * blk16, prop + ((size_t)t * Nt + t) * blk16, blk16 * sizeof(double2),
-                             cudaMemcpyDeviceToDevice, c.s));
   Combos cb(Nt);
   const int cL = cb.use(q[P3], q[P4]), cSq = cb.use(q[P2], q[P1]), cDt = cb.use(q[P1], q[P2]);
   std::vector<char> on_tf(Nt, 0), on_ti(Nt, 0);
@@ -945,7 +938,8 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
     cb.need[cL][p / Nt] = cb.need[cSq][p % Nt] = cb.need[cDt][p % Nt] = 1;
   }
   std::vector<const double2*> M;
-  CTR_TRY(per_t_products(c, diag, el, WS_RPHI, cb.list, cb.need, M));
+  // tau(t, t) of the full perambulator
+  CTR_TRY(per_t_products(c, prop, (size_t)(Nt + 1) * blk16, el, WS_RPHI, cb.list, cb.need, 16 * (4 * (size_t)Nt + 4), M));
   // co-factors per time slice: K [tf][16], Jsq, Jdt [ti][16] (block (row, column) of the co-factor)
   double2 *Ks = nullptr, *Js = nullptr, *Jd = nullptr;
   if (g) {
@@ -961,7 +955,10 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
                         + (g ? 48 + 32 + 8 : 0)           // Rw, S, K; U; O
                         + (g && hor ? 32 + 32 + 32 + 8 : 0);  // Y; Z; Q; N
   const size_t per_pair = blocks * N2 * sizeof(double2);
-  const int batch = std::max(1, std::min((int)pairs.size(), (int)(sets_budget() / per_pair)));
+  // what the per-time-slice products and co-factors leave of the budget
+  const size_t fixed = ((size_t)4 + (g ? 3 : 0)) * Nt * blk16 * sizeof(double2);
+  const size_t budget = CHAIN_BUDGET - std::min(CHAIN_BUDGET, fixed);
+  const int batch = (int)std::max<size_t>(1, std::min(pairs.size(), budget / per_pair));
   for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
     const int np = (int)pb.ent.size();
     void* mem;
@@ -1258,7 +1255,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
     }
   }
   const size_t per_sl = 64 * N2 * sizeof(double2);
-  const size_t chunk = std::max<size_t>(1, std::min(sl.size(), sets_budget() / per_sl));
+  const size_t chunk = std::max<size_t>(1, std::min(sl.size(), budget / per_sl));
   for (size_t s0 = 0; s0 < sl.size(); s0 += chunk) {
     const size_t ns = std::min(chunk, sl.size() - s0);
     void* mem;
@@ -1267,7 +1264,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
     PairList pl;
     for (size_t k = 0; k < ns; k++) {
       const Slice& S = sl[s0 + k];
-      const double2* D = diag + (size_t)S.t * blk16;
+      const double2* D = prop + (size_t)S.t * (Nt + 1) * blk16;
       double2* o = (double2*)mem + k * 64 * N2;  // tau Pb, F Pa, Pa tau, Pb F
       GridTask A = make_grid(16, 1, 1, kOne, 0, 0), B = make_grid(16, 1, 1, kOne, 0, 0);
       for (int b = 0; b < 16; b++) {

@@ -68,12 +68,14 @@ GridTask make_grid(int nslab, int nb, int nterm, const float* w, int adag, int b
 // One stage on the call's engine: plain tasks, or grids (stacked along M on the split engine).
 int run_stage(const Ctx& c, const std::vector<ZTask>& tasks, int slot);
 int run_grids(const Ctx& c, const std::vector<GridTask>& g, int slot);
-int per_t_products(const Ctx& c, const double2* diag, const std::vector<Elem>& el, int slot,
+int per_t_products(const Ctx& c, const double2* diag, size_t dstride, const std::vector<Elem>& el, int slot,
                    const std::vector<std::pair<int, int>>& combos, const std::vector<std::vector<char>>& need,
-                   std::vector<const double2*>& M);
+                   size_t cap, std::vector<const double2*>& M);
 // One call's own elementals, [nt][nev][nev] each; set[k]: the first of them with the k-th one's address.
 std::vector<Elem> elems(int nev, const std::vector<const double*>& p, int32_t* set);
-// Scratch budget of a batch of pairs.
+// Scratch budget of a batch of pairs: of a momentum-set call, and of every other call, which
+// has to run beside a caller's own tensors.
 size_t sets_budget();
+constexpr size_t CHAIN_BUDGET = (size_t)3 << 30;
 
 }  // namespace ctr

@@ -292,15 +292,17 @@ size_t sets_budget() {
 // Per time slice: M(a, b, t) = Phi_a(t) taud(t) Phi_b(t), 16 consecutive blocks at
 // M[combo * Nt + t], for the (a, b) combos and the t flagged in need.  Two stages
 // of grids: Phi_a taud_blk for every a of a time slice stacked along M against
-// taud_blk, then its 16 blocks stacked against every Phi_b that follows a.
-int per_t_products(const Ctx& c, const double2* diag, const std::vector<Elem>& el, int slot,
+// taud_blk, then its 16 blocks stacked against every Phi_b that follows a.  taud(t) =
+// diag + t * dstride.  The time slices run in groups where all their Phi_a taud
+// would make it more than `cap` blocks (0: no limit).
+int per_t_products(const Ctx& c, const double2* diag, size_t dstride, const std::vector<Elem>& el, int slot,
                    const std::vector<std::pair<int, int>>& combos, const std::vector<std::vector<char>>& need,
-                   std::vector<const double2*>& M) {
+                   size_t cap, std::vector<const double2*>& M) {
   const int Nt = c.Nt, nc = (int)combos.size();
   const size_t N2 = c.N2, blk16 = 16 * N2;
   auto P = [&](int q, int t) { return el[q].p + (size_t)t * el[q].stride; };
   M.assign((size_t)nc * Nt, nullptr);
-  size_t nblk = 0;
+  size_t nblk = 0, ntmp = 0;
   std::vector<std::vector<int>> as(Nt);  // distinct first elementals of each time slice
   for (int t = 0; t < Nt; t++)
     for (int ci = 0; ci < nc; ci++)
@@ -308,45 +310,60 @@ int per_t_products(const Ctx& c, const double2* diag, const std::vector<Elem>& e
         nblk += 16;
         if (std::find(as[t].begin(), as[t].end(), combos[ci].first) == as[t].end()) as[t].push_back(combos[ci].first);
       }
-  for (auto& v : as) nblk += 16 * v.size();
-  void* mem;
-  CTR_TRY(workspace(slot).get(nblk * N2 * sizeof(double2), &mem));
-  double2* next = (double2*)mem;
-  std::vector<GridTask> g0, g1;
-  for (int t = 0; t < Nt; t++) {
-    const int na = (int)as[t].size();
-    if (!na) continue;
-    double2* tmp = next;  // block b of the a-th elemental at (b * na + a)
-    next += (size_t)16 * na * N2;
-    for (int jb = 0; jb < 2; jb++) {
-      GridTask G = make_grid(na, 8, 1, kOne, 0, 0);
-      for (int k = 0; k < na; k++) G.A[k] = P(as[t][k], t);
-      for (int j = 0; j < 8; j++) {
-        G.B[j][0] = diag + (size_t)t * blk16 + (size_t)(8 * jb + j) * N2;
-        G.C0[j] = tmp + (size_t)(8 * jb + j) * na * N2;
-      }
-      g0.push_back(std::move(G));
+  const size_t room = cap == 0 ? ~(size_t)0 : cap - std::min(cap, nblk);
+  std::vector<int> ends;  // of the groups of time slices
+  for (int t = 0, t0 = 0, used = 0; t < Nt; t++) {
+    const int n = 16 * (int)as[t].size();
+    if (t > t0 && (size_t)(used + n) > room) {
+      ends.push_back(t0 = t);
+      used = 0;
     }
-    for (int k = 0; k < na; k++) {
-      std::vector<int> cs;
-      for (int ci = 0; ci < nc; ci++)
-        if (need[ci][t] && combos[ci].first == as[t][k]) cs.push_back(ci);
-      for (size_t c0 = 0; c0 < cs.size(); c0 += 8) {
-        GridTask G = make_grid(16, (int)std::min<size_t>(8, cs.size() - c0), 1, kOne, 0, 0);
-        for (int b = 0; b < 16; b++) G.A[b] = tmp + ((size_t)b * na + k) * N2;
-        for (int j = 0; j < G.nb; j++) {
-          const int ci = cs[c0 + j];
-          G.B[j][0] = P(combos[ci].second, t);
-          G.C0[j] = next;
-          M[(size_t)ci * Nt + t] = next;
-          next += blk16;
-        }
-        g1.push_back(std::move(G));
-      }
-    }
+    used += n;
+    ntmp = std::max<size_t>(ntmp, used);
   }
-  CTR_TRY(run_grids(c, g0, WS_TASKS));
-  return run_grids(c, g1, WS_TASKS2);
+  ends.push_back(Nt);
+  void* mem;
+  CTR_TRY(workspace(slot).get((nblk + ntmp) * N2 * sizeof(double2), &mem));
+  double2 *next = (double2*)mem, *const tmp0 = next + nblk * N2;
+  for (size_t e = 0; e < ends.size(); e++) {
+    std::vector<GridTask> g0, g1;
+    double2* tnext = tmp0;
+    for (int t = e ? ends[e - 1] : 0; t < ends[e]; t++) {
+      const int na = (int)as[t].size();
+      if (!na) continue;
+      double2* tmp = tnext;  // block b of the a-th elemental at (b * na + a)
+      tnext += (size_t)16 * na * N2;
+      for (int jb = 0; jb < 2; jb++) {
+        GridTask G = make_grid(na, 8, 1, kOne, 0, 0);
+        for (int k = 0; k < na; k++) G.A[k] = P(as[t][k], t);
+        for (int j = 0; j < 8; j++) {
+          G.B[j][0] = diag + (size_t)t * dstride + (size_t)(8 * jb + j) * N2;
+          G.C0[j] = tmp + (size_t)(8 * jb + j) * na * N2;
+        }
+        g0.push_back(std::move(G));
+      }
+      for (int k = 0; k < na; k++) {
+        std::vector<int> cs;
+        for (int ci = 0; ci < nc; ci++)
+          if (need[ci][t] && combos[ci].first == as[t][k]) cs.push_back(ci);
+        for (size_t c0 = 0; c0 < cs.size(); c0 += 8) {
+          GridTask G = make_grid(16, (int)std::min<size_t>(8, cs.size() - c0), 1, kOne, 0, 0);
+          for (int b = 0; b < 16; b++) G.A[b] = tmp + ((size_t)b * na + k) * N2;
+          for (int j = 0; j < G.nb; j++) {
+            const int ci = cs[c0 + j];
+            G.B[j][0] = P(combos[ci].second, t);
+            G.C0[j] = next;
+            M[(size_t)ci * Nt + t] = next;
+            next += blk16;
+          }
+          g1.push_back(std::move(G));
+        }
+      }
+    }
+    CTR_TRY(run_grids(c, g0, WS_TASKS));
+    CTR_TRY(run_grids(c, g1, WS_TASKS2));
+  }
+  return CTR_OK;
 }
 
 // Distinct values in ascending order, and the index of each of 0 .. n - 1.
@@ -366,7 +383,7 @@ static std::vector<int> index_of(std::vector<int>& v, int n) {
 // each set's entries are bitwise those of a call of its own.
 int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* prop_rows, const double* prop_diag,
               const std::vector<Elem>& el, int nset, const int32_t* sets, double* corr, cudaStream_t s, int engine,
-              const std::vector<int>* plist) {
+              bool sets_call, const std::vector<int>* plist) {
   Ctx c{N, Nt, (size_t)N * N, s, engine};
   if (engine == CTR_ENGINE_SPLIT && !plist) g_refined_last = 0;
   const size_t N2 = c.N2, blk16 = 16 * N2;
@@ -398,7 +415,8 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
   }
   std::vector<const double2*> M;
   // a recomputation (plist) keeps its own per-time-slice products
-  CTR_TRY(per_t_products(c, diag, el, plist ? WS_RPHI : WS_PHI, cb.list, cb.need, M));
+  CTR_TRY(per_t_products(c, diag, blk16, el, plist ? WS_RPHI : WS_PHI, cb.list, cb.need,
+                         sets_call ? 0 : 16 * (4 * (size_t)Nt + 4), M));
   const std::vector<int> icl = index_of(CL, (int)cb.list.size()), icr = index_of(CR, (int)cb.list.size());
   const int nCL = (int)CL.size(), nCR = (int)CR.size();
   // elementals on the sink side (P3, P4) and on the source side (P1, P2)
@@ -445,7 +463,8 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
   const size_t blk_pair = 16 * (size_t)(nCR + nCL + nW + nU + (iso == 0 ? nW + nF : 0));
   const size_t tr_pair = (size_t)nset * (iso == 0 ? 48 : 32) + 16 * (size_t)nTW;
   const size_t per_pair = blk_pair * N2 * sizeof(double2) + tr_pair * (sizeof(double2) + sizeof(double));
-  const int batch = std::max(1, std::min(npairs, (int)(sets_budget() / std::max<size_t>(per_pair, 1))));
+  const size_t budget = sets_call ? sets_budget() : CHAIN_BUDGET;
+  const int batch = std::max(1, std::min(npairs, (int)(budget / std::max<size_t>(per_pair, 1))));
   Refine rf;
   CTR_TRY(refine_begin(c, (size_t)nset * npairs * 5, WS_REFINE, rf));
   for (const PairBatch& pb : pair_batches(tau, blk16, Nt, tf_begin, rows, batch, plist)) {
@@ -651,7 +670,8 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
                         std::vector<int> pl;
                         while (u1 < units.size() && units[u1] / npairs == k) pl.push_back(units[u1++] % npairs);
                         CTR_TRY(pipi_core(N, Nt, tf_begin, tf_end, iso, prop_rows, prop_diag, elc, 1,
-                                          set_copy.data() + 4 * k, (double*)(out + u0 * 5), ls, CTR_ENGINE_FP64, &pl));
+                                          set_copy.data() + 4 * k, (double*)(out + u0 * 5), ls, CTR_ENGINE_FP64, false,
+                                          &pl));
                         u0 = u1;
                       }
                       return CTR_OK;
@@ -850,12 +870,12 @@ bool sink_plan(const std::vector<Vertex>& V, SinkPlan& P) {
 // lib/calculate_rhopi_core.h: coef * Tr[Phi_ip(tf) tau_{s5s6} Phi_P2(ti)
 // taud(ti)_{s1s2} Phi_P1(ti) tau_{s3s2}^dag] with s6 = s1, s4 = s3 and coef =
 // c(iop, s3, s5) g5(s1), so the sum over s1 is (T G R)_{s5 s2}; the triangle's
-// sum over s3 is (T G R)_{s1 s5} alike.  gram: the closing traces may run as
-// Gram products (split engine).
+// sum over s3 is (T G R)_{s1 s5} alike.  sets_call: the closing traces may run as
+// Gram products (split engine), and the batches take the sets' budget.
 int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* prop_rows, const double* prop_diag,
                        const std::vector<Elem>& el, const double* mom5, const double* mom2, int nset,
                        const int32_t* sets, const std::vector<int>& idirs, double* rhopi, double* tri,
-                       double* hor_fish, cudaStream_t s, int engine, bool gram_ok, const std::vector<int>* plist,
+                       double* hor_fish, cudaStream_t s, int engine, bool sets_call, const std::vector<int>* plist,
                        const std::vector<int>* tlist) {
   Ctx c{N, Nt, (size_t)N * N, s, engine};
   const bool rerun = plist || tlist;
@@ -878,7 +898,8 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   const int nC = (int)cb.list.size();
   std::vector<const double2*> M;
   // a recomputation keeps its own R, so that the caller's stays valid
-  CTR_TRY(per_t_products(c, diag, el, rerun ? WS_RPHI : WS_PHI, cb.list, cb.need, M));
+  CTR_TRY(per_t_products(c, diag, blk16, el, rerun ? WS_RPHI : WS_PHI, cb.list, cb.need,
+                         sets_call ? 0 : 16 * (2 * (size_t)Nt + 4), M));
   std::vector<int32_t> sc(sets, sets + 2 * nset);
   std::vector<Elem> elc(el);
 
@@ -997,13 +1018,14 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   const size_t blk_pair = 16 * ((size_t)nC + nops);
   const size_t tr_pair = (size_t)nset * (uniq.size() + (tri ? 32 : 0));
   const size_t per_pair = blk_pair * N2 * sizeof(double2) + tr_pair * (sizeof(double2) + sizeof(double));
-  const int batch = std::max(1, std::min(npairs, (int)(sets_budget() / std::max<size_t>(per_pair, 1))));
+  const size_t budget = sets_call ? sets_budget() : CHAIN_BUDGET;
+  const int batch = std::max(1, std::min(npairs, (int)(budget / std::max<size_t>(per_pair, 1))));
   // closing-trace form on the split engine (chains.trace_form): when it is known
   // to be the Gram products, the FP64 trace tasks are not built
   const std::string trace_shape =
       "nev=" + std::to_string(N) + ",m=" + std::to_string(4 * nC) + ",n=" + std::to_string(4 * nops);
   int known_form = 0;
-  const bool gram = c.engine == CTR_ENGINE_SPLIT && gram_ok;
+  const bool gram = c.engine == CTR_ENGINE_SPLIT && sets_call;
   const bool fp64_traces_needed = !gram ||
                                   !tune_peek("chains.trace_form", trace_shape, 2, 1, &known_form) || known_form == 0;
   Refine rf_rp, rf_tr;
@@ -1040,7 +1062,7 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   const int nH = (int)sp.H.size();
   const size_t per_pair_sink = 16 * ((size_t)nops + nH) * N2 * sizeof(double2) +
                                (size_t)nH * nC * (sizeof(double2) + sizeof(double));
-  const int batch_sink = std::max(1, std::min(npairs, (int)(sets_budget() / per_pair_sink)));
+  const int batch_sink = std::max(1, std::min(npairs, (int)(budget / per_pair_sink)));
   // 9 sink times of 14 rows fill a 128-row tile of the Gram product
   for (const PairBatch& pb : sink ? pair_batches(tau, blk16, Nt, tf_begin, rows, batch_sink, plist, 18)
                                   : std::vector<PairBatch>()) {
@@ -1399,7 +1421,7 @@ int ctr_pipi(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin,
   int32_t set[4];
   const std::vector<ctr::Elem> el = ctr::elems(nev, {p1, p2, p3, p4}, set);
   return ctr::pipi_core(nev, nt, tf_begin, tf_end, isospin, prop_rows, prop_diag, el, 1, set, corr,
-                        (cudaStream_t)stream, engine, nullptr);
+                        (cudaStream_t)stream, engine, false, nullptr);
 }
 
 int ctr_pipi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin, const double* prop_rows,
@@ -1414,7 +1436,7 @@ int ctr_pipi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, int iso
     if (sets[k] < 0 || sets[k] >= nphi)
       return ctr::fail(CTR_ERR_ARG, "ctr_pipi_sets: elemental index %d not in [0,%d)", sets[k], nphi);
   return ctr::pipi_core(nev, nt, tf_begin, tf_end, isospin, prop_rows, prop_diag, ctr::elems(nev, phi, nphi), nset,
-                        sets, corr, (cudaStream_t)stream, engine, nullptr);
+                        sets, corr, (cudaStream_t)stream, engine, true, nullptr);
 }
 
 int ctr_rhopi_sigmapi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, const double* prop_rows,
