@@ -729,6 +729,9 @@ std::vector<int> weighted_pairs(int Nt, int nout, const double2* w) {
   return p;
 }
 
+// Host tables of a batch.
+constexpr size_t TABLE_BUDGET = (size_t)64 << 20;
+
 // rho (lib/calculate_rho_core.h): a spin row is coef * t, t = Tr[A_cd Bt_ab] with
 // A = tau_cd Phi_L(ti) and Bt = tau_ab^dag Phi_R(tf)^dag, so f_k d/df_k of t is
 // diag(Bt A) at Phi_L's right index and diag(A Bt) at Phi_R's left one.  Cut at the
@@ -757,7 +760,10 @@ int rho_vjp(const Ctx& c, const double2* prop, const double2* phis, const double
     }
   const int nL = (int)Ls.size(), nR = (int)Rs.size(), kinds = grad ? 2 : 1;
   const size_t per_pair = 16 * (size_t)kinds * (nL + nR) * N2 * sizeof(double2);
-  const int batch = (int)std::max<size_t>(1, std::min(pairs.size(), CHAIN_BUDGET / per_pair));
+  // a pair's terms, at most 48 outputs of them; a batch's tables pass through a pinned
+  // staging buffer, so they are bounded as well as its blocks
+  const size_t table = 48 * (sizeof(PairGroup) + 16 * (size_t)kinds * sizeof(PairTerm));
+  const int batch = (int)std::max<size_t>(1, std::min({pairs.size(), CHAIN_BUDGET / per_pair, TABLE_BUDGET / table}));
   for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
     const int np = (int)pb.ent.size();
     void* mem;
@@ -958,7 +964,8 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
   // what the per-time-slice products and co-factors leave of the budget
   const size_t fixed = ((size_t)4 + (g ? 3 : 0)) * Nt * blk16 * sizeof(double2);
   const size_t budget = CHAIN_BUDGET - std::min(CHAIN_BUDGET, fixed);
-  const int batch = (int)std::max<size_t>(1, std::min(pairs.size(), budget / per_pair));
+  const size_t table = 64 * sizeof(DiagTask) + 72 * sizeof(PairTerm) + 5 * sizeof(PairGroup);
+  const int batch = (int)std::max<size_t>(1, std::min({pairs.size(), budget / per_pair, TABLE_BUDGET / table}));
   for (const PairBatch& pb : pair_batches(prop, blk16, Nt, 0, Nt, batch, &pairs)) {
     const int np = (int)pb.ent.size();
     void* mem;

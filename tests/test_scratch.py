@@ -55,3 +55,18 @@ def test_single_calls_keep_to_three_gigabytes(cuda, kind):
                 api.pipi_profile_vjp(tau, *p, f, w, 0, engine="fp64")
 
     assert _growth(call) <= 5 * 1024 * MB
+
+
+def test_gradient_tables_are_bounded(cuda):
+    """Every output of a rho gradient weighted at a small Nev: the pair tables pass through
+    a pinned buffer, in batches of 64 MB."""
+    n, nt = 2, 96
+    tau, mom5 = _gauss(nt, nt, 4, 4, n, n), _gauss(nt, 5, n, n)
+    f = torch.rand(n, dtype=torch.float64, device="cuda") + 0.5
+
+    def call(rows):
+        w = torch.zeros((nt, nt, 48), dtype=torch.complex128, device="cuda")
+        w[:rows or nt] = 1.0
+        api.rho_profile_vjp(tau, mom5, f, w, engine="fp64")
+
+    assert _growth(call) <= 400 * MB
