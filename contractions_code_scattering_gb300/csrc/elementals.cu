@@ -223,8 +223,9 @@ __global__ void __launch_bounds__(256) el_sum_kernel(const ElTask* __restrict__ 
   }
 }
 
-// Launches of at most EL_PART_BYTES of partial tiles each.
-constexpr size_t EL_PART_BYTES = (size_t)512 << 20;
+// Launches of at most EL_PART_BYTES of partial tiles each: 3300 tiles of 50 x 50, 7 waves of
+// them (7 momenta on 16^3, Nev = 100: 128 ms with 128 to 512 MB, 135 with 64).
+constexpr size_t EL_PART_BYTES = (size_t)128 << 20;
 
 template <int TE, int RX, int RY>
 int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const double2* phase, long long V,
@@ -237,18 +238,28 @@ int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const
   for (const ElTask& T : tasks) units += (long long)T.nterm * (T.self ? nti * (nti + 1) / 2 : nti * nti);
   // pieces a product: enough that the launch has about 16 CTAs an SM (its last
   // wave then costs a few percent), none shorter than 512 of K
-  const int nsplit = (int)std::max<long long>(1, std::min((16LL * nsm + units - 1) / units, K / 512));
+  int nsplit = (int)std::max<long long>(1, std::min((16LL * nsm + units - 1) / units, K / 512));
   void* d_tasks;
   CTR_TRY(upload(WS_TASKS, tasks.data(), tasks.size() * sizeof(ElTask), &d_tasks, s));
-  const size_t max_parts = EL_PART_BYTES / ((size_t)TE * TE * sizeof(double2));
+  // partial tiles of a launch; fewer, and longer pieces, where memory is short
+  const size_t tile_bytes = (size_t)TE * TE * sizeof(double2);
+  size_t max_parts = std::min<size_t>(EL_PART_BYTES / tile_bytes, (size_t)units * nsplit);
+  void* part;
+  for (;;) {
+    nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, max_parts / 3));
+    const int rc = workspace(WS_ROWS).get(max_parts * tile_bytes, &part);
+    if (rc == CTR_OK) break;
+    if (rc != CTR_ERR_ALLOC || max_parts <= 3 || capturing()) return rc;
+    cudaGetLastError();
+    max_parts = std::max<size_t>(3, max_parts / 2);
+  }
   std::vector<ElPiece> pieces;
   std::vector<int4> tiles;
   auto flush = [&]() -> int {
     if (pieces.empty()) return CTR_OK;
-    void *d[2], *part;
+    void* d[2];
     CTR_TRY(upload_group(WS_TASKS2, {{pieces.data(), pieces.size() * sizeof(ElPiece)},
                                      {tiles.data(), tiles.size() * sizeof(int4)}}, d, s));
-    CTR_TRY(workspace(WS_ROWS).get(pieces.size() * TE * TE * sizeof(double2), &part));
     {
       TimedLaunch tl(s, "el_gemm");
       el_gemm_kernel<TE, RX, RY><<<(unsigned)pieces.size(), (TE / RX) * (TE / RY), 0, s>>>(

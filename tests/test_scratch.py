@@ -70,3 +70,12 @@ def test_gradient_tables_are_bounded(cuda):
         api.rho_profile_vjp(tau, mom5, f, w, engine="fp64")
 
     assert _growth(call) <= 400 * MB
+
+
+def test_elementals_partial_tiles(cuda):
+    """The partial tiles of the elementals: 128 MB beside the derivative fields and phases."""
+    n, nt, l = 100, 4, 8
+    v = _gauss(nt, n, l, l, l, 3)
+    links = _gauss(nt, l, l, l, 3, 3, 3)
+    moms = [(a, b, c) for a in range(4) for b in range(4) for c in range(8)]
+    assert _growth(lambda rows: api.elementals(v, moms[:rows or len(moms)], links=links)) <= 240 * MB
