@@ -235,7 +235,11 @@ int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const
   CTR_CUDA(cudaGetDevice(&dev));
   CTR_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   long long units = 0;  // products of one tile
-  for (const ElTask& T : tasks) units += (long long)T.nterm * (T.self ? nti * (nti + 1) / 2 : nti * nti);
+  int most = 1;         // of one task's
+  for (const ElTask& T : tasks) {
+    units += (long long)T.nterm * (T.self ? nti * (nti + 1) / 2 : nti * nti);
+    most = std::max(most, T.nterm);
+  }
   // pieces a product: enough that the launch has about 16 CTAs an SM (its last
   // wave then costs a few percent), none shorter than 512 of K
   int nsplit = (int)std::max<long long>(1, std::min((16LL * nsm + units - 1) / units, K / 512));
@@ -246,12 +250,12 @@ int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const
   size_t max_parts = std::min<size_t>(EL_PART_BYTES / tile_bytes, (size_t)units * nsplit);
   void* part;
   for (;;) {
-    nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, max_parts / 3));
+    nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, max_parts / most));
     const int rc = workspace(WS_ROWS).get(max_parts * tile_bytes, &part);
     if (rc == CTR_OK) break;
-    if (rc != CTR_ERR_ALLOC || max_parts <= 3 || capturing()) return rc;
+    if (rc != CTR_ERR_ALLOC || max_parts <= (size_t)most || capturing()) return rc;
     cudaGetLastError();
-    max_parts = std::max<size_t>(3, max_parts / 2);
+    max_parts = std::max<size_t>(most, max_parts / 2);
   }
   std::vector<ElPiece> pieces;
   std::vector<int4> tiles;
