@@ -688,6 +688,29 @@ int profiled(int N, long long nmat, const double* phi, const double* f, int slot
   return CTR_OK;
 }
 
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// A gradient's correlators, of which the caller's array need only hold doubles: the kernels
+// write p, 16-byte aligned, and close() copies it to the array where it is not.
+struct CorrOut {
+  double* to;
+  size_t n;
+  double2* p = nullptr;
+  CorrOut(double* corr, size_t entries) : to(corr), n(entries) {}
+  int open() {
+    p = (double2*)to;
+    void* m;
+    if (aligned16(to)) return CTR_OK;
+    CTR_TRY(workspace(WS_ADJ_CORR).get(n * sizeof(double2), &m));
+    p = (double2*)m;
+    return CTR_OK;
+  }
+  int close(cudaStream_t s) const {
+    if (p != (double2*)to) CTR_CUDA(cudaMemcpyAsync(to, p, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    return CTR_OK;
+  }
+};
+
 int check_f(int N, const double* f, cudaStream_t s) {
   std::vector<double> h(N);
   CTR_CUDA(cudaMemcpyAsync(h.data(), f, N * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1380,8 +1403,11 @@ int ctr_rho_profile_vjp(int engine, int nev, int nt, const double* prop, const d
   CTR_CUDA(cudaStreamSynchronize(s));
   double2* phis;
   CTR_TRY(profiled(nev, (long long)nt * 5, mom5, f, WS_PHI, &phis, s));
-  return rho_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, (const double2*)prop, phis, f, (const double2*)hw.data(),
-                 (double2*)corr, grad);
+  CorrOut out(corr, (size_t)nt * nt * 48);
+  CTR_TRY(out.open());
+  CTR_TRY(rho_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, (const double2*)prop, phis, f, (const double2*)hw.data(),
+                  out.p, grad));
+  return out.close(s);
 }
 
 int ctr_pipi_profile_vjp(int engine, int nev, int nt, int isospin, const double* prop, const double* p1,
@@ -1404,13 +1430,22 @@ int ctr_pipi_profile_vjp(int engine, int nev, int nt, int isospin, const double*
   void* mem;
   CTR_TRY(workspace(WS_PHI).get(el.size() * n1 * sizeof(double2), &mem));
   for (size_t k = 0; k < el.size(); k++) {
+    if (!aligned16(el[k].p)) {  // p1..p4 need only hold doubles
+      void* raw;
+      CTR_TRY(workspace(WS_SCRATCH).get(n1 * sizeof(double2), &raw));
+      CTR_CUDA(cudaMemcpyAsync(raw, el[k].p, n1 * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+      el[k].p = (const double2*)raw;
+    }
     TimedLaunch tl(s, "apply_profile");
     apply_profile_kernel<<<1024, 256, 0, s>>>(el[k].p, (double2*)mem + k * n1, f, nev, nt);
     CTR_CUDA(cudaGetLastError());
     el[k].p = (const double2*)mem + k * n1;
   }
-  return pipi_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, isospin, (const double2*)prop, el, set, f,
-                  (const double2*)hw.data(), (double2*)corr, grad);
+  CorrOut out(corr, (size_t)nt * nt * 5);
+  CTR_TRY(out.open());
+  CTR_TRY(pipi_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, isospin, (const double2*)prop, el, set, f,
+                   (const double2*)hw.data(), out.p, grad));
+  return out.close(s);
 }
 
 }  // extern "C"
