@@ -58,6 +58,13 @@ __device__ inline double block_sum_256(double v) {
   return r;  // valid in thread 0
 }
 
+// |c| of a row's coefficient; exact where it is real or imaginary, as the tables' are.
+__device__ __forceinline__ double coef_abs(float re, float im) {
+  if (im == 0.f) return fabs((double)re);
+  if (re == 0.f) return fabs((double)im);
+  return sqrt((double)re * re + (double)im * im);
+}
+
 // Block sums of two FP64 values: lanes 0-15 of each warp carry the first, 16-31
 // the second (5 adds a warp instead of 10: each holds the FP64 pipe for 16
 // clocks), then the warps' sums in order.  Thread k < 2 returns value k.

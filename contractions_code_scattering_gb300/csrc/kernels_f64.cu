@@ -311,7 +311,7 @@ __device__ __forceinline__ float abs1_scaled_f32(double2 v) { return abs_scaled_
 // reduction tree is fixed, so results are bitwise reproducible.
 template <int TPB>
 __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restrict__ tasks, int ntask, int N) {
-  __shared__ float reda[TPB / 32];
+  __shared__ double reda[TPB / 32];
   const int t = blockIdx.x;
   if (t >= ntask) return;
   const TraceTask& T = tasks[t];
@@ -341,8 +341,9 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
     }
   }
   if (want_abs) {
-    for (int o = 16; o; o >>= 1) abf += __shfl_xor_sync(0xffffffffu, abf, o);
-    if ((threadIdx.x & 31) == 0) reda[threadIdx.x >> 5] = abf;
+    double ab = (double)abf;
+    for (int o = 16; o; o >>= 1) ab += __shfl_xor_sync(0xffffffffu, ab, o);
+    if ((threadIdx.x & 31) == 0) reda[threadIdx.x >> 5] = ab;
   }
   const double v = block_sum2<TPB>(re, im);
   if (threadIdx.x >= 32) return;
@@ -351,11 +352,11 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
     const double2 z = make_double2(v, vi);
     *T.out = T.mode & 2 ? z : cmul(make_double2((double)T.coef[0], (double)T.coef[1]), z);
     if (want_abs) {
-      float ab = reda[0];
+      double ab = reda[0];
 #pragma unroll
       for (int w = 1; w < TPB / 32; w++) ab += reda[w];
       // 2^-80 = 2^(-2 TRACE_ABS_SHIFT)
-      *T.absout = (double)sqrtf(T.coef[0] * T.coef[0] + T.coef[1] * T.coef[1]) * ((double)ab * 0x1p-80);
+      *T.absout = coef_abs(T.coef[0], T.coef[1]) * (ab * 0x1p-80);
     }
   }
 }
@@ -505,7 +506,7 @@ __global__ void rowsum_coef_refine_kernel(const double2* __restrict__ tr, const 
     const double2 v = tr[t];
     re += cr * v.x - ci * v.y;
     im += cr * v.y + ci * v.x;
-    sc += (double)sqrtf(coef[2 * r] * coef[2 * r] + coef[2 * r + 1] * coef[2 * r + 1]) * trabs[t];
+    sc += coef_abs(coef[2 * r], coef[2 * r + 1]) * trabs[t];
   }
   out[(size_t)p * nout + o] = make_double2(re, im);
   // flagged: an error estimate above the tolerance, a NaN (a product whose

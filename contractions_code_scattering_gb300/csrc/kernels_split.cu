@@ -1877,16 +1877,16 @@ __device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
   return s + __shfl_xor_sync(0xffffffffu, s, 1);
 }
 
-// The same for four FP32 values: each lane returns the sum of value lane >> 3.
-__device__ __forceinline__ float warp_sum4(const float (&v)[4], int lane) {
-  float a[2];
+// The same for four values: each lane returns the sum of value lane >> 3.
+__device__ __forceinline__ double warp_sum4(const double (&v)[4], int lane) {
+  double a[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    const float keep = (lane & 16) ? v[2 + i] : v[i], give = (lane & 16) ? v[i] : v[2 + i];
+    const double keep = (lane & 16) ? v[2 + i] : v[i], give = (lane & 16) ? v[i] : v[2 + i];
     a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
   }
-  const float keep = (lane & 8) ? a[1] : a[0], give = (lane & 8) ? a[0] : a[1];
-  float s = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+  const double keep = (lane & 8) ? a[1] : a[0], give = (lane & 8) ? a[0] : a[1];
+  double s = keep + __shfl_xor_sync(0xffffffffu, give, 8);
   s += __shfl_xor_sync(0xffffffffu, s, 4);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
   return s + __shfl_xor_sync(0xffffffffu, s, 1);
@@ -1957,11 +1957,9 @@ __global__ void __launch_bounds__(TPB) trace_quads_kernel(const TraceGroup* __re
       }
     }
   }
-  // A warp's FP64 add holds the FP64 pipe for 16 clocks, so the eight sums go
-  // through a reduce-scatter (4 + 2 + 1 + 1 + 1 adds a warp instead of 8 x 5) and
-  // the four error scales, which need a few bits, stay in FP32.
-  __shared__ double red[NW][8];
-  __shared__ float reda[NW][4];
+  // A warp's FP64 add holds the FP64 pipe for 16 clocks, so the eight sums and the four
+  // error scales go through reduce-scatters (9 and 6 adds a warp instead of 12 x 5).
+  __shared__ double red[NW][8], reda[NW][4];
   const int lane = threadIdx.x & 31;
   double v[8];
 #pragma unroll
@@ -1970,14 +1968,15 @@ __global__ void __launch_bounds__(TPB) trace_quads_kernel(const TraceGroup* __re
     v[2 * k + 1] = (double)si[k] + (double)ei[k];
   }
   const double tot = warp_sum8(v, lane);
-  const float tota = warp_sum4(sa, lane);
+  const double va[4] = {(double)sa[0], (double)sa[1], (double)sa[2], (double)sa[3]};
+  const double tota = warp_sum4(va, lane);
   if ((lane & 3) == 0) red[threadIdx.x >> 5][lane >> 2] = tot;
   if ((lane & 7) == 0) reda[threadIdx.x >> 5][lane >> 3] = tota;
   __syncthreads();
   if (threadIdx.x < nt) {
     const int t = threadIdx.x, k = G.ta[t] * 2 + G.tb[t];
     double re = red[0][2 * k], im = red[0][2 * k + 1];
-    float ab = reda[0][k];
+    double ab = reda[0][k];
 #pragma unroll
     for (int w = 1; w < NW; w++) {
       re += red[w][2 * k];
@@ -1988,7 +1987,7 @@ __global__ void __launch_bounds__(TPB) trace_quads_kernel(const TraceGroup* __re
     const TraceRow T = rt[r];
     const double2 c = make_double2((double)T.coef[0], (double)T.coef[1]);
     rows[(size_t)q * nrows + r] = cmul(c, make_double2(re, im));
-    rabs[(size_t)q * nrows + r] = (double)(sqrtf(T.coef[0] * T.coef[0] + T.coef[1] * T.coef[1]) * ab);
+    rabs[(size_t)q * nrows + r] = coef_abs(T.coef[0], T.coef[1]) * ab;
   }
 }
 

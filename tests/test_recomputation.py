@@ -64,3 +64,26 @@ def test_cancelling_twins_are_flagged(cuda, sets_call):
     ref, got = run("fp64"), run("split")
     assert lib().ctr_split_refined() == got.numel()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("power", [-76, 70])
+def test_scaled_coefficients_flag_the_same_entries(cuda, power):
+    """Coefficients whose squares leave FP32's range: the two-sided form recomputes the
+    same entries as for coefficients near 1, with values scaled by the power of two."""
+    nt, n, nout = 2, 16, 40
+    rng = np.random.default_rng(998)
+    prop = _dev(synth.make_prop(nt, n, seed=999), cuda)
+    phi = _dev(np.stack([synth.make_phi_random(nt, n, rng) for _ in range(2)], axis=1), cuda)
+    rows = np.concatenate([rng.integers(0, 4, (160, 4)), rng.integers(0, 2, (160, 2))], axis=1).astype(np.int16)
+    coef = rng.integers(1, 4, (160, 2)).astype(np.float32)
+    oi = np.repeat(np.arange(nout, dtype=np.int32), 4)
+    check(lib().ctr_split_set_refine(4e-13))  # flags some of the entries
+    try:
+        ref = api.twosided(prop, phi, rows, coef, oi, nout, engine="split")
+        flagged = lib().ctr_split_refined()
+        got = api.twosided(prop, phi, rows, np.ldexp(coef, power).astype(np.float32), oi, nout, engine="split")
+        assert 0 < flagged < ref.numel()
+        assert lib().ctr_split_refined() == flagged
+    finally:
+        check(lib().ctr_split_set_refine(1e-9))
+    assert torch.equal(got, ref * 2.0 ** power)
