@@ -1031,13 +1031,17 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   Refine rf_rp, rf_tr;
   if (rhopi) CTR_TRY(refine_begin(c, (size_t)nset * nd * npairs * 4, WS_REFINE, rf_rp));
   if (tri) CTR_TRY(refine_begin(c, (size_t)nset * npairs * 2, WS_SPLITJOBS3, rf_tr));
-  // The sink form takes its place where it costs less, per pair: the terms' block
-  // products instead of 64 a set, and its rows to slice for the Gram product (16
-  // blocks a row; a block's slices and its share of that product take about 0.65 of
-  // a block product) instead of a set's and an operator's.  With every output that
-  // is from 11 sets on, for the triangle alone from 2.  Measured, 27 sets at Nev =
-  // 128, Lt = 48, 8 sink times: block products 158 -> 78 ms, slices, Gram products
-  // and sums of the traces 48 -> 26 ms; the call 254 -> 155 ms.
+  // The sink form takes its place where it costs less.  In block products a pair: the
+  // terms' products, a quarter dearer each (two terms of K, four columns of blocks), instead
+  // of 64 a set, and 10.4 for each row of 16 blocks that a Gram product has, its tiles of
+  // 128 rows and 48 columns counted whole (0.65 of a block product a block's slices and its
+  // share of that product): nH rows a sink time of a batch and a column a set, once a
+  // t_src, against a row a set and a column an operator.  At least 11 sets with every
+  // output, 9 for rho -> pi pi and 2 for the triangle, where the tiles are full.  Measured
+  // (Nev = 128, Lt = 32, ms, with X / sink form): 8 sink times, 11 and 27 sets, every output
+  // 72 / 70 and 137 / 75, triangle 65 / 25 and 130 / 31; 4 sink times, every output 38 / 41
+  // and 74 / 47, triangle of 2 and 3 sets 15.7 / 16.4 and 18.2 / 16.8; one sink time,
+  // triangle of 2, 16 and 27 sets 4.8 / 12.4, 16.1 / 17.0 and 25.1 / 21.1.
   SinkPlan sp;
   bool sink = gram && !fp64_traces_needed;
   if (sink) {
@@ -1060,11 +1064,19 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
     sink = sink_plan(V, sp) && sp.products + 10.4 * sp.H.size() < 64.0 * nC + 10.4 * (nC + nops);
   }
   const int nH = (int)sp.H.size();
+  // sink times a batch: their rows fill two tiles of a t_src's Gram product
+  const int hmax = std::max(1, 256 / std::max(1, nH));
+  if (sink) {
+    auto tiles = [](int n, int size) { return (double)((n + size - 1) / size * size); };
+    const int h = std::min(rows, hmax);
+    const double rows_sink = (tiles(h * nH, 128) + tiles(nC, 48)) / h;
+    const double rows_x = (tiles(4 * nC, 128) + tiles(4 * nops, 48)) / 4;  // four products a pair, of 4 of the 16 blocks
+    sink = 1.25 * sp.products + 10.4 * rows_sink < 64.0 * nC + 10.4 * rows_x;
+  }
   const size_t per_pair_sink = 16 * ((size_t)nops + nH) * N2 * sizeof(double2) +
                                (size_t)nH * nC * (sizeof(double2) + sizeof(double));
   const int batch_sink = std::max(1, std::min(npairs, (int)(budget / per_pair_sink)));
-  // 9 sink times of 14 rows fill a 128-row tile of the Gram product
-  for (const PairBatch& pb : sink ? pair_batches(tau, blk16, Nt, tf_begin, rows, batch_sink, plist, 18)
+  for (const PairBatch& pb : sink ? pair_batches(tau, blk16, Nt, tf_begin, rows, batch_sink, plist, hmax)
                                   : std::vector<PairBatch>()) {
     const int np = (int)pb.ent.size(), ng = (int)pb.by_ti.size();
     void* mem;
