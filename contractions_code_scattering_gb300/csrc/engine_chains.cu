@@ -795,6 +795,36 @@ struct SinkPlan {
   int products = 0;                                         // block products of the terms, per pair
 };
 
+// A term's blocks H_{s1 s2} may cancel in their sum over s3, and their norms, the scales of
+// the Gram product's rows, with them: each row's scale is at least what the sum has
+// without cancellation, (sum_k |Op tau_{s5_k s1}|^2 |tau_{s3_k s2}|^2 / Nev)^(1/2) for H_{s1 s2}
+// against |R_{s1 s2}|.  0.78 takes the two factors' norms of |Re| + |Im| to a product's,
+// so that the two scales agree where nothing cancels.  One CTA a (pair, term).
+__global__ void __launch_bounds__(32) sink_scale_kernel(const SinkTerm* __restrict__ terms, int nH, int nops, int nC,
+                                                        int Nt, double per_nev, const double* __restrict__ nO,
+                                                        const double* __restrict__ nT, const double* __restrict__ nR,
+                                                        const int* __restrict__ ti, double* __restrict__ tra) {
+  __shared__ double est[16];
+  const int i = blockIdx.x / nH;
+  if (threadIdx.x < 16) {
+    const SinkTerm& T = terms[blockIdx.x - i * nH];
+    const int s1 = threadIdx.x / 4, s2 = threadIdx.x & 3;
+    double e = 0.0;
+    for (int k = 0; k < T.n; k++) {
+      const double a = nO[((size_t)i * 16 + T.s5[k] * 4 + s1) * nops + T.slab] * nT[(size_t)i * 16 + T.s3[k] * 4 + s2];
+      e += a * a;
+    }
+    est[threadIdx.x] = 0.78 * sqrt(e * per_nev);
+  }
+  __syncwarp();
+  for (int ci = threadIdx.x; ci < nC; ci += 32) {
+    double a = 0.0;
+    for (int b = 0; b < 16; b++) a += est[b] * nR[((size_t)ci * Nt + ti[i]) * 16 + b];
+    double& t = tra[(size_t)blockIdx.x * nC + ci];
+    t = fmax(t, a);
+  }
+}
+
 // False where a vertex's coefficients are not +-1 times one of them.  Two vertices
 // of one operator that differ in the sign of half their spins (gamma_x and gamma_y)
 // share two terms of two spins each, a and b: one is a + b, the other a - b.
@@ -1076,6 +1106,19 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   const size_t per_pair_sink = 16 * ((size_t)nops + nH) * N2 * sizeof(double2) +
                                (size_t)nH * nC * (sizeof(double2) + sizeof(double));
   const int batch_sink = std::max(1, std::min(npairs, (int)(budget / per_pair_sink)));
+  // norms of R (for the call), of Op tau and of tau (for a batch)
+  const bool scales = sink && (rf_rp.on || rf_tr.on);
+  double *nR = nullptr, *nO = nullptr, *nT = nullptr;
+  if (scales) {
+    void* p;
+    CTR_TRY(workspace(WS_SINKNORM).get(16 * ((size_t)nC * Nt + (size_t)batch_sink * (nops + 1)) * sizeof(double), &p));
+    nR = (double*)p;
+    nO = nR + (size_t)16 * nC * Nt;
+    nT = nO + (size_t)16 * batch_sink * nops;
+    void* d;
+    CTR_TRY(upload(WS_MISC, M.data(), M.size() * sizeof(const double2*), &d, c.s));
+    CTR_TRY(launch_block_norms((const double2* const*)d, nC * Nt, 16, N, nR, c.s));
+  }
   for (const PairBatch& pb : sink ? pair_batches(tau, blk16, Nt, tf_begin, rows, batch_sink, plist, hmax)
                                   : std::vector<PairBatch>()) {
     const int np = (int)pb.ent.size(), ng = (int)pb.by_ti.size();
@@ -1172,6 +1215,23 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
         }
     }
     CTR_TRY(gram_rows(N, gr, trv, tra, c.s));
+    if (scales) {
+      std::vector<const double2*> bases;
+      for (int i = 0; i < np; i++) bases.push_back(Oblk(0, i, 0));
+      bases.insert(bases.end(), pb.T.begin(), pb.T.end());
+      void* d[3];
+      CTR_TRY(upload_group(WS_ROWTASKS,
+                           {{bases.data(), bases.size() * sizeof(const double2*)},
+                            {sp.H.data(), sp.H.size() * sizeof(SinkTerm)},
+                            {pb.ti.data(), pb.ti.size() * sizeof(int)}},
+                           d, c.s));
+      CTR_TRY(launch_block_norms((const double2* const*)d[0], np, 16 * nops, N, nO, c.s));
+      CTR_TRY(launch_block_norms((const double2* const*)d[0] + np, np, 16, N, nT, c.s));
+      TimedLaunch tl(c.s, "sink_scale");
+      sink_scale_kernel<<<np * nH, 32, 0, c.s>>>((const SinkTerm*)d[1], nH, nops, nC, Nt, 1.0 / N, nO, nT, nR,
+                                                 (const int*)d[2], tra);
+      CTR_CUDA(cudaGetLastError());
+    }
     std::vector<RowItems*> items;
     for (RowItems& r : it) items.push_back(&r);
     CTR_TRY(upload_items(c, items));

@@ -91,6 +91,8 @@ int launch_zgemm_f64(const ZTask* d_tasks, int ntask, int N, cudaStream_t s, con
 int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s);
 // The launch alone, not counted or timed.
 int launch_trace_f64_untimed(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s);
+// out[i * per + k] = (sum (|Re x| + |Im x|)^2)^(1/2) over the k-th of `per` consecutive blocks at base[i].
+int launch_block_norms(const double2* const* d_base, int nbase, int per, int N, double* out, cudaStream_t s);
 // loop[t] = sum_s Tr[tau(t,t)_ss Phi(t)] for diag [Nt][4][4][N][N], mom [Nt][N][N].
 int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s);
 int launch_rowsum_coef(const double2* tr, int ntr, const int* off, const int* idx, const int* tix, const float* coef,

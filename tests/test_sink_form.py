@@ -93,3 +93,23 @@ def test_sink_form_replayed(cuda, tol):
         g.close()
     finally:
         check(lib().ctr_split_set_refine(1e-9))
+
+
+@pytest.mark.parametrize("rhopi", [False, True])
+def test_cancelling_sink_terms_are_flagged(cuda, rhopi):
+    """tau_{2 s} = tau_{0 s} and tau_{3 s} = tau_{1 s} up to 1e-8: the triangle's sum over the
+    closing spin, which the sink form takes inside its products, cancels to 1e-8 of its
+    terms, so every entry has to be recomputed."""
+    nt, n = 8, 10
+    prop, phi, mom5, mom2 = _inputs(cuda, nt, n, 1400)
+    rng = np.random.default_rng(1401)
+    for a, b in ((2, 0), (3, 1)):
+        prop[:, :, a] = prop[:, :, b] * (1.0 + 1e-8 * rng.normal(size=prop[:, :, b].shape))
+    tp = _dev(prop, cuda)
+    diag = api.prop_diag(_dev(synth.make_prop(nt, n, seed=1402), cuda))
+    run = lambda engine: api.run_contract_rhopi_sigmapi_sets(tp, diag, phi, SETS[:11], mom5, mom2, engine=engine,
+                                                             rhopi=rhopi, triangle=True, hor_fish=False)
+    ref = run("fp64")
+    got, launches = _sink_launches(lambda: run("split"))
+    assert launches > 0 and lib().ctr_split_refined() >= ref["triangle"].numel()
+    assert torch.equal(got["triangle"], ref["triangle"])
