@@ -98,14 +98,9 @@ int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, do
 int launch_rowsum_coef(const double2* tr, int ntr, const int* off, const int* idx, const int* tix, const float* coef,
                        int nout, int npair, double2* out, cudaStream_t s);
 int launch_source_average(int Nt, int ncorr, const double2* corr, double scale, double2* avg, cudaStream_t s);
-// Row sums as launch_rowsum (out stride nout) plus per-entry refinement flags:
-// entries with eps_over_tol * sum(rabs) > |out| append (pair_base + p) * nout + o to list.
-int launch_rowsum_refine(const double2* rows, const double* rabs, int nrows, const int* off, const int* idx, int nout,
-                         int npair, double2* out, double eps_over_tol, int* count, int* list, int pair_base,
-                         cudaStream_t s);
-// Row sums over shared traces: out[p][o] = sum over rows r of output o (CSR off/idx) of
-// coef[r] * tr[p][tix[r]]; the error scale sum |coef[r]| trabs[p][tix[r]] flags entries
-// as launch_rowsum_refine does.
+// The same with per-entry refinement flags: entry p * nout + o of trace values and error
+// scales tr, trabs [npair][ntr] is listed in list (+ pair_base * nout) and counted where
+// eps_over_tol times its scale sum |coef| trabs exceeds its magnitude.
 int launch_rowsum_coef_refine(const double2* tr, const double* trabs, int ntr, const int* off, const int* idx,
                               const int* tix, const float* coef, int nout, int npair, double2* out,
                               double eps_over_tol, int* count, int* list, int pair_base, cudaStream_t s);

@@ -477,30 +477,6 @@ __global__ void rowsum_coef_kernel(const double2* __restrict__ tr, int ntr, cons
   out[g] = make_double2(re, im);
 }
 
-__global__ void rowsum_refine_kernel(const double2* __restrict__ rows, const double* __restrict__ rabs, int nrows,
-                                     const int* __restrict__ off, const int* __restrict__ idx, int nout, int npair,
-                                     double2* __restrict__ out, double eps_over_tol, int* __restrict__ count,
-                                     int* __restrict__ list, int pair_base) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= npair * nout) return;
-  const int p = g / nout, o = g % nout;
-  double re = 0.0, im = 0.0, sc = 0.0;
-  for (int k = off[o]; k < off[o + 1]; k++) {
-    const size_t r = (size_t)p * nrows + idx[k];
-    re += rows[r].x;
-    im += rows[r].y;
-    sc += rabs[r];
-  }
-  out[(size_t)p * nout + o] = make_double2(re, im);
-  // flagged: an error estimate above the tolerance (or not a number), or an
-  // error scale that underflowed while the value did not
-  const double mag = sqrt(re * re + im * im);
-  if (eps_over_tol > 0.0 && (!(sc * eps_over_tol <= mag) || (sc == 0.0 && mag > 0.0))) {
-    const int slot = atomicAdd(count, 1);
-    list[slot] = (pair_base + p) * nout + o;
-  }
-}
-
 // Smallest trusted error scale sum |coef| sum |A||B| of a float-float entry.
 constexpr double FF_MIN_SCALE = 0x1p-90;
 
@@ -703,18 +679,6 @@ int launch_source_average(int Nt, int ncorr, const double2* corr, double scale, 
   if (n == 0) return CTR_OK;
   TimedLaunch tl(s, "source_average");
   source_average_kernel<<<(n + 255) / 256, 256, 0, s>>>(Nt, ncorr, corr, scale, avg);
-  CTR_CUDA(cudaGetLastError());
-  return CTR_OK;
-}
-
-int launch_rowsum_refine(const double2* rows, const double* rabs, int nrows, const int* off, const int* idx, int nout,
-                         int npair, double2* out, double eps_over_tol, int* count, int* list, int pair_base,
-                         cudaStream_t s) {
-  const int n = npair * nout;
-  if (n == 0) return CTR_OK;
-  TimedLaunch tl(s, "rowsum_refine");
-  rowsum_refine_kernel<<<(n + 255) / 256, 256, 0, s>>>(rows, rabs, nrows, off, idx, nout, npair, out, eps_over_tol,
-                                                        count, list, pair_base);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
 }

@@ -870,14 +870,9 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
 #pragma unroll
     for (int s = 0; s < C::NS; s++) {
       const uint32_t re = slice_pair(Ur[0], nr[0], Ur[1], nr[1], s), im = slice_pair(Ui[0], ni[0], Ui[1], ni[1], s);
-      if (C::PACK) {
-        *(uint32_t*)(d + (s * 3 + 0) * C::B_SUB) = im ^ BF16X2_SIGNS;
-        *(uint32_t*)(d + (s * 3 + 1) * C::B_SUB) = re;
-        *(uint32_t*)(d + (s * 3 + 2) * C::B_SUB) = im;
-      } else {
-        *(uint32_t*)(d + (s * 2 + 0) * C::B_SUB) = re;
-        *(uint32_t*)(d + (s * 2 + 1) * C::B_SUB) = im;
-      }
+      *(uint32_t*)(d + (s * 3 + 0) * C::B_SUB) = im ^ BF16X2_SIGNS;
+      *(uint32_t*)(d + (s * 3 + 1) * C::B_SUB) = re;
+      *(uint32_t*)(d + (s * 3 + 2) * C::B_SUB) = im;
     }
   }
 }
@@ -999,7 +994,7 @@ __device__ __forceinline__ void issue_row(uint32_t tbase, uint64_t a, uint64_t b
     const uint64_t b = desc_at(bdesc, ((j * 3 + (P ? 0 : 1)) * C::B_SUB) >> 4);
     // the first MMA of level l in a tile is Xr of pair (0, l)
     const uint32_t accum = (!first_chunk || !(I == 0 && P == 0 && j <= C::NL - 1)) ? 1u : 0u;
-    umma_f16<op>(tbase + (uint32_t)C::acc_col(0, lvl), a, b, idesc_bf16_f32(SPLIT_M, 2 * C::BN, false), accum);
+    umma_f16<op>(tbase + (uint32_t)C::acc_col(0, lvl), a, b, idesc_bf16_f32(SPLIT_M, 2 * C::BN), accum);
     issue_row<C, G, I, P, j + 1, true>(tbase, a, bdesc, first_chunk);
   }
 }
@@ -1012,7 +1007,6 @@ __device__ __forceinline__ void issue_row(uint32_t tbase, uint64_t a, uint64_t b
 // sums the pairs (I + q, J - q).
 template <class C, int G, int STEP = 1, int I = 0>
 __device__ __forceinline__ void issue_pairs(uint32_t tbase, uint64_t adesc, uint64_t bdesc, bool first_chunk) {
-  static_assert(C::PACK, "packed complex operands");
   if constexpr (I < C::NS) {
     constexpr int a = I / STEP * 2 * C::A_SUB;
     issue_row<C, G, I, 0, 0, false>(tbase, desc_at(adesc, a >> 4), bdesc, first_chunk);

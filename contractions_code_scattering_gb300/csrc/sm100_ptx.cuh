@@ -216,11 +216,10 @@ __device__ __forceinline__ uint64_t sdesc_kmajor_noswz(uint32_t saddr, uint32_t 
 }
 
 // Instruction descriptor of kind::f16 with bf16 A/B, f32 D, both K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool negA) {
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4)                        // D format f32
          | (1u << 7)                      // A format bf16
          | (1u << 10)                     // B format bf16
-         | ((negA ? 1u : 0u) << 13)       // negate A
          | ((uint32_t)(N >> 3) << 17)     // N / 8
          | ((uint32_t)(M >> 4) << 24);    // M / 16
 }

@@ -32,30 +32,29 @@ constexpr int SPLIT_MAXBLK = 32;
 //    N = 48 (10 x 48 = 480 TMEM columns); the epilogue sums the levels exactly
 //    in 64-bit integers, so products keep ~2^-53 of their row/column scales.
 //
-// Packed complex MMAs (PACK): the right operand keeps three planes per slice,
+// Packed complex MMAs: the right operand keeps three planes per slice,
 // -Yi, Yr, Yi, adjacent along N, so that the complex product takes two MMAs of
 // width 2 BN per slice pair, Xr [Yr | Yi] and Xi [-Yi | Yr], into one [Re | Im]
 // accumulator per level (instead of four MMAs of width BN); the left operand
 // tile is then read from shared memory half as often per flop.
-template <int NS_, int NL_, int BN_, bool PACK_, bool INT_OUT_, bool LONG_ = false>
+template <int NS_, int NL_, int BN_, bool INT_OUT_, bool LONG_ = false>
 struct SplitCfg {
   static constexpr int NS = NS_, NL = NL_, BN = BN_;
   static constexpr bool LONG = LONG_;  // K above 128: levels 0 and 1 drained piece by piece
-  static constexpr bool PACK = PACK_;
   static constexpr bool INT_OUT = INT_OUT_;  // epilogue: complex128 via exact integer sums (else float-float)
   static constexpr int EPI_WARPS = 16;             // 4 per TMEM lane quadrant, splitting the columns
   static constexpr int EPI_CW = 4;                 // columns per TMEM load in the epilogue
-  static constexpr int B_PLANES = PACK ? 3 : 2;
+  static constexpr int B_PLANES = 3;
   static constexpr int A_SUB = SPLIT_M * SPLIT_K * 2;
   static constexpr int B_SUB = BN * SPLIT_K * 2;
   static constexpr int A_STAGE = NS * 2 * A_SUB;
   static constexpr int B_STAGE = NS * B_PLANES * B_SUB;
   // TMEM column of accumulator (part 0 = Re / 1 = Im, level l)
-  __host__ __device__ static constexpr int acc_col(int part, int l) { return PACK ? (l * 2 + part) * BN : (part * NL + l) * BN; }
+  __host__ __device__ static constexpr int acc_col(int part, int l) { return (l * 2 + part) * BN; }
 };
-using CfgStd = SplitCfg<SPLIT_NSLICE, 4, SPLIT_N, true, false>;
-using CfgHP = SplitCfg<6, 5, 48, true, true>;
-using CfgHPLong = SplitCfg<6, 5, 48, true, true, true>;  // CfgHP's operands, any number of chunks
+using CfgStd = SplitCfg<SPLIT_NSLICE, 4, SPLIT_N, false>;
+using CfgHP = SplitCfg<6, 5, 48, true>;
+using CfgHPLong = SplitCfg<6, 5, 48, true, true>;  // CfgHP's operands, any number of chunks
 static_assert(CfgStd::B_STAGE == SPLIT_B_STAGE && CfgStd::A_STAGE == SPLIT_A_STAGE, "standard stage sizes");
 static_assert(CfgStd::BN % (CfgStd::EPI_CW * (CfgStd::EPI_WARPS / 4)) == 0 &&
                   CfgHP::BN % (CfgHP::EPI_CW * (CfgHP::EPI_WARPS / 4)) == 0,
