@@ -203,14 +203,15 @@ int prepare_for_capture();
 // ---------------------------------------------------------------- autotuner
 // Knob choices keyed by "knob|shape" (tune.cpp).  tune_mode() is 0 while the
 // thread records a graph.  tune_resolve returns the forced value, the cached
-// choice, a fresh measurement of run(c) for c < ncand (mode >= 1), or dflt.
+// choice, a fresh measurement of run(c) for c < ncand (mode >= 1; for c < nmeasure where
+// that is given, the others being kernels among them), or dflt.
 int tune_mode();
 std::string tune_key(const char* knob, const std::string& shape);
 int tune_forced(const char* knob);
 bool tune_lookup(const std::string& key, int* choice);
 void tune_store(const std::string& key, int choice, const std::vector<double>& ms);
 int tune_resolve(const char* knob, const std::string& shape, int ncand, int dflt, cudaStream_t s,
-                 const std::function<int(int)>& run, int* choice);
+                 const std::function<int(int)>& run, int* choice, int nmeasure = 0);
 // The choice tune_resolve will return when it will not measure (forced, cached or
 // mode 0): true and *choice set; false when it would measure the candidates.
 bool tune_peek(const char* knob, const std::string& shape, int ncand, int dflt, int* choice);

@@ -452,7 +452,8 @@ int twosided_split(int N, int Nt, int tf_begin, int tf_end, const double* prop_r
                                (const float4* const*)d_tt + np, ldA, ldB, np, N, R, Rabs, variant, stream);
     };
     int variant = 0;
-    CTR_TRY(tune_resolve("trace_rows", shape, TRACE_VARIANTS + 3, TRACE_VARIANTS + 1, stream, traces, &variant));
+    CTR_TRY(tune_resolve("trace_rows", shape, TRACE_VARIANTS + 3, TRACE_VARIANTS + 1, stream, traces, &variant,
+                         N <= TRACE_WARP_NEV ? TRACE_VARIANTS + 2 : 0));
     CTR_TRY(traces(variant));
     return launch_rowsum_coef_refine(R, Rabs, ntr, (const int*)d_csr, (const int*)d_csr + (nout + 1),
                                      (const int*)d_tix, (const float*)d_rcoef, nout, np,

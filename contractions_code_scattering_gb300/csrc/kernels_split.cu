@@ -2579,14 +2579,6 @@ int launch_trace_groups(const TraceGroup* d_groups, int ngroups, int maxcols, co
   return CTR_OK;
 }
 
-// Up to this Nev a group gets one warp: its Nev^2 elements are too few to pay
-// for a cross-warp reduction, and with 32 CTAs an SM the loads in flight still
-// cover the latency.  Measured (rho, 256 pairs, trace_quads in us; one warp /
-// 128 threads / 64 threads before the reduce-scatter): Nev = 16: 272 / 1175 /
-// 731, 32: 548 / 1417 / 1047, 64: 1887 / 2288 / 2173.  The gain over 128 threads
-// is down to the shorter reduction by Nev = 64, so larger blocks keep them.
-constexpr int TRACE_WARP_NEV = 64;
-
 int launch_trace_quads(const TraceGroup* d_groups, int ngroups, const TraceRow* d_rows, int nrows,
                        const float4* const* d_abase, const float4* const* d_bbase, int lda, int ldb, int npair,
                        int nev, double2* rows, double* rabs, int variant, cudaStream_t s) {

@@ -77,7 +77,7 @@ bool tune_peek(const char* knob, const std::string& shape, int ncand, int dflt, 
 }
 
 int tune_resolve(const char* knob, const std::string& shape, int ncand, int dflt, cudaStream_t s,
-                 const std::function<int(int)>& run, int* choice) {
+                 const std::function<int(int)>& run, int* choice, int nmeasure) {
   const int forced = tune_forced(knob);
   if (forced >= 0) {
     if (forced >= ncand) return fail(CTR_ERR_ARG, "tuning knob %s forced to %d, which is not below %d", knob, forced, ncand);
@@ -90,6 +90,7 @@ int tune_resolve(const char* knob, const std::string& shape, int ncand, int dflt
     *choice = dflt;
     return CTR_OK;
   }
+  if (nmeasure > 0) ncand = nmeasure;
   cudaEvent_t e0, e1;
   CTR_CUDA(cudaEventCreate(&e0));
   CTR_CUDA(cudaEventCreate(&e1));
