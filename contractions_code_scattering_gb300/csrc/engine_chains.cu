@@ -809,12 +809,13 @@ __global__ void __launch_bounds__(32) sink_scale_kernel(const SinkTerm* __restri
   if (threadIdx.x < 16) {
     const SinkTerm& T = terms[blockIdx.x - i * nH];
     const int s1 = threadIdx.x / 4, s2 = threadIdx.x & 3;
-    double e = 0.0;
+    double a[4], m = 0.0, e = 0.0;
     for (int k = 0; k < T.n; k++) {
-      const double a = nO[((size_t)i * 16 + T.s5[k] * 4 + s1) * nops + T.slab] * nT[(size_t)i * 16 + T.s3[k] * 4 + s2];
-      e += a * a;
+      a[k] = nO[((size_t)i * 16 + T.s5[k] * 4 + s1) * nops + T.slab] * nT[(size_t)i * 16 + T.s3[k] * 4 + s2];
+      m = fmax(m, a[k]);
     }
-    est[threadIdx.x] = 0.78 * sqrt(e * per_nev);
+    for (int k = 0; k < T.n && m > 0.0; k++) e += (a[k] / m) * (a[k] / m);
+    est[threadIdx.x] = 0.78 * m * sqrt(e * per_nev);
   }
   __syncwarp();
   for (int ci = threadIdx.x; ci < nC; ci += 32) {

@@ -361,21 +361,6 @@ __global__ void __launch_bounds__(TPB) trace_f64_kernel(const TraceTask* __restr
   }
 }
 
-// Norms of blocks, in FP32 and over the range of the traces' error scales.  One CTA a block.
-__global__ void __launch_bounds__(256) block_norms_kernel(const double2* const* __restrict__ base, int per, int n2,
-                                                          double* __restrict__ out) {
-  const int i = blockIdx.x / per;
-  const double2* x = base[i] + (size_t)(blockIdx.x - i * per) * n2;
-  float s = 0.f;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < n2; e += 256) {
-    const float a = abs1_scaled_f32(x[e]);
-    s = fmaf(a, a, s);
-  }
-  const double t = block_sum_256((double)s);
-  if (threadIdx.x == 0) out[blockIdx.x] = sqrt(t) * 0x1p-40;  // 2^-TRACE_ABS_SHIFT
-}
-
 // ---------------------------------------------------------- unit-spin loop
 // loop[t] = sum_s Tr[tau(t,t)_ss Phi(t)] = Tr[(sum_s tau(t,t)_ss) Phi(t)].  The
 // FP64 pipe is the bound: summing the four spin blocks first takes 6 adds + 4
@@ -623,14 +608,6 @@ int launch_trace_f64(const TraceTask* d_tasks, int ntask, int N, cudaStream_t s)
   if (ntask == 0) return CTR_OK;
   TimedLaunch tl(s, "trace_f64");
   return launch_trace_f64_untimed(d_tasks, ntask, N, s);
-}
-
-int launch_block_norms(const double2* const* d_base, int nbase, int per, int N, double* out, cudaStream_t s) {
-  if (nbase == 0) return CTR_OK;
-  TimedLaunch tl(s, "block_norms");
-  block_norms_kernel<<<nbase * per, 256, 0, s>>>(d_base, per, N * N, out);
-  CTR_CUDA(cudaGetLastError());
-  return CTR_OK;
 }
 
 int launch_loop_unity(const double2* diag, const double2* mom, int N, int Nt, double2* loop, cudaStream_t s) {

@@ -2138,6 +2138,45 @@ __global__ void __launch_bounds__(128) gram_trace_sum_kernel(const GramTrace* __
   if (tra) tra[T.slot] = sqrt(c.x * c.x + c.y * c.y) * ab;
 }
 
+// Norms (sum (|Re x| + |Im x|)^2)^(1/2) of blocks over the whole range of doubles: a thread
+// sums squares in FP32 relative to 2^E, E the largest exponent it has met but for 2^30.
+// One CTA a block, read once.
+__global__ void __launch_bounds__(256) block_norms_kernel(const double2* const* __restrict__ base, int per, int n2,
+                                                          double* __restrict__ out) {
+  __shared__ int sE[8];
+  __shared__ float ss[8];
+  const int i = blockIdx.x / per;
+  const double2* x = base[i] + (size_t)(blockIdx.x - i * per) * n2;
+  int E = -30000;
+  float s = 0.f;
+  // s 2^(2 k) for k <= 0; 2^-126 stands for less
+  auto down = [](float v, int k) { return v * __int_as_float((127 + max(2 * k, -126)) << 23); };
+  auto rel = [&](double v) { return ((__double2hiint(v) >> 20) & 0x7FF) == 0 ? 0.f : abs_rel_f32(v, E); };
+#pragma unroll 4
+  for (int e = threadIdx.x; e < n2; e += 256) {
+    const double2 v = x[e];
+    const int b = max(f64_exp_bound(v.x), f64_exp_bound(v.y));
+    if (b > E + 30) {
+      s = down(s, max(E - b, -1000));
+      E = b;
+    }
+    const float a = rel(v.x) + rel(v.y);
+    s = fmaf(a, a, s);
+  }
+  auto add = [&](int E2, float s2) {
+    const int m = max(E, E2);
+    s = down(s, max(E - m, -1000)) + down(s2, max(E2 - m, -1000));
+    E = m;
+  };
+  for (int o = 16; o; o >>= 1) add(__shfl_xor_sync(0xffffffffu, E, o), __shfl_xor_sync(0xffffffffu, s, o));
+  if ((threadIdx.x & 31) == 0) sE[threadIdx.x >> 5] = E, ss[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) add(sE[w], ss[w]);
+    out[blockIdx.x] = s > 0.f ? (double)sqrtf(s) * pow2d(E) : (s == 0.f ? 0.0 : (double)s);
+  }
+}
+
 // Values of Gram products whose every entry is wanted: group g's blocks b < nblk
 // (instances (g * nblk + b) * npiece + p) add up, with the sign of bit b of
 // `negative`, into trv[rowbase[g * mrows + r] + c] for c < ncols; rows whose base is
@@ -2347,6 +2386,14 @@ int launch_slice_gram(bool right, const double2* const* d_blk, int ngroup, int n
     slice_gram_kernel<CfgHP, false><<<(unsigned)(grid * (SPLIT_M / 8)), 256, GRAM_SLICE_SMEM, s>>>(
         d_blk, nrows, ntile, n2, npiece, nchunk, out, exps, norms);
   }
+  CTR_CUDA(cudaGetLastError());
+  return CTR_OK;
+}
+
+int launch_block_norms(const double2* const* d_base, int nbase, int per, int N, double* out, cudaStream_t s) {
+  if (nbase == 0) return CTR_OK;
+  TimedLaunch tl(s, "block_norms");
+  block_norms_kernel<<<nbase * per, 256, 0, s>>>(d_base, per, N * N, out);
   CTR_CUDA(cudaGetLastError());
   return CTR_OK;
 }

@@ -113,3 +113,23 @@ def test_cancelling_sink_terms_are_flagged(cuda, rhopi):
     got, launches = _sink_launches(lambda: run("split"))
     assert launches > 0 and lib().ctr_split_refined() >= ref["triangle"].numel()
     assert torch.equal(got["triangle"], ref["triangle"])
+
+
+@pytest.mark.parametrize("power", [-200, 70, 200])
+def test_sink_scales_follow_the_data(cuda, power):
+    """tau times a power of two: the same entries are recomputed, and the values are those
+    of the unscaled call times its square."""
+    nt, n = 8, 9
+    prop, phi, mom5, mom2 = _inputs(cuda, nt, n, 1500)
+    diag = api.prop_diag(_dev(prop, cuda))
+    run = lambda tau: api.run_contract_rhopi_sigmapi_sets(_dev(tau, cuda), diag, phi, SETS[:11], mom5, mom2,
+                                                          engine="split", hor_fish=False)
+    check(lib().ctr_split_set_refine(1e-13))
+    try:
+        (ref, launches), flagged = _sink_launches(lambda: run(prop)), lib().ctr_split_refined()
+        got = run(prop * 2.0 ** power)
+        assert launches > 0 and 0 < flagged < ref["rhopi"].numel() and lib().ctr_split_refined() == flagged
+    finally:
+        check(lib().ctr_split_set_refine(1e-9))
+    for k in ref:
+        assert torch.equal(got[k], ref[k] * 2.0 ** (2 * power)), k
