@@ -969,6 +969,14 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
   std::vector<const double2*> M;
   // tau(t, t) of the full perambulator
   CTR_TRY(per_t_products(c, prop, (size_t)(Nt + 1) * blk16, el, WS_RPHI, cb.list, cb.need, 16 * (4 * (size_t)Nt + 4), M));
+  // The co-factors K and J carry the weights through block products, whose operands flush
+  // to zero below 2^-1000: they take the weights relative to a power of two.
+  double wmax = 0.0;
+  for (int p : pairs)
+    for (int k = 0; k < 2; k++)
+      wmax = std::max({wmax, std::fabs(w[(size_t)p * 5 + k].x), std::fabs(w[(size_t)p * 5 + k].y)});
+  const int wexp = wmax > 0.0 && std::isfinite(wmax) ? std::max(-1000, std::min(1000, std::ilogb(wmax))) : 0;
+  const double wdown = std::ldexp(1.0, -wexp), wup = std::ldexp(1.0, wexp);
   // co-factors per time slice: K [tf][16], Jsq, Jdt [ti][16] (block (row, column) of the co-factor)
   double2 *Ks = nullptr, *Js = nullptr, *Jd = nullptr;
   if (g) {
@@ -1134,7 +1142,8 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
       }
       if (!g) continue;
       // Rw = w_sq Rsq + w_dt Rdt, S = T G Rw, K = S T^dag (the leading G is a sign of its row)
-      const double2 a = make_double2(wp[0].x * wsq, wp[0].y * wsq), b = make_double2(wp[1].x * wdt, wp[1].y * wdt);
+      const double2 a = make_double2(wp[0].x * wdown * wsq, wp[0].y * wdown * wsq),
+                    b = make_double2(wp[1].x * wdown * wdt, wp[1].y * wdown * wdt);
       for (int k = 0; k < 16; k++) {
         comb.begin(bR[i] + (size_t)k * N2, false);
         comb.term(M[(size_t)cSq * Nt + ti] + (size_t)k * N2, a);
@@ -1263,7 +1272,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
           for (int i : mi) {
             const double2 wv = w[(size_t)pairs[pb.ent[i]] * 5 + k];
             const double sc = k ? wdt : wsq;
-            sum.term(rc(bJ[i], b / 4, b % 4), make_double2(wv.x * sc, wv.y * sc));
+            sum.term(rc(bJ[i], b / 4, b % 4), make_double2(wv.x * wdown * sc, wv.y * wdown * sc));
           }
         }
     CTR_TRY(sum.run((int)N2, c.s));
@@ -1320,7 +1329,7 @@ int pipi_vjp(const Ctx& c, int iso, const double2* prop, const std::vector<Elem>
         g0.push_back(std::move(C));
         g0.push_back(std::move(E));
       }
-      pl.begin(make_double2(1.0, 0.0));
+      pl.begin(make_double2(1.0, 0.0), nullptr, wup);
       for (int b = 0; b < 16; b++) {
         const int bt = (b % 4) * 4 + b / 4;  // tau_ab against F_ba
         const int u = G5[S.row_sign ? b % 4 : b / 4] < 0 ? 2 : 0;

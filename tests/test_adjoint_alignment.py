@@ -1,4 +1,4 @@
-"""Profile gradients with caller arrays that are aligned to doubles only."""
+"""Profile gradients: caller arrays that are aligned to doubles only, and the range of the weights."""
 import ctypes
 
 import numpy as np
@@ -51,3 +51,19 @@ def test_arrays_aligned_to_doubles(cuda, engine):
         torch.cuda.synchronize()
         assert out[0] == 0 and torch.equal(out[1:], torch.view_as_real(ref).reshape(-1))
         assert torch.equal(g, grad)
+
+
+@pytest.mark.parametrize("engine", ["fp64", "split"])
+@pytest.mark.parametrize("power", [-1005, 900])
+def test_pipi_gradient_weight_range(cuda, engine, power):
+    """Weights near the ends of the doubles' range scale the pi pi gradient, to rounding."""
+    nt, n = 3, 8
+    rng = np.random.default_rng(65)
+    prop = torch.from_numpy(synth.make_prop(nt, n, seed=66)).to(cuda)
+    ps = [torch.from_numpy(synth.make_phi_random(nt, n, rng)).to(cuda) for _ in range(4)]
+    f = torch.from_numpy(rng.uniform(0.5, 1.5, n)).to(cuda)
+    w = torch.zeros((nt, nt, 5), dtype=torch.complex128, device=cuda)
+    w[..., :2] = torch.from_numpy(rng.normal(size=(nt, nt, 2)) + 1j * rng.normal(size=(nt, nt, 2))).to(cuda)
+    _, ref = api.pipi_profile_vjp(prop, *ps, f, w, 0, engine=engine)
+    _, got = api.pipi_profile_vjp(prop, *ps, f, w * 2.0 ** power, 0, engine=engine)
+    assert (got * 2.0 ** -power - ref).abs().max() <= 1e-13 * ref.abs().max()
