@@ -1414,7 +1414,7 @@ int ctr_rho_profile_vjp(int engine, int nev, int nt, const double* prop, const d
   CTR_TRY(profiled(nev, (long long)nt * 5, mom5, f, WS_PHI, &phis, s));
   CorrOut out(corr, (size_t)nt * nt * 48);
   CTR_TRY(out.open());
-  CTR_TRY(rho_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, (const double2*)prop, phis, f, (const double2*)hw.data(),
+  CTR_TRY(rho_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine, true}, (const double2*)prop, phis, f, (const double2*)hw.data(),
                   out.p, grad));
   return out.close(s);
 }
@@ -1452,7 +1452,7 @@ int ctr_pipi_profile_vjp(int engine, int nev, int nt, int isospin, const double*
   }
   CorrOut out(corr, (size_t)nt * nt * 5);
   CTR_TRY(out.open());
-  CTR_TRY(pipi_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine}, isospin, (const double2*)prop, el, set, f,
+  CTR_TRY(pipi_vjp(Ctx{nev, nt, (size_t)nev * nev, s, engine, true}, isospin, (const double2*)prop, el, set, f,
                    (const double2*)hw.data(), out.p, grad));
   return out.close(s);
 }

@@ -17,6 +17,7 @@ struct Ctx {
   size_t N2;
   cudaStream_t s;
   int engine = CTR_ENGINE_FP64;
+  bool full = false;  // split engine: grids of more than 128 k at full scale
 };
 
 // Elemental of a call: Phi(t) = p + t * stride (an [Nt][N][N] array, or one momentum

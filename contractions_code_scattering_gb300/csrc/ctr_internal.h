@@ -146,7 +146,8 @@ struct GridTask {
   float w[4];
   int nslab, nb, nterm, adag, bdag;
 };
-int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t stream);
+// full: products of more than 128 k with operands at full scale (SplitGemmBatch::full).
+int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t stream, bool full);
 
 // Closing traces Tr-Had(X, Y) = sum_e X_e conj(Y_e) of many left and right
 // blocks that meet in groups, as Gram products on the split engine: group g has

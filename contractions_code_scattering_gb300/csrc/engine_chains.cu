@@ -52,7 +52,7 @@ int run_traces(const Ctx& c, const std::vector<TraceTask>& t) {
 // FP64 engine runs them as plain tasks.
 int run_grids(const Ctx& c, const std::vector<GridTask>& g, int slot) {
   if (g.empty()) return CTR_OK;
-  if (c.engine == CTR_ENGINE_SPLIT) return zgemm_split_grids(c.N, g, c.s);
+  if (c.engine == CTR_ENGINE_SPLIT) return zgemm_split_grids(c.N, g, c.s, c.full);
   std::vector<ZTask> t;
   for (const GridTask& G : g)
     for (int sl = 0; sl < G.nslab; sl++)

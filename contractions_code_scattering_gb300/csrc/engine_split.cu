@@ -896,6 +896,7 @@ int zgemm_split_tasks(int N, const ZTask* tasks, int ntask, cudaStream_t stream)
                                       (const int*)d_bexp, stream));
       SplitGemmBatch G{(const SplitGemmInst*)d_gi, 1, ntiles, nchunk, N, nb * N, SPLIT_M, nullptr, 1, N, 1};
       G.step = split_tail_step(K);
+      G.full = 1;
       CTR_TRY(launch_split_gemm(G, ni, d_err, stream));
       if (!capturing()) g_split_products += (double)ni * nb * nterm;
     }
@@ -915,7 +916,7 @@ namespace ctr {
 // once per distinct right side of a launch.  Pieces of equal shape (terms,
 // right blocks, slabs) form one persistent launch; the epilogue writes slab s of
 // right block j at C0[j] + s Nev^2, i.e. row s Nev + r of the piece.
-int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t stream) {
+int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t stream, bool full) {
   if (grids.empty()) return CTR_OK;
   if (N > SPLIT_MAXK) return fail(CTR_ERR_UNSUPPORTED, "split engine supports Nev <= %d (got %d)", SPLIT_MAXK, N);
   int* d_err;
@@ -945,6 +946,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
     const int nterm = std::get<0>(bk.first), nb = std::get<1>(bk.first), ns = std::get<2>(bk.first);
     const int K = nterm * N, nchunk = cdiv(K, SPLIT_K), ntiles = cdiv(nb * N, CfgHP::BN),
               mtiles = cdiv(ns * N, SPLIT_M);
+    const int eplus = K > 128 && !full ? 1 : 0;
     const size_t l_b = align256((size_t)mtiles * nchunk * CfgHP::A_STAGE), le_b = align256((size_t)mtiles * SPLIT_M * 4);
     const size_t r_b = align256((size_t)ntiles * nchunk * CfgHP::B_STAGE), re_b = align256((size_t)ntiles * CfgHP::BN * 4);
     const size_t per = l_b + le_b + r_b + re_b;  // one left and at most one distinct right per piece
@@ -1000,6 +1002,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
           L.nslab = pc.ns;
           L.nterm = nterm;
           L.dag = G.adag;
+          L.eplus = eplus;
           L.out = lbase + lj.size() * (l_b + le_b);
           L.exps = (int*)(L.out + l_b);
           lt = lid.emplace(key, (int)lj.size()).first;
@@ -1017,6 +1020,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
           R.nb = nb;
           R.nterm = nterm;
           R.dag = G.bdag;
+          R.eplus = eplus;
           for (int j = 0; j < nb; j++)
             for (int q = 0; q < nterm; q++) {
               R.b[j][q] = G.B[j][q];
@@ -1042,6 +1046,7 @@ int zgemm_split_grids(int N, const std::vector<GridTask>& grids, cudaStream_t st
       SplitGemmBatch B{(const SplitGemmInst*)d_gi, mtiles, ntiles, nchunk, ns * N, nb * N, mtiles * SPLIT_M,
                        nullptr, 1, N, 1};
       B.step = split_tail_step(K);
+      B.full = full;
       // persistent tile walk (N tiles or M tiles innermost), autotuned per tile shape
       // by re-launching the GEMM on the same operands (it rewrites the same outputs)
       char gshape[96];

@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(256) slice_stack_left_kernel(const SliceStackL
         if (b > -30000) e = max(e, b + J.wexp[q]);
       }
     }
-    const int E = e < -1000 ? 0 : e;
+    const int E = (e < -1000 ? 0 : e) + J.eplus;
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[g] = E;
   }
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(128) slice_task_right_kernel(const SliceTaskRJ
         e = max(e, bexp[((size_t)J.bi[jb][q] * 2 + (dag ? 0 : 1)) * nev + c]);
       }
     }
-    const int E = e < -1000 ? 0 : e;
+    const int E = (e < -1000 ? 0 : e) + J.eplus;
     sexp[threadIdx.x] = E;
     if (kc == 0) J.exps[n] = E;  // exps sized ntiles * BN (padding columns get 0)
   }
@@ -1115,14 +1115,17 @@ __global__ void __launch_bounds__(gemm_threads<C>(), 1)
   // Nev = 57 741 -> 704 us, Nev = 100 9.25 -> 8.98 ms); shorter tiles are bound by their
   // epilogue, which the second wait only lengthens (Nev = 32 223 -> 242 us).
   const bool early = g.nchunk >= 4;
-  // The pieces of a tile of more than 128 k, 4 to 8 chunks each, at whose ends levels 0 and 1
-  // and the last level are drained into the epilogue's 64-bit sums.  Level 0 then stays
-  // below 2^24 units, where FP32 sums are exact, for any data and with operands at full
-  // scale: halved instead (the digits of both then reach 512 k), products of four terms
-  // lost two bits.  The last level, truncated by the tensor core at each MMA, gets an error
-  // that grows with the chunks summed.  Error of a four-term product of Gaussian blocks,
-  // largest entries 1: 4.8e-15 -> 8e-16 at Nev = 100 (one term 8e-16); the drains cost 1.5 to
-  // 4 % of a call (pi pi sets 166 -> 173 ms, profile 25.6 -> 26.1).
+  // The pieces of a tile of more than 128 k at full scale, 4 to 8 chunks each, at whose ends
+  // levels 0 and 1 and the last level are drained into the epilogue's 64-bit sums.  Level
+  // 0 then stays below 2^24 units, where FP32 sums are exact, for any data.  With the
+  // operands' leading digits halved instead, which reach 512 k in one sum, products lose
+  // two bits, and the last level, truncated by the tensor core at each MMA, gets an error
+  // that grows with the chunks summed.  Root mean square error of four-term products of
+  // Gaussian blocks at Nev = 100, relative: halved 4.8e-15, in pieces 8e-16 (one term
+  // 8e-16).  A drain costs 2 to 3 K clocks of a tile: 25 chunks 5.29 -> 5.80 ms a launch, 16
+  // chunks 2.92 -> 3.19, 10 chunks 0.76 -> 0.92.  So the form is for sums that no error
+  // estimate watches, the profile gradients (25.6 -> 26.1 ms), and for callers' own
+  // products; the chain calls' entries are checked one by one and keep the halved digits.
   const uint32_t pieces = C::LONG ? (g.nchunk + 7) / 8 : 1;
   if (warp == 0) {
     if (lane == 0) {
@@ -2549,8 +2552,7 @@ int launch_split_gemm(const SplitGemmBatch& g, int ninst, int* d_err, cudaStream
   if (ninst == 0) return CTR_OK;
   if (g.hp) {
     if (g.out_mode != 1 || g.levels) return fail(CTR_ERR_ARG, "split GEMM: the high-precision tiles write complex128");
-    // (Gram products halve their leading digits instead: their pieces' errors are far below their scales)
-    if (!gram && g.nchunk > 8)
+    if (g.full && g.nchunk > 8)
       return launch_split_gemm_cfg<CfgHPLong>(g, ninst, d_err, s, "split_gemm_hp", &g_split_mma_flops);
     return gram ? launch_split_gemm_cfg<CfgHP>(g, ninst, d_err, s, "gram_gemm", &g_gram_mma_flops)
                 : launch_split_gemm_cfg<CfgHP>(g, ninst, d_err, s, "split_gemm_hp", &g_split_mma_flops);

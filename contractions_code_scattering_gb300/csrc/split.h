@@ -54,7 +54,7 @@ struct SplitCfg {
 };
 using CfgStd = SplitCfg<SPLIT_NSLICE, 4, SPLIT_N, false>;
 using CfgHP = SplitCfg<6, 5, 48, true>;
-using CfgHPLong = SplitCfg<6, 5, 48, true, true>;  // CfgHP's operands, any number of chunks
+using CfgHPLong = SplitCfg<6, 5, 48, true, true>;  // CfgHP's tiles above 128 k, operands at full scale
 static_assert(CfgStd::B_STAGE == SPLIT_B_STAGE && CfgStd::A_STAGE == SPLIT_A_STAGE, "standard stage sizes");
 static_assert(CfgStd::BN % (CfgStd::EPI_CW * (CfgStd::EPI_WARPS / 4)) == 0 &&
                   CfgHP::BN % (CfgHP::EPI_CW * (CfgHP::EPI_WARPS / 4)) == 0,
@@ -112,12 +112,15 @@ struct SplitGemmBatch {
   int hp;            // 0: CfgStd operands and tiles, 1: CfgHP's (out_mode 1 only)
   int order;         // persistent tile walk: 0 N tiles innermost, 1 M tiles innermost
   int step;          // split_tail_step(K) of operands sliced that way, 0 or 1 otherwise
+  int full;          // above 128 k: 1 for operands at full scale (CfgHPLong), 0 for halved ones
 };
 
 // Operands of the task form C = sum_q w_q op(A_q) op(B_q) (q < nterm <= 4),
 // concatenated along K (term q occupies k in [q N, (q+1) N)).  Left: rows of
 // the A side with the weights applied; right: up to SPLIT_TASK_NB output blocks
 // stacked along N.  dag bit q (left) / bit 4j+q (right): conjugate transpose.
+// eplus = 1 halves the leading digit (|d_0| <= 128) so that level 0 stays exact for
+// K <= 512 in one sum (SplitGemmBatch::full = 0).
 // The scale exponents come from per-block tables: bi indexes a table of
 // [2][nev] ints per distinct block of the launch (row-wise and column-wise
 // exponent bounds, launch_block_exp); wexp is the exponent of the power-of-two
@@ -134,7 +137,7 @@ struct SliceTaskLJob {
 struct SliceTaskRJob {
   const double2* b[SPLIT_TASK_NB][4];
   int bi[SPLIT_TASK_NB][4];
-  int nb, nterm, dag;
+  int nb, nterm, dag, eplus;
   uint8_t* out;  // [ntiles][nchunk][CfgHP::B_STAGE]
   int* exps;     // [ntiles * CfgHP::BN]
 };
@@ -149,7 +152,7 @@ struct SliceStackLJob {
   int bi[SPLIT_STACK][4];
   float w[4];
   int wexp[4];
-  int nslab, nterm, dag;
+  int nslab, nterm, dag, eplus;
   uint8_t* out;  // [mtiles][nchunk][CfgHP::A_STAGE]
   int* exps;     // [mtiles * SPLIT_M]
 };
