@@ -1,7 +1,8 @@
 // Chain diagrams: rho->pipi, pipi->pipi (I=1, I=0), loop-unity, sigma->pipi,
-// on either engine: every GEMM stage below is a list of block-product tasks
-// that runs on the FP64 tile kernel or on the split-precision tensor-core
-// engine (zgemm_split_tasks); the closing traces are FP64 in both.
+// on either engine: every GEMM stage below is a list of block products that runs on
+// the FP64 tile kernel or on the split-precision tensor-core engine.  The closing
+// traces are FP64 on both, but for the momentum-set calls of rho->pipi and sigma->pipi
+// on the split engine, which take them as Gram products.
 //
 // The reference evaluates every spin row as an independent chain of 2-6 Nev^3
 // products (lib/calculate_{rhopi,pipi_*,sigmapi_*,loop_unity}_core.h).  The
@@ -225,8 +226,8 @@ struct TracePlan {
   }
 };
 
-// (set, pair) item of a pi pi batch: 112 trace slots in the layout of
-// pipi_combine_kernel, combined into corr[ent * 5 ..].
+// (set, pair) item of a pi pi batch: 112 trace slots (16 each of square, double triangle,
+// horizontal double triangle and the four twins; -1: none), combined into corr[ent * 5 ..].
 __global__ void pipi_combine_sets_kernel(const double2* __restrict__ trv, const double* __restrict__ trabs,
                                          const int* __restrict__ slots, const int* __restrict__ ent, int nitem, int iso,
                                          double2* __restrict__ corr, double eps_over_tol, int* __restrict__ count,
@@ -444,9 +445,12 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
   int nF = 0;
   for (auto& v : FK) nF += (int)v.size();
   // star / fish twin traces (sink elemental, source elemental): (4, 1), (3, 2), (3, 1), (4, 2)
-  // of every set, a term for each of tau's 16 blocks.  (I = 0 has Tr[Phi_x Pm(y)_cc] for
-  // less, 151 instead of 165 ms for 19 sets at Nev = 100 and 4 sink times, but a Pm that
-  // cancels in its spin sum takes the traces' error scales down with it.)
+  // of every set, a term for each of tau's 16 blocks; on the FP64 engine at I = 0 the 4
+  // Tr[Phi_x Pm(y)_cc] instead (Nev = 32, 64 pairs: 6.4 -> 5.9 ms).  The split engine would
+  // gain as much (19 sets, Nev = 100, 4 sink times: 165 against 151 ms), but where Pm cancels in
+  // its spin sum those traces' error scales fall with it, and entries that need a
+  // recomputation go without.
+  const bool from_pm = iso == 0 && engine == CTR_ENGINE_FP64;
   std::map<std::pair<int, int>, int> twk;
   std::vector<std::pair<int, int>> TW;
   std::vector<int> twin(4 * nset);
@@ -459,9 +463,9 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       twin[4 * k + h] = it->second;
     }
   }
-  const int nTW = (int)TW.size();
-  const size_t blk_pair = 16 * (size_t)(nCR + nCL + nW + nU + (iso == 0 ? nW + nF : 0));
-  const size_t tr_pair = (size_t)nset * (iso == 0 ? 48 : 32) + 16 * (size_t)nTW;
+  const int nTW = (int)TW.size(), ntw = from_pm ? 4 : 16;  // traces a twin
+  const size_t blk_pair = 16 * (size_t)(nCR + nCL + nW + (from_pm ? 0 : nU) + (iso == 0 ? nW + nF : 0));
+  const size_t tr_pair = (size_t)nset * (iso == 0 ? 48 : 32) + ntw * (size_t)nTW;
   const size_t per_pair = blk_pair * N2 * sizeof(double2) + tr_pair * (sizeof(double2) + sizeof(double));
   const size_t budget = sets_call ? sets_budget() : CHAIN_BUDGET;
   const int batch = std::max(1, std::min(npairs, (int)(budget / std::max<size_t>(per_pair, 1))));
@@ -478,7 +482,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       used += nblk * N2;
       return p;
     };
-    std::vector<double2*> bS((size_t)ng * nCR), bV(ng), bW((size_t)nh * nCL), bY(nh), bP(np, nullptr);
+    std::vector<double2*> bS((size_t)ng * nCR), bV(ng), bW((size_t)nh * nCL), bY(nh, nullptr), bP(np, nullptr);
     std::vector<std::vector<double2*>> bF(np, std::vector<double2*>(nW, nullptr));
     for (int g = 0; g < ng; g++) {
       const size_t m = pb.by_ti[g].size();
@@ -488,7 +492,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
     for (int h = 0; h < nh; h++) {
       const size_t m = pb.by_tf[h].size();
       for (int ci = 0; ci < nCL; ci++) bW[(size_t)h * nCL + ci] = alloc(16 * m);
-      bY[h] = alloc(16 * (size_t)nU * m);
+      if (!from_pm) bY[h] = alloc(16 * (size_t)nU * m);
     }
     for (int i = 0; i < np && iso == 0; i++) {
       bP[i] = alloc(16 * (size_t)nW);
@@ -564,7 +568,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
         g0.push_back(std::move(G));
       }
       // Y(q) = tau_b^dag Phi_q(tf): slab (pair, block b), right block q
-      for (int q0 = 0; q0 < nU; q0 += 8) {
+      for (int q0 = 0; q0 < nU && !from_pm; q0 += 8) {
         GridTask G = make_grid(16 * m, std::min(8, nU - q0), 1, kOne, 1, 0);
         for (int pp = 0; pp < m; pp++)
           for (int b = 0; b < 16; b++) G.A[pp * 16 + b] = pb.T[mem_i[pp]] + b * N2;
@@ -614,12 +618,13 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       return fail(CTR_ERR_ALLOC, "pi pi: batch arena overflow");
     TracePlan tp;
     tp.tt.reserve(ntr);
-    std::vector<int> slots, ent, tws(16 * (size_t)nTW);
+    std::vector<int> slots, ent, tws(ntw * (size_t)nTW);
     slots.reserve((size_t)np * nset * 112);
     for (int i = 0; i < np; i++) {
       for (int t = 0; t < nTW; t++)
-        for (int b = 0; b < 16; b++)
-          tws[t * 16 + b] = tp.add(Vblk(iw[TW[t].second], i, b), Yblk(iu[TW[t].first], i, b), 1.f, 0.f, 1);
+        for (int b = 0; b < ntw; b++)
+          tws[t * ntw + b] = from_pm ? tp.add(P(TW[t].first, pb.tf[i]), Pblk(iw[TW[t].second], i, b, b), 1.f, 0.f, 1)
+                                     : tp.add(Vblk(iw[TW[t].second], i, b), Yblk(iu[TW[t].first], i, b), 1.f, 0.f, 1);
       for (int k = 0; k < nset; k++) {
         const int* q = sets + 4 * k;
         for (int cr : {cSq[k], cDt[k]})
@@ -637,7 +642,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
           slots.push_back(tp.add(Fb, Gb, 1.f, 0.f, 1));
         }
         for (int h = 0; h < 4; h++)
-          for (int b = 0; b < 16; b++) slots.push_back(tws[twin[4 * k + h] * 16 + b]);
+          for (int b = 0; b < 16; b++) slots.push_back(b < ntw ? tws[twin[4 * k + h] * ntw + b] : -1);
         ent.push_back(k * npairs + pb.ent[i]);
       }
     }
