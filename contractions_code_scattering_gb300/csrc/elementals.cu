@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(256) el_sum_kernel(const ElTask* __restrict__ 
   }
 }
 
-// Launches of at most EL_PART_BYTES of partial tiles each: 3300 tiles of 50 x 50, 7 waves of
-// them (7 momenta on 16^3, Nev = 100: 128 ms with 128 to 512 MB, 135 with 64).
+// Launches of at most EL_PART_BYTES of partial tiles each, whole waves of CTAs: 7 of them
+// for tiles of 50 x 50.
 constexpr size_t EL_PART_BYTES = (size_t)128 << 20;
 
 template <int TE, int RX, int RY>
@@ -247,7 +247,11 @@ int launch_el_gemm(const std::vector<ElTask>& tasks, int nev, long long K, const
   CTR_TRY(upload(WS_TASKS, tasks.data(), tasks.size() * sizeof(ElTask), &d_tasks, s));
   // partial tiles of a launch; fewer, and longer pieces, where memory is short
   const size_t tile_bytes = (size_t)TE * TE * sizeof(double2);
-  size_t max_parts = std::min<size_t>(EL_PART_BYTES / tile_bytes, (size_t)units * nsplit);
+  int resident = 1;
+  CTR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, el_gemm_kernel<TE, RX, RY>, (TE / RX) * (TE / RY), 0));
+  const size_t wave = (size_t)nsm * std::max(1, resident);
+  size_t max_parts = EL_PART_BYTES / tile_bytes;
+  max_parts = std::min<size_t>(max_parts - (max_parts > wave ? max_parts % wave : 0), (size_t)units * nsplit);
   void* part;
   for (;;) {
     nsplit = (int)std::max<size_t>(1, std::min<size_t>(nsplit, max_parts / most));
