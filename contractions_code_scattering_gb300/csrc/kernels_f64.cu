@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(LOOP_TPB) loop_unity_kernel(const double2* __r
   __shared__ double part[16];  // in CTA 0: the CTAs' partial sums
   if (ncta > 1) cluster_arrive();
   const int t = blockIdx.x / ncta, rank = blockIdx.x - t * ncta;
-  const unsigned n2 = (unsigned)N * N;  // Nev <= 4096
+  const unsigned n2 = (unsigned)N * N;  // below 2^32: 2^16 x 2^16 blocks would fill a terabyte a time slice
   const double2* T = diag + (size_t)t * 16 * n2;
   const double2* P = mom + (size_t)t * n2;
   const unsigned e1 = (unsigned)((unsigned long long)n2 * (rank + 1) / ncta);

@@ -903,7 +903,7 @@ static_assert(2 * CfgStd::NL * CfgStd::BN <= (int)TMEM_COLS && 2 * CfgHP::NL * C
 
 // I * 2^e as a double, rounded to nearest even; integer operations only, as few as
 // there are: 24 a thread of the epilogue, whose stores they hold up (triangles at
-// Nev = 32 1.82 -> 1.66 ms, Nev = 64 6.80 -> 6.58)
+// Nev = 32 1.82 -> 1.74 ms, Nev = 64 6.80 -> 6.58)
 // (normal results; magnitudes below 2^-1022 flush to zero).
 __device__ __forceinline__ double i2d_scaled(long long I, int e) {
   const uint32_t m = (uint32_t)(I >> 63);

@@ -111,7 +111,8 @@ int ctr_pipi(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin,
  * elemental; set s contracts with P1..P4 = phi[:, sets[4s + k]] (k = 0..3, host array
  * [nset][4]).  corr [nset][tf_end-tf_begin][Nt][5], each set's entries as ctr_pipi gives them.
  * Block products and traces that several sets share (e.g. Phi(q) tau, tau Phi(q) tau^dag for the
- * sets (p, -p) and (-p, p), L T and T^dag L of sets with the same sink pair) are computed once
+ * sets (p, -p) and (-p, p), T G R of sets with the same source pair, T^dag L of those with
+ * the same sink pair) are computed once
  * per batch of (t_sink, t_src) pairs. */
 int ctr_pipi_sets(int engine, int nev, int nt, int tf_begin, int tf_end, int isospin, const double* prop_rows,
                   const double* prop_diag, const double* phi, int nphi, int nset, const int32_t* sets, double* corr,
