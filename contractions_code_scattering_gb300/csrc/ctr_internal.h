@@ -98,7 +98,7 @@ enum {
   WS_GRAM,          // sliced operands and partial products of Gram traces
   WS_GRAMJOBS,      // their block, instance and pointer tables
   WS_GRAMTRACES,    // their trace lists
-  WS_SINKNORM,      // norms of the sink form's operands
+  WS_NORMS,         // norms of the operands of multi-term products
   WS_ADJ_CORR,      // its correlators where the caller's array is not 16-byte aligned
   WS_ADJ_SUM,       // per-time-slice co-factors of a profile gradient
   WS_COUNT

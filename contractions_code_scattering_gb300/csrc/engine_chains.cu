@@ -228,10 +228,18 @@ struct TracePlan {
 
 // (set, pair) item of a pi pi batch: 112 trace slots (16 each of square, double triangle,
 // horizontal double triangle and the four twins; -1: none), combined into corr[ent * 5 ..].
+//
+// A block of S = T G R or W = T^dag L may cancel in its sum of four terms, and the error
+// scales of square and double triangle with it.  They are at least what the sums have
+// without cancellation: 0.78^2 / Nev sum_ab (sum_k |T_ak|^2 |R_kb|^2)^(1/2) (sum_c |T_cb|^2
+// |L_ca|^2)^(1/2) from the blocks' norms nT (of a pair), nM (of L and R per time slice; row
+// terms[4 it] of nT, rows terms[4 it + 1..3] of nM for L, Rsq and Rdt), times the 0.78 that
+// a sum of |S| |W| has of the product of their norms.
 __global__ void pipi_combine_sets_kernel(const double2* __restrict__ trv, const double* __restrict__ trabs,
                                          const int* __restrict__ slots, const int* __restrict__ ent, int nitem, int iso,
                                          double2* __restrict__ corr, double eps_over_tol, int* __restrict__ count,
-                                         int* __restrict__ list) {
+                                         int* __restrict__ list, const int* __restrict__ terms,
+                                         const double* __restrict__ nT, const double* __restrict__ nM, double per_nev) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= nitem) return;
   const int* sl = slots + (size_t)it * 112;
@@ -248,6 +256,24 @@ __global__ void pipi_combine_sets_kernel(const double2* __restrict__ trv, const 
     }
     sum[g] = make_double2(re, im);
     ab[g] = a;
+  }
+  if (trabs) {
+    const int* m = terms + 4 * (size_t)it;
+    const double *T = nT + 16 * (size_t)m[0], *L = nM + 16 * (size_t)m[1];
+    for (int g = 0; g < 2; g++) {
+      const double* R = nM + 16 * (size_t)m[2 + g];
+      double f = 0.0;
+      for (int b = 0; b < 16; b++) {
+        double es = 0.0, ew = 0.0;
+        for (int k = 0; k < 4; k++) {
+          const double s = T[(b & 12) + k] * R[4 * k + (b & 3)], w = T[4 * k + (b & 3)] * L[4 * k + (b >> 2)];
+          es += s * s;
+          ew += w * w;
+        }
+        f += sqrt(es) * sqrt(ew);
+      }
+      ab[g] = fmax(ab[g], 0.47 * per_nev * f);
+    }
   }
   const double2 star = cmul(sum[3], sum[4]);
   const double2 fish = cmul(sum[5], sum[6]);
@@ -471,6 +497,15 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
   const int batch = std::max(1, std::min(npairs, (int)(budget / std::max<size_t>(per_pair, 1))));
   Refine rf;
   CTR_TRY(refine_begin(c, (size_t)nset * npairs * 5, WS_REFINE, rf));
+  double *nM = nullptr, *nT = nullptr;  // norms of L and R (for the call), of T (for a batch)
+  if (rf.on) {
+    void *p, *d;
+    CTR_TRY(workspace(WS_NORMS).get(16 * (M.size() + (size_t)batch) * sizeof(double), &p));
+    nM = (double*)p;
+    nT = nM + 16 * M.size();
+    CTR_TRY(upload(WS_MISC, M.data(), M.size() * sizeof(const double2*), &d, s));
+    CTR_TRY(launch_block_norms((const double2* const*)d, (int)M.size(), 16, N, nM, s));
+  }
   for (const PairBatch& pb : pair_batches(tau, blk16, Nt, tf_begin, rows, batch, plist)) {
     const int np = (int)pb.ent.size(), ng = (int)pb.by_ti.size(), nh = (int)pb.by_tf.size();
     void* mem;
@@ -618,7 +653,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       return fail(CTR_ERR_ALLOC, "pi pi: batch arena overflow");
     TracePlan tp;
     tp.tt.reserve(ntr);
-    std::vector<int> slots, ent, tws(ntw * (size_t)nTW);
+    std::vector<int> slots, ent, terms, tws(ntw * (size_t)nTW);
     slots.reserve((size_t)np * nset * 112);
     for (int i = 0; i < np; i++) {
       for (int t = 0; t < nTW; t++)
@@ -644,6 +679,7 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
         for (int h = 0; h < 4; h++)
           for (int b = 0; b < 16; b++) slots.push_back(b < ntw ? tws[twin[4 * k + h] * ntw + b] : -1);
         ent.push_back(k * npairs + pb.ent[i]);
+        terms.insert(terms.end(), {i, cL[k] * Nt + pb.tf[i], cSq[k] * Nt + pb.ti[i], cDt[k] * Nt + pb.ti[i]});
       }
     }
     for (size_t k = 0; k < tp.tt.size(); k++) {
@@ -651,15 +687,20 @@ int pipi_core(int N, int Nt, int tf_begin, int tf_end, int iso, const double* pr
       if (tra) tp.tt[k].absout = tra + k;
     }
     CTR_TRY(run_traces(c, tp.tt));
-    void* d[2];
-    CTR_TRY(upload_group(WS_MISC, {{slots.data(), slots.size() * sizeof(int)}, {ent.data(), ent.size() * sizeof(int)}},
+    void* d[4];
+    CTR_TRY(upload_group(WS_MISC,
+                         {{slots.data(), slots.size() * sizeof(int)},
+                          {ent.data(), ent.size() * sizeof(int)},
+                          {terms.data(), terms.size() * sizeof(int)},
+                          {pb.T.data(), pb.T.size() * sizeof(const double2*)}},
                          d, s));
+    if (rf.on) CTR_TRY(launch_block_norms((const double2* const*)d[3], np, 16, N, nT, s));
     {
       TimedLaunch tl(s, "pipi_combine");
       const int nitem = (int)ent.size();
       pipi_combine_sets_kernel<<<(nitem + 127) / 128, 128, 0, s>>>(trv, tra, (const int*)d[0], (const int*)d[1], nitem,
                                                                    iso, (double2*)corr, rf.eps_over_tol, rf.count,
-                                                                   rf.list);
+                                                                   rf.list, (const int*)d[2], nT, nM, 1.0 / N);
       CTR_CUDA(cudaGetLastError());
     }
   }
@@ -1117,7 +1158,7 @@ int rhopi_sigmapi_core(int N, int Nt, int tf_begin, int tf_end, const double* pr
   double *nR = nullptr, *nO = nullptr, *nT = nullptr;
   if (scales) {
     void* p;
-    CTR_TRY(workspace(WS_SINKNORM).get(16 * ((size_t)nC * Nt + (size_t)batch_sink * (nops + 1)) * sizeof(double), &p));
+    CTR_TRY(workspace(WS_NORMS).get(16 * ((size_t)nC * Nt + (size_t)batch_sink * (nops + 1)) * sizeof(double), &p));
     nR = (double*)p;
     nO = nR + (size_t)16 * nC * Nt;
     nT = nO + (size_t)16 * batch_sink * nops;

@@ -2143,12 +2143,16 @@ __global__ void __launch_bounds__(128) gram_trace_sum_kernel(const GramTrace* __
 
 // Norms (sum (|Re x| + |Im x|)^2)^(1/2) of blocks over the whole range of doubles: a thread
 // sums squares in FP32 relative to 2^E, E the largest exponent it has met but for 2^30.
-// One CTA a block, read once.
+// One CTA a block, read once; 0 where there is none.
 __global__ void __launch_bounds__(256) block_norms_kernel(const double2* const* __restrict__ base, int per, int n2,
                                                           double* __restrict__ out) {
   __shared__ int sE[8];
   __shared__ float ss[8];
   const int i = blockIdx.x / per;
+  if (!base[i]) {
+    if (threadIdx.x == 0) out[blockIdx.x] = 0.0;
+    return;
+  }
   const double2* x = base[i] + (size_t)(blockIdx.x - i * per) * n2;
   int E = -30000;
   float s = 0.f;

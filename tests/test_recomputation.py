@@ -87,3 +87,27 @@ def test_scaled_coefficients_flag_the_same_entries(cuda, power):
     finally:
         check(lib().ctr_split_set_refine(1e-9))
     assert torch.equal(got, ref * 2.0 ** power)
+
+
+@pytest.mark.parametrize("iso", [0, 1])
+@pytest.mark.parametrize("side", ["sink", "source"])
+def test_cancelling_block_sums_are_flagged(cuda, iso, side):
+    """Square and double triangle where W = T^dag L or S = T G R cancels in its spin sum:
+    rows (columns, with gamma_5) of tau alike up to 1e-8 and those of tau(t, t) opposite.
+    All pairs have to take the FP64 engine's values."""
+    nt, n = 2, 20
+    prop = synth.make_prop(nt, n, seed=1005)
+    rng = np.random.default_rng(1006)
+    diag = rng.normal(size=(nt, 4, 4, n, n)) + 1j * rng.normal(size=(nt, 4, 4, n, n))
+    near = lambda x: x * (1.0 + 1e-8 * rng.normal(size=x.shape))
+    for a, b in ((2, 0), (3, 1)):
+        if side == "sink":
+            prop[:, :, a], diag[:, a] = near(prop[:, :, b]), -diag[:, b]
+        else:
+            prop[:, :, :, a], diag[:, a] = near(prop[:, :, :, b]), diag[:, b]
+    ps = [_dev(synth.make_phi_random(nt, n, rng), cuda) for _ in range(4)]
+    run = lambda engine: api.run_contract_pipi(_dev(prop, cuda), _dev(diag, cuda), *ps, iso, engine=engine,
+                                               tf_range=(0, nt))
+    ref, got = run("fp64"), run("split")
+    assert lib().ctr_split_refined() == got.numel()
+    assert torch.equal(got, ref)
